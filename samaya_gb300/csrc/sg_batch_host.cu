@@ -3,12 +3,16 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
 #include <limits>
 #include <numeric>
+#include <queue>
 #include <random>
+#include <utility>
 
 #include "../../include/sg_pdlp.h"
 #include "sg_batch.cuh"
+#include "sg_cluster_layout.h"
 
 namespace sg {
 
@@ -29,6 +33,12 @@ Batch::~Batch() {
                   const_cast<void*>(static_cast<const void*>(u_.ck_off)),
                   const_cast<void*>(static_cast<const void*>(u_.mask_off))}) {
     if (p) cudaFree(p);
+  }
+  if (wait_host_) cudaFreeHost(wait_host_);
+  if (groups_.fork) cudaEventDestroy(groups_.fork);
+  for (int mode = 0; mode < kModes; ++mode) {
+    if (groups_.join[mode]) cudaEventDestroy(groups_.join[mode]);
+    if (groups_.stream[mode]) cudaStreamDestroy(groups_.stream[mode]);
   }
   if (stream_) cudaStreamDestroy(stream_);
 }
@@ -65,8 +75,8 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
     return SG_ERR_INVALID_ARGUMENT;
   }
   // Host layout of the matrices.
-  std::vector<long long> nnz_off(nmat + 1, 0), kptr_off(nmat + 1, 0), tptr_off(nmat + 1, 0),
-      col_off(nmat + 1, 0), row_off(nmat + 1, 0), cp_off(nmat + 1, 0);
+  std::vector<long long> nnz_off(nmat + 1, 0), col_off(nmat + 1, 0), row_off(nmat + 1, 0),
+      cp_off(nmat + 1, 0);
   for (int g = 0; g < nmat; ++g) {
     if (mat_m[g] < 0 || mat_n[g] < 0) {
       if (err) *err = "negative dimension";
@@ -86,8 +96,6 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
       }
     }
     nnz_off[g + 1] = nnz_off[g] + nnz;
-    kptr_off[g + 1] = kptr_off[g] + mat_m[g] + 1;
-    tptr_off[g + 1] = tptr_off[g] + mat_n[g] + 1;
     col_off[g + 1] = col_off[g] + mat_n[g];
     row_off[g + 1] = row_off[g] + mat_m[g];
   }
@@ -96,9 +104,15 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
     if (err) *err = "null matrix arrays";
     return SG_ERR_INVALID_ARGUMENT;
   }
-  std::vector<int> kptr(kptr_off[nmat]), tptr(tptr_off[nmat]), kidx(std::max(total_nnz, 1LL)),
-      tidx(std::max(total_nnz, 1LL));
-  std::vector<double> kval(std::max(total_nnz, 1LL)), tval(std::max(total_nnz, 1LL));
+  // Per matrix: the rows of A and of A' in their order (sg_cluster_layout.h), then the elements,
+  // each operator's column numbers replaced by the other's positions.
+  std::vector<StartLen> ksl(std::max(row_off[nmat], 1LL)), tsl(std::max(col_off[nmat], 1LL));
+  std::vector<int> kperm(ksl.size()), tperm(tsl.size()), slice(2 * static_cast<size_t>(nmat));
+  std::vector<long long> k_off(nmat + 1, 0), t_off(nmat + 1, 0), kd_off(nmat + 1, 0),
+      td_off(nmat + 1, 0);
+  std::vector<StartLen> kdesc, tdesc;
+  std::vector<RowOrder> korder(nmat), torder(nmat);
+  std::vector<std::vector<int>> kptr(nmat);
   int max_m = 0;
   for (int g = 0; g < nmat; ++g) {
     const int m = mat_m[g], n = mat_n[g];
@@ -106,26 +120,60 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
     const int64_t* cp = mat_colptr + cp_off[g];
     const int32_t* ri = mat_rowidx + nnz_off[g];
     const double* va = mat_val + nnz_off[g];
-    int* tp = tptr.data() + tptr_off[g];
-    for (int j = 0; j <= n; ++j) tp[j] = static_cast<int>(cp[j]);
     for (long long p = 0; p < cp[n]; ++p) {
       if (ri[p] < 0 || ri[p] >= m || !std::isfinite(va[p])) {
         if (err) *err = "bad matrix entry";
         return SG_ERR_INVALID_ARGUMENT;
       }
-      tidx[nnz_off[g] + p] = ri[p];
-      tval[nnz_off[g] + p] = va[p];
     }
-    int* kp = kptr.data() + kptr_off[g];
-    std::fill(kp, kp + m + 1, 0);
+    std::vector<int>& kp = kptr[g];
+    kp.assign(static_cast<size_t>(m) + 1, 0);
     for (long long p = 0; p < cp[n]; ++p) ++kp[ri[p] + 1];
     for (int i = 0; i < m; ++i) kp[i + 1] += kp[i];
-    std::vector<int> next(kp, kp + m);
+    std::vector<int> tp(static_cast<size_t>(n) + 1);
+    for (int j = 0; j <= n; ++j) tp[j] = static_cast<int>(cp[j]);
+    korder[g] = order_rows(kp.data(), m);
+    torder[g] = order_rows(tp.data(), n);
+    slice[2 * g] = korder[g].slice;
+    slice[2 * g + 1] = torder[g].slice;
+    kd_off[g + 1] = kd_off[g] + slices_of(korder[g]);
+    td_off[g + 1] = td_off[g] + slices_of(torder[g]);
+    kdesc.resize(kd_off[g + 1]);
+    tdesc.resize(td_off[g + 1]);
+    const long long kn =
+        place_rows(kp.data(), korder[g], ksl.data() + row_off[g], kdesc.data() + kd_off[g]);
+    const long long tn =
+        place_rows(tp.data(), torder[g], tsl.data() + col_off[g], tdesc.data() + td_off[g]);
+    if (kn >= std::numeric_limits<int>::max() || tn >= std::numeric_limits<int>::max()) {
+      if (err) *err = "matrix too large for 32-bit offsets";
+      return SG_ERR_TOO_LARGE;
+    }
+    k_off[g + 1] = k_off[g] + kn;
+    t_off[g + 1] = t_off[g] + tn;
+    std::copy(korder[g].perm.begin(), korder[g].perm.end(), kperm.begin() + row_off[g]);
+    std::copy(torder[g].perm.begin(), torder[g].perm.end(), tperm.begin() + col_off[g]);
+  }
+  std::vector<int> kidx(std::max(k_off[nmat], 1LL)), tidx(std::max(t_off[nmat], 1LL));
+  std::vector<double> kval(kidx.size()), tval(tidx.size());
+  for (int g = 0; g < nmat; ++g) {
+    const int n = mat_n[g];
+    const int64_t* cp = mat_colptr + cp_off[g];
+    const int32_t* ri = mat_rowidx + nnz_off[g];
+    const double* va = mat_val + nnz_off[g];
+    std::fill(kidx.begin() + k_off[g], kidx.begin() + k_off[g + 1], n);  // padding
+    std::fill(tidx.begin() + t_off[g], tidx.begin() + t_off[g + 1], mat_m[g]);
+    std::vector<int> done(static_cast<size_t>(mat_m[g]), 0);  // nonzeros of each row placed
     for (int j = 0; j < n; ++j) {
+      const int tpos = torder[g].pos[j];
+      const StartLen& ts = tsl[col_off[g] + tpos];
       for (long long p = cp[j]; p < cp[j + 1]; ++p) {
-        const int q = next[ri[p]]++;
-        kidx[nnz_off[g] + q] = j;
-        kval[nnz_off[g] + q] = va[p];
+        const int kpos = korder[g].pos[ri[p]];
+        const long long tq = t_off[g] + place_of(ts, static_cast<int>(p - cp[j]));
+        tidx[tq] = kpos;
+        tval[tq] = va[p];
+        const long long kq = k_off[g] + place_of(ksl[row_off[g] + kpos], done[ri[p]]++);
+        kidx[kq] = tpos;
+        kval[kq] = va[p];
       }
     }
   }
@@ -142,7 +190,8 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
     vec_off[i + 1] = vec_off[i] + nt;
     yrow_off[i + 1] = yrow_off[i] + mat_m[g];
     // Keep every instance's block 16-byte aligned.
-    long long elems = 8 * nt + 4 * static_cast<long long>(mat_m[g]);
+    long long elems = instance_elements(mat_n[g], mat_m[g], slice[2 * g + 1], slice[2 * g],
+                                        precision == 1);
     const long long align = 16 / static_cast<long long>(tsz);
     elems = (elems + align - 1) / align * align;
     state_off[i + 1] = state_off[i] + elems;
@@ -202,48 +251,68 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   };
   int* d_mm = nullptr;
   int* d_mn = nullptr;
-  long long *d_nz = nullptr, *d_kpo = nullptr, *d_tpo = nullptr, *d_co = nullptr, *d_ro = nullptr;
+  long long *d_ko = nullptr, *d_to = nullptr, *d_co = nullptr, *d_ro = nullptr;
   SG_B_TRY(up(&d_mm, mat_m, nmat));
   SG_B_TRY(up(&d_mn, mat_n, nmat));
-  SG_B_TRY(up(&d_nz, nnz_off.data(), nmat + 1));
-  SG_B_TRY(up(&d_kpo, kptr_off.data(), nmat + 1));
-  SG_B_TRY(up(&d_tpo, tptr_off.data(), nmat + 1));
+  SG_B_TRY(up(&d_ko, k_off.data(), nmat + 1));
+  SG_B_TRY(up(&d_to, t_off.data(), nmat + 1));
   SG_B_TRY(up(&d_co, col_off.data(), nmat + 1));
   SG_B_TRY(up(&d_ro, row_off.data(), nmat + 1));
   v.mat_m = d_mm;
   v.mat_n = d_mn;
-  v.mat_nnz_off = d_nz;
-  v.mat_kptr_off = d_kpo;
-  v.mat_tptr_off = d_tpo;
+  v.mat_k_off = d_ko;
+  v.mat_t_off = d_to;
   v.mat_col_off = d_co;
   v.mat_row_off = d_ro;
-  int *d_kp = nullptr, *d_ki = nullptr, *d_tp = nullptr, *d_ti = nullptr;
+  int *d_ki = nullptr, *d_ti = nullptr, *d_kperm = nullptr, *d_tperm = nullptr, *d_sl = nullptr;
+  StartLen *d_ksl = nullptr, *d_tsl = nullptr, *d_kdesc = nullptr, *d_tdesc = nullptr;
+  long long *d_kdo = nullptr, *d_tdo = nullptr;
   double *d_kv0 = nullptr, *d_tv0 = nullptr;
-  SG_B_TRY(up(&d_kp, kptr.data(), kptr.size()));
-  SG_B_TRY(up(&d_ki, kidx.data(), total_nnz));
-  SG_B_TRY(up(&d_tp, tptr.data(), tptr.size()));
-  SG_B_TRY(up(&d_ti, tidx.data(), total_nnz));
-  SG_B_TRY(up(&d_kv0, kval.data(), total_nnz));
-  SG_B_TRY(up(&d_tv0, tval.data(), total_nnz));
-  v.k_ptr = d_kp;
+  SG_B_TRY(up(&d_ksl, ksl.data(), ksl.size()));
+  SG_B_TRY(up(&d_tsl, tsl.data(), tsl.size()));
+  SG_B_TRY(up(&d_kdesc, kdesc.data(), kdesc.size()));
+  SG_B_TRY(up(&d_tdesc, tdesc.data(), tdesc.size()));
+  SG_B_TRY(up(&d_kdo, kd_off.data(), nmat + 1));
+  SG_B_TRY(up(&d_tdo, td_off.data(), nmat + 1));
+  SG_B_TRY(up(&d_kperm, kperm.data(), kperm.size()));
+  SG_B_TRY(up(&d_tperm, tperm.data(), tperm.size()));
+  SG_B_TRY(up(&d_sl, slice.data(), slice.size()));
+  SG_B_TRY(up(&d_ki, kidx.data(), kidx.size()));
+  SG_B_TRY(up(&d_ti, tidx.data(), tidx.size()));
+  SG_B_TRY(up(&d_kv0, kval.data(), kval.size()));
+  SG_B_TRY(up(&d_tv0, tval.data(), tval.size()));
+  static_assert(sizeof(StartLen) == sizeof(int2), "row starts layout");
+  v.k_sl = reinterpret_cast<const int2*>(d_ksl);
+  v.t_sl = reinterpret_cast<const int2*>(d_tsl);
+  v.k_desc = reinterpret_cast<const int2*>(d_kdesc);
+  v.t_desc = reinterpret_cast<const int2*>(d_tdesc);
+  v.mat_kd_off = d_kdo;
+  v.mat_td_off = d_tdo;
+  v.k_perm = d_kperm;
+  v.t_perm = d_tperm;
+  v.mat_slice = d_sl;
   v.k_idx = d_ki;
-  v.t_ptr = d_tp;
   v.t_idx = d_ti;
   v.k_val0 = d_kv0;
   v.t_val0 = d_tv0;
-  SG_B_TRY(b->alloc(&v.k_val, total_nnz));
-  SG_B_TRY(b->alloc(&v.t_val, total_nnz));
+  SG_B_TRY(b->alloc(&v.k_val, kval.size()));
+  SG_B_TRY(b->alloc(&v.t_val, tval.size()));
   v.fp32 = precision == 1 ? 1 : 0;
   if (v.fp32) {
-    SG_B_TRY(b->alloc(&v.k_val32, total_nnz));
-    SG_B_TRY(b->alloc(&v.t_val32, total_nnz));
+    SG_B_TRY(b->alloc(&v.k_val32, kval.size()));
+    SG_B_TRY(b->alloc(&v.t_val32, tval.size()));
   }
   SG_B_TRY(b->alloc(&v.cs, col_off[nmat]));
   SG_B_TRY(b->alloc(&v.rs, row_off[nmat]));
-  SG_B_TRY(b->alloc(&v.cn, col_off[nmat]));
-  SG_B_TRY(b->alloc(&v.rn, row_off[nmat]));
-  SG_B_TRY(b->alloc(&v.pu, row_off[nmat]));
-  SG_B_TRY(b->alloc(&v.pv, col_off[nmat]));
+  SG_B_TRY(b->alloc(&v.ics, col_off[nmat]));
+  SG_B_TRY(b->alloc(&v.irs, row_off[nmat]));
+  v.spill = nullptr;
+  for (int g = 0; g < nmat && v.spill == nullptr; ++g) {
+    if (cluster_vector_bytes(mat_n[g], mat_m[g], slice[2 * g + 1], slice[2 * g], 1,
+                             sizeof(double)) > kClusterSmemMax) {
+      SG_B_TRY(b->alloc(&v.spill, col_off[nmat] + row_off[nmat] + 2 * nmat));
+    }
+  }
   SG_B_TRY(b->alloc(&v.info, nmat));
   const double* d_u0 = nullptr;
   SG_B_TRY(up(&d_u0, u0.data(), u0.size()));
@@ -251,7 +320,6 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   int* d_im = nullptr;
   long long *d_vo = nullptr, *d_yo = nullptr, *d_so = nullptr;
   double *d_c = nullptr, *d_l = nullptr, *d_u = nullptr;
-  int* d_order = nullptr;
   SG_B_TRY(up(&d_im, inst_mat, count));
   SG_B_TRY(up(&d_vo, vec_off.data(), count + 1));
   SG_B_TRY(up(&d_yo, yrow_off.data(), count + 1));
@@ -259,7 +327,6 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   SG_B_TRY(up(&d_c, cost, vec_off[count]));
   SG_B_TRY(up(&d_l, lower, vec_off[count]));
   SG_B_TRY(up(&d_u, upper, vec_off[count]));
-  SG_B_TRY(up(&d_order, order.data(), count));
   v.inst_mat = d_im;
   v.vec_off = d_vo;
   v.row_off = d_yo;
@@ -267,18 +334,20 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   v.cost = d_c;
   v.lower = d_l;
   v.upper = d_u;
-  v.order = d_order;
   unsigned char* st = nullptr;
   SG_B_TRY(b->alloc(&st, static_cast<size_t>(state_off[count]) * tsz));
   v.state = st;
   SG_B_TRY(b->alloc(&v.x_out, vec_off[count]));
   SG_B_TRY(b->alloc(&v.y_out, yrow_off[count]));
   SG_B_TRY(b->alloc(&v.results, count));
-  SG_B_TRY(b->alloc(&v.queue, 1));
+  SG_B_TRY(b->alloc(&v.queue, kModes));
   unsigned long long* dl = nullptr;
   SG_B_TRY(b->alloc(&dl, 1));
   v.deadline = dl;
-  v.total_nnz = total_nnz;
+  SG_B_TRY(b->alloc(&v.wait_error, 1));
+  SG_B_CUDA(cudaMemset(v.wait_error, 0, sizeof(int)));
+  SG_B_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&b->wait_host_), sizeof(int),
+                          cudaHostAllocDefault));
   v.max_iter = max_iter;
   v.tol = tol;
   v.algorithm = algorithm == 1 || algorithm == 2 ? algorithm : 0;
@@ -286,12 +355,161 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   // single-LP engine does (the enhanced PDHG keeps 0.36 here: measured no faster at 0.1 on the
   // batched node relaxations).
   v.art_frac = v.algorithm == 2 ? 0.1 : 0.36;
-  int dev = 0, sms = 148;
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  b->grid_ = std::max(1, std::min(count, 2 * sms));
+  cudaDeviceGetAttribute(&b->sms_, cudaDevAttrMultiProcessorCount, dev);
+  b->mat_m_.assign(mat_m, mat_m + nmat);
+  b->mat_n_.assign(mat_n, mat_n + nmat);
+  b->inst_mat_.assign(inst_mat, inst_mat + count);
+  b->mat_slice_ = slice;
+  b->mat_nnz_.resize(nmat);
+  for (int g = 0; g < nmat; ++g) b->mat_nnz_[g] = nnz_off[g + 1] - nnz_off[g];
+  b->order_ = std::move(order);
+  SG_B_TRY(b->make_plan(Kind::kSetup, &b->setup_plan_));
+  SG_B_TRY(b->make_plan(Kind::kSolve, &b->solve_plan_));
   *out = b;
   return SG_OK;
+}
+
+// Cluster size, shared memory and clusters of one kernel: the size with the shortest estimated
+// finish when the instances go to the clusters largest first. The estimate of an iteration, in
+// microseconds, is fitted to measured ones of random LPs from 100 x 250 to 5,000 x 10,000 and
+// facility-location LPs, 1 to 600 of them, at every size (within 20%; e.g. FP64, 1 LP of
+// 1,500 x 3,000: 34.9 / 20.0 / 10.4 / 7.4 / 6.7 with 1 / 2 / 4 / 8 / 16 CTAs; 160 LPs of
+// 500 x 1,200: 15.3 / 17.6 / 21.5 / 32.2 / 84.9).
+int Batch::make_plan(Kind kind, ClusterPlan* plan) {
+  const bool setup = kind == Kind::kSetup;
+  const bool fp32 = kind == Kind::kSolve && v_.fp32;
+  const size_t elem = fp32 ? sizeof(float) : sizeof(double);
+  const int count = setup ? static_cast<int>(mat_m_.size()) : v_.count;
+  // Two FP64 CTAs share an SM; FP32 ones take it for themselves.
+  const int per_sm = fp32 ? 1 : 2;
+  const size_t limit = fp32 ? kClusterSmemMax : kClusterSmemHalf;
+  auto vector_bytes = [&](int g, int size) {
+    return cluster_vector_bytes(mat_n_[g], mat_m_[g], mat_slice_[2 * g + 1], mat_slice_[2 * g],
+                                size, elem);
+  };
+  auto all_bytes = [&](int g, int size) {
+    const int ks = mat_slice_[2 * g], ts = mat_slice_[2 * g + 1];
+    const long long kslices = share_rows(mat_m_[g], ks, size) >> ks;
+    const long long tslices = share_rows(mat_n_[g], ts, size) >> ts;
+    return vector_bytes(g, size) +
+           (setup                  ? 0
+            : kind == Kind::kSolve ? solve_state_bytes(tslices, kslices, elem)
+                                   : unroll_state_bytes(tslices, kslices, kind == Kind::kAdjoint));
+  };
+  std::vector<std::pair<double, int>> work(count);  // an iteration's time by one CTA, the matrix
+  bool fits = true;  // every instance's gathered vectors in shared memory
+  for (int i = 0; i < count; ++i) {
+    const int g = setup ? i : inst_mat_[i];
+    const double rows = static_cast<double>(mat_m_[g]) + mat_n_[g];
+    const double nnz = static_cast<double>(mat_nnz_[g]);
+    work[i] = {fp32 ? 2.7e-4 * (2 * nnz + 3 * rows) : 5.6e-4 * (2 * nnz + 5 * rows), g};
+    fits = fits && vector_bytes(g, 2) <= kClusterSmemMax;
+  }
+  std::sort(work.begin(), work.end(), std::greater<std::pair<double, int>>());
+  // The sizes' exchanges and epilogues.
+  const int sizes[5] = {1, 2, 4, 8, 16};
+  const double fixed64[5] = {0.7, 2.2, 3.4, 4.2, 5.2};
+  const double fixed32[5] = {5.4, 6.4, 6.8, 7.7, 8.7};
+  // The setup's passes end in reductions over the cluster (the same unit: a thirtieth of it; 64
+  // LPs of 500 x 1,200: 0.66 / 0.55 / 0.61 / 1.09 ms with 1 / 2 / 4 / 8 CTAs).
+  const double fixed_setup[5] = {5.5, 9.0, 9.9, 10.6, 11.3};
+  const double* fixed = setup ? fixed_setup : fp32 ? fixed32 : fixed64;
+  plan->size = 1;
+  double best_time = -1.0;
+  for (int k = 0; k < 5; ++k) {
+    const int size = sizes[k];
+    if (size > 1 && !fits) break;
+    // Clusters at once (SMs of a GPC left over by clusters of 8 and 16: an eighth or more).
+    const int slots = std::max(1, per_sm * sms_ / size - (size >= 8 ? per_sm * sms_ / size / 8 : 0));
+    const bool shared_sm = !fp32 && static_cast<long long>(std::min(count, slots)) * size > sms_;
+    // Largest first, each to the cluster that is free first.
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+    for (int c = 0; c < std::min(count, slots); ++c) free_at.push(0.0);
+    double end = 0.0;
+    for (const auto& w : work) {
+      const double own = w.first / size;
+      double t = own + fixed[k];
+      // The FP64 pipe of a shared SM; a state left in device memory (160 LPs of 2,000 x 4,000:
+      // 72 us with 2 CTAs, 48 with 4, which hold it).
+      if (shared_sm) t = setup ? 1.25 * t : std::max(t, 1.15 * own);
+      if (!setup && !fp32 && all_bytes(w.second, size) > limit) t *= 1.45;
+      t += free_at.top();
+      free_at.pop();
+      free_at.push(t);
+      end = std::max(end, t);
+    }
+    if (best_time < 0 || end < best_time) {
+      best_time = end;
+      plan->size = size;
+    }
+  }
+  const int best = plan->size;
+  plan->clusters = std::max(1, per_sm * sms_ / best);
+  plan->threads = fp32 ? kThreads32 : kThreads64;
+  if (setup) {
+    // One launch for all matrices; a matrix whose vectors do not fit leaves them in device
+    // memory.
+    for (int g = 0; g < count; ++g) {
+      const size_t vec = vector_bytes(g, best);
+      if (vec <= kClusterSmemMax) plan->smem[0] = std::max(plan->smem[0], vec);
+    }
+    return SG_OK;
+  }
+  // Every instance in the mode that keeps the most in shared memory, FP64 ones within half of it
+  // (two CTAs to an SM) as long as their vectors allow that.
+  std::vector<int> lists[kModes];
+  for (int i : order_) {
+    const int g = inst_mat_[i];
+    const size_t vec = vector_bytes(g, best);
+    const size_t all = all_bytes(g, best);
+    const int mode = all <= limit             ? kAllShared
+                     : vec <= kClusterSmemMax ? kVectorsShared
+                                              : kInDevice;
+    const size_t need = mode == kAllShared ? all : mode == kVectorsShared ? vec : 0;
+    lists[mode].push_back(i);
+    plan->smem[mode] = std::max(plan->smem[mode], need);
+  }
+  int used = 0;
+  for (int mode = 0; mode < kModes; ++mode) {
+    if (lists[mode].empty()) continue;
+    ++used;
+    int* d = nullptr;
+    const int rc = alloc(&d, lists[mode].size());
+    if (rc != SG_OK) return rc;
+    if (cudaMemcpy(d, lists[mode].data(), lists[mode].size() * sizeof(int),
+                   cudaMemcpyHostToDevice) != cudaSuccess) {
+      return SG_ERR_CUDA;
+    }
+    plan->group[mode].inst = d;
+    plan->group[mode].count = static_cast<int>(lists[mode].size());
+  }
+  if (used > 1 && groups_.fork == nullptr) {
+    cudaError_t e = cudaEventCreateWithFlags(&groups_.fork, cudaEventDisableTiming);
+    for (int mode = 1; mode < kModes; ++mode) {
+      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&groups_.stream[mode], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&groups_.join[mode], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) return SG_ERR_CUDA;
+  }
+  return SG_OK;
+}
+
+// Waits for the stream; a wait inside a kernel that gave up is an error too.
+cudaError_t Batch::finish(std::string* err) {
+  cudaError_t e = cudaMemcpyAsync(wait_host_, v_.wait_error, sizeof(int), cudaMemcpyDeviceToHost,
+                                  stream_);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess && *wait_host_ != 0) {
+    cudaMemset(v_.wait_error, 0, sizeof(int));
+    e = cudaErrorUnknown;
+    if (err) *err = "an exchange between the CTAs of a cluster did not complete";
+    return e;
+  }
+  if (e != cudaSuccess && err) *err = cudaGetErrorString(e);
+  return e;
 }
 
 int Batch::solve(InstResult* results, double* x, double* y, double* device_ms, std::string* err) {
@@ -301,17 +519,21 @@ int Batch::solve(InstResult* results, double* x, double* y, double* device_ms, s
   cudaEventRecord(e0, stream_);
   const unsigned long long budget =
       time_limit_ > 0 ? static_cast<unsigned long long>(time_limit_ * 1e9) : 0ull;
-  launch_batch(v_, grid_, budget, stream_);
+  cudaError_t e = launch_batch(v_, setup_plan_, solve_plan_, budget, groups_, stream_);
   cudaEventRecord(e1, stream_);
-  cudaError_t e = cudaStreamSynchronize(stream_);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  std::string why;
+  if (e == cudaSuccess) {
+    e = finish(&why);
+  } else {
+    why = cudaGetErrorString(e);
+  }
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   if (device_ms) *device_ms = ms;
   if (e != cudaSuccess) {
-    if (err) *err = std::string("batch solve: ") + cudaGetErrorString(e);
+    if (err) *err = "batch solve: " + why;
     return SG_ERR_CUDA;
   }
   if (results) {
@@ -403,11 +625,24 @@ int Batch::unroll(int iterations, int every, double* v_out, std::string* err) {
     u_.every = every;
     u_.nck = nck;
   }
-  launch_batch_setup(v_, stream_);
-  launch_unroll(v_, u_, 0, grid_, stream_);
-  cudaError_t e = cudaStreamSynchronize(stream_);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  if (forward_plan_.size == 0) {
+    int rc = make_plan(Kind::kForward, &forward_plan_);
+    if (rc == SG_OK) rc = make_plan(Kind::kAdjoint, &adjoint_plan_);
+    if (rc != SG_OK) {
+      forward_plan_ = ClusterPlan();
+      if (err) *err = "unroll plan: out of memory";
+      return rc;
+    }
+  }
+  std::string why;
+  cudaError_t e = launch_batch_setup(v_, setup_plan_, stream_);
+  if (e == cudaSuccess) e = launch_unroll(v_, u_, forward_plan_, 0, groups_, stream_);
   if (e != cudaSuccess) return fail(e, "unroll");
+  e = finish(&why);
+  if (e != cudaSuccess) {
+    if (err) *err = "unroll: " + why;
+    return SG_ERR_CUDA;
+  }
   if (v_out) {
     e = cudaMemcpy(v_out, u_.v_out, sizeof(double) * total_vec_, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail(e, "unroll download");
@@ -433,11 +668,15 @@ int Batch::unroll_adjoint(const double* grad_v, double* grad_cost, double* grad_
   cudaError_t e = cudaMemcpy(const_cast<double*>(u_.grad_v), grad_v,
                              sizeof(double) * total_vec_, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return fail(e, "adjoint upload");
-  launch_batch_setup(v_, stream_);
-  launch_unroll(v_, u_, 1, grid_, stream_);
-  e = cudaStreamSynchronize(stream_);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  std::string why;
+  e = launch_batch_setup(v_, setup_plan_, stream_);
+  if (e == cudaSuccess) e = launch_unroll(v_, u_, adjoint_plan_, 1, groups_, stream_);
   if (e != cudaSuccess) return fail(e, "adjoint");
+  e = finish(&why);
+  if (e != cudaSuccess) {
+    if (err) *err = "adjoint: " + why;
+    return SG_ERR_CUDA;
+  }
   const std::pair<double*, const double*> outs[3] = {
       {grad_cost, u_.grad_cost}, {grad_lower, u_.grad_lower}, {grad_upper, u_.grad_upper}};
   for (const auto& o : outs) {

@@ -1,0 +1,713 @@
+// The batched solve: persistent clusters that run whole PDLP solves (see sg_batch.cu).
+//
+// FP64 steps are bound by the FP64 pipe (busy 47-53% of the time) and by the walks' load latency
+// before a cluster's exchange; FP32 ones by the instructions around each nonzero (addresses,
+// bounds of the row). One CTA per LP (a block barrier a half step, unsorted rows, the nonzeros
+// of a row side by side, averages and evaluation sums in separate passes) took 25.4 ms for 256
+// iterations of 160 random LPs of 100-2,500 rows in FP64, clusters of four 13.4 ms; 512
+// Halpern iterations of 256 facility-location nodes (40 x 160) with FP32 storage 53.6 ms,
+// now, still a CTA per LP, 21.4 ms.
+#pragma once
+
+#include "sg_batch_device.cuh"
+
+namespace sg {
+
+// ------------------------------------------------------------------------------------------
+// Solve: persistent clusters, one instance at a time.
+
+namespace {
+
+struct Meas {
+  double rp, rd, rg, pobj, dobj;
+};
+
+__device__ __forceinline__ Meas finish7(const double* s, double amc, double amr, double cnorm,
+                                        int m) {
+  Meas r;
+  const double ps = 1.0 + amc * sqrt(s[4]) + sqrt(s[5]);
+  const double ds = 1.0 + amr * sqrt(s[6]) + cnorm;
+  const double gs = 1.0 + fabs(s[2]) + fabs(s[3]);
+  r.rp = m > 0 ? sqrt(s[0]) / ps : 0.0;
+  r.rd = m > 0 ? sqrt(s[1]) / ds : 0.0;
+  r.rg = (s[2] - s[3]) / gs;
+  r.pobj = s[2];
+  r.dobj = s[3];
+  return r;
+}
+
+__device__ __forceinline__ double kkt_w(double w, const Meas& e) {
+  return sqrt(w * w * e.rp * e.rp + e.rd * e.rd / (w * w) + e.rg * e.rg);
+}
+
+// The state of the own columns and rows that every iteration reads, one array after another
+// (array k of own entry l, position p): the point, the sum since the restart (FP32: the running
+// average; Halpern: the anchor) and the scaled problem; the rows' extrapolated point (negated),
+// dual and its sum.
+enum : int {
+  kPoint = 0, kSum = 1, kCost = 2, kLower = 3, kUpper = 4, kBar = 5, kDual = 6, kDualSum = 7
+};
+constexpr int kColArrays = 5, kRowArrays = 8;  // solve_state_bytes
+
+// Slice by slice, 32 entries of each array (a constant distance between a row's values): in shared
+// memory the CTA's own slices, in device memory all slices.
+template <typename T, int MODE>
+struct alignas(16) SolveState {
+  T* device;                   // not kAllShared: the columns' arrays
+  long long rows_device;       // and how far on the rows' are
+  unsigned cols_at, rows_at;   // kAllShared: offsets
+  unsigned rank, size;
+  __device__ __forceinline__ T* col_base() const {
+    if constexpr (MODE == kAllShared) return reinterpret_cast<T*>(sg_smem + cols_at);
+    return device;
+  }
+  __device__ __forceinline__ T* row_base() const {
+    if constexpr (MODE == kAllShared) return reinterpret_cast<T*>(sg_smem + rows_at);
+    return device + rows_device;
+  }
+  __device__ __forceinline__ T& col(int k, const At& at) const {
+    if constexpr (MODE == kAllShared) {
+      return reinterpret_cast<T*>(sg_smem + cols_at)[(at.ls * kColArrays + k) * 32 + at.lane];
+    } else {
+      return device[(static_cast<long long>(at.ls * size + rank) * kColArrays + k) * 32 + at.lane];
+    }
+  }
+  __device__ __forceinline__ T& row(int k, const At& at) const {
+    if constexpr (MODE == kAllShared) {
+      return reinterpret_cast<T*>(sg_smem + rows_at)[(at.ls * kRowArrays + k) * 32 + at.lane];
+    } else {
+      return device[rows_device +
+                    (static_cast<long long>(at.ls * size + rank) * kRowArrays + k) * 32 + at.lane];
+    }
+  }
+};
+
+// One operator's state arrays (the columns' or the rows') in a walk: entry k of the own row `at`.
+template <typename T, int MODE, int ARRAYS>
+struct StepState {
+  Array<T, MODE == kAllShared> base;
+  unsigned rank, size;
+  struct Entry {
+    Array<T, MODE == kAllShared> e;
+    __device__ __forceinline__ T get(int k) const { return e.get(32 * k); }
+    __device__ __forceinline__ void set(int k, T v) const { e.set(32 * k, v); }
+  };
+  __device__ __forceinline__ Entry at(const At& a) const {
+    Entry r{base};
+    if constexpr (MODE == kAllShared) {
+      r.e.a += (a.ls * (ARRAYS * 32) + a.lane) * static_cast<int>(sizeof(T));
+    } else {
+      r.e.a += static_cast<long long>(a.ls * static_cast<int>(size) + static_cast<int>(rank)) *
+                   (ARRAYS * 32) + a.lane;
+    }
+    return r;
+  }
+};
+
+// Device storage of an instance beside the state: the second point (the restart point, or
+// Halpern's T(z)), the columns' saved extrapolated point, by position.
+template <typename T>
+struct Second {
+  T* st;  // x (n), r (m), y (m), saved (n)
+  int n, m;
+  __device__ __forceinline__ T& x(int p) const { return st[p]; }
+  __device__ __forceinline__ T& r(int p) const { return st[n + p]; }
+  __device__ __forceinline__ T& y(int p) const { return st[n + m + p]; }
+  __device__ __forceinline__ T& saved(int p) const { return st[n + 2 * m + p]; }
+};
+
+// The average of `count` points whose sum is s (FP64; FP32 keeps the average itself).
+__device__ __forceinline__ double average(double s, double inv_count) { return s * inv_count; }
+__device__ __forceinline__ float average(float s, double) { return s; }
+
+template <typename T, int MODE>
+__device__ __forceinline__ StepState<T, MODE, kColArrays> col_state(const SolveState<T, MODE>& S) {
+  return {S.col_base(), S.rank, S.size};
+}
+template <typename T, int MODE>
+__device__ __forceinline__ StepState<T, MODE, kRowArrays> row_state(const SolveState<T, MODE>& S) {
+  return {S.row_base(), S.rank, S.size};
+}
+
+// The given problem and the scales of an instance, by position.
+struct Given {
+  const int *kperm, *tperm;
+  const double *cost, *lower, *upper;  // (columns, rows) in the caller's order
+  const double *cs, *rs, *ics, *irs;
+  int n;
+};
+
+// What the walks need of an instance, in shared memory (sh_copy); evaluate_point is a call of its
+// own, so that its registers are not the step's.
+template <typename T, int MODE>
+struct EvalContext {
+  MatShare<T> M;
+  Exchange<T, MODE> ex;
+  SolveState<T, MODE> S;
+  Second<T> Z;
+  Given G;
+  T weight[64], rest[64];  // run_steps
+};
+
+// One PDHG iteration (FP64: sums since the restart in place of running averages, one addition
+// less each, and the row's own term as the sum's start). xs has been put, not waited for; so it
+// is afterwards.
+template <typename T, int MODE>
+__device__ __forceinline__ bool classic_step(const EvalContext<T, MODE>* ctx, T tau, T sig,
+                                             T ta, T tb) {
+  constexpr bool kF64 = sizeof(T) == 8;
+  {
+    const auto K = sh_copy(&ctx->M.K);
+    const auto ex = sh_copy(&ctx->ex);
+    const auto R = row_state(sh_copy(&ctx->S));
+    const Sender<T, MODE, 1> y_out(ex);
+    const bool ok = walk_rows<true, false>(
+        K, Gather<T, MODE>{ex.xs()},
+        [&](const At& at) { return kF64 ? R.at(at).get(kBar) : T(0); },
+        [&](const At& at, T s) {
+          const auto e = R.at(at);
+          const T res = kF64 ? s : s + e.get(kBar);
+          const T yn = e.get(kDual) + sig * res;
+          e.set(kDual, yn);
+          y_out.put(at, yn);
+          const T lo = e.get(kLower);
+          const T up = e.get(kUpper);
+          const T r = e.get(kPoint);
+          if constexpr (kF64) {
+            e.set(kDualSum, e.get(kDualSum) + yn);
+            // An equality row's logical is its bound from the first step on: a warp of such
+            // rows skips the logicals.
+            const bool steady = same_bits(lo, up) && same_bits(r, lo);
+            const unsigned here = __activemask();
+            if (__any_sync(here, !steady)) {
+              keep_branch(here);
+              const T rn = clamp_to(r - tau * (e.get(kCost) - yn), lo, up);
+              e.set(kPoint, rn);
+              e.set(kBar, fma(-2.0, rn, r));
+              e.set(kSum, e.get(kSum) + rn);
+            } else {
+              e.set(kBar, -lo);
+            }
+          } else {
+            const T rn = clamp_to(r - tau * (e.get(kCost) - yn), lo, up);
+            e.set(kPoint, rn);
+            e.set(kBar, -(rn + (rn - r)));
+            e.set(kDualSum, tb * e.get(kDualSum) + ta * yn);
+            e.set(kSum, tb * e.get(kSum) + ta * rn);
+          }
+        },
+        [&]() { return ex.wait(0); });
+    if (!ok) return false;
+  }
+  const auto Kt = sh_copy(&ctx->M.Kt);
+  const auto ex = sh_copy(&ctx->ex);
+  const auto C = col_state(sh_copy(&ctx->S));
+  const Sender<T, MODE, 0> x_out(ex);
+  return walk_rows<true, false>(
+      Kt, Gather<T, MODE>{ex.ys()},
+      [&](const At& at) { return kF64 ? C.at(at).get(kCost) : T(0); },
+      [&](const At& at, T s) {
+        const auto e = C.at(at);
+        const T x = e.get(kPoint);
+        const T g = kF64 ? s : e.get(kCost) + s;
+        const T v = clamp_to(x - tau * g, e.get(kLower), e.get(kUpper));
+        e.set(kPoint, v);
+        x_out.put(at, kF64 ? fma(T(2), v, -x) : v + (v - x));
+        e.set(kSum, kF64 ? e.get(kSum) + v : tb * e.get(kSum) + ta * v);
+      },
+      [&]() { return ex.wait(1); });
+}
+
+// One reflected Halpern iteration z+ = N + w (z0 - N), N = 2 T(z) - z, w = 1 / (k + 2) (k:
+// iterations since the restart), T the PDHG map in primal-first order, as the single-LP engine's
+// halpern_primal / halpern_dual kernels compute it; the anchor is in the sums' place, and T(z)
+// (the point the evaluation, the restarts and the answer use) is written when it is `measured`.
+// ys has been put, not waited for; so it is afterwards.
+template <typename T, int MODE>
+__device__ __forceinline__ bool halpern_step(const EvalContext<T, MODE>* ctx, T tau, T sig, T w,
+                                             bool measured) {
+  constexpr bool kF64 = sizeof(T) == 8;
+  const Second<T>& Z = ctx->Z;
+  {
+    const auto Kt = sh_copy(&ctx->M.Kt);
+    const auto ex = sh_copy(&ctx->ex);
+    const auto C = col_state(sh_copy(&ctx->S));
+    const Sender<T, MODE, 0> x_out(ex);
+    const bool ok = walk_rows<true, false>(
+        Kt, Gather<T, MODE>{ex.ys()},
+        [&](const At& at) { return kF64 ? C.at(at).get(kCost) : T(0); },
+        [&](const At& at, T s) {
+          const auto e = C.at(at);
+          const T x = e.get(kPoint);
+          const T g = kF64 ? s : e.get(kCost) + s;
+          const T xh = clamp_to(x - tau * g, e.get(kLower), e.get(kUpper));
+          const T refl = kF64 ? fma(T(2), xh, -x) : xh + (xh - x);
+          x_out.put(at, refl);
+          e.set(kPoint, refl + w * (e.get(kSum) - refl));
+          if (measured) Z.x(at.p) = xh;
+        },
+        [&]() { return ex.wait(1); });
+    if (!ok) return false;
+  }
+  const auto K = sh_copy(&ctx->M.K);
+  const auto ex = sh_copy(&ctx->ex);
+  const auto R = row_state(sh_copy(&ctx->S));
+  const Sender<T, MODE, 1> y_out(ex);
+  return walk_rows<true, false>(
+      K, Gather<T, MODE>{ex.xs()}, Zero<T>(),
+      [&](const At& at, T s) {
+        const auto e = R.at(at);
+        const T y = e.get(kDual);
+        const T r = e.get(kPoint);
+        const T rh = clamp_to(r - tau * (e.get(kCost) - y), e.get(kLower), e.get(kUpper));
+        const T rrefl = kF64 ? fma(T(2), rh, -r) : rh + (rh - r);
+        const T yh = y + sig * (s - rrefl);
+        const T yrefl = kF64 ? fma(T(2), yh, -y) : yh + (yh - y);
+        const T yn = yrefl + w * (e.get(kDualSum) - yrefl);
+        e.set(kDual, yn);
+        y_out.put(at, yn);
+        e.set(kPoint, rrefl + w * (e.get(kSum) - rrefl));
+        if (measured) {
+          Z.y(at.p) = yh;
+          Z.r(at.p) = rh;
+        }
+      },
+      [&]() { return ex.wait(0); });
+}
+
+// `count` iterations from iteration t (k since the restart) on, the last of them measured; xs
+// (Halpern: ys) put, not waited for, before and after. (Inlined: in a called function every global
+// load takes two more instructions for its descriptor.)
+template <typename T, int MODE, bool HALPERN>
+__device__ __forceinline__ bool run_steps(EvalContext<T, MODE>* ctx, int count, long long k,
+                                       T tau, T sig) {
+  // The steps' weights, a thread each (a double division by every thread of every step would
+  // take the FP64 pipe for 4,000 clocks a step).
+  __syncthreads();
+  if (threadIdx.x < count) {
+    ctx->weight[threadIdx.x] = static_cast<T>(
+        1.0 / static_cast<double>(k + static_cast<int>(threadIdx.x) + (HALPERN ? 2 : 1)));
+    ctx->rest[threadIdx.x] = static_cast<T>(
+        1.0 - 1.0 / static_cast<double>(k + static_cast<int>(threadIdx.x) + 1));
+  }
+  __syncthreads();
+  bool ok = true;
+  for (int i = 0; i < count && ok; ++i) {
+    if constexpr (HALPERN) {
+      ok = halpern_step<T, MODE>(ctx, tau, sig, ctx->weight[i], i == count - 1);
+    } else {
+      ok = classic_step<T, MODE>(ctx, tau, sig, ctx->weight[i], ctx->rest[i]);
+    }
+  }
+  return ok;
+}
+
+// One iterate's sums (7 evaluation sums in the original space, pdlp.cpp:411-488, and the restart
+// distances of v and y) into e: which 0 the current point, 1 the average, 2 Halpern's T(z). The
+// evaluated vectors take the place of xs and ys.
+template <typename T, int MODE>
+__device__ __noinline__ bool evaluate_point(const EvalContext<T, MODE>* ctx, int which,
+                                            double inv_k, double (&e)[9]) {
+  constexpr bool kF64 = sizeof(T) == 8;
+  const MatShare<T>& M = ctx->M;
+  const Exchange<T, MODE>& ex = ctx->ex;
+  const SolveState<T, MODE>& S = ctx->S;
+  const Second<T>& Z = ctx->Z;
+  const Given& G = ctx->G;
+  auto vx = [&](const At& at) -> T {
+    return which == 0 ? S.col(kPoint, at)
+           : which == 1 ? static_cast<T>(average(S.col(kSum, at), inv_k)) : Z.x(at.p);
+  };
+  auto vy = [&](const At& at) -> T {
+    return which == 0 ? S.row(kDual, at)
+           : which == 1 ? static_cast<T>(average(S.row(kDualSum, at), inv_k)) : Z.y(at.p);
+  };
+  auto vr = [&](const At& at) -> T {
+    if (which == 2) return Z.r(at.p);
+    if (which == 0) return S.row(kPoint, at);
+    if (kF64 && S.row(kLower, at) == S.row(kUpper, at)) return S.row(kLower, at);
+    return static_cast<T>(average(S.row(kSum, at), inv_k));
+  };
+  const bool halpern = which == 2;
+#pragma unroll
+  for (int q = 0; q < 9; ++q) e[q] = 0.0;
+  each_own(M.Kt, [&](const At& at) { ex.put_x(at, vx(at)); });
+  each_own(M.K, [&](const At& at) { ex.put_y(at, vy(at)); });
+  bool good = ex.wait(0);
+  good = ex.wait(1) && good;
+  if (!good) return false;
+  const int m = M.m;
+  walk_rows<true, false>(M.K, GatherD<T>{ex.xs()}, Zero<double>(), [&](const At& at, double s) {
+    const int k = G.n + G.kperm[at.p];
+    const double irs = G.irs[at.p];
+    const double rv = static_cast<double>(vr(at));
+    const double yv = static_cast<double>(vy(at));
+    const double value = rv * irs;
+    const double yo = yv * G.rs[at.p];
+    const double c = G.cost[k];
+    const double g = c - yo;
+    const double ep = s * irs - value;
+    const double lo = G.lower[k];
+    const double up = G.upper[k];
+    e[0] += ep * ep;
+    e[5] += value * value;
+    e[6] += yo * yo;
+    e[2] += c * value;
+    const double lam = lam_of(g, lo, up);
+    e[1] += (g - lam) * (g - lam);
+    if (lam > 0.0) e[3] += lam * lo;
+    if (lam < 0.0) e[3] += lam * up;
+    const double dv = rv - static_cast<double>(halpern ? S.row(kSum, at) : Z.r(at.p));
+    const double dy = yv - static_cast<double>(halpern ? S.row(kDualSum, at) : Z.y(at.p));
+    e[7] += dv * dv;
+    e[8] += dy * dy;
+  }, Ready());
+  walk_rows<true, false>(M.Kt, GatherD<T>{ex.ys()}, Zero<double>(), [&](const At& at, double s) {
+    const int k = G.tperm[at.p];
+    const double xv = static_cast<double>(vx(at));
+    const double value = xv * G.cs[at.p];
+    const double c = G.cost[k];
+    const double g = c + (m > 0 ? s * G.ics[at.p] : 0.0);
+    const double lo = G.lower[k];
+    const double up = G.upper[k];
+    e[4] += value * value;
+    e[2] += c * value;
+    const double lam = lam_of(g, lo, up);
+    e[1] += (g - lam) * (g - lam);
+    if (lam > 0.0) e[3] += lam * lo;
+    if (lam < 0.0) e[3] += lam * up;
+    const double dv = xv - static_cast<double>(halpern ? S.col(kSum, at) : Z.x(at.p));
+    e[7] += dv * dv;
+  }, Ready());
+  return true;
+}
+
+// Runs one instance; false when a wait gave up. Storage, products and step sums in T (GB300's
+// FP64 pipe is small), the evaluation in FP64.
+template <typename T, int MODE, bool halpern>
+__device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
+                               EvalContext<T, MODE>* ctx, unsigned rank,
+                               unsigned size) {
+  constexpr bool kF64 = sizeof(T) == 8;
+  const int g = b.inst_mat[inst];
+  const T* kval = reinterpret_cast<const T*>(kF64 ? static_cast<const void*>(b.k_val)
+                                                  : static_cast<const void*>(b.k_val32));
+  const T* tval = reinterpret_cast<const T*>(kF64 ? static_cast<const void*>(b.t_val)
+                                                  : static_cast<const void*>(b.t_val32));
+  MatShare<T> M = mat_share<T>(b, g, kval, tval, rank, size);
+  const int m = M.m;
+  const int n = M.n;
+  const long long nt = static_cast<long long>(n) + m;
+  const long long vo = b.vec_off[inst];
+  const Given G{M.kperm, M.tperm, b.cost + vo, b.lower + vo, b.upper + vo,
+                b.cs + b.mat_col_off[g], b.rs + b.mat_row_off[g], b.ics + b.mat_col_off[g],
+                b.irs + b.mat_row_off[g], n};
+  const MatInfo mi = b.info[g];
+  // Device storage (instance_elements): the gathered vectors where they do not fit, the second
+  // points, the state where it does not fit.
+  T* st = reinterpret_cast<T*>(b.state) + b.state_off[inst];
+  const Second<T> Z{st + nt + 2, n, m};
+  Exchange<T, MODE> ex = make_exchange<T, MODE>(M, sh, st, rank, size);
+  SolveState<T, MODE> S;
+  S.device = st + 3 * nt + 2;
+  S.rows_device = (share_rows(n, M.Kt.slice, 1) >> M.Kt.slice) * 32 * kColArrays;
+  S.cols_at = static_cast<unsigned>(cluster_vector_bytes(n, m, M.Kt.slice, M.K.slice,
+                                                         static_cast<int>(size), sizeof(T)));
+  S.rows_at = S.cols_at + M.Kt.slices() * static_cast<unsigned>(32 * kColArrays * sizeof(T));
+  S.rank = rank;
+  S.size = size;
+  if (threadIdx.x == 0) {
+    ctx->M = M;
+    ctx->ex = ex;
+    ctx->S = S;
+    ctx->Z = Z;
+    ctx->G = G;
+  }
+  // Scaled problem, zero iterates, ||c||.
+  double nrm[3] = {0.0, 0.0, 0.0};
+  each_own(M.Kt, [&](const At& at) {
+    const int k = G.tperm[at.p];
+    const double sc = G.cs[at.p];
+    const double c0 = G.cost[k];
+    const double c = c0 * sc;
+    S.col(kCost, at) = static_cast<T>(c);
+    S.col(kLower, at) = static_cast<T>(G.lower[k] / sc);
+    S.col(kUpper, at) = static_cast<T>(G.upper[k] / sc);
+    S.col(kPoint, at) = S.col(kSum, at) = Z.x(at.p) = T(0);
+    nrm[0] += c0 * c0;
+    nrm[1] += c * c;
+  });
+  each_own(M.K, [&](const At& at) {
+    const int k = n + G.kperm[at.p];
+    const double r = G.rs[at.p];
+    const double c0 = G.cost[k];
+    const double lo = G.lower[k] * r;
+    const double up = G.upper[k] * r;
+    S.row(kCost, at) = static_cast<T>(c0 * r);
+    S.row(kLower, at) = static_cast<T>(lo);
+    S.row(kUpper, at) = static_cast<T>(up);
+    S.row(kPoint, at) = S.row(kSum, at) = S.row(kBar, at) = T(0);
+    S.row(kDual, at) = S.row(kDualSum, at) = Z.r(at.p) = Z.y(at.p) = T(0);
+    nrm[0] += c0 * c0;
+    const double bb = fmax(isfinite(lo) ? fabs(lo) : 0.0, isfinite(up) ? fabs(up) : 0.0);
+    nrm[2] += bb * bb;
+  });
+  cluster_reduce<3>(nrm, sh, rank, size);
+  const double c_norm = sqrt(nrm[0]);
+  double omega = 1.0;
+  if (b.algorithm >= 1) {
+    const double cn = sqrt(nrm[1]), bn = sqrt(nrm[2]);
+    omega = (cn > 1e-10 && bn > 1e-10) ? cn / bn : 1.0;
+  }
+  const double eta = mi.eta;
+  double tau = eta / omega, sigma = eta * omega;
+  long long max_iter = b.max_iter;
+  if (max_iter <= 0) {
+    max_iter = 10000LL * nt / 10;
+    if (max_iter < 10000LL) max_iter = 10000LL;
+    if (max_iter > 1000000LL) max_iter = 1000000LL;
+  }
+  double kar = INFINITY, kprev = INFINITY;
+  long long t = 0, k_since = 0, restarts = 0;
+  int status = kIterationLimit;
+  int result_avg = 0;
+  double inv_k = 1.0;  // 1 / iterations since the restart, at an evaluation
+  Meas final_meas{0, 0, 0, 0, 0};
+  bool ok = true;
+  // The gathered vector the first step reads.
+  if (halpern) {
+    each_own(M.K, [&](const At& at) { ex.put_y(at, T(0)); });
+  } else {
+    each_own(M.Kt, [&](const At& at) { ex.put_x(at, T(0)); });
+  }
+  while (t < max_iter) {
+    // The iterations up to the next evaluation.
+    long long steps = 64 - t % 64;
+    if (steps > max_iter - t) steps = max_iter - t;
+    ok = run_steps<T, MODE, halpern>(ctx, static_cast<int>(steps), k_since, static_cast<T>(tau),
+                                     static_cast<T>(sigma));
+    t += steps;
+    k_since += steps;
+    ok = ok && ex.wait(halpern ? 1 : 0);
+    if (!ok) break;
+    // Evaluation of the current and the average iterate; Halpern: only T(z) (the Halpern iterate
+    // itself can leave the bounds).
+    if (!halpern) {
+      each_own(M.Kt, [&](const At& at) { Z.saved(at.p) = ex.xs()[at.p]; });
+      inv_k = 1.0 / static_cast<double>(k_since);
+    }
+    // a: the current iterate's 7 sums, the average's 7, the distances (v, y) of each, and
+    // whether the time limit has passed (asked by one thread, so that all agree).
+    double a[19];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) a[q] = 0.0;
+    for (int w = halpern ? 1 : 0; w < 2 && ok; ++w) {
+      cluster_sync(size);  // every CTA has read xs and ys, their last entries in place
+      double e[9];
+      ok = evaluate_point<T, MODE>(ctx, halpern ? 2 : w, inv_k, e);
+      if (w == 0) {
+#pragma unroll
+        for (int q = 0; q < 7; ++q) a[q] = e[q];
+        a[14] = e[7];
+        a[15] = e[8];
+      } else {
+#pragma unroll
+        for (int q = 0; q < 7; ++q) a[7 + q] = e[q];
+        a[16] = e[7];
+        a[17] = e[8];
+      }
+    }
+    if (!ok) break;
+    if (rank == 0 && threadIdx.x == 0) {
+      const unsigned long long deadline = *b.deadline;
+      if (deadline != 0ull && globaltimer_ns() > deadline) a[18] = 1.0;
+    }
+    cluster_reduce<19>(a, sh, rank, size);
+    const Meas mc = finish7(a, mi.a_norm_max_col, mi.at_norm_max_row, c_norm, m);
+    const Meas ma = finish7(a + 7, mi.a_norm_max_col, mi.at_norm_max_row, c_norm, m);
+    const double tol = b.tol;
+    if (!halpern && mc.rp < tol && mc.rd < tol && fabs(mc.rg) < tol) {
+      status = kOptimal;
+      final_meas = mc;
+      break;
+    }
+    if (ma.rp < tol && ma.rd < tol && fabs(ma.rg) < tol) {
+      status = kOptimal;
+      result_avg = 1;
+      final_meas = ma;
+      break;
+    }
+    final_meas = halpern ? ma : mc;
+    // Restart (pdlp.cpp:1069-1131); the Halpern iteration restarts to T(z).
+    const double kc = kkt_w(omega, mc), ka = kkt_w(omega, ma);
+    const bool to_avg = halpern || ka < kc;
+    const double cand = halpern ? ka : fmin(kc, ka);
+    if (!(kar < INFINITY)) kar = cand;
+    const bool restart = cand <= 0.2 * kar || (cand <= 0.8 * kar && cand > kprev) ||
+                         static_cast<double>(k_since) >= b.art_frac * static_cast<double>(t);
+    kprev = cand;
+    if (restart) {
+      const double dx = sqrt(to_avg ? a[16] : a[14]);
+      const double dy = sqrt(to_avg ? a[17] : a[15]);
+      if (dx > 1e-10 && dy > 1e-10) {
+        omega = exp(0.5 * log(dy / dx) + 0.5 * log(omega));
+        tau = eta / omega;
+        sigma = eta * omega;
+      }
+      // The candidate becomes the point, the extrapolated point and the anchor; a sum starts
+      // again from nothing (an FP32 average is replaced by the first step's weight 1).
+      each_own(M.Kt, [&](const At& at) {
+        const T v = halpern  ? Z.x(at.p)
+                    : to_avg ? static_cast<T>(average(S.col(kSum, at), inv_k))
+                             : S.col(kPoint, at);
+        S.col(kPoint, at) = v;
+        if (halpern) {
+          S.col(kSum, at) = v;
+        } else {
+          Z.x(at.p) = v;
+          Z.saved(at.p) = v;
+          if (kF64) S.col(kSum, at) = T(0);
+        }
+      });
+      each_own(M.K, [&](const At& at) {
+        T v, y;
+        if (halpern) {
+          v = Z.r(at.p);
+          y = Z.y(at.p);
+        } else if (to_avg) {
+          v = kF64 && S.row(kLower, at) == S.row(kUpper, at)
+                  ? S.row(kLower, at)
+                  : static_cast<T>(average(S.row(kSum, at), inv_k));
+          y = static_cast<T>(average(S.row(kDualSum, at), inv_k));
+        } else {
+          v = S.row(kPoint, at);
+          y = S.row(kDual, at);
+        }
+        S.row(kPoint, at) = v;
+        S.row(kDual, at) = y;
+        if (halpern) {
+          S.row(kSum, at) = v;
+          S.row(kDualSum, at) = y;
+        } else {
+          S.row(kBar, at) = -v;
+          Z.r(at.p) = v;
+          Z.y(at.p) = y;
+          if (kF64) S.row(kSum, at) = S.row(kDualSum, at) = T(0);
+        }
+      });
+      k_since = 0;
+      kar = cand;
+      kprev = INFINITY;
+      ++restarts;
+    }
+    if (a[18] != 0.0) {
+      status = kTimeLimit;
+      break;
+    }
+    // The gathered vector the next iteration reads first.
+    if (halpern) {
+      each_own(M.K, [&](const At& at) { ex.put_y(at, S.row(kDual, at)); });
+    } else {
+      each_own(M.Kt, [&](const At& at) { ex.put_x(at, Z.saved(at.p)); });
+    }
+  }
+  // Entries put after the last evaluation are taken in before anyone goes on.
+  if (ok && status == kIterationLimit) ok = ex.wait(halpern ? 1 : 0);
+  __syncthreads();
+  // Answer in the LpProblem's space (Halpern: T(z), within the bounds).
+  double* xo = b.x_out + vo;
+  double* yo = b.y_out + b.row_off[inst];
+  each_own(M.Kt, [&](const At& at) {
+    const T v = halpern      ? Z.x(at.p)
+                : result_avg ? static_cast<T>(average(S.col(kSum, at), inv_k))
+                             : S.col(kPoint, at);
+    xo[G.tperm[at.p]] = static_cast<double>(v) * G.cs[at.p];
+  });
+  each_own(M.K, [&](const At& at) {
+    T v, y;
+    if (halpern) {
+      v = Z.r(at.p);
+      y = Z.y(at.p);
+    } else if (result_avg) {
+      v = kF64 && S.row(kLower, at) == S.row(kUpper, at)
+              ? S.row(kLower, at)
+              : static_cast<T>(average(S.row(kSum, at), inv_k));
+      y = static_cast<T>(average(S.row(kDualSum, at), inv_k));
+    } else {
+      v = S.row(kPoint, at);
+      y = S.row(kDual, at);
+    }
+    xo[n + G.kperm[at.p]] = static_cast<double>(v) / G.rs[at.p];
+    yo[G.kperm[at.p]] = static_cast<double>(y) * G.rs[at.p];
+  });
+  if (rank == 0 && threadIdx.x == 0) {
+    InstResult& r = b.results[inst];
+    r.status = ok ? status : kNumericalError;
+    r.iterations = status == kIterationLimit ? max_iter : t;
+    r.rel_primal = final_meas.rp;
+    r.rel_dual = final_meas.rd;
+    r.rel_gap = final_meas.rg;
+    r.primal_obj = final_meas.pobj;
+    r.dual_obj = final_meas.dobj;
+    r.restarts = restarts;
+  }
+  if (!ok && threadIdx.x == 0) atomicExch(b.wait_error, 1);
+  return ok;
+}
+
+// The next position of the work queue, the same for every thread of the cluster.
+__device__ __forceinline__ int next_instance(unsigned* queue, ClusterShared& sh, unsigned rank,
+                                             unsigned size) {
+  cluster_sync(size);  // the last instance is done, its position read by all
+  if (rank == 0 && threadIdx.x == 0) {
+    const unsigned q = atomicAdd(queue, 1u);
+    for (unsigned p = 0; p < size; ++p) st_cluster(map_rank(shared_addr(&sh.next), p), q);
+  }
+  cluster_sync(size);
+  return sh.next;
+}
+
+}  // namespace
+
+template <typename T>
+constexpr int solve_threads() {
+  return sizeof(T) == 8 ? kThreads64 : kThreads32;
+}
+
+template <typename T, int MODE, bool HALPERN>
+__global__ void __launch_bounds__(solve_threads<T>(), sizeof(T) == 8 ? 2 : 1)
+    batch_solve_kernel(BatchView b, InstanceList list) {
+  __shared__ ClusterShared sh;
+  __shared__ EvalContext<T, MODE> ctx;
+  const unsigned rank = cluster_rank();
+  const unsigned size = cluster_size();
+  cluster_init(sh, size);
+  for (;;) {
+    const int q = next_instance(b.queue + MODE, sh, rank, size);
+    if (q >= list.count) break;
+    if (!solve_instance<T, MODE, HALPERN>(b, list.inst[q], sh, &ctx, rank, size)) break;
+  }
+  cluster_sync(size);
+}
+
+template <typename T>
+cudaError_t launch_solve(const BatchView& b, const ClusterPlan& p, int mode, cudaStream_t s) {
+  const InstanceList list = p.group[mode];
+  const int clusters = list.count < p.clusters ? list.count : p.clusters;
+  auto go = [&](auto kernel) {
+    return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], s, b, list);
+  };
+  const bool h = b.algorithm == 2;
+  if (mode == kAllShared) {
+    return h ? go(batch_solve_kernel<T, kAllShared, true>)
+             : go(batch_solve_kernel<T, kAllShared, false>);
+  }
+  if (mode == kVectorsShared) {
+    return h ? go(batch_solve_kernel<T, kVectorsShared, true>)
+             : go(batch_solve_kernel<T, kVectorsShared, false>);
+  }
+  return h ? go(batch_solve_kernel<T, kInDevice, true>)
+           : go(batch_solve_kernel<T, kInDevice, false>);
+}
+
+}  // namespace sg
