@@ -314,7 +314,8 @@ int Engine::create_from_device(Engine** out, const DeviceLp& d, const Options& o
     delete e;
     return code;
   }
-  rc = e->set_active_rows(d.row_inert, &why);
+  rc = e->upload_chunk(&why);
+  if (rc == kOk) rc = e->set_active_rows(d.row_inert, &why);
   if (rc == kOk) rc = e->find_neighbours(&why);
   if (rc == kOk) rc = e->tune_tiles(&why);
   if (rc != kOk) {
@@ -800,6 +801,7 @@ int Engine::alloc_all(std::string* err) {
   const size_t nb = static_cast<size_t>(nnz_);
   SG_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   for (auto& ev : ev_) SG_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  plan_chunk();
   // The nonzero arrays carry kSegPad zeroed elements after the last nonzero: a staged segment's
   // bulk copies end at the 4-aligned position above it.
   auto layout = [&](Carver& c) {
@@ -838,6 +840,19 @@ int Engine::alloc_all(std::string* err) {
     for (double** p : {&rhs_ev_, &rs_, &rn_, &pu_, &u0_, &y_out_, &ray_out_}) c.take(p, m);
     for (double** p : {&cs_, &cn_, &pv_, &inv_cs_}) c.take(p, static_cast<size_t>(n_));
     c.take(&inv_rs_, m);
+    if (chunk_size_ > 0 || chunk32_size_ > 0) {
+      for (DevClusterOp* op : {&Kc_, &Ktc_}) {
+        c.take(&op->sl, op->sl_host.size());
+        c.take(&op->desc, op->desc_host.size());
+        c.take(&op->perm, op->order.perm.size());
+        c.take(&op->pos, op->order.pos.size());
+        c.take(&op->idx, static_cast<size_t>(op->elements));
+        c.take(&op->val, static_cast<size_t>(op->elements));
+        if (chunk32_size_ > 0) c.take(&op->val32, static_cast<size_t>(op->elements));
+      }
+      c.take(&chunk_second_, nt + m);
+      if (chunk32_size_ > 0) c.take(&chunk_second32_, nt + m);
+    }
     c.take(&partial_, static_cast<size_t>(4096) * kMaxSums);
     c.take(&counter_, 8);
     c.take(&ctl_, 1);
@@ -874,6 +889,99 @@ int Engine::alloc_all(std::string* err) {
   memset(ctl_host_, 0, sizeof(Ctl));
   configure_kernels();
   return kOk;
+}
+
+// Whether the chunk's iterations run on a cluster (chunk_kernel), and on how many CTAs: up to where
+// 16 SMs take as long as the step launches do. Measured, us an iteration with its share of the
+// evaluation, w = 2 nnz + 5 (n + m), step launches against 4 / 8 / 16 CTAs:
+//   FP64  200 x 500 (w 9,500)        11.8 against 5.4 / 5.7 / 6.1
+//         777 x 2,049 (39,000)       12.2 against 7.1 / 6.0 / 6.5
+//         2,000 x 5,000 (95,000)     12.6 against 10.4 / 8.4 / 7.0
+//         5,000 x 10,000 (195,000)   12.9 against - / 13.3 / 10.6
+//   FP32  200 x 500                  9.7 against 4.4 / 4.7 / 5.2
+//         5,000 x 10,000             10.9 against 11.4 / 9.2 / 7.6
+void Engine::plan_chunk() {
+  if (m_ <= 0 || n_ <= 0 || nnz_ <= 0) return;
+  const long long work = 2 * nnz_ + 5 * (static_cast<long long>(n_) + m_);
+  constexpr long long kMost64 = 220000, kMost32 = 300000;
+  if (work > kMost32) return;
+  const int size = work <= 20000 ? 4 : work <= 45000 ? 8 : 16;
+  Kc_.order = order_rows(K_.host_ptr.data(), m_);
+  Ktc_.order = order_rows(Kt_.host_ptr.data(), n_);
+  auto fits = [&](size_t elem) {
+    return chunk_fits(chunk_smem_bytes(n_, m_, Ktc_.order.slice, Kc_.order.slice, size, elem));
+  };
+  auto longest = [](const std::vector<int>& ptr) {
+    int most = 0;
+    for (size_t r = 0; r + 1 < ptr.size(); ++r) most = std::max(most, ptr[r + 1] - ptr[r]);
+    return most;
+  };
+  if (work <= kMost64 && fits(sizeof(double))) chunk_size_ = size;
+  // FP32 sums keep the step kernels' order: rows longer than kWarpRowMin have another. (The
+  // refinement's inner problems have a right-hand side, which these steps do not read.)
+  if (switch_ && fits(sizeof(float)) &&
+      std::max(longest(K_.host_ptr), longest(Kt_.host_ptr)) <= kWarpRowMin) {
+    chunk32_size_ = size;
+  }
+  if (chunk_size_ == 0 && chunk32_size_ == 0) return;
+  for (auto p : {std::make_pair(&Kc_, &K_), std::make_pair(&Ktc_, &Kt_)}) {
+    DevClusterOp& c = *p.first;
+    c.sl_host.resize(p.second->rows);
+    c.desc_host.resize(slices_of(c.order));
+    c.elements =
+        place_rows(p.second->host_ptr.data(), c.order, c.sl_host.data(), c.desc_host.data());
+  }
+}
+
+// The layout's arrays (the column numbers by a kernel: the operators are in device memory).
+int Engine::upload_chunk(std::string* err) {
+  if (chunk_size_ == 0 && chunk32_size_ == 0) return kOk;
+  cudaStream_t s = stream_;
+  for (DevClusterOp* c : {&Kc_, &Ktc_}) {
+    const int other = c == &Kc_ ? n_ : m_;
+    auto up = [&](void* dst, const void* src, size_t bytes) {
+      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
+    };
+    SG_TRY(up(c->sl, c->sl_host.data(), c->sl_host.size() * sizeof(StartLen)));
+    SG_TRY(up(c->desc, c->desc_host.data(), c->desc_host.size() * sizeof(StartLen)));
+    SG_TRY(up(c->perm, c->order.perm.data(), c->order.perm.size() * sizeof(int)));
+    SG_TRY(up(c->pos, c->order.pos.data(), c->order.pos.size() * sizeof(int)));
+    // Padding: value 0, the other operator's entry past the last.
+    const std::vector<int> pad(static_cast<size_t>(c->elements), other);
+    SG_TRY(up(c->idx, pad.data(), pad.size() * sizeof(int)));
+    SG_TRY(cudaMemsetAsync(c->val, 0, c->elements * sizeof(double), s));
+    if (c->val32) SG_TRY(cudaMemsetAsync(c->val32, 0, c->elements * sizeof(float), s));
+  }
+  launch_chunk_indices(chunk_view64(), K_.view64(), Kt_.view64(), s);
+  SG_TRY(cudaGetLastError());
+  SG_TRY(cudaStreamSynchronize(s));
+  return kOk;
+}
+
+namespace {
+
+template <typename T>
+ClusterOp<T> cluster_op(const DevClusterOp& c, T* val) {
+  return ClusterOp<T>{reinterpret_cast<const int2*>(c.sl), reinterpret_cast<const int2*>(c.desc),
+                      c.perm, c.pos, c.idx, val, c.order.slice};
+}
+
+}  // namespace
+
+ChunkView<double> Engine::chunk_view64() const {
+  return ChunkView<double>{cluster_op(Kc_, Kc_.val), cluster_op(Ktc_, Ktc_.val), chunk_second_,
+                           n_, m_, chunk_size_,
+                           chunk_smem_bytes(n_, m_, Ktc_.order.slice, Kc_.order.slice,
+                                            std::max(chunk_size_, 1), sizeof(double)),
+                           wait_error_};
+}
+
+ChunkView<float> Engine::chunk_view32() const {
+  return ChunkView<float>{cluster_op(Kc_, Kc_.val32), cluster_op(Ktc_, Ktc_.val32),
+                          chunk_second32_, n_, m_, chunk32_size_,
+                          chunk_smem_bytes(n_, m_, Ktc_.order.slice, Kc_.order.slice,
+                                           std::max(chunk32_size_, 1), sizeof(float)),
+                          wait_error_};
 }
 
 template <typename T>
@@ -993,6 +1101,7 @@ int Engine::setup_device(const double* rhs_orig) {
     }
   }
   launch_apply_scaling(K, Kt, rs_, cs_, nnz_, s);
+  if (chunk_size_ > 0) launch_chunk_values(chunk_view64(), K, Kt, s);
   launch_reciprocals(cs_, inv_cs_, n_, s);
   launch_reciprocals(rs_, inv_rs_, m_, s);
   launch_scale_vectors(n_, m_, cs_, rs_, cost_orig_, lower_orig_, upper_orig_, nullptr,
@@ -1043,14 +1152,20 @@ int Engine::equilibration(double* col_scale, double* row_scale, double* op_norm,
 namespace {
 
 // The kernels of one chunk; returns how many launches it records.
-// Ks is K over the active rows (the steps), K over every row (evaluation and detection).
+// Ks is K over the active rows (the steps), K over every row (evaluation and detection);
+// c.size > 0: the iterations in one cluster launch.
 template <typename T>
-int enqueue_chunk(Ctl* ctl, const OpView<T>& Ks, const OpView<T>& K, const OpView<T>& Kt,
+int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const OpView<T>& K,
+                  const OpView<T>& Kt,
                   const IterView<T>& it, const EvalView& ev, const RedView& red,
                   double* scratch_n, int gsk, int gst, int gk, int gt, bool halpern,
                   cudaStream_t s) {
   int kernels = 0;
-  for (int j = 0; j < kCheckFrequency; ++j) {
+  if (c.size > 0) {
+    launch_chunk(ctl, c, it, halpern, s);
+    kernels = 1;
+  }
+  for (int j = 0; j < kCheckFrequency && c.size == 0; ++j) {
     if (Ks.ts.ntiles > 0) ++kernels;
     if (Kt.ts.ntiles > 0) ++kernels;
     if (halpern) {
@@ -1072,7 +1187,7 @@ int enqueue_chunk(Ctl* ctl, const OpView<T>& Ks, const OpView<T>& K, const OpVie
 }  // namespace
 
 void Engine::enqueue_chunk_body() {
-  chunk_kernels_ = enqueue_chunk(ctl_, K_.step64(), K_.view64(), Kt_.view64(),
+  chunk_kernels_ = enqueue_chunk(ctl_, chunk_view64(), K_.step64(), K_.view64(), Kt_.view64(),
                                  iter_view(it64_), eval_view(), red_view(), scratch_n_,
                                  grid_step_k_, grid_step_t_, grid_k_, grid_t_,
                                  opt_.algorithm == 2, stream_);
@@ -1096,7 +1211,7 @@ int Engine::capture_chunk32() {
   IterView<float> it = iter_view(it32_);
   it.rhs = it32_.rhs;
   SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  chunk32_kernels_ = enqueue_chunk(ctl32_, K_.step32(), K_.view32(), Kt_.view32(), it,
+  chunk32_kernels_ = enqueue_chunk(ctl32_, chunk_view32(), K_.step32(), K_.view32(), Kt_.view32(), it,
                                    inner_eval_view(), red_view(), scratch_n_, grid_step_k_,
                                    grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2,
                                    stream_);
@@ -1176,8 +1291,8 @@ int Engine::run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, C
   return kOk;
 }
 
-// A staged segment's bulk copy that never completed (its bounded wait gave up) makes the
-// launch's sums unusable: the call reports it (and the flag is cleared).
+// A staged segment's bulk copy or a cluster's exchange that never completed (its bounded wait gave
+// up) makes the launch's sums unusable: the call reports it (and the flag is cleared).
 int Engine::check_wait_error(std::string* err) {
   int flag = 0;
   if (cudaMemcpy(&flag, wait_error_, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) {
@@ -1186,7 +1301,7 @@ int Engine::check_wait_error(std::string* err) {
   }
   if (flag == 0) return kOk;
   cudaMemset(wait_error_, 0, sizeof(int));
-  if (err) *err = "a bulk copy into shared memory did not complete";
+  if (err) *err = "a copy into shared memory did not complete";
   return kErrCuda;
 }
 
@@ -1333,6 +1448,7 @@ int Engine::prepare_fp32() {
   const long long nb = nnz_;
   launch_convert(K_.val, K_.val32, nb, s);
   launch_convert(Kt_.val, Kt_.val32, nb, s);
+  if (chunk32_size_ > 0) launch_chunk_values(chunk_view32(), K_.view32(), Kt_.view32(), s);
   SG_TRY(cudaMemcpyAsync(ctl32_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToDevice, s));
   launch_setup_norms(ctl32_, K_.view64(), Kt_.view64(), it64_.cost, red_view(), grid_k_, grid_t_,
                      s);

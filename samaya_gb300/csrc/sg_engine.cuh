@@ -10,6 +10,8 @@
 #include <string>
 #include <vector>
 
+#include "sg_chunk.cuh"
+#include "sg_cluster_layout.h"
 #include "sg_kernels.cuh"
 #include "sg_refine.cuh"
 
@@ -159,6 +161,20 @@ struct DevOp {
   OpView<float> step32() const { return OpView<float>{ptr, idx, val32, rows, step_tileset()}; }
 };
 
+// An operator in the cluster kernels' layout (sg_chunk.cu), beside its CSR arrays.
+struct DevClusterOp {
+  RowOrder order;
+  std::vector<StartLen> sl_host, desc_host;
+  long long elements = 0;
+  StartLen* sl = nullptr;
+  StartLen* desc = nullptr;
+  int* perm = nullptr;
+  int* pos = nullptr;
+  int* idx = nullptr;
+  double* val = nullptr;
+  float* val32 = nullptr;
+};
+
 // Iterate storage of one precision.
 template <typename T>
 struct DevIter {
@@ -283,6 +299,16 @@ class Engine {
   int finish_fp64(SolveInfo* info, double t0, long long iterations_before, double* x, double* y,
                   double* dual_ray, double* primal_ray);
   void enqueue_chunk_body();
+  // The cluster form of the chunk's iterations: whether and on how many CTAs (0: step launches),
+  // its arrays and views.
+  void plan_chunk();
+  int upload_chunk(std::string* err);
+  int chunk_size_ = 0, chunk32_size_ = 0;
+  DevClusterOp Kc_, Ktc_;
+  double* chunk_second_ = nullptr;
+  float* chunk_second32_ = nullptr;
+  ChunkView<double> chunk_view64() const;
+  ChunkView<float> chunk_view32() const;
   int check(cudaError_t e, const char* what);
   TileShape default_shape(const DevOp& op) const;
   int set_tiles(DevOp* op, const TileShape& shape);
