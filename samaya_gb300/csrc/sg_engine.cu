@@ -762,16 +762,21 @@ int Engine::tune_tiles(std::string* err) {
     }
   }
   dfree(long_terms_);
-  const int maxlong = std::max(std::max(std::max(K_.nlong, K_.st_nlong), Kt_.nlong), 1);
+  const int maxlong = std::max(std::max(K_.nlong + Kt_.nlong, K_.st_nlong), 1);
   if (dalloc(&long_terms_, static_cast<size_t>(maxlong) * kMaxSums) != cudaSuccess) {
     if (err) *err = "out of device memory";
     return kErrOutOfMemory;
   }
-  // Grids: persistent CTAs for the evaluation kernels (2 per SM; 4 per SM measured no faster
-  // on the transportation LP); one CTA per tile for the step kernels.
-  const int eval_cap = sm_count_ * 2;
+  // Grids: persistent CTAs for the evaluation kernels (4 per SM: the transportation LP's solve of
+  // 512 FP32 iterations 21.0 ms at 2, 20.6 at 4, 20.7 at 6); one CTA per tile for the step kernels.
+  const int eval_cap = sm_count_ * 4;
   grid_k_ = std::max(1, std::min(K_.ntiles, eval_cap));
   grid_t_ = std::max(1, std::min(Kt_.ntiles, eval_cap));
+  // The setup's passes, few registers a thread: as many CTAs as fit (the power-law LP of 400,000 x
+  // 800,000, 192 iterations: 18.9 ms at 2 per SM, 18.3 at 4, 17.8 at 8).
+  const int setup_cap = sm_count_ * 8;
+  grid_setup_k_ = std::max(1, std::min(K_.ntiles, setup_cap));
+  grid_setup_t_ = std::max(1, std::min(Kt_.ntiles, setup_cap));
   grid_step_k_ = std::max(1, std::min(K_.step_tiles(), 65535));
   grid_full_k_ = std::max(1, std::min(K_.ntiles, 65535));
   grid_step_t_ = std::max(1, std::min(Kt_.ntiles, 65535));
@@ -1031,6 +1036,18 @@ RedView Engine::red_view() const {
   return r;
 }
 
+namespace {
+
+// V[0] to Vrst and Y[0] to Yrst lie one after another in the arena: a memset each.
+template <typename T>
+cudaError_t zero_iterates(const DevIter<T>& it, size_t nt, size_t m, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(it.V[0], 0, (it.Vrst + nt - it.V[0]) * sizeof(T), s);
+  return e != cudaSuccess ? e
+                          : cudaMemsetAsync(it.Y[0], 0, (it.Yrst + m - it.Y[0]) * sizeof(T), s);
+}
+
+}  // namespace
+
 // Device setup (pdlp.cpp:260-316, 377-394, 490-492): working values from the originals,
 // residual-scale constants, Ruiz, A_eq, scaled vectors, operator norm and step sizes; iterates
 // zeroed. Asynchronous on the engine's stream.
@@ -1038,16 +1055,10 @@ int Engine::setup_device(const double* rhs_orig) {
   (void)rhs_orig;
   cudaStream_t s = stream_;
   const size_t nt = static_cast<size_t>(n_) + m_;
-  const size_t nb = static_cast<size_t>(nnz_);
   std::string* err = nullptr;
-  if (nb > 0) {
-    SG_TRY(cudaMemcpyAsync(K_.val, K_.val_orig, nb * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    SG_TRY(cudaMemcpyAsync(Kt_.val, Kt_.val_orig, nb * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  }
   SG_TRY(cudaMemcpyAsync(cost_ev_, cost_orig_, nt * sizeof(double), cudaMemcpyDeviceToDevice, s));
   SG_TRY(cudaMemcpyAsync(lower_ev_, lower_orig_, nt * sizeof(double), cudaMemcpyDeviceToDevice, s));
   SG_TRY(cudaMemcpyAsync(upper_ev_, upper_orig_, nt * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  SG_TRY(cudaMemsetAsync(ctl_, 0, sizeof(Ctl), s));
   // Constant fields of the control block.
   Ctl h;
   memset(&h, 0, sizeof(h));
@@ -1076,51 +1087,36 @@ int Engine::setup_device(const double* rhs_orig) {
   // takes 1,984 instead of 2,112 FP64 iterations.
   h.art_frac = opt_.artificial_restart > 0 ? opt_.artificial_restart
                                            : (opt_.algorithm == 0 ? 0.36 : 0.1);
-  SG_TRY(cudaMemcpyAsync(ctl_, &h, sizeof(Ctl), cudaMemcpyHostToDevice, s));
-  SG_TRY(cudaStreamSynchronize(s));  // h lives on this stack frame
   const OpView<double> K = K_.view64();
   const OpView<double> Kt = Kt_.view64();
+  // The given values, which the scaling reads.
+  OpView<double> K0 = K, Kt0 = Kt;
+  K0.val = K_.val_orig;
+  Kt0.val = Kt_.val_orig;
   const RedView red = red_view();
-  // Scale factors start at 1.
-  {
-    std::vector<double> ones(std::max(nt, static_cast<size_t>(1)), 1.0);
-    SG_TRY(cudaMemcpyAsync(cs_, ones.data(), static_cast<size_t>(n_) * sizeof(double),
-                           cudaMemcpyHostToDevice, s));
-    SG_TRY(cudaMemcpyAsync(rs_, ones.data(), static_cast<size_t>(m_) * sizeof(double),
-                           cudaMemcpyHostToDevice, s));
-    SG_TRY(cudaStreamSynchronize(s));
-  }
-  launch_setup_norms(ctl_, K, Kt, cost_orig_, red, grid_k_, grid_t_, s);
+  launch_setup_begin(ctl_, h, n_, m_, cs_, cn_, rs_, rn_, s);
+  launch_setup_norms(ctl_, K0, Kt0, cost_orig_, red, grid_k_, grid_t_, s);
   if (m_ > 0 && n_ > 0) {
     if (opt_.algorithm >= 1) {
-      launch_enhanced_scaling(K, Kt, rs_, cs_, rn_, cn_, grid_k_, grid_t_, s);
+      launch_enhanced_scaling(K0, Kt0, rs_, cs_, rn_, cn_, grid_setup_k_, grid_setup_t_, s);
     } else {
-      for (int pass = 0; pass < 10; ++pass) {
-        launch_ruiz_pass(ctl_, K, Kt, rs_, cs_, rn_, cn_, red, grid_k_, grid_t_, s);
-      }
+      launch_ruiz(ctl_, K0, Kt0, rs_, cs_, rn_, cn_, red, grid_setup_k_, grid_setup_t_, s);
     }
   }
-  launch_apply_scaling(K, Kt, rs_, cs_, nnz_, s);
+  launch_apply_scaling(K, Kt, K_.val_orig, Kt_.val_orig, rs_, cs_, nnz_, s);
   if (chunk_size_ > 0) launch_chunk_values(chunk_view64(), K, Kt, s);
-  launch_reciprocals(cs_, inv_cs_, n_, s);
-  launch_reciprocals(rs_, inv_rs_, m_, s);
-  launch_scale_vectors(n_, m_, cs_, rs_, cost_orig_, lower_orig_, upper_orig_, nullptr,
-                       it64_.cost, it64_.lower, it64_.upper, nullptr, s);
+  launch_scale_vectors(n_, m_, cs_, rs_, cost_orig_, lower_orig_, upper_orig_, it64_.cost,
+                       it64_.lower, it64_.upper, inv_cs_, inv_rs_, s);
   if (m_ > 0) {
     SG_TRY(cudaMemcpyAsync(pu_, u0_, static_cast<size_t>(m_) * sizeof(double),
                            cudaMemcpyDeviceToDevice, s));
   }
-  launch_power_iteration(ctl_, K, Kt, pu_, pv_, red, 20, grid_k_, grid_t_, s);
+  launch_power_iteration(ctl_, K, Kt, pu_, pv_, red, 20, grid_setup_k_, grid_setup_t_, s);
   if (opt_.algorithm >= 1) {
     launch_primal_weight_init(ctl_, n_, m_, it64_.cost, it64_.lower, it64_.upper, red, s);
   }
   // Iterates start at zero (pdlp.cpp:323-329).
-  for (double* p : {it64_.V[0], it64_.V[1], it64_.Vbar, it64_.Verg, it64_.Vrst}) {
-    SG_TRY(cudaMemsetAsync(p, 0, nt * sizeof(double), s));
-  }
-  for (double* p : {it64_.Y[0], it64_.Y[1], it64_.Yerg, it64_.Yrst}) {
-    SG_TRY(cudaMemsetAsync(p, 0, static_cast<size_t>(m_) * sizeof(double), s));
-  }
+  SG_TRY(zero_iterates(it64_, nt, static_cast<size_t>(m_), s));
   SG_TRY(cudaGetLastError());
   return kOk;
 }
@@ -1243,22 +1239,22 @@ IterView<double> Engine::master_view() {
   return v;
 }
 
-// Replays a chunk graph until the device says done, keeping a few chunks in flight; the host
-// only reads the control block back (an event per chunk).
+// Replays a chunk graph until the device says done, one chunk running and one behind it; the host
+// only reads the control block back (an event per chunk). The device's iteration counter starts
+// at t0 and every chunk advances it by kCheckFrequency until max_iter, so no more chunks are
+// launched than reach it (a chunk after the end is 142 empty launches, 0.2 ms; three in flight
+// left two of them behind every solve).
 int Engine::run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, Ctl* ctl,
-                     int kernels_per_chunk, long long max_iter) {
+                     int kernels_per_chunk, long long t0, long long max_iter) {
   std::string* err = nullptr;
-  constexpr int kInflight = 3;
+  constexpr int kInflight = 2;
   int head = 0;  // oldest in flight
   int count = 0;
   long long launches = 0;
-  // Every chunk advances the device's iteration counter by kCheckFrequency until the limit, so
-  // a correct run needs at most this many launches; the bound keeps the host loop finite even
-  // if the device never reported done.
-  const long long launch_cap = max_iter / kCheckFrequency + 2 * kInflight + 4;
+  const long long launch_cap =
+      std::max<long long>(1, (max_iter - t0 + kCheckFrequency - 1) / kCheckFrequency);
   for (;;) {
-    if (launches >= launch_cap) break;
-    while (count < kInflight) {
+    while (count < kInflight && launches < launch_cap) {
       const int slot = (head + count) % 4;
       SG_TRY(cudaGraphLaunch(exec, stream_));
       SG_TRY(cudaMemcpyAsync(ctl_host_, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_));
@@ -1266,6 +1262,7 @@ int Engine::run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, C
       ++count;
       ++launches;
     }
+    if (count == 0) break;
     SG_TRY(cudaEventSynchronize(ev_[head]));
     head = (head + 1) % 4;
     --count;
@@ -1343,7 +1340,7 @@ int Engine::solve_fp64(SolveInfo* info, double* x, double* y, double* dual_ray,
   const double deadline = opt_.time_limit > 0 ? t0 + opt_.time_limit : 0.0;
   const double t_setup = now_s();
   info->setup_seconds = t_setup - t0;
-  rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, max_iterations());
+  rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, 0, max_iterations());
   if (rc != kOk) return rc;
   return finish_fp64(info, t0, 0, x, y, dual_ray, primal_ray);
 }
@@ -1441,7 +1438,6 @@ void finish_host(const Ctl& c, const double* s, double* rp, double* rd, double* 
 // of the equilibrated operators, the FP32 control block (the FP64 one's step size and initial
 // weight, the norms of the equilibrated matrix for its relative residuals), its chunk graph.
 int Engine::prepare_fp32() {
-  std::string* err = nullptr;
   cudaStream_t s = stream_;
   int rc = setup_device(nullptr);
   if (rc != kOk) return rc;
@@ -1449,17 +1445,9 @@ int Engine::prepare_fp32() {
   launch_convert(K_.val, K_.val32, nb, s);
   launch_convert(Kt_.val, Kt_.val32, nb, s);
   if (chunk32_size_ > 0) launch_chunk_values(chunk_view32(), K_.view32(), Kt_.view32(), s);
-  SG_TRY(cudaMemcpyAsync(ctl32_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToDevice, s));
+  launch_ir_begin(ctl32_, ctl_, s);
   launch_setup_norms(ctl32_, K_.view64(), Kt_.view64(), it64_.cost, red_view(), grid_k_, grid_t_,
                      s);
-  SG_TRY(cudaStreamSynchronize(s));
-  {
-    Ctl h;
-    SG_TRY(cudaMemcpy(&h, ctl32_, sizeof(Ctl), cudaMemcpyDeviceToHost));
-    h.ir_omega0 = h.omega;
-    h.q_norm = 0.0;
-    SG_TRY(cudaMemcpy(ctl32_, &h, sizeof(Ctl), cudaMemcpyHostToDevice));
-  }
   return capture_chunk32();
 }
 
@@ -1509,12 +1497,7 @@ int Engine::solve_switched(SolveInfo* info, double* x, double* y, double* dual_r
   const IrView irv = ir_view();
   launch_ir_scales(ctl32_, 0, 1e4, s);
   launch_ir_build(ctl32_, irv, 0, s);
-  for (float* p : {it32_.V[0], it32_.V[1], it32_.Vbar, it32_.Verg, it32_.Vrst}) {
-    SG_TRY(cudaMemsetAsync(p, 0, nt * sizeof(float), s));
-  }
-  for (float* p : {it32_.Y[0], it32_.Y[1], it32_.Yerg, it32_.Yrst}) {
-    SG_TRY(cudaMemsetAsync(p, 0, static_cast<size_t>(m_) * sizeof(float), s));
-  }
+  SG_TRY(zero_iterates(it32_, nt, static_cast<size_t>(m_), s));
   launch_norm_into(cost_in_, static_cast<long long>(nt), red_view(), &ctl32_->c_norm, s);
   launch_norm_into(rhs_in_, m_, red_view(), &ctl32_->q_norm, s);
   const long long max_iter = max_iterations();
@@ -1522,7 +1505,7 @@ int Engine::solve_switched(SolveInfo* info, double* x, double* y, double* dual_r
   if (opt_.time_limit > 0) launch_set_deadline(ctl32_, opt_.time_limit - (now_s() - t0), s);
   const double deadline = opt_.time_limit > 0 ? t0 + opt_.time_limit : 0.0;
   info->setup_seconds = now_s() - t0;
-  rc = run_loop(deadline, info, chunk32_exec_, ctl32_, chunk32_kernels_, max_iter);
+  rc = run_loop(deadline, info, chunk32_exec_, ctl32_, chunk32_kernels_, 0, max_iter);
   if (rc != kOk) return rc;
   const long long fp32_restarts = ctl_host_->restarts;
   const long long fp32_evals = ctl_host_->evaluations;
@@ -1530,7 +1513,7 @@ int Engine::solve_switched(SolveInfo* info, double* x, double* y, double* dual_r
   IterView<float> it32 = iter_view(it32_);
   launch_continue(ctl_, ctl32_, it32, iter_view(it64_), s);
   if (opt_.time_limit > 0) launch_set_deadline(ctl_, opt_.time_limit - (now_s() - t0), s);
-  rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, max_iter);
+  rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, ctl_host_->t, max_iter);
   if (rc != kOk) return rc;
   rc = finish_fp64(info, t0, 0, x, y, dual_ray, primal_ray);
   info->restarts += fp32_restarts;
@@ -1593,7 +1576,7 @@ int Engine::solve_refined(SolveInfo* info, double* x, double* y, double* dual_ra
     launch_norm_into(rhs_in_, m_, red_view(), &ctl32_->q_norm, s);
     launch_ir_reset(ctl32_, opt_.inner_tol, budget, kStallEvaluations, s);
     if (opt_.time_limit > 0) launch_set_deadline(ctl32_, opt_.time_limit - (now_s() - t0), s);
-    rc = run_loop(deadline, info, chunk32_exec_, ctl32_, chunk32_kernels_, budget);
+    rc = run_loop(deadline, info, chunk32_exec_, ctl32_, chunk32_kernels_, 0, budget);
     if (rc != kOk) return rc;
     total_iters += ctl_host_->t;
     if (round == 0) {
@@ -1641,7 +1624,7 @@ int Engine::solve_refined(SolveInfo* info, double* x, double* y, double* dual_ra
     const long long left = inner_max - total_iters;
     launch_restart_at_point(ctl_, round0_omega, iter_view(it64_), left, s);
     if (opt_.time_limit > 0) launch_set_deadline(ctl_, opt_.time_limit - (now_s() - t0), s);
-    rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, left);
+    rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, 0, left);
     if (rc != kOk) return rc;
     const long long restarts = info->restarts, evaluations = info->evaluations;
     rc = finish_fp64(info, t0, total_iters, x, y, dual_ray, primal_ray);

@@ -286,7 +286,7 @@ class Engine {
   EvalView eval_view() const;
   RedView red_view() const;
   int run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, Ctl* ctl,
-               int kernels_per_chunk, long long max_iter);
+               int kernels_per_chunk, long long t0, long long max_iter);
   int capture_chunk32();
   long long max_iterations() const;
   IterView<double> master_view();
@@ -330,6 +330,7 @@ class Engine {
   int check_wait_error(std::string* err);
   // grid_step_k_: the dual steps of the solves (active rows); grid_full_k_: every row.
   int grid_k_ = 1, grid_t_ = 1, grid_step_k_ = 1, grid_step_t_ = 1, grid_full_k_ = 1;
+  int grid_setup_k_ = 1, grid_setup_t_ = 1;
   int sm_count_ = 148;
   bool fp32_ = false;
   bool switch_ = false;   // FP32 PDLP, then FP64 PDLP from its answer

@@ -1338,102 +1338,182 @@ struct RuizProd {
   }
 };
 
-struct RuizEpi {
-  const double* own;
-  double* norm;
-  __device__ __forceinline__ void row(int r, const double (&s)[1]) { norm[r] = sqrt(s[0]) * own[r]; }
-  __device__ __forceinline__ void long_row(int, int r, const double (&s)[1]) { row(r, s); }
+// A scaling pass: every column (rows of K', the first grid_t CTAs) and every row (rows of K)
+// takes its statistic with the old scales and writes its new scale to the other buffer, so a
+// pass is one launch and needs no scratch vectors. (As three launches, K' and K statistics and
+// an update, 22 passes' worth took 1.7 ms of a 1,000 x 2,000 transportation LP's solve: the
+// update's square root and quotient alone 64 us of FP64 pipe a pass.)
+struct ScalePair {
+  const double* cs;
+  const double* rs;
+  double* cs_new;
+  double* rs_new;
 };
 
-__global__ void __launch_bounds__(kBlock) ruiz_norm_kernel(const Ctl* c, OpView<double> A,
-                                                           const double* own, const double* other,
-                                                           double* norm) {
-  if (c->ruiz_done) return;
-  RuizEpi epi{own, norm};
-  run_tiles<double, double, 1>(A.ts, A.ptr, A.idx, A.val, RuizProd{other}, epi);
-}
-
-// Scale update of one Ruiz pass (pdlp.cpp:154-178) over columns then rows.
-__global__ void __launch_bounds__(kBlock) ruiz_update_kernel(Ctl* c, int n, int m, double* cs,
-                                                             const double* cn, double* rs,
-                                                             const double* rn, RedView red) {
-  if (c->ruiz_done) return;
-  __shared__ double scratch[kMaxSums * (kBlock / 32)];
-  double a[1] = {0.0};
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + m; k += gridDim.x * blockDim.x) {
-    double* sc = k < n ? cs + k : rs + (k - n);
-    const double nv = k < n ? cn[k] : rn[k - n];
-    if (nv > 0) {
-      const double old = *sc;
-      double s = old / nv;
-      s = fmax(1e-8, fmin(1e8, s));
-      if (fabs(s - old) / fmax(fabs(old), 1.0) > 0.1) a[0] = 1.0;
-      *sc = s;
-    }
+// The reference's pass (pdlp.cpp:109-187): scale / norm within [1e-8, 1e8], the norm sqrt(sum)
+// times the scale; `changed` when a scale moved by more than a tenth.
+struct RuizEpi {
+  const double* own;
+  double* out;
+  double changed[1];
+  double* long_terms;
+  __device__ __forceinline__ double update(int r, double sum) const {
+    const double old = own[r];
+    const double nv = sqrt(sum) * old;
+    const double s = nv > 0 ? fmax(1e-8, fmin(1e8, old / nv)) : old;
+    out[r] = s;
+    return fabs(s - old) / fmax(fabs(old), 1.0) > 0.1 ? 1.0 : 0.0;
   }
-  grid_reduce<1, 1u>(a, red.partial, red.counter, scratch,
-                     [c](const double (&t)[1]) { c->ruiz_done = t[0] > 0.0 ? 0 : 1; });
+  __device__ __forceinline__ void row(int r, const double (&s)[1]) {
+    changed[0] = fmax(changed[0], update(r, s[0]));
+  }
+  __device__ __forceinline__ void long_row(int lrow, int r, const double (&s)[1]) {
+    long_terms[lrow * kMaxSums] = update(r, s[0]);
+  }
+};
+
+__global__ void __launch_bounds__(kBlock) ruiz_pass_kernel(Ctl* c, OpView<double> K,
+                                                           OpView<double> Kt, ScalePair sc,
+                                                           RedView red, int grid_t) {
+  if (c->ruiz_done) {
+    // No pass since has moved a scale: both buffers take the current ones.
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Kt.rows + K.rows;
+         k += gridDim.x * blockDim.x) {
+      if (k < Kt.rows) {
+        sc.cs_new[k] = sc.cs[k];
+      } else {
+        sc.rs_new[k - Kt.rows] = sc.rs[k - Kt.rows];
+      }
+    }
+    return;
+  }
+  RuizEpi epi{nullptr, nullptr, {0.0}, nullptr};
+  const int b = blockIdx.x;
+  if (b < grid_t) {
+    epi.own = sc.cs;
+    epi.out = sc.cs_new;
+    epi.long_terms = red.long_terms + static_cast<size_t>(K.ts.nlong) * kMaxSums;
+    run_tiles<double, double, 1>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, RuizProd{sc.rs}, epi, b, grid_t);
+  } else {
+    epi.own = sc.rs;
+    epi.out = sc.rs_new;
+    epi.long_terms = red.long_terms;
+    run_tiles<double, double, 1>(K.ts, K.ptr, K.idx, K.val, RuizProd{sc.cs}, epi, b - grid_t,
+                                 gridDim.x - grid_t);
+  }
+  grid_reduce<1, 1u>(epi.changed, red.partial, red.counter, smem_red(),
+                     [c](const double (&t)[1]) { c->ruiz_done = t[0] > 0.0 ? 0 : 1; },
+                     red.long_terms, K.ts.nlong + Kt.ts.nlong);
 }
 
 // A_eq = D_r A D_c on both operators: K entries (a rs_i) cs_j, K' entries (a cs_j) rs_i, the
-// association of apply_equilibration for A and A' (pdlp.cpp:204, 265-266). Rows by binary
-// search in the row starts.
-__device__ __forceinline__ int row_of(const int* ptr, int rows, int k) {
-  int lo = 0, hi = rows;  // ptr[lo] <= k < ptr[hi]
-  while (hi - lo > 1) {
+// association of apply_equilibration for A and A' (pdlp.cpp:204, 265-266). A warp takes 256
+// consecutive nonzeros: two of its lanes find the first's and the last's row in the row starts,
+// each nonzero's own row lies between (a search over all rows for every nonzero took 118 us for
+// the 4 million of a 1,000 x 2,000 transportation LP).
+__device__ __forceinline__ int row_between(const int* ptr, int lo, int hi, int k) {
+  while (hi - lo > 1) {  // ptr[lo] <= k < ptr[hi]
     const int mid = (lo + hi) >> 1;
-    if (ptr[mid] <= k) lo = mid; else hi = mid;
+    if (__ldg(ptr + mid) <= k) lo = mid; else hi = mid;
   }
   return lo;
 }
 
-__global__ void apply_scaling_kernel(OpView<double> K, OpView<double> Kt, const double* rs,
-                                     const double* cs, long long nnz) {
-  for (long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; k < nnz;
-       k += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int kk = static_cast<int>(k);
-    const int i = row_of(K.ptr, K.rows, kk);
-    const int j = K.idx[kk];
-    K.val[kk] = K.val[kk] * rs[i] * cs[j];
-    const int jj = row_of(Kt.ptr, Kt.rows, kk);
-    const int ii = Kt.idx[kk];
-    Kt.val[kk] = Kt.val[kk] * cs[jj] * rs[ii];
+__device__ __forceinline__ void scale_nonzeros(const OpView<double>& A, const double* given,
+                                               const double* own, const double* other, int k0,
+                                               int k1) {
+  const int lane = threadIdx.x & 31;
+  const int edge = lane == 0 ? k0 : k1 - 1;
+  int found = 0;
+  if (lane < 2) found = row_between(A.ptr, 0, A.rows, edge);
+  const int r0 = __shfl_sync(0xffffffffu, found, 0);
+  const int r1 = __shfl_sync(0xffffffffu, found, 1) + 1;
+  for (int k = k0 + lane; k < k1; k += 32) {
+    const int r = row_between(A.ptr, r0, r1, k);
+    A.val[k] = given[k] * __ldg(own + r) * __ldg(other + A.idx[k]);
   }
 }
 
-__global__ void scale_vectors_kernel(int n, int m, const double* cs, const double* rs,
-                                     const double* cost, const double* lower, const double* upper,
-                                     const double* rhs, double* cost_eq, double* lower_eq,
-                                     double* upper_eq, double* rhs_eq) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + m; k += gridDim.x * blockDim.x) {
-    if (k < n) {
-      cost_eq[k] = cost[k] * cs[k];
-      lower_eq[k] = lower[k] / cs[k];
-      upper_eq[k] = upper[k] / cs[k];
+__global__ void __launch_bounds__(kBlock) apply_scaling_kernel(
+    OpView<double> K, OpView<double> Kt, const double* k_given, const double* t_given,
+    const double* __restrict__ rs, const double* __restrict__ cs, int nnz) {
+  constexpr int kPerWarp = 256;
+  const int parts = (nnz + kPerWarp - 1) / kPerWarp;
+  const int warps = gridDim.x * (kBlock / 32);
+  for (int w = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); w < 2 * parts; w += warps) {
+    const bool rows = w < parts;
+    const int k0 = (rows ? w : w - parts) * kPerWarp;
+    const int k1 = min(k0 + kPerWarp, nnz);
+    if (rows) {
+      scale_nonzeros(K, k_given, rs, cs, k0, k1);
     } else {
-      const double r = rs[k - n];
-      cost_eq[k] = cost[k] * r;
-      lower_eq[k] = lower[k] * r;
-      upper_eq[k] = upper[k] * r;
-      if (rhs != nullptr) rhs_eq[k - n] = rhs[k - n] * r;
+      scale_nonzeros(Kt, t_given, cs, rs, k0, k1);
     }
   }
 }
 
-// Power iteration (pdlp.cpp:36-103) on A_eq: v = A' u, u = A v, sigma = |u| / |v|.
+// A column's bound over its scale. 0 and infinity, the usual bounds, stay: a warp of such skips
+// the quotient (150 us for 2 million columns with two quotients each, on the FP64 pipe).
+__device__ __forceinline__ double bound_over(double b, double scale) {
+  const long long mag = __double_as_longlong(b) & 0x7fffffffffffffffLL;
+  const bool stays = mag == 0 || mag == 0x7ff0000000000000LL;
+  const unsigned here = __activemask();
+  if (__any_sync(here, !stays)) {
+    __syncwarp(here);  // a branch, not predicated instructions
+    if (!stays) b = b / scale;
+  }
+  return b;
+}
+
+// The equilibrated cost and bounds, and the scales' reciprocals.
+__global__ void scale_vectors_kernel(int n, int m, const double* cs, const double* rs,
+                                     const double* cost, const double* lower, const double* upper,
+                                     double* cost_eq, double* lower_eq, double* upper_eq,
+                                     double* inv_cs, double* inv_rs) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + m; k += gridDim.x * blockDim.x) {
+    if (k < n) {
+      const double c = cs[k];
+      inv_cs[k] = 1.0 / c;
+      cost_eq[k] = cost[k] * c;
+      lower_eq[k] = bound_over(lower[k], c);
+      upper_eq[k] = bound_over(upper[k], c);
+    } else {
+      const double r = rs[k - n];
+      inv_rs[k - n] = 1.0 / r;
+      cost_eq[k] = cost[k] * r;
+      lower_eq[k] = lower[k] * r;
+      upper_eq[k] = upper[k] * r;
+    }
+  }
+}
+
+// Power iteration (pdlp.cpp:36-103) on A_eq: v = A' u, u = A v, sigma = |u| / |v|. In place of
+// u / |u| the A' product takes u times a power of two that brings |u| into [1, 2): sigma does
+// not see the length, the scaling is exact, and the quotients' launch between two products goes
+// (21 of 63, 19 us each for 400,000 rows).
 struct StoreSqEpi {
   double* out;
+  double scale;  // a power of two
   double acc[1];
   double* long_terms;
   __device__ __forceinline__ void row(int r, const double (&s)[1]) {
-    out[r] = s[0];
-    acc[0] += s[0] * s[0];
+    const double v = s[0] * scale;
+    out[r] = v;
+    acc[0] += v * v;
   }
   __device__ __forceinline__ void long_row(int lrow, int r, const double (&s)[1]) {
-    out[r] = s[0];
-    long_terms[lrow * kMaxSums] = s[0] * s[0];
+    const double v = s[0] * scale;
+    out[r] = v;
+    long_terms[lrow * kMaxSums] = v * v;
   }
 };
+
+// 2^-e for norm = f 2^e, f in [1, 2) (norm zero or not normal: 1).
+__device__ __forceinline__ double inverse_power(double norm) {
+  const int e = (__double2hiint(norm) >> 20) & 0x7ff;
+  if (e == 0 || e >= 0x7fe) return 1.0;
+  return __hiloint2double((0x7fe - e) << 20, 0);
+}
 
 __global__ void __launch_bounds__(kBlock) power_spmv_kernel(Ctl* c, OpView<double> A,
                                                             const double* x, double* y,
@@ -1441,6 +1521,7 @@ __global__ void __launch_bounds__(kBlock) power_spmv_kernel(Ctl* c, OpView<doubl
   if (c->power_done) return;
   StoreSqEpi epi;
   epi.out = y;
+  epi.scale = which == 0 ? inverse_power(c->power_unorm) : 1.0;
   epi.acc[0] = 0.0;
   epi.long_terms = red.long_terms;
   run_tiles<double, double, 1>(A.ts, A.ptr, A.idx, A.val, Gather1<double, double>{x}, epi);
@@ -1459,14 +1540,6 @@ __global__ void __launch_bounds__(kBlock) power_spmv_kernel(Ctl* c, OpView<doubl
       }
     }
   }, red.long_terms, A.ts.nlong);
-}
-
-__global__ void scale_by_norm_kernel(const Ctl* c, double* u, int m, int first) {
-  if (!first && c->power_done) return;
-  const double nrm = c->power_unorm;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    u[i] = u[i] / nrm;
-  }
 }
 
 __global__ void power_finish_kernel(Ctl* c) {
@@ -1537,30 +1610,30 @@ struct AbsProd {
   }
 };
 
-struct StatEpi {
+// scale / sqrt(statistic times scale) where that is positive.
+struct RescaleEpi {
   const double* own;
-  double* stat;
-  __device__ __forceinline__ void row(int r, const double (&s)[1]) { stat[r] = s[0] * own[r]; }
+  double* out;
+  __device__ __forceinline__ void row(int r, const double (&s)[1]) {
+    const double old = own[r];
+    const double stat = s[0] * old;
+    out[r] = stat > 0.0 ? old * rsqrt(stat) : old;
+  }
   __device__ __forceinline__ void long_row(int, int r, const double (&s)[1]) { row(r, s); }
 };
 
 template <bool MAXRED>
-__global__ void __launch_bounds__(kBlock) abs_stat_kernel(OpView<double> A, const double* own,
-                                                          const double* other, double* stat) {
-  StatEpi epi{own, stat};
-  run_tiles<double, double, 1, AbsProd, StatEpi, MAXRED>(A.ts, A.ptr, A.idx, A.val,
-                                                         AbsProd{other}, epi);
-}
-
-// scale /= sqrt(stat) where stat > 0, columns then rows.
-__global__ void sqrt_rescale_kernel(int n, int m, double* cs, const double* cn, double* rs,
-                                    const double* rn) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + m; k += gridDim.x * blockDim.x) {
-    if (k < n) {
-      if (cn[k] > 0.0) cs[k] = cs[k] / sqrt(cn[k]);
-    } else {
-      if (rn[k - n] > 0.0) rs[k - n] = rs[k - n] / sqrt(rn[k - n]);
-    }
+__global__ void __launch_bounds__(kBlock) abs_pass_kernel(OpView<double> K, OpView<double> Kt,
+                                                          ScalePair sc, int grid_t) {
+  const int b = blockIdx.x;
+  if (b < grid_t) {
+    RescaleEpi epi{sc.cs, sc.cs_new};
+    run_tiles<double, double, 1, AbsProd, RescaleEpi, MAXRED>(
+        Kt.ts, Kt.ptr, Kt.idx, Kt.val, AbsProd{sc.rs}, epi, b, grid_t);
+  } else {
+    RescaleEpi epi{sc.rs, sc.rs_new};
+    run_tiles<double, double, 1, AbsProd, RescaleEpi, MAXRED>(
+        K.ts, K.ptr, K.idx, K.val, AbsProd{sc.cs}, epi, b - grid_t, gridDim.x - grid_t);
   }
 }
 
@@ -1661,11 +1734,11 @@ void configure_kernels() {
   cudaFuncSetAttribute(det_farkas_cols_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(det_farkas_cols_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(max_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(ruiz_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(ruiz_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(power_spmv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(spmv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(abs_stat_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(abs_stat_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(abs_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(abs_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
 }
 
 template <typename T>
@@ -1842,39 +1915,28 @@ void launch_reciprocals(const double* a, double* out, int count, cudaStream_t s)
                                                                                      count);
 }
 
-void launch_ruiz_pass(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt, double* rs,
-                      double* cs, double* rn, double* cn, const RedView& red, int grid_k,
-                      int grid_t, cudaStream_t s) {
-  // Column norms (rows of K'), then row norms (rows of K), both with the old scales.
-  ruiz_norm_kernel<<<grid_t, kBlock, tile_smem_bytes(Kt.ts, 1, 8), s>>>(ctl, Kt, cs, rs, cn);
-  ruiz_norm_kernel<<<grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(ctl, K, rs, cs, rn);
-  const int nt = K.rows + Kt.rows;
-  ruiz_update_kernel<<<vec_grid(nt) < 1024 ? vec_grid(nt) : 1024, kBlock, 0, s>>>(
-      ctl, Kt.rows, K.rows, cs, cn, rs, rn, red);
+void launch_ruiz(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt, double* rs,
+                 double* cs, double* rn, double* cn, const RedView& red, int grid_k, int grid_t,
+                 cudaStream_t s) {
+  const size_t sm = tile_smem_bytes(K.ts, 1, 8);
+  for (int pass = 0; pass < 10; ++pass) {
+    const ScalePair sc = pass % 2 == 0 ? ScalePair{cs, rs, cn, rn} : ScalePair{cn, rn, cs, rs};
+    ruiz_pass_kernel<<<grid_t + grid_k, kBlock, sm, s>>>(ctl, K, Kt, sc, red, grid_t);
+  }
 }
 
 void launch_enhanced_scaling(const OpView<double>& K, const OpView<double>& Kt, double* rs,
                              double* cs, double* rn, double* cn, int grid_k, int grid_t,
                              cudaStream_t s) {
-  const int n = Kt.rows;
-  const int m = K.rows;
-  const int g = vec_grid(n + m);
-  for (int pass = 0; pass < 10; ++pass) {
-    if (Kt.ts.ntiles > 0) {
-      abs_stat_kernel<true><<<grid_t, kBlock, tile_smem_bytes(Kt.ts, 1, 8), s>>>(Kt, cs, rs, cn);
+  const size_t sm = tile_smem_bytes(K.ts, 1, 8);
+  for (int pass = 0; pass < 11; ++pass) {
+    const ScalePair sc = pass % 2 == 1 ? ScalePair{cs, rs, cn, rn} : ScalePair{cn, rn, cs, rs};
+    if (pass < 10) {
+      abs_pass_kernel<true><<<grid_t + grid_k, kBlock, sm, s>>>(K, Kt, sc, grid_t);
+    } else {
+      abs_pass_kernel<false><<<grid_t + grid_k, kBlock, sm, s>>>(K, Kt, sc, grid_t);
     }
-    if (K.ts.ntiles > 0) {
-      abs_stat_kernel<true><<<grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(K, rs, cs, rn);
-    }
-    sqrt_rescale_kernel<<<g, kBlock, 0, s>>>(n, m, cs, cn, rs, rn);
   }
-  if (Kt.ts.ntiles > 0) {
-    abs_stat_kernel<false><<<grid_t, kBlock, tile_smem_bytes(Kt.ts, 1, 8), s>>>(Kt, cs, rs, cn);
-  }
-  if (K.ts.ntiles > 0) {
-    abs_stat_kernel<false><<<grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(K, rs, cs, rn);
-  }
-  sqrt_rescale_kernel<<<g, kBlock, 0, s>>>(n, m, cs, cn, rs, rn);
 }
 
 void launch_primal_weight_init(Ctl* ctl, int n, int m, const double* cost_eq,
@@ -1884,18 +1946,39 @@ void launch_primal_weight_init(Ctl* ctl, int n, int m, const double* cost_eq,
   primal_weight_init_kernel<<<g, kBlock, 0, s>>>(ctl, n, m, cost_eq, lower_eq, upper_eq, red);
 }
 
-void launch_apply_scaling(const OpView<double>& K, const OpView<double>& Kt, const double* rs,
+void launch_apply_scaling(const OpView<double>& K, const OpView<double>& Kt,
+                          const double* k_given, const double* t_given, const double* rs,
                           const double* cs, long long nnz, cudaStream_t s) {
   if (nnz == 0) return;
-  apply_scaling_kernel<<<vec_grid(nnz), kBlock, 0, s>>>(K, Kt, rs, cs, nnz);
+  apply_scaling_kernel<<<vec_grid(nnz / 4), kBlock, 0, s>>>(K, Kt, k_given, t_given, rs, cs,
+                                                            static_cast<int>(nnz));
 }
 
 void launch_scale_vectors(int n, int m, const double* cs, const double* rs, const double* cost,
-                          const double* lower, const double* upper, const double* rhs,
-                          double* cost_eq, double* lower_eq, double* upper_eq, double* rhs_eq,
+                          const double* lower, const double* upper, double* cost_eq,
+                          double* lower_eq, double* upper_eq, double* inv_cs, double* inv_rs,
                           cudaStream_t s) {
-  scale_vectors_kernel<<<vec_grid(n + m), kBlock, 0, s>>>(n, m, cs, rs, cost, lower, upper, rhs,
-                                                          cost_eq, lower_eq, upper_eq, rhs_eq);
+  scale_vectors_kernel<<<vec_grid(n + m), kBlock, 0, s>>>(n, m, cs, rs, cost, lower, upper,
+                                                          cost_eq, lower_eq, upper_eq, inv_cs,
+                                                          inv_rs);
+}
+
+// The start of a solve's setup: the control block, and both scale buffers at 1.
+__global__ void setup_begin_kernel(Ctl* ctl, Ctl value, int n, int m, double* cs, double* cn,
+                                   double* rs, double* rn) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ctl = value;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + m; k += gridDim.x * blockDim.x) {
+    if (k < n) {
+      cs[k] = cn[k] = 1.0;
+    } else {
+      rs[k - n] = rn[k - n] = 1.0;
+    }
+  }
+}
+
+void launch_setup_begin(Ctl* ctl, const Ctl& value, int n, int m, double* cs, double* cn,
+                        double* rs, double* rn, cudaStream_t s) {
+  setup_begin_kernel<<<vec_grid(n + m), kBlock, 0, s>>>(ctl, value, n, m, cs, cn, rs, rn);
 }
 
 void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt,
@@ -1905,7 +1988,6 @@ void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<doub
   if (m > 0) {
     const int gm = vec_grid(m) < 1024 ? vec_grid(m) : 1024;
     sum_sq_kernel<<<gm, kBlock, 0, s>>>(u, m, red, &ctl->power_unorm);
-    scale_by_norm_kernel<<<gm, kBlock, 0, s>>>(ctl, u, m, 1);
     for (int it = 0; it < iters; ++it) {
       if (Kt.ts.ntiles > 0) {
         power_spmv_kernel<<<grid_t, kBlock, tile_smem_bytes(Kt.ts, 1, 8), s>>>(ctl, Kt, u, v, red, 0);
@@ -1913,7 +1995,6 @@ void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<doub
       if (K.ts.ntiles > 0) {
         power_spmv_kernel<<<grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(ctl, K, v, u, red, 1);
       }
-      scale_by_norm_kernel<<<gm, kBlock, 0, s>>>(ctl, u, m, 0);
     }
   }
   power_finish_kernel<<<1, 32, 0, s>>>(ctl);

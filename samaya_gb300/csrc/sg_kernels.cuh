@@ -102,9 +102,10 @@ void launch_setup_norms(Ctl* ctl, const OpView<double>& K, const OpView<double>&
 void launch_reciprocals(const double* a, double* out, int count, cudaStream_t s);
 void launch_row_neighbours(int m, const int* ptr, const int* idx, unsigned char* out,
                            cudaStream_t s);
-void launch_ruiz_pass(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt, double* rs,
-                      double* cs, double* rn, double* cn, const RedView& red, int grid_k,
-                      int grid_t, cudaStream_t s);
+// The reference's Ruiz scaling, 10 passes; cn and rn the other buffers (all four at 1 before).
+void launch_ruiz(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt, double* rs,
+                 double* cs, double* rn, double* cn, const RedView& red, int grid_k, int grid_t,
+                 cudaStream_t s);
 // Enhanced preconditioning: 10 passes of infinity-norm Ruiz, then Pock-Chambolle (alpha = 1).
 void launch_enhanced_scaling(const OpView<double>& K, const OpView<double>& Kt, double* rs,
                              double* cs, double* rn, double* cn, int grid_k, int grid_t,
@@ -113,12 +114,16 @@ void launch_enhanced_scaling(const OpView<double>& K, const OpView<double>& Kt, 
 void launch_primal_weight_init(Ctl* ctl, int n, int m, const double* cost_eq,
                                const double* lower_eq, const double* upper_eq,
                                const RedView& red, cudaStream_t s);
-void launch_apply_scaling(const OpView<double>& K, const OpView<double>& Kt, const double* rs,
+// K.val and Kt.val from the given values.
+void launch_apply_scaling(const OpView<double>& K, const OpView<double>& Kt,
+                          const double* k_given, const double* t_given, const double* rs,
                           const double* cs, long long nnz, cudaStream_t s);
 void launch_scale_vectors(int n, int m, const double* cs, const double* rs, const double* cost,
-                          const double* lower, const double* upper, const double* rhs,
-                          double* cost_eq, double* lower_eq, double* upper_eq, double* rhs_eq,
+                          const double* lower, const double* upper, double* cost_eq,
+                          double* lower_eq, double* upper_eq, double* inv_cs, double* inv_rs,
                           cudaStream_t s);
+void launch_setup_begin(Ctl* ctl, const Ctl& value, int n, int m, double* cs, double* cn,
+                        double* rs, double* rn, cudaStream_t s);
 void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt,
                             double* u, double* v, const RedView& red, int iters, int grid_k,
                             int grid_t, cudaStream_t s);

@@ -125,6 +125,13 @@ __global__ void __launch_bounds__(kBlock) ir_cols_kernel(Ctl* c, OpView<double> 
 }
 
 // Scale factors of the correction problem and its starting primal weight.
+__global__ void ir_begin_kernel(Ctl* c32, const Ctl* __restrict__ c64) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  *c32 = *c64;
+  c32->ir_omega0 = c64->omega;
+  c32->q_norm = 0.0;
+}
+
 __global__ void ir_scales_kernel(Ctl* c, int round, double growth) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (round == 0) {
@@ -343,6 +350,10 @@ void launch_ir_residual(Ctl* c32, const OpView<double>& K, const OpView<double>&
                         const IrView& v, int grid_k, int grid_t, cudaStream_t s) {
   ir_rows_kernel<<<grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(c32, K, v);
   ir_cols_kernel<<<grid_t, kBlock, tile_smem_bytes(Kt.ts, 1, 8), s>>>(c32, Kt, v);
+}
+
+void launch_ir_begin(Ctl* c32, const Ctl* c64, cudaStream_t s) {
+  ir_begin_kernel<<<1, 32, 0, s>>>(c32, c64);
 }
 
 void launch_ir_scales(Ctl* c32, int round, double growth, cudaStream_t s) {

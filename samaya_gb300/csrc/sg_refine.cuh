@@ -29,6 +29,8 @@ struct IrView {
 void configure_refine_kernels();
 void launch_ir_residual(Ctl* c32, const OpView<double>& K, const OpView<double>& Kt,
                         const IrView& v, int grid_k, int grid_t, cudaStream_t s);
+// The FP32 control block from the FP64 one; its primal weight is the inner problems' first.
+void launch_ir_begin(Ctl* c32, const Ctl* c64, cudaStream_t s);
 void launch_ir_scales(Ctl* c32, int round, double growth, cudaStream_t s);
 void launch_ir_build(const Ctl* c32, const IrView& v, int round, cudaStream_t s);
 void launch_ir_update(const Ctl* c32, const IterView<float>& it, const IrView& v, int round,

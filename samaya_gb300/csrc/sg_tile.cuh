@@ -100,7 +100,10 @@ __device__ __forceinline__ double* smem_red() {
 
 template <bool MAXRED, typename ACC>
 __device__ __forceinline__ ACC combine(ACC a, ACC b) {
-  if constexpr (MAXRED) {
+  if constexpr (MAXRED && sizeof(ACC) == 8) {
+    // Magnitudes: their bits compare as integers (GB300's FP64 pipe is small).
+    return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+  } else if constexpr (MAXRED) {
     return a > b ? a : b;
   } else {
     return a + b;
@@ -312,13 +315,16 @@ __device__ __forceinline__ void group_tile(const TileSet& ts, const Tile& tile, 
 // Epi: void row(int r, const ACC (&s)[NV]) for rows of kind-0 tiles (lane 0 of the row's team),
 //      void long_row(int lrow, int r, const ACC (&s)[NV]) for a split row (thread 0 of the CTA
 //      that completes it).
-// MAXRED: each row's products are combined by max instead of + (norm statistics).
+// MAXRED: each row's products, none negative, are combined by max instead of + (norm statistics).
+// The CTA takes every step-th tile from `first` on (all CTAs of the grid share the tiles unless
+// a launch covers two operators).
 // WIDE: unroll the warp-per-row loop 8 deep (4 otherwise) and the segment loop 4 deep (2).
 template <typename T, typename ACC, int NV, typename Prod, typename Epi, bool MAXRED = false,
           bool WIDE = false, bool GROUPS = false>
 __device__ __forceinline__ void run_tiles(const TileSet& ts, const int* __restrict__ ptr,
                                           const int* __restrict__ idx,
-                                          const T* __restrict__ val, const Prod& prod, Epi& epi) {
+                                          const T* __restrict__ val, const Prod& prod, Epi& epi,
+                                          int first = blockIdx.x, int step = gridDim.x) {
   const int tid = threadIdx.x;
   __shared__ bool last_seg;
   double* red = smem_red();
@@ -338,7 +344,7 @@ __device__ __forceinline__ void run_tiles(const TileSet& ts, const int* __restri
       __syncthreads();
     }
   }
-  for (int ti = blockIdx.x; ti < ts.ntiles; ti += gridDim.x) {
+  for (int ti = first; ti < ts.ntiles; ti += step) {
     const Tile tile = ts.tiles[ti];
     if constexpr (GROUPS) {
       static_assert(NV == 1 && !MAXRED, "kind-3 tiles carry one plain sum per row");
