@@ -1161,15 +1161,16 @@ int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const Op
     launch_chunk(ctl, c, it, halpern, s);
     kernels = 1;
   }
+  const bool both = Ks.ts.ntiles > 0 && Kt.ts.ntiles > 0;
   for (int j = 0; j < kCheckFrequency && c.size == 0; ++j) {
     if (Ks.ts.ntiles > 0) ++kernels;
     if (Kt.ts.ntiles > 0) ++kernels;
     if (halpern) {
-      launch_halpern_primal(ctl, Kt, it, j, gst, s);
-      launch_halpern_dual(ctl, Ks, it, j, gsk, s);
+      launch_halpern_primal(ctl, Kt, it, j, gst, s, j > 0);
+      launch_halpern_dual(ctl, Ks, it, j, gsk, s, both);
     } else {
-      launch_dual_step(ctl, Ks, it, j, gsk, s);
-      launch_primal_step(ctl, Kt, it, j, gst, s);
+      launch_dual_step(ctl, Ks, it, j, gsk, s, j > 0);
+      launch_primal_step(ctl, Kt, it, j, gst, s, both);
     }
   }
   launch_eval(ctl, K, Kt, it, ev, red, gk, gt, -1, s, halpern);

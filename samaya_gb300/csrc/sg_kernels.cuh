@@ -63,19 +63,21 @@ struct RedView {
 
 constexpr int kEvalSums = 18;
 
+// behind: the launch before it on the stream is a step of the same chunk (it starts while that
+// one ends).
 template <typename T>
 void launch_dual_step(const Ctl* ctl, const OpView<T>& K, const IterView<T>& it, int j,
-                      int grid, cudaStream_t s);
+                      int grid, cudaStream_t s, bool behind = false);
 template <typename T>
 void launch_primal_step(const Ctl* ctl, const OpView<T>& Kt, const IterView<T>& it, int j,
-                        int grid, cudaStream_t s);
+                        int grid, cudaStream_t s, bool behind = false);
 // Reflected Halpern PDHG steps (primal launch first, then dual; see sg_kernels.cu).
 template <typename T>
 void launch_halpern_primal(const Ctl* ctl, const OpView<T>& Kt, const IterView<T>& it, int j,
-                           int grid, cudaStream_t s);
+                           int grid, cudaStream_t s, bool behind = false);
 template <typename T>
 void launch_halpern_dual(const Ctl* ctl, const OpView<T>& K, const IterView<T>& it, int j,
-                         int grid, cudaStream_t s);
+                         int grid, cudaStream_t s, bool behind = false);
 template <typename T>
 // second_only: measure the second slot (Verg, Yerg) alone; the first slot's sums are 0 (the
 // Halpern solves decide on T(z) only).
