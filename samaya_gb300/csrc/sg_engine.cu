@@ -218,6 +218,7 @@ Engine::~Engine() {
   dfree(long_terms_);
   dfree(arena_);
   if (ctl_host_) cudaFreeHost(ctl_host_);
+  if (seam_host_) cudaFreeHost(seam_host_);
   for (auto& e : ev_) {
     if (e) cudaEventDestroy(e);
   }
@@ -1714,15 +1715,8 @@ int Engine::seam_set_original(const double* cs, const double* rs, const double* 
 int Engine::seam_ctl_write(double tau, double sigma, long long t, long long k,
                            long long max_iter) {
   std::string* err = nullptr;
-  SG_TRY(cudaStreamSynchronize(stream_));
-  SG_TRY(cudaMemcpy(ctl_host_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost));
-  ctl_host_->tau = tau;
-  ctl_host_->sigma = sigma;
-  ctl_host_->t = t;
-  ctl_host_->k = k;
-  ctl_host_->done = 0;
-  ctl_host_->max_iter = max_iter;
-  SG_TRY(cudaMemcpy(ctl_, ctl_host_, sizeof(Ctl), cudaMemcpyHostToDevice));
+  launch_step_ctl(ctl_, tau, sigma, t, k, max_iter, stream_);
+  SG_TRY(cudaGetLastError());
   return kOk;
 }
 
@@ -1772,17 +1766,17 @@ int Engine::seam_halpern_step(double tau, double sigma, long long k) {
 
 namespace {
 
+// src as T; `h` is the staging of a conversion, which must outlive the copy.
 template <typename T>
-int upload_as(const double* src, T* dst, size_t count, cudaStream_t s) {
-  if (count == 0) return kOk;
-  std::vector<T> h(count);
-  for (size_t i = 0; i < count; ++i) h[i] = static_cast<T>(src[i]);
-  if (cudaMemcpyAsync(dst, h.data(), count * sizeof(T), cudaMemcpyHostToDevice, s) !=
-      cudaSuccess) {
-    return kErrCuda;
+cudaError_t upload_as(const double* src, T* dst, size_t count, std::vector<T>* h,
+                      cudaStream_t s) {
+  if (count == 0) return cudaSuccess;
+  const void* from = src;
+  if constexpr (!std::is_same<T, double>::value) {
+    h->assign(src, src + count);
+    from = h->data();
   }
-  // The staging vector must outlive the copy.
-  return cudaStreamSynchronize(s) == cudaSuccess ? kOk : kErrCuda;
+  return cudaMemcpyAsync(dst, from, count * sizeof(T), cudaMemcpyHostToDevice, s);
 }
 
 template <typename T>
@@ -1799,17 +1793,19 @@ int download_as(const T* src, double* dst, size_t count) {
 template <typename T>
 int set_iterate_state(DevIter<T>& it, int p, size_t nt, size_t m, const double* v,
                       const double* y, const double* v0, const double* y0, cudaStream_t s) {
-  int rc = kOk;
-  for (T* dst : {it.V[p], it.Vbar}) {
-    if (rc == kOk) rc = upload_as(v, dst, nt, s);
+  std::vector<T> h[4];
+  cudaError_t e = upload_as(v, it.V[p], nt, &h[0], s);
+  if (e == cudaSuccess) {
+    e = cudaMemcpyAsync(it.Vbar, it.V[p], nt * sizeof(T), cudaMemcpyDeviceToDevice, s);
   }
-  if (rc == kOk) rc = upload_as(v0, it.Vrst, nt, s);
-  if (rc == kOk) rc = upload_as(y, it.Y[p], m, s);
-  if (rc == kOk) rc = upload_as(y0, it.Yrst, m, s);
-  if (rc != kOk) return rc;
-  if (cudaMemsetAsync(it.Verg, 0, nt * sizeof(T), s) != cudaSuccess) return kErrCuda;
-  if (m > 0 && cudaMemsetAsync(it.Yerg, 0, m * sizeof(T), s) != cudaSuccess) return kErrCuda;
-  return kOk;
+  if (e == cudaSuccess) e = upload_as(v0, it.Vrst, nt, &h[1], s);
+  if (e == cudaSuccess) e = upload_as(y, it.Y[p], m, &h[2], s);
+  if (e == cudaSuccess) e = upload_as(y0, it.Yrst, m, &h[3], s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(it.Verg, 0, nt * sizeof(T), s);
+  if (e == cudaSuccess && m > 0) e = cudaMemsetAsync(it.Yerg, 0, m * sizeof(T), s);
+  // The staging and the caller's vectors are free again when this returns.
+  const cudaError_t done = cudaStreamSynchronize(s);
+  return e == cudaSuccess && done == cudaSuccess ? kOk : kErrCuda;
 }
 
 }  // namespace
@@ -1846,9 +1842,7 @@ int Engine::seam_set_state(int precision, const double* v, const double* y, cons
   } else {
     rc = set_iterate_state(it64_, p, nt, m, v, y, v0, y0, s);
   }
-  if (rc != kOk) return rc;
-  SG_TRY(cudaStreamSynchronize(s));
-  return kOk;
+  return rc;
 }
 
 int Engine::seam_advance() {
@@ -1871,8 +1865,8 @@ int Engine::seam_eval_launch() {
                 grid_k_, grid_t_, parity, stream_);
   }
   SG_TRY(cudaGetLastError());
+  SG_TRY(cudaMemcpyAsync(ctl_host_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_));
   SG_TRY(cudaStreamSynchronize(stream_));
-  SG_TRY(cudaMemcpy(ctl_host_, ctl_, sizeof(Ctl), cudaMemcpyDeviceToHost));
   return kOk;
 }
 
@@ -1925,8 +1919,35 @@ int Engine::seam_download(double* v, double* v_new, double* y, double* y_new, do
   const size_t nt = static_cast<size_t>(n_) + m_;
   const size_t m = static_cast<size_t>(m_);
   const int p = static_cast<int>(seam_steps_ & 1);
-  SG_TRY(cudaStreamSynchronize(stream_));
   int rc = kOk;
+  // Small FP64 iterates come over in one copy each into pinned memory and one wait (a copy into
+  // pageable memory waits for itself).
+  const size_t total = 3 * (nt + m);
+  constexpr size_t kPinned = 32768;
+  if (!seam_fp32_ && total <= kPinned) {
+    if (seam_host_ == nullptr) {
+      SG_TRY(cudaHostAlloc(reinterpret_cast<void**>(&seam_host_), kPinned * sizeof(double),
+                           cudaHostAllocDefault));
+    }
+    const std::tuple<const double*, double*, size_t> parts[6] = {
+        {it64_.V[p], v, nt},         {it64_.V[p ^ 1], v_new, nt}, {it64_.Y[p], y, m},
+        {it64_.Y[p ^ 1], y_new, m},  {it64_.Verg, v_erg, nt},     {it64_.Yerg, y_erg, m}};
+    double* at = seam_host_;
+    for (const auto& [src, dst, count] : parts) {
+      if (dst != nullptr && count > 0) {
+        SG_TRY(cudaMemcpyAsync(at, src, count * sizeof(double), cudaMemcpyDeviceToHost, stream_));
+      }
+      at += count;
+    }
+    SG_TRY(cudaStreamSynchronize(stream_));
+    at = seam_host_;
+    for (const auto& [src, dst, count] : parts) {
+      if (dst != nullptr && count > 0) memcpy(dst, at, count * sizeof(double));
+      at += count;
+    }
+    return kOk;
+  }
+  SG_TRY(cudaStreamSynchronize(stream_));
   auto get = [&](auto& it) {
     if (rc == kOk) rc = download_as(it.V[p], v, nt);
     if (rc == kOk) rc = download_as(it.V[p ^ 1], v_new, nt);

@@ -369,6 +369,7 @@ class Engine {
   char* arena_ = nullptr;
   size_t arena_bytes_ = 0;
   Ctl* ctl_host_ = nullptr;       // pinned
+  double* seam_host_ = nullptr;   // pinned, made by the first seam_download of a small LP
   cudaStream_t stream_ = nullptr;
   cudaGraphExec_t chunk_exec_ = nullptr;
   cudaGraph_t chunk_graph_ = nullptr;

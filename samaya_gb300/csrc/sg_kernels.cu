@@ -2033,6 +2033,22 @@ void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<doub
 
 void launch_init_state(Ctl* ctl, cudaStream_t s) { init_state_kernel<<<1, 32, 0, s>>>(ctl); }
 
+__global__ void step_ctl_kernel(Ctl* c, double tau, double sigma, long long t, long long k,
+                                long long max_iter) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  c->tau = tau;
+  c->sigma = sigma;
+  c->t = t;
+  c->k = k;
+  c->done = 0;
+  c->max_iter = max_iter;
+}
+
+void launch_step_ctl(Ctl* ctl, double tau, double sigma, long long t, long long k,
+                     long long max_iter, cudaStream_t s) {
+  step_ctl_kernel<<<1, 32, 0, s>>>(ctl, tau, sigma, t, k, max_iter);
+}
+
 void launch_set_deadline(Ctl* ctl, double seconds, cudaStream_t s) {
   const double ns = seconds * 1e9;
   const unsigned long long budget = ns > 1.8e19 ? 18000000000000000000ull

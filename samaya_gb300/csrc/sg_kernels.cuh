@@ -130,6 +130,9 @@ void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<doub
                             double* u, double* v, const RedView& red, int iters, int grid_k,
                             int grid_t, cudaStream_t s);
 void launch_init_state(Ctl* ctl, cudaStream_t s);
+// The control block of a single step (the inner seam).
+void launch_step_ctl(Ctl* ctl, double tau, double sigma, long long t, long long k,
+                     long long max_iter, cudaStream_t s);
 void launch_set_deadline(Ctl* ctl, double seconds, cudaStream_t s);
 
 template <typename Src, typename Dst>
