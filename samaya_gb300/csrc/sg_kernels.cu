@@ -171,12 +171,27 @@ struct PrimalEpi {
     p.xerg = static_cast<ACC>(xerg[j]);
     return p;
   }
-  __device__ __forceinline__ void row(int j, const ACC (&s)[1], const Pre& p) {
-    ACC xn = p.x - tau * (p.c + s[0]);
+  // The column's new values, written to x_new, xbar and xerg.
+  static constexpr int kIn = 3, kOut = 3;
+  __device__ __forceinline__ void update(const Pre& p, ACC s, ACC (&o)[kOut]) const {
+    ACC xn = p.x - tau * (p.c + s);
     xn = clampv<ACC>(xn, p.l, p.u);
-    x_new[j] = static_cast<T>(xn);
-    xbar[j] = static_cast<T>(extrapolate<ACC>(xn, p.x));
-    xerg[j] = static_cast<T>(beta * p.xerg + alpha * xn);
+    o[0] = xn;
+    o[1] = extrapolate<ACC>(xn, p.x);
+    o[2] = beta * p.xerg + alpha * xn;
+  }
+  __device__ __forceinline__ void row(int j, const ACC (&s)[1], const Pre& p) {
+    ACC o[kOut];
+    update(p, s[0], o);
+    x_new[j] = static_cast<T>(o[0]);
+    xbar[j] = static_cast<T>(o[1]);
+    xerg[j] = static_cast<T>(o[2]);
+  }
+  // The vectors that Pre reads beside the bounds, and those that update fills.
+  __device__ __forceinline__ const T* in(int k) const { return k == 0 ? x : k == 1 ? c : xerg; }
+  __device__ __forceinline__ T* out(int k) const { return k == 0 ? x_new : k == 1 ? xbar : xerg; }
+  __device__ __forceinline__ static Pre pre(const ACC (&v)[kIn], ACC l, ACC u) {
+    return Pre{v[0], v[1], l, u, v[2]};
   }
   __device__ __forceinline__ void row(int j, const ACC (&s)[1]) { row(j, s, load(j)); }
   __device__ __forceinline__ void long_row(int, int j, const ACC (&s)[1]) { row(j, s); }
@@ -198,6 +213,78 @@ __device__ __forceinline__ void let_next_start() {
 }
 __device__ __forceinline__ void wait_for_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A primal step over an operator of exactly two nonzeros a column (the columns of a transportation
+// or network-flow LP): a thread takes kWide<T> consecutive columns, 16 bytes of every vector, so
+// that all its loads are 16 bytes wide and on their way together. Bound by memory (68 bytes a
+// column in FP32, shared bounds not counted). A column a thread and 256 after another (run_tiles)
+// had half the bytes in flight and twice the instructions.
+template <typename T>
+constexpr int kWide = 16 / static_cast<int>(sizeof(T));
+
+template <typename T>
+__device__ __forceinline__ void load_wide(const T* p, T (&v)[kWide<T>]) {
+  *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+}
+template <typename T>
+__device__ __forceinline__ void store_wide(T* p, const T (&v)[kWide<T>]) {
+  *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(v);
+}
+
+template <typename T, typename Epi>
+__device__ __forceinline__ void two_nonzero_columns(const OpView<T>& Kt, const T* y, Epi& epi) {
+  using ACC = Acc<T>;
+  constexpr int W = kWide<T>;
+  const int n = Kt.rows;
+  const int j0 = (blockIdx.x * kBlock + threadIdx.x) * W;
+  if (j0 + W > n) {
+    for (int j = j0; j < n; ++j) {
+      ACC s[1] = {ACC(0)};
+      for (int q = 2 * j; q < 2 * j + 2; ++q) s[0] += ldg(Kt.val + q) * y[ldg(Kt.idx + q)];
+      epi.row(j, s);
+    }
+    return;
+  }
+  alignas(16) int idx[2 * W];
+  alignas(16) T val[2][W];
+  alignas(16) T in[Epi::kIn][W];
+  alignas(16) T lo[W], up[W];
+#pragma unroll
+  for (int k = 0; k < W / 2; ++k) {
+    *reinterpret_cast<int4*>(idx + 4 * k) =
+        __ldg(reinterpret_cast<const int4*>(Kt.idx + 2 * static_cast<size_t>(j0)) + k);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    *reinterpret_cast<float4*>(val[k]) =
+        __ldg(reinterpret_cast<const float4*>(Kt.val + 2 * static_cast<size_t>(j0)) + k);
+  }
+#pragma unroll
+  for (int k = 0; k < Epi::kIn; ++k) load_wide(epi.in(k) + j0, in[k]);
+  if (!epi.b.uniform) {
+    load_wide(epi.b.l + j0, lo);
+    load_wide(epi.b.u + j0, up);
+  }
+  alignas(16) T out[Epi::kOut][W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    ACC s = ACC(0);
+#pragma unroll
+    for (int q = 2 * w; q < 2 * w + 2; ++q) s += val[q / W][q % W] * y[idx[q]];
+    ACC v[Epi::kIn], o[Epi::kOut];
+#pragma unroll
+    for (int k = 0; k < Epi::kIn; ++k) v[k] = in[k][w];
+    epi.update(Epi::pre(v, epi.b.uniform ? epi.b.lo : lo[w], epi.b.uniform ? epi.b.hi : up[w]), s,
+               o);
+#pragma unroll
+    for (int k = 0; k < Epi::kOut; ++k) out[k][w] = static_cast<T>(o[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < Epi::kOut; ++k) {
+    T* p = epi.out(k);
+    if (p != nullptr) store_wide(p + j0, out[k]);
+  }
 }
 
 // The scalars of one step launch. FP64 kernels compute them once per CTA (thread 0) and share
@@ -252,6 +339,7 @@ __device__ __forceinline__ StepScalars<ACC> step_scalars(const Ctl* __restrict__
 //   1: 128 registers, the warp-per-row and segment loops unrolled twice as deep (operators of
 //      long rows, whose few CTAs need more loads in flight each; at 3 CTAs per SM, 80
 //      registers, no faster on the transportation LP);
+//   3 (primal steps only): operators of two nonzeros a column (two_nonzero_columns);
 //   2 (dual steps only): variant 0 plus the kind-3 row groups and the staged kind-1 segments
 //      of a tile set that has them.
 // (Measured and not kept: a third variant loading a short row's first three pairs of
@@ -260,6 +348,7 @@ template <typename T>
 constexpr int step_min_blocks(int variant, bool dual) {
   if (variant == 1) return 2;
   if (variant == 2) return sizeof(T) == 8 ? 3 : 4;
+  if (variant == 3) return 4;
   if (sizeof(T) == 8) return dual ? 4 : 5;
   return dual ? 5 : 6;
 }
@@ -320,9 +409,13 @@ __global__ void __launch_bounds__(kBlock, step_min_blocks<T>(VAR, false)) primal
   epi.beta = sc.beta;
   wait_for_previous();
   if (idle) return;
-  Gather1<T, ACC> g{it.y(p ^ 1)};
-  run_tiles<T, ACC, 1, Gather1<T, ACC>, PrimalEpi<T, ACC>, false, VAR == 1>(
-      Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+  if constexpr (VAR == 3) {
+    two_nonzero_columns<T>(Kt, it.y(p ^ 1), epi);
+  } else {
+    Gather1<T, ACC> g{it.y(p ^ 1)};
+    run_tiles<T, ACC, 1, Gather1<T, ACC>, PrimalEpi<T, ACC>, false, VAR == 1>(
+        Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -376,12 +469,28 @@ struct HalpernPrimalEpi {
     p.x0 = static_cast<ACC>(x0[j]);
     return p;
   }
-  __device__ __forceinline__ void row(int j, const ACC (&s)[1], const Pre& p) {
-    const ACC xh = clampv<ACC>(p.x - tau * (p.c + s[0]), p.l, p.u);
+  // The column's new values, written to x_new, xbar and (when `hat`) xhat.
+  static constexpr int kIn = 3, kOut = 3;
+  __device__ __forceinline__ void update(const Pre& p, ACC s, ACC (&o)[kOut]) const {
+    const ACC xh = clampv<ACC>(p.x - tau * (p.c + s), p.l, p.u);
     const ACC refl = extrapolate<ACC>(xh, p.x);
-    if (hat) xhat[j] = static_cast<T>(xh);
-    xbar[j] = static_cast<T>(refl);
-    x_new[j] = static_cast<T>(halpern_mix<ACC>(refl, p.x0, w));
+    o[0] = halpern_mix<ACC>(refl, p.x0, w);
+    o[1] = refl;
+    o[2] = xh;
+  }
+  __device__ __forceinline__ void row(int j, const ACC (&s)[1], const Pre& p) {
+    ACC o[kOut];
+    update(p, s[0], o);
+    if (hat) xhat[j] = static_cast<T>(o[2]);
+    xbar[j] = static_cast<T>(o[1]);
+    x_new[j] = static_cast<T>(o[0]);
+  }
+  __device__ __forceinline__ const T* in(int k) const { return k == 0 ? x : k == 1 ? c : x0; }
+  __device__ __forceinline__ T* out(int k) const {
+    return k == 0 ? x_new : k == 1 ? xbar : hat ? xhat : nullptr;
+  }
+  __device__ __forceinline__ static Pre pre(const ACC (&v)[kIn], ACC l, ACC u) {
+    return Pre{v[0], v[1], l, u, v[2]};
   }
   __device__ __forceinline__ void row(int j, const ACC (&s)[1]) { row(j, s, load(j)); }
   __device__ __forceinline__ void long_row(int, int j, const ACC (&s)[1]) { row(j, s); }
@@ -460,9 +569,13 @@ __global__ void __launch_bounds__(kBlock, step_min_blocks<T>(VAR, false)) halper
   epi.hat = halpern_writes_hat(ctl, t, j);
   wait_for_previous();
   if (idle) return;
-  Gather1<T, ACC> g{it.y(p)};
-  run_tiles<T, ACC, 1, Gather1<T, ACC>, HalpernPrimalEpi<T, ACC>, false, VAR == 1>(
-      Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+  if constexpr (VAR == 3) {
+    two_nonzero_columns<T>(Kt, it.y(p), epi);
+  } else {
+    Gather1<T, ACC> g{it.y(p)};
+    run_tiles<T, ACC, 1, Gather1<T, ACC>, HalpernPrimalEpi<T, ACC>, false, VAR == 1>(
+        Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+  }
 }
 
 template <typename T, int VAR>
@@ -1798,20 +1911,39 @@ void launch_dual_step(const Ctl* ctl, const OpView<T>& K, const IterView<T>& it,
                  ctl, K, it, j, grid, dual_smem_bytes<T>(K.ts), behind, s);
 }
 
+// The launch of a primal step: columns of two nonzeros, or tiles.
+template <typename T>
+int primal_variant(const TileSet& ts) {
+  return ts.uniform_len == 2 ? 3 : ts.variant == 1 ? 1 : 0;
+}
+template <typename T>
+int primal_grid(const OpView<T>& Kt, int grid) {
+  constexpr int kColumns = kBlock * kWide<T>;
+  return Kt.ts.uniform_len == 2 ? (Kt.rows + kColumns - 1) / kColumns : grid;
+}
+
 template <typename T>
 void launch_primal_step(const Ctl* ctl, const OpView<T>& Kt, const IterView<T>& it, int j,
                         int grid, cudaStream_t s, bool behind) {
   if (Kt.ts.ntiles == 0) return;
-  launch_step<T>(Kt.ts.variant == 1 ? primal_step_kernel<T, 1> : primal_step_kernel<T, 0>, ctl, Kt,
-                 it, j, grid, tile_smem_bytes(Kt.ts, 1, sizeof(T)), behind, s);
+  const int v = primal_variant<T>(Kt.ts);
+  launch_step<T>(v == 3   ? primal_step_kernel<T, 3>
+                 : v == 1 ? primal_step_kernel<T, 1>
+                          : primal_step_kernel<T, 0>,
+                 ctl, Kt, it, j, primal_grid(Kt, grid), tile_smem_bytes(Kt.ts, 1, sizeof(T)),
+                 behind, s);
 }
 
 template <typename T>
 void launch_halpern_primal(const Ctl* ctl, const OpView<T>& Kt, const IterView<T>& it, int j,
                            int grid, cudaStream_t s, bool behind) {
   if (Kt.ts.ntiles == 0) return;
-  launch_step<T>(Kt.ts.variant == 1 ? halpern_primal_kernel<T, 1> : halpern_primal_kernel<T, 0>,
-                 ctl, Kt, it, j, grid, tile_smem_bytes(Kt.ts, 1, sizeof(T)), behind, s);
+  const int v = primal_variant<T>(Kt.ts);
+  launch_step<T>(v == 3   ? halpern_primal_kernel<T, 3>
+                 : v == 1 ? halpern_primal_kernel<T, 1>
+                          : halpern_primal_kernel<T, 0>,
+                 ctl, Kt, it, j, primal_grid(Kt, grid), tile_smem_bytes(Kt.ts, 1, sizeof(T)),
+                 behind, s);
 }
 
 template <typename T>
