@@ -65,6 +65,12 @@ struct TileSet {
   int* wait_error;  // set to 1 when a bounded wait for a bulk copy gave up (staged sets)
 };
 
+// Whether the infeasibility and unboundedness checks run at the evaluation after iteration t
+// (every eighth evaluation past 1,000 iterations, pdlp.cpp:715-1043).
+__host__ __device__ inline bool detection_due(long long t) {
+  return t - 1 > 1000 && (t / kCheckFrequency) % 8 == 0;
+}
+
 constexpr int kSegChunk = 2048;  // nonzeros per bulk-copied chunk of a staged segment
 constexpr int kSegPad = 4;       // padding elements after an operator's nonzeros
 

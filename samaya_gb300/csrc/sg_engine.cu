@@ -199,10 +199,10 @@ int device_info(int* major, int* minor, char* name, size_t len) {
 
 Engine::~Engine() {
   if (stream_) cudaStreamSynchronize(stream_);
-  if (chunk_exec_) cudaGraphExecDestroy(chunk_exec_);
-  if (chunk_graph_) cudaGraphDestroy(chunk_graph_);
-  if (chunk32_exec_) cudaGraphExecDestroy(chunk32_exec_);
-  if (chunk32_graph_) cudaGraphDestroy(chunk32_graph_);
+  for (ChunkGraph* g : {&chunk_[0], &chunk_[1], &chunk32_}) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    if (g->graph) cudaGraphDestroy(g->graph);
+  }
   // The buffers sized by the problem live in the arena; the tile sets and the rest are their
   // own allocations.
   for (DevOp* op : {&K_, &Kt_}) {
@@ -1155,7 +1155,7 @@ template <typename T>
 int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const OpView<T>& K,
                   const OpView<T>& Kt,
                   const IterView<T>& it, const EvalView& ev, const RedView& red,
-                  double* scratch_n, int gsk, int gst, int gk, int gt, bool halpern,
+                  double* scratch_n, int gsk, int gst, int gk, int gt, bool halpern, bool detect,
                   cudaStream_t s) {
   int kernels = 0;
   if (c.size > 0) {
@@ -1175,46 +1175,48 @@ int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const Op
     }
   }
   launch_eval(ctl, K, Kt, it, ev, red, gk, gt, -1, s, halpern);
-  launch_decide_a(ctl, s);
-  launch_detect(ctl, K, Kt, it, ev, red, scratch_n, nullptr, gk, gt, s);
-  launch_decide_b(ctl, s);
+  if (detect) {
+    launch_decide_a(ctl, s);
+    launch_detect(ctl, K, Kt, it, ev, red, scratch_n, nullptr, gk, gt, s);
+    launch_decide_b(ctl, s);
+  } else {
+    launch_decide(ctl, s);
+  }
   launch_restart(ctl, it, s);
-  return kernels + 2 + 1 + 6 + 1 + 1;
+  return kernels + 2 + (detect ? 8 : 1) + 1;
 }
 
 }  // namespace
 
-void Engine::enqueue_chunk_body() {
-  chunk_kernels_ = enqueue_chunk(ctl_, chunk_view64(), K_.step64(), K_.view64(), Kt_.view64(),
-                                 iter_view(it64_), eval_view(), red_view(), scratch_n_,
-                                 grid_step_k_, grid_step_t_, grid_k_, grid_t_,
-                                 opt_.algorithm == 2, stream_);
-}
-
-int Engine::capture_chunk() {
-  if (chunk_exec_ != nullptr) return kOk;
+// One graph without the detection kernels (six launches, 15 us with nothing to do), one with
+// them, made when the first evaluation that runs them comes up.
+int Engine::capture_chunk(bool detect) {
+  ChunkGraph& g = chunk_[detect ? 1 : 0];
+  if (g.exec != nullptr) return kOk;
   std::string* err = nullptr;
   SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  enqueue_chunk_body();
-  SG_TRY(cudaStreamEndCapture(stream_, &chunk_graph_));
-  SG_TRY(cudaGraphInstantiate(&chunk_exec_, chunk_graph_, 0));
+  g.kernels = enqueue_chunk(ctl_, chunk_view64(), K_.step64(), K_.view64(), Kt_.view64(),
+                            iter_view(it64_), eval_view(), red_view(), scratch_n_, grid_step_k_,
+                            grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, detect, stream_);
+  SG_TRY(cudaStreamEndCapture(stream_, &g.graph));
+  SG_TRY(cudaGraphInstantiate(&g.exec, g.graph, 0));
   return kOk;
 }
 
 // The FP32 inner solves' chunk: FP32 operators and iterates, the correction problem's
 // right-hand side, evaluation in the equilibrated space (unit scales), its own control block.
 int Engine::capture_chunk32() {
-  if (chunk32_exec_ != nullptr) return kOk;
+  if (chunk32_.exec != nullptr) return kOk;
   std::string* err = nullptr;
   IterView<float> it = iter_view(it32_);
   it.rhs = it32_.rhs;
   SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  chunk32_kernels_ = enqueue_chunk(ctl32_, chunk_view32(), K_.step32(), K_.view32(), Kt_.view32(), it,
+  chunk32_.kernels = enqueue_chunk(ctl32_, chunk_view32(), K_.step32(), K_.view32(), Kt_.view32(), it,
                                    inner_eval_view(), red_view(), scratch_n_, grid_step_k_,
-                                   grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2,
+                                   grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, false,
                                    stream_);
-  SG_TRY(cudaStreamEndCapture(stream_, &chunk32_graph_));
-  SG_TRY(cudaGraphInstantiate(&chunk32_exec_, chunk32_graph_, 0));
+  SG_TRY(cudaStreamEndCapture(stream_, &chunk32_.graph));
+  SG_TRY(cudaGraphInstantiate(&chunk32_.exec, chunk32_.graph, 0));
   return kOk;
 }
 
@@ -1246,8 +1248,9 @@ IterView<double> Engine::master_view() {
 // at t0 and every chunk advances it by kCheckFrequency until max_iter, so no more chunks are
 // launched than reach it (a chunk after the end is 142 empty launches, 0.2 ms; three in flight
 // left two of them behind every solve).
-int Engine::run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, Ctl* ctl,
-                     int kernels_per_chunk, long long t0, long long max_iter) {
+int Engine::run_loop(double deadline_s, SolveInfo* info, bool fp32, long long t0,
+                     long long max_iter) {
+  Ctl* ctl = fp32 ? ctl32_ : ctl_;
   std::string* err = nullptr;
   constexpr int kInflight = 2;
   int head = 0;  // oldest in flight
@@ -1258,7 +1261,14 @@ int Engine::run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, C
   for (;;) {
     while (count < kInflight && launches < launch_cap) {
       const int slot = (head + count) % 4;
-      SG_TRY(cudaGraphLaunch(exec, stream_));
+      // The FP32 phases and the Halpern iteration run no detection.
+      const long long t = std::min(t0 + (launches + 1) * kCheckFrequency, max_iter);
+      const bool detect = !fp32 && opt_.algorithm != 2 && m_ > 0 && detection_due(t);
+      const int rc = fp32 ? capture_chunk32() : capture_chunk(detect);
+      if (rc != kOk) return rc;
+      const ChunkGraph& g = fp32 ? chunk32_ : chunk_[detect ? 1 : 0];
+      SG_TRY(cudaGraphLaunch(g.exec, stream_));
+      info->kernel_launches += g.kernels;
       SG_TRY(cudaMemcpyAsync(ctl_host_, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream_));
       SG_TRY(cudaEventRecord(ev_[slot], stream_));
       ++count;
@@ -1286,7 +1296,6 @@ int Engine::run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, C
   SG_TRY(cudaStreamSynchronize(stream_));
   SG_TRY(cudaMemcpy(ctl_host_, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
   info->graph_launches += launches;
-  info->kernel_launches += launches * kernels_per_chunk;
   return kOk;
 }
 
@@ -1335,14 +1344,14 @@ int Engine::solve_fp64(SolveInfo* info, double* x, double* y, double* dual_ray,
   const double t0 = now_s();
   int rc = setup_device(nullptr);
   if (rc != kOk) return rc;
-  rc = capture_chunk();
+  rc = capture_chunk(false);
   if (rc != kOk) return rc;
   // Deadline on the device clock (%globaltimer), checked by the decision kernel.
   if (opt_.time_limit > 0) launch_set_deadline(ctl_, opt_.time_limit - (now_s() - t0), stream_);
   const double deadline = opt_.time_limit > 0 ? t0 + opt_.time_limit : 0.0;
   const double t_setup = now_s();
   info->setup_seconds = t_setup - t0;
-  rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, 0, max_iterations());
+  rc = run_loop(deadline, info, false, 0, max_iterations());
   if (rc != kOk) return rc;
   return finish_fp64(info, t0, 0, x, y, dual_ray, primal_ray);
 }
@@ -1492,7 +1501,7 @@ int Engine::solve_switched(SolveInfo* info, double* x, double* y, double* dual_r
   cudaStream_t s = stream_;
   int rc = prepare_fp32();
   if (rc != kOk) return rc;
-  rc = capture_chunk();
+  rc = capture_chunk(false);
   if (rc != kOk) return rc;
   const size_t nt = static_cast<size_t>(n_) + m_;
   // FP32 phase: the correction problem of round 0 is the equilibrated problem itself.
@@ -1507,7 +1516,7 @@ int Engine::solve_switched(SolveInfo* info, double* x, double* y, double* dual_r
   if (opt_.time_limit > 0) launch_set_deadline(ctl32_, opt_.time_limit - (now_s() - t0), s);
   const double deadline = opt_.time_limit > 0 ? t0 + opt_.time_limit : 0.0;
   info->setup_seconds = now_s() - t0;
-  rc = run_loop(deadline, info, chunk32_exec_, ctl32_, chunk32_kernels_, 0, max_iter);
+  rc = run_loop(deadline, info, true, 0, max_iter);
   if (rc != kOk) return rc;
   const long long fp32_restarts = ctl_host_->restarts;
   const long long fp32_evals = ctl_host_->evaluations;
@@ -1515,7 +1524,7 @@ int Engine::solve_switched(SolveInfo* info, double* x, double* y, double* dual_r
   IterView<float> it32 = iter_view(it32_);
   launch_continue(ctl_, ctl32_, it32, iter_view(it64_), s);
   if (opt_.time_limit > 0) launch_set_deadline(ctl_, opt_.time_limit - (now_s() - t0), s);
-  rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, ctl_host_->t, max_iter);
+  rc = run_loop(deadline, info, false, ctl_host_->t, max_iter);
   if (rc != kOk) return rc;
   rc = finish_fp64(info, t0, 0, x, y, dual_ray, primal_ray);
   info->restarts += fp32_restarts;
@@ -1578,7 +1587,7 @@ int Engine::solve_refined(SolveInfo* info, double* x, double* y, double* dual_ra
     launch_norm_into(rhs_in_, m_, red_view(), &ctl32_->q_norm, s);
     launch_ir_reset(ctl32_, opt_.inner_tol, budget, kStallEvaluations, s);
     if (opt_.time_limit > 0) launch_set_deadline(ctl32_, opt_.time_limit - (now_s() - t0), s);
-    rc = run_loop(deadline, info, chunk32_exec_, ctl32_, chunk32_kernels_, 0, budget);
+    rc = run_loop(deadline, info, true, 0, budget);
     if (rc != kOk) return rc;
     total_iters += ctl_host_->t;
     if (round == 0) {
@@ -1621,12 +1630,12 @@ int Engine::solve_refined(SolveInfo* info, double* x, double* y, double* dual_ra
   if (status == kIterationLimit && total_iters < inner_max) {
     // The refinement did not reach the tolerance: the FP64 PDLP continues from the refined
     // point (restarted there, with the first round's primal weight).
-    rc = capture_chunk();
+    rc = capture_chunk(false);
     if (rc != kOk) return rc;
     const long long left = inner_max - total_iters;
     launch_restart_at_point(ctl_, round0_omega, iter_view(it64_), left, s);
     if (opt_.time_limit > 0) launch_set_deadline(ctl_, opt_.time_limit - (now_s() - t0), s);
-    rc = run_loop(deadline, info, chunk_exec_, ctl_, chunk_kernels_, 0, left);
+    rc = run_loop(deadline, info, false, 0, left);
     if (rc != kOk) return rc;
     const long long restarts = info->restarts, evaluations = info->evaluations;
     rc = finish_fp64(info, t0, total_iters, x, y, dual_ray, primal_ray);

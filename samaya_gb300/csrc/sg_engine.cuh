@@ -280,13 +280,12 @@ class Engine {
   Engine() = default;
   int alloc_all(std::string* err);
   int setup_device(const double* rhs_orig);
-  int capture_chunk();
+  int capture_chunk(bool detect);
   template <typename T>
   IterView<T> iter_view(DevIter<T>& it);
   EvalView eval_view() const;
   RedView red_view() const;
-  int run_loop(double deadline_s, SolveInfo* info, cudaGraphExec_t exec, Ctl* ctl,
-               int kernels_per_chunk, long long t0, long long max_iter);
+  int run_loop(double deadline_s, SolveInfo* info, bool fp32, long long t0, long long max_iter);
   int capture_chunk32();
   long long max_iterations() const;
   IterView<double> master_view();
@@ -298,7 +297,6 @@ class Engine {
   IrView ir_view();
   int finish_fp64(SolveInfo* info, double t0, long long iterations_before, double* x, double* y,
                   double* dual_ray, double* primal_ray);
-  void enqueue_chunk_body();
   // The cluster form of the chunk's iterations: whether and on how many CTAs (0: step launches),
   // its arrays and views.
   void plan_chunk();
@@ -371,9 +369,12 @@ class Engine {
   Ctl* ctl_host_ = nullptr;       // pinned
   double* seam_host_ = nullptr;   // pinned, made by the first seam_download of a small LP
   cudaStream_t stream_ = nullptr;
-  cudaGraphExec_t chunk_exec_ = nullptr;
-  cudaGraph_t chunk_graph_ = nullptr;
-  int chunk_kernels_ = 0;
+  struct ChunkGraph {
+    cudaGraphExec_t exec = nullptr;
+    cudaGraph_t graph = nullptr;
+    int kernels = 0;
+  };
+  ChunkGraph chunk_[2];  // without and with the detection kernels
   long long seam_steps_ = 0;
   bool seam_mode_ = false;
   bool seam_fp32_ = false;   // the seam's steps, evaluation and download use the FP32 set
@@ -383,9 +384,7 @@ class Engine {
   // Mixed-precision path: the inner solves' control block and graph, the correction problem
   // (FP64 evaluation copy), unit scales for its evaluation, and the residual vectors.
   Ctl* ctl32_ = nullptr;
-  cudaGraphExec_t chunk32_exec_ = nullptr;
-  cudaGraph_t chunk32_graph_ = nullptr;
-  int chunk32_kernels_ = 0;
+  ChunkGraph chunk32_;
   double* ones_n_ = nullptr;
   double* ones_m_ = nullptr;
   double* cost_in_ = nullptr;

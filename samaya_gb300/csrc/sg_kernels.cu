@@ -217,9 +217,9 @@ __device__ __forceinline__ void wait_for_previous() {
 
 // A primal step over an operator of exactly two nonzeros a column (the columns of a transportation
 // or network-flow LP): a thread takes kWide<T> consecutive columns, 16 bytes of every vector, so
-// that all its loads are 16 bytes wide and on their way together. Bound by memory (68 bytes a
-// column in FP32, shared bounds not counted). A column a thread and 256 after another (run_tiles)
-// had half the bytes in flight and twice the instructions.
+// that all its loads are 16 bytes wide and on their way together. Bound by memory (36 bytes a
+// column in FP32, shared bounds not counted; 2 million columns 14.5 us by run_tiles, a column a
+// thread and 256 after another, 10.3 so).
 template <typename T>
 constexpr int kWide = 16 / static_cast<int>(sizeof(T));
 
@@ -1007,30 +1007,12 @@ __device__ void set_answer(Ctl* c, int status, const Meas& e, long long iteratio
   c->done = 1;
 }
 
-// Termination test after the evaluation; schedules the detection checks.
-__global__ void decide_a_kernel(Ctl* c) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  c->restart_pending = 0;
-  c->detect_pending = 0;
-  if (c->done) return;
+// Termination test after the evaluation (cur, avg: its measures); schedules the detection checks.
+__device__ __forceinline__ void decide_termination(Ctl* c, const Meas& cur, const Meas& avg) {
   long long steps = c->max_iter - c->t;
   if (steps > kCheckFrequency) steps = kCheckFrequency;
   const long long t_new = c->t + steps;
-  const long long iter = t_new - 1;
-  double s_cur[7], s_avg[7];
-  for (int q = 0; q < 7; ++q) {
-    s_cur[q] = c->eval_c[q] + c->eval_r[q];
-    s_avg[q] = c->eval_c[7 + q] + c->eval_r[7 + q];
-  }
-  const Meas cur = finish_sums(c, s_cur);
-  const Meas avg = finish_sums(c, s_avg);
   c->evaluations += 1;
-  const double wc[5] = {cur.rp, cur.rd, cur.rg, cur.pobj, cur.dobj};
-  const double wa[5] = {avg.rp, avg.rd, avg.rg, avg.pobj, avg.dobj};
-  for (int q = 0; q < 5; ++q) {
-    c->meas[0][q] = wc[q];
-    c->meas[1][q] = wa[q];
-  }
   if (!c->halpern && converged(cur, c->tol)) {
     set_answer(c, kOptimal, cur, t_new, 0);
     c->t = t_new;
@@ -1055,23 +1037,18 @@ __global__ void decide_a_kernel(Ctl* c) {
       return;
     }
   }
-  c->detect_pending =
-      (!c->no_detect && iter > 1000 && c->m > 0 && ((iter + 1) / kCheckFrequency) % 8 == 0) ? 1
-                                                                                              : 0;
+  c->detect_pending = !c->no_detect && detection_due(t_new) && c->m > 0 ? 1 : 0;
   for (int q = 0; q < 8; ++q) c->det_flags[q] = 0;
 }
 
 // Detection verdict, then PDLP's adaptive restart and primal-weight update; advances the
 // iteration counters and applies the iteration and time limits.
-__global__ void decide_b_kernel(Ctl* c) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (c->done) return;
+__device__ __forceinline__ void decide_restart(Ctl* c, const Meas& cur, const Meas& avg,
+                                               double kkt_cur, double kkt_avg) {
   long long steps = c->max_iter - c->t;
   if (steps > kCheckFrequency) steps = kCheckFrequency;
   const long long t_new = c->t + steps;
   const long long iter = t_new - 1;
-  Meas cur{c->meas[0][0], c->meas[0][1], c->meas[0][2], c->meas[0][3], c->meas[0][4]};
-  Meas avg{c->meas[1][0], c->meas[1][1], c->meas[1][2], c->meas[1][3], c->meas[1][4]};
   if (c->detect_pending) {
     if (c->det_flags[0]) {
       set_answer(c, kInfeasible, cur, t_new, 0);
@@ -1086,8 +1063,6 @@ __global__ void decide_b_kernel(Ctl* c) {
   }
   const long long k_new = c->k + steps;
   const double omega = c->omega;
-  const double kkt_cur = kkt_weighted(omega, cur);
-  const double kkt_avg = kkt_weighted(omega, avg);
   const bool to_average = c->halpern || kkt_avg < kkt_cur;
   const double cand = to_average ? kkt_avg : kkt_cur;
   if (!(c->kkt_at_restart < INFINITY)) c->kkt_at_restart = cand;
@@ -1124,6 +1099,54 @@ __global__ void decide_b_kernel(Ctl* c) {
   if (c->deadline_ns != 0ull && globaltimer_ns() > c->deadline_ns) {
     set_answer(c, kTimeLimit, ans ? avg : cur, c->t, ans);
   }
+}
+
+// The decisions by one warp: the termination test (FIRST), the restart (LAST), or both when no
+// detection is due between them. Bound by latency: on the control block in device memory, every
+// read behind a write to it, the two kernels took 20 us (under a profiler's cold caches); here it
+// is copied to shared memory, and two lanes measure the two iterates side by side.
+template <bool FIRST, bool LAST>
+__global__ void decide_kernel(Ctl* ctl) {
+  __shared__ __align__(16) unsigned long long copy[(sizeof(Ctl) + 7) / 8];
+  static_assert(sizeof(Ctl) % 8 == 0, "copied by 8 bytes");
+  constexpr int kWords = sizeof(Ctl) / 8;
+  const int lane = threadIdx.x;
+  unsigned long long* from = reinterpret_cast<unsigned long long*>(ctl);
+  for (int k = lane; k < kWords; k += 32) copy[k] = from[k];
+  __syncwarp();
+  Ctl* c = reinterpret_cast<Ctl*>(copy);
+  if (FIRST) {
+    if (lane == 0) {
+      c->restart_pending = 0;
+      c->detect_pending = 0;
+    }
+    __syncwarp();
+  }
+  const bool done = c->done != 0;
+  if (!done && lane < 2) {
+    // Lane 0 the current iterate, lane 1 the average.
+    Meas e;
+    if (FIRST) {
+      double s[7];
+      for (int q = 0; q < 7; ++q) s[q] = c->eval_c[7 * lane + q] + c->eval_r[7 * lane + q];
+      e = finish_sums(c, s);
+      const double w[5] = {e.rp, e.rd, e.rg, e.pobj, e.dobj};
+      for (int q = 0; q < 5; ++q) c->meas[lane][q] = w[q];
+    } else {
+      e = Meas{c->meas[lane][0], c->meas[lane][1], c->meas[lane][2], c->meas[lane][3],
+               c->meas[lane][4]};
+    }
+    const double kkt = LAST ? kkt_weighted(c->omega, e) : 0.0;
+    const double kkt_avg = __shfl_sync(3u, kkt, 1);
+    __syncwarp(3u);
+    if (lane == 0) {
+      const Meas avg{c->meas[1][0], c->meas[1][1], c->meas[1][2], c->meas[1][3], c->meas[1][4]};
+      if (FIRST) decide_termination(c, e, avg);
+      if (LAST && !c->done) decide_restart(c, e, avg, kkt, kkt_avg);
+    }
+  }
+  __syncwarp();
+  for (int k = lane; k < kWords; k += 32) from[k] = copy[k];
 }
 
 // Restart at the candidate (pdhg_core.cu:362-380 + advance()): it becomes the current point
@@ -1983,8 +2006,9 @@ void launch_eval(Ctl* ctl, const OpView<T>& K, const OpView<T>& Kt, const IterVi
   }
 }
 
-void launch_decide_a(Ctl* ctl, cudaStream_t s) { decide_a_kernel<<<1, 32, 0, s>>>(ctl); }
-void launch_decide_b(Ctl* ctl, cudaStream_t s) { decide_b_kernel<<<1, 32, 0, s>>>(ctl); }
+void launch_decide(Ctl* ctl, cudaStream_t s) { decide_kernel<true, true><<<1, 32, 0, s>>>(ctl); }
+void launch_decide_a(Ctl* ctl, cudaStream_t s) { decide_kernel<true, false><<<1, 32, 0, s>>>(ctl); }
+void launch_decide_b(Ctl* ctl, cudaStream_t s) { decide_kernel<false, true><<<1, 32, 0, s>>>(ctl); }
 
 template <typename T>
 void launch_restart(const Ctl* ctl, const IterView<T>& it, cudaStream_t s) {

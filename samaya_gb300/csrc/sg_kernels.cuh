@@ -84,6 +84,8 @@ template <typename T>
 void launch_eval(Ctl* ctl, const OpView<T>& K, const OpView<T>& Kt, const IterView<T>& it,
                  const EvalView& ev, const RedView& red, int grid_k, int grid_t,
                  int fixed_parity, cudaStream_t s, bool second_only = false);
+// The decisions after an evaluation; a and b around launch_detect where detection is due.
+void launch_decide(Ctl* ctl, cudaStream_t s);
 void launch_decide_a(Ctl* ctl, cudaStream_t s);
 void launch_decide_b(Ctl* ctl, cudaStream_t s);
 template <typename T>
