@@ -58,12 +58,12 @@ struct Gather {
 };
 
 // A matrix's share of one CTA.
-template <typename T>
+template <typename T, typename Share = RowShare<T>>
 struct MatShare {
   int m, n;
   long long kz, tz;        // first element of A's and A''s arrays
   const int *kperm, *tperm;  // position -> row, column
-  RowShare<T> K, Kt;       // own rows of A and of A'
+  Share K, Kt;             // own rows of A and of A'
   int nr, nc;              // own rows and columns, whole slices
 };
 

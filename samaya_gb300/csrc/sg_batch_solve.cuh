@@ -246,8 +246,8 @@ __device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
       ctx->rest[threadIdx.x] = static_cast<T>(1.0 - 1.0 / (k + 1.0));
     }
     __syncthreads();
-    ok = run_steps<T, MODE, halpern>(ctx, static_cast<int>(steps), static_cast<T>(tau),
-                                     static_cast<T>(sigma), [] {});
+    ok = run_steps<halpern, T, MODE, RowShare<T>, SolveState<T, MODE>>(
+        ctx, static_cast<int>(steps), static_cast<T>(tau), static_cast<T>(sigma), [] {});
     t += steps;
     k_since += steps;
     ok = ok && ex.wait(halpern ? 1 : 0);

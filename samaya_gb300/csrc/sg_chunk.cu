@@ -2,10 +2,11 @@
 // one thread-block cluster.
 //
 // Launched step by step, an iteration of a small LP is two kernels of five dependent L2 round
-// trips each and two launches, 12-17 us whatever its size; here the iterates stay in the cluster's
-// shared memory, the nonzeros in its L1 caches, and a half step ends in an exchange: 5.4 us for a
-// random LP of 200 x 500 (FP64, bound by the exchanges and the loads' latency), 10.6 for one of
-// 5,000 x 10,000 (bound by the FP64 pipes of 16 SMs). Engine::plan_chunk says where it is taken.
+// trips each and two launches, 9-17 us whatever its size; here the iterates and the matrix stay in
+// the cluster's shared memory, and a half step ends in an exchange: 3.3 us for a random LP of 200 x
+// 500 (FP64, bound by latency: loads, chains of FP64 operations, exchanges), 7.1 for one of 3,500 x
+// 7,000 (bound by the FP64 pipes of 16 SMs). With the batched solves' walks, a row on a lane and
+// the nonzeros in L1, these took 4.4 and 7.9. Engine::plan_chunk says where this kernel is taken.
 #include "sg_chunk.cuh"
 #include "sg_cluster_steps.cuh"
 
@@ -13,7 +14,224 @@ namespace sg {
 
 namespace {
 
-constexpr int kChunkThreads = 512;
+// A CTA's share of an operator in tasks, its elements and tasks in shared memory.
+template <typename T>
+struct alignas(16) TaskShare {
+  using Value = T;
+  static constexpr bool kTasks = true;
+  int own;                            // rows
+  int first;                          // position of the first
+  unsigned rank, size;
+  unsigned val_at, idx_at, task_at;   // shared addresses
+  unsigned sums_at;
+  int tasks, pad;
+  int shared_rows, filled;            // the first rows take several lanes; the last have no nonzeros
+
+  __device__ __forceinline__ int4 task(int t) const {
+    int4 v;
+    asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(task_at + 16 * t)
+                 : "memory");
+    return v;
+  }
+
+  // f(at, init(at) + sum) for every own row. Where a row has a lane to itself, the lane runs f; the
+  // sums of rows on several lanes, a shuffle tree's, go to shared memory, and a thread per row runs
+  // f after them. (With a lane per row everywhere, as walk_one has it, an LP of 200 x 500 left 12
+  // of 16 warps idle, and one warp's 20 nonzeros took 3,500 of an iteration's 7,800 clocks.)
+  template <typename Prod, typename Init, typename F, typename Ready>
+  __device__ __forceinline__ bool walk(const Prod& prod, const Init& init, const F& f,
+                                       const Ready& ready) const {
+    // B steps' elements loaded while the B before are summed (of the same task or the warp's task
+    // before).
+    constexpr int B = sizeof(T) == 8 ? 4 : 8;
+    const int lane = threadIdx.x & 31;
+    T a[B];
+    unsigned j[B];
+    auto fetch = [&](const int4& d, int k) {
+      const unsigned val = val_at + (d.x + lane + 32 * k) * static_cast<int>(sizeof(T));
+      const unsigned idx = idx_at + (d.x + lane + 32 * k) * 2;
+      const int left = d.y - k;
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        if (u < left) {
+          a[u] = sh_load(val + 32 * u * static_cast<int>(sizeof(T)), T());
+          j[u] = sh_load_u16(idx + 64 * u);
+        }
+      }
+    };
+    int t = threadIdx.x >> 5;
+    int4 d = t < tasks ? task(t) : make_int4(0, 0, 0, 0);
+    fetch(d, 0);
+    if (!ready()) return false;
+    while (t < tasks) {
+      t += kChunkThreads / 32;
+      const int4 dn = t < tasks ? task(t) : make_int4(0, 0, 0, 0);
+      T s = T(0);
+      for (int k = 0;; k += B) {
+        T ca[B];
+        unsigned cj[B];
+        const bool more = k + B < d.y;
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+          ca[u] = a[u];
+          cj[u] = j[u];
+        }
+        fetch(more ? d : dn, more ? k + B : 0);
+        const int left = d.y - k;
+        if (left >= B) {
+          if constexpr (sizeof(T) == 8) keep_branch(0xffffffffu);
+#pragma unroll
+          for (int u = 0; u < B; ++u) s = s + prod(ca[u], static_cast<int>(cj[u]));
+        } else {
+#pragma unroll
+          for (int u = 0; u < B - 1; ++u) {
+            if (u < left) {
+              if constexpr (sizeof(T) == 8) keep_branch(0xffffffffu);
+              s = s + prod(ca[u], static_cast<int>(cj[u]));
+            }
+          }
+        }
+        if (!more) break;
+      }
+      const int lanes = d.w >> 8;
+      if (lanes == 0) {
+        if (lane < (d.w & 255)) {
+          const int l = d.z + lane;
+          const At at{l, 0, l, first + l};
+          f(at, init(at) + s);
+        }
+      } else {
+        for (int o = (1 << lanes) >> 1; o > 0; o >>= 1) {
+          s = s + __shfl_xor_sync(0xffffffffu, s, o);
+        }
+        const int r = lane >> lanes;
+        if ((lane & ((1 << lanes) - 1)) == 0 && r < (d.w & 255)) {
+          sh_store(sums_at + (d.z + r) * static_cast<int>(sizeof(T)), s);
+        }
+      }
+      d = dn;
+    }
+    const int rest = shared_rows + own - filled;
+    if (rest == 0) return true;
+    __syncthreads();
+    for (int k = threadIdx.x; k < rest; k += kChunkThreads) {
+      const bool sum = k < shared_rows;
+      const int l = sum ? k : k - shared_rows + filled;
+      const At at{l, 0, l, first + l};
+      T s = init(at);
+      if (sum) s = s + sh_load(sums_at + l * static_cast<int>(sizeof(T)), T());
+      f(at, s);
+    }
+    return true;
+  }
+};
+
+// f(at) for every own row.
+template <typename T, typename F>
+__device__ __forceinline__ void each_own(const TaskShare<T>& A, const F& f) {
+  for (int l = threadIdx.x; l < A.own; l += blockDim.x) f(At{l, 0, l, A.first + l});
+}
+
+// The state in shared memory, array after array (SolveState's, without slices).
+template <typename T>
+struct alignas(16) FlatState {
+  unsigned cols_at, rows_at;      // shared addresses
+  unsigned cols_bytes, rows_bytes;  // of an array
+  struct Entry {
+    unsigned a, array;
+    __device__ __forceinline__ T get(int k) const { return sh_load(a + k * array, T()); }
+    __device__ __forceinline__ void set(int k, T v) const { sh_store(a + k * array, v); }
+  };
+  struct Arrays {
+    unsigned base, array;
+    __device__ __forceinline__ Entry at(const At& p) const {
+      return Entry{base + p.l * static_cast<unsigned>(sizeof(T)), array};
+    }
+  };
+  __device__ __forceinline__ Entry col(const At& at) const {
+    return Arrays{cols_at, cols_bytes}.at(at);
+  }
+  __device__ __forceinline__ Entry row(const At& at) const {
+    return Arrays{rows_at, rows_bytes}.at(at);
+  }
+};
+template <typename T>
+__device__ __forceinline__ typename FlatState<T>::Arrays col_state(const FlatState<T>& S) {
+  return {S.cols_at, S.cols_bytes};
+}
+template <typename T>
+__device__ __forceinline__ typename FlatState<T>::Arrays row_state(const FlatState<T>& S) {
+  return {S.rows_at, S.rows_bytes};
+}
+
+template <typename T>
+__device__ __forceinline__ TaskShare<T> task_share(const ChunkOp<T>& op, int rows, unsigned rank,
+                                                   unsigned size, unsigned sums_at) {
+  const unsigned base = shared_addr(sg_smem);
+  TaskShare<T> s;
+  s.own = rows > static_cast<int>(rank)
+              ? (rows - static_cast<int>(rank) - 1) / static_cast<int>(size) + 1
+              : 0;
+  s.first = static_cast<int>(rank) * op.per;
+  s.rank = rank;
+  s.size = size;
+  s.val_at = base + op.val_at;
+  s.idx_at = base + op.idx_at;
+  s.task_at = base + op.task_at;
+  s.sums_at = base + sums_at;
+  s.tasks = op.task_off[rank + 1] - op.task_off[rank];
+  s.filled = op.filled[2 * rank];
+  s.shared_rows = op.filled[2 * rank + 1];
+  return s;
+}
+
+// The CTA's block of an operator to shared memory.
+template <typename T>
+__device__ __forceinline__ void load_block(const ChunkOp<T>& op, unsigned rank) {
+  T* val = reinterpret_cast<T*>(sg_smem + op.val_at);
+  unsigned short* idx = reinterpret_cast<unsigned short*>(sg_smem + op.idx_at);
+  int4* task = reinterpret_cast<int4*>(sg_smem + op.task_at);
+  const int e0 = op.elem_off[rank];
+  const int elems = op.elem_off[rank + 1] - e0;
+  for (int k = threadIdx.x; k < elems; k += kChunkThreads) {
+    val[k] = op.val[e0 + k];
+    idx[k] = op.idx[e0 + k];
+  }
+  const int t0 = op.task_off[rank];
+  const int tasks = op.task_off[rank + 1] - t0;
+  for (int k = threadIdx.x; k < tasks; k += kChunkThreads) task[k] = op.task[t0 + k];
+}
+
+// Masks of the own columns (which 0) or rows (1): the CTAs that own the other operator's rows of
+// their nonzeros (`per` positions each).
+template <typename T>
+__device__ __forceinline__ void task_masks(const TaskShare<T>& A, int per, unsigned short* mask,
+                                           ClusterShared& sh, int which) {
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < A.tasks; t += kChunkThreads / 32) {
+    const int4 d = A.task(t);
+    const int lanes = d.w >> 8;
+    unsigned m = 0;
+    for (int k = 0; k < d.y; ++k) {
+      const int j = static_cast<int>(sh_load_u16(A.idx_at + (d.x + lane + 32 * k) * 2));
+      const unsigned owner = static_cast<unsigned>(j / per);  // size: padding
+      if (owner < A.size) m |= 1u << (owner ^ A.rank);
+    }
+    for (int o = (1 << lanes) >> 1; o > 0; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+    const int r = lane >> lanes;
+    if ((lane & ((1 << lanes) - 1)) == 0 && r < (d.w & 255)) {
+      m &= ~1u;
+      mask[d.z + r] = static_cast<unsigned short>(m);
+      while (m != 0u) {
+        const unsigned q = __ffs(m) - 1;
+        m &= m - 1u;
+        atomicAdd(&sh.count[which][q], 1u);
+      }
+    }
+  }
+}
 
 template <typename T, bool HALPERN>
 __global__ void __launch_bounds__(kChunkThreads, 1)
@@ -21,7 +239,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   constexpr int MODE = kAllShared;
   constexpr bool kF64 = sizeof(T) == 8;
   __shared__ ClusterShared sh;
-  __shared__ StepContext<T, MODE> ctx;
+  __shared__ StepContext<T, MODE, TaskShare<T>, FlatState<T>> ctx;
   if (ctl->done) return;
   const long long t = ctl->t;
   const long long k0 = ctl->k;
@@ -32,26 +250,41 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   const unsigned size = cluster_size();
   cluster_init(sh, size);
   const int n = c.n;
-  MatShare<T> M;
+  load_block(c.K, rank);
+  load_block(c.Kt, rank);
+  MatShare<T, TaskShare<T>> M;
   M.m = c.m;
   M.n = n;
   M.kz = M.tz = 0;
   M.kperm = c.K.perm;
   M.tperm = c.Kt.perm;
-  M.K = RowShare<T>{c.K.sl, c.K.desc, c.K.idx, c.K.val, c.m, c.K.slice, rank, size};
-  M.Kt = RowShare<T>{c.Kt.sl, c.Kt.desc, c.Kt.idx, c.Kt.val, n, c.Kt.slice, rank, size};
-  M.nr = M.K.own();
-  M.nc = M.Kt.own();
-  const Second<T> Z{c.second, n, c.m};
-  const Exchange<T, MODE> ex = make_exchange<T, MODE>(M, sh, nullptr, rank, size);
-  SolveState<T, MODE> S;
-  S.device = nullptr;
-  S.rows_device = 0;
-  S.cols_at = static_cast<unsigned>(cluster_vector_bytes(n, c.m, c.Kt.slice, c.K.slice,
-                                                         static_cast<int>(size), sizeof(T)));
-  S.rows_at = S.cols_at + M.Kt.slices() * static_cast<unsigned>(32 * kColArrays * sizeof(T));
-  S.rank = rank;
-  S.size = size;
+  M.K = task_share(c.K, c.m, rank, size, c.sums_at);
+  M.Kt = task_share(c.Kt, n, rank, size, c.sums_at);
+  M.nr = M.K.own;
+  M.nc = M.Kt.own;
+  const Second<T> Z{c.second, c.np, c.mp};
+  Exchange<T, MODE> ex;
+  ex.sh = &sh;
+  ex.rank = rank;
+  ex.size = size;
+  ex.device = nullptr;
+  ex.xs_at = 0u;
+  ex.ys_at = (c.np + 1) * static_cast<unsigned>(sizeof(T));
+  ex.cmask_at = ex.ys_at + (c.mp + 1) * static_cast<unsigned>(sizeof(T));
+  ex.rmask_at = ex.cmask_at + M.nc * 2;
+  if (threadIdx.x == 0) ex.xs()[c.np] = ex.ys()[c.mp] = T(0);
+  for (int k = threadIdx.x; k < M.nc + M.nr; k += kChunkThreads) ex.cmask()[k] = 0;
+  if (threadIdx.x < 2 * kMaxCluster) (&sh.count[0][0])[threadIdx.x] = 0;
+  __syncthreads();
+  task_masks(M.Kt, c.K.per, ex.cmask(), sh, 0);
+  task_masks(M.K, c.Kt.per, ex.rmask(), sh, 1);
+  settle_counts(ex);
+  const unsigned base = shared_addr(sg_smem);
+  FlatState<T> S;
+  S.cols_at = base + c.cols_at;
+  S.rows_at = base + c.rows_at;
+  S.cols_bytes = M.nc * static_cast<unsigned>(sizeof(T));
+  S.rows_bytes = M.nr * static_cast<unsigned>(sizeof(T));
   if (threadIdx.x == 0) {
     ctx.M = M;
     ctx.ex = ex;
@@ -73,44 +306,44 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   auto sum_of = [&](T average) { return !kF64 ? average : k0 == 0 ? T(0) : average * count; };
   each_own(M.Kt, [&](const At& at) {
     const int j = M.tperm[at.p];
-    S.col(kPoint, at) = v[j];
-    S.col(kSum, at) = HALPERN ? it.Vrst[j] : sum_of(it.Verg[j]);
-    S.col(kCost, at) = it.cost[j];
-    S.col(kLower, at) = it.xb_uniform ? it.xb_lo : it.lower[j];
-    S.col(kUpper, at) = it.xb_uniform ? it.xb_hi : it.upper[j];
+    S.col(at).set(kPoint, v[j]);
+    S.col(at).set(kSum, HALPERN ? it.Vrst[j] : sum_of(it.Verg[j]));
+    S.col(at).set(kCost, it.cost[j]);
+    S.col(at).set(kLower, it.xb_uniform ? it.xb_lo : it.lower[j]);
+    S.col(at).set(kUpper, it.xb_uniform ? it.xb_hi : it.upper[j]);
     if (!HALPERN) ex.put_x(at, it.Vbar[j]);
   });
   each_own(M.K, [&](const At& at) {
     const int i = M.kperm[at.p];
     const int q = n + i;
-    S.row(kPoint, at) = v[q];
-    S.row(kCost, at) = it.cost[q];
-    S.row(kLower, at) = it.lower[q];
-    S.row(kUpper, at) = it.upper[q];
-    S.row(kDual, at) = y[i];
+    S.row(at).set(kPoint, v[q]);
+    S.row(at).set(kCost, it.cost[q]);
+    S.row(at).set(kLower, it.lower[q]);
+    S.row(at).set(kUpper, it.upper[q]);
+    S.row(at).set(kDual, y[i]);
     if (HALPERN) {
-      S.row(kSum, at) = it.Vrst[q];
-      S.row(kDualSum, at) = it.Yrst[i];
+      S.row(at).set(kSum, it.Vrst[q]);
+      S.row(at).set(kDualSum, it.Yrst[i]);
       ex.put_y(at, y[i]);
     } else {
-      S.row(kSum, at) = sum_of(it.Verg[q]);
-      S.row(kDualSum, at) = sum_of(it.Yerg[i]);
-      S.row(kBar, at) = -it.Vbar[q];
+      S.row(at).set(kSum, sum_of(it.Verg[q]));
+      S.row(at).set(kDualSum, sum_of(it.Yerg[i]));
+      S.row(at).set(kBar, -it.Vbar[q]);
     }
   });
   __syncthreads();
-  bool ok = run_steps<T, MODE, HALPERN>(
+  bool ok = run_steps<HALPERN, T, MODE, TaskShare<T>, FlatState<T>>(
       &ctx, steps, static_cast<T>(ctl->tau), static_cast<T>(ctl->sigma), [&] {
         // The other buffers hold the iterate before the last.
         const int other = static_cast<int>((t + steps + 1) & 1);
         __syncthreads();
         each_own(ctx.M.Kt, [&](const At& at) {
-          it.v(other)[ctx.M.tperm[at.p]] = ctx.S.col(kPoint, at);
+          it.v(other)[ctx.M.tperm[at.p]] = ctx.S.col(at).get(kPoint);
         });
         each_own(ctx.M.K, [&](const At& at) {
           const int i = ctx.M.kperm[at.p];
-          it.v(other)[ctx.M.n + i] = ctx.S.row(kPoint, at);
-          it.y(other)[i] = ctx.S.row(kDual, at);
+          it.v(other)[ctx.M.n + i] = ctx.S.row(at).get(kPoint);
+          it.y(other)[i] = ctx.S.row(at).get(kDual);
         });
       });
   ok = ok && ex.wait(HALPERN ? 1 : 0);
@@ -120,27 +353,27 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
     auto average_of = [&](T sum) { return kF64 ? sum * inv : sum; };
     each_own(M.Kt, [&](const At& at) {
       const int j = M.tperm[at.p];
-      it.v(now)[j] = S.col(kPoint, at);
+      it.v(now)[j] = S.col(at).get(kPoint);
       it.Vbar[j] = ex.xs()[at.p];
-      it.Verg[j] = HALPERN ? Z.x(at.p) : average_of(S.col(kSum, at));
+      it.Verg[j] = HALPERN ? Z.x(at.p) : average_of(S.col(at).get(kSum));
     });
     each_own(M.K, [&](const At& at) {
       const int i = M.kperm[at.p];
       const int q = n + i;
-      it.v(now)[q] = S.row(kPoint, at);
-      it.y(now)[i] = S.row(kDual, at);
+      it.v(now)[q] = S.row(at).get(kPoint);
+      it.y(now)[i] = S.row(at).get(kDual);
       if (HALPERN) {
         it.Verg[q] = Z.r(at.p);
         it.Yerg[i] = Z.y(at.p);
       } else {
-        const T lo = S.row(kLower, at);
-        it.Vbar[q] = -S.row(kBar, at);
-        it.Yerg[i] = average_of(S.row(kDualSum, at));
+        const T lo = S.row(at).get(kLower);
+        it.Vbar[q] = -S.row(at).get(kBar);
+        it.Yerg[i] = average_of(S.row(at).get(kDualSum));
         // An FP64 step leaves the sums of equality rows, whose logicals are their bound from
         // the first step on, to this.
-        it.Verg[q] = kF64 && lo == S.row(kUpper, at)
+        it.Verg[q] = kF64 && lo == S.row(at).get(kUpper)
                          ? average_of(sum_of(it.Verg[q]) + static_cast<T>(steps) * lo)
-                         : average_of(S.row(kSum, at));
+                         : average_of(S.row(at).get(kSum));
       }
     });
   } else if (threadIdx.x == 0) {
@@ -160,14 +393,15 @@ __global__ void chunk_fill_kernel(ChunkView<T> c, OpView<T> K, OpView<T> Kt) {
     const bool rows = w < c.m;
     const int r = rows ? w : w - c.m;
     const OpView<T>& A = rows ? K : Kt;
-    const ClusterOp<T>& C = rows ? c.K : c.Kt;
+    const ChunkOp<T>& C = rows ? c.K : c.Kt;
     const int* other = rows ? c.Kt.pos : c.K.pos;
     const int b = A.ptr[r];
-    const int2 sl = C.sl[C.pos[r]];
-    for (int k = lane; k < sl.y; k += 32) {
-      const int at = nonzero_at(sl.x, sl.y, k);
+    const int len = A.ptr[r + 1] - b;
+    const int2 place = C.row[C.pos[r]];
+    for (int k = lane; k < len; k += 32) {
+      const int at = place.x + ((k >> place.y) << 5) + (k & ((1 << place.y) - 1));
       if constexpr (INDICES) {
-        C.idx[at] = other[A.idx[b + k]];
+        C.idx[at] = static_cast<unsigned short>(other[A.idx[b + k]]);
       } else {
         C.val[at] = A.val[b + k];
       }
@@ -182,13 +416,35 @@ int fill_grid(int rows) {
 
 }  // namespace
 
-size_t chunk_smem_bytes(int n, int m, int tslice, int kslice, int size, size_t elem) {
-  return cluster_vector_bytes(n, m, tslice, kslice, size, elem) +
-         solve_state_bytes(share_rows(n, tslice, size) >> tslice,
-                           share_rows(m, kslice, size) >> kslice, elem);
+template <typename T>
+bool place_chunk(ChunkView<T>* v, const TaskLayout& k, const TaskLayout& t) {
+  const size_t nc = t.per;
+  const size_t nr = k.per;
+  v->np = t.positions();
+  v->mp = k.positions();
+  v->K.per = k.per;
+  v->Kt.per = t.per;
+  if (v->np > 65535 || v->mp > 65535) return false;  // 16-bit column numbers
+  // The gathered vectors and the masks come first (chunk_kernel).
+  size_t at = (static_cast<size_t>(v->np) + v->mp + 2) * sizeof(T) + 2 * (nc + nr);
+  auto take = [&](size_t bytes) {
+    at = (at + 15) & ~static_cast<size_t>(15);
+    const unsigned here = static_cast<unsigned>(at);
+    at += bytes;
+    return here;
+  };
+  v->cols_at = take(kColArrays * nc * sizeof(T));
+  v->rows_at = take(kRowArrays * nr * sizeof(T));
+  v->sums_at = take((nc > nr ? nc : nr) * sizeof(T));
+  v->K.val_at = take(k.most_elems * sizeof(T));
+  v->Kt.val_at = take(t.most_elems * sizeof(T));
+  v->K.idx_at = take(k.most_elems * sizeof(unsigned short));
+  v->Kt.idx_at = take(t.most_elems * sizeof(unsigned short));
+  v->K.task_at = take(k.most_tasks * sizeof(Task));
+  v->Kt.task_at = take(t.most_tasks * sizeof(Task));
+  v->smem = at;
+  return at <= kClusterSmemMax;
 }
-
-bool chunk_fits(size_t smem) { return smem <= kClusterSmemMax; }
 
 template <typename T>
 void launch_chunk_indices(const ChunkView<T>& c, const OpView<T>& K, const OpView<T>& Kt,
@@ -211,8 +467,12 @@ cudaError_t launch_chunk(Ctl* ctl, const ChunkView<T>& c, const IterView<T>& it,
   return halpern ? go(chunk_kernel<T, true>) : go(chunk_kernel<T, false>);
 }
 
+template bool place_chunk<double>(ChunkView<double>*, const TaskLayout&, const TaskLayout&);
+template bool place_chunk<float>(ChunkView<float>*, const TaskLayout&, const TaskLayout&);
 template void launch_chunk_indices<double>(const ChunkView<double>&, const OpView<double>&,
                                            const OpView<double>&, cudaStream_t);
+template void launch_chunk_indices<float>(const ChunkView<float>&, const OpView<float>&,
+                                          const OpView<float>&, cudaStream_t);
 template void launch_chunk_values<double>(const ChunkView<double>&, const OpView<double>&,
                                           const OpView<double>&, cudaStream_t);
 template void launch_chunk_values<float>(const ChunkView<float>&, const OpView<float>&,

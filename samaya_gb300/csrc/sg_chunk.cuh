@@ -1,35 +1,45 @@
 // The iterations between two evaluations of a small LP in one launch (see sg_chunk.cu).
 #pragma once
 
+#include "sg_cluster_layout.h"
 #include "sg_kernels.cuh"
 
 namespace sg {
 
-// An operator in the cluster kernels' layout (sg_cluster.cuh).
+constexpr int kChunkThreads = 512;
+
+// An operator in tasks (sg_cluster_layout.h), and where a CTA keeps its block of it in shared
+// memory (bytes).
 template <typename T>
-struct ClusterOp {
-  const int2* sl;
-  const int2* desc;
-  const int* perm;  // position -> row
-  const int* pos;   // row -> position
-  int* idx;
+struct ChunkOp {
+  const int* perm;   // position -> row
+  const int* pos;    // row -> position
+  const int2* row;   // per position: first element, log2 lanes
+  const int4* task;
+  const int* task_off;
+  const int* elem_off;
+  const int* filled;
+  unsigned short* idx;
   T* val;
-  int slice;        // log2 of the rows of a slice
+  int per;           // positions of a CTA
+  unsigned val_at, idx_at, task_at;
 };
 
 template <typename T>
 struct ChunkView {
-  ClusterOp<T> K, Kt;
-  T* second;        // n + 2m: Halpern's T(z) by position
+  ChunkOp<T> K, Kt;
+  T* second;        // Halpern's T(z), by position
   int n, m;
-  int size;         // CTAs of the cluster
+  int np, mp;       // positions of the columns and rows
+  int size;         // CTAs of the cluster; 0: the LP takes step launches
+  unsigned cols_at, rows_at, sums_at;  // the state of the own columns and rows, a walk's sums
   size_t smem;
   int* wait_error;  // set to 1 when a bounded wait gave up
 };
 
-// Shared memory of a CTA that holds its share of an LP, and whether it fits.
-size_t chunk_smem_bytes(int n, int m, int tslice, int kslice, int size, size_t elem);
-bool chunk_fits(size_t smem);
+// Sets the places in shared memory and smem; false when they do not fit.
+template <typename T>
+bool place_chunk(ChunkView<T>* v, const TaskLayout& k, const TaskLayout& t);
 // The column numbers of both operators, from their CSR arrays.
 template <typename T>
 void launch_chunk_indices(const ChunkView<T>& c, const OpView<T>& K, const OpView<T>& Kt,

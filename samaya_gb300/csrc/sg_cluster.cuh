@@ -89,6 +89,23 @@ __device__ __forceinline__ void st_async(unsigned addr, float v, unsigned bar) {
       : "memory");
 }
 
+__device__ __forceinline__ void st_async_if(unsigned on, unsigned addr, double v, unsigned bar) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n"
+      " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];\n}" ::"r"(
+          addr),
+      "l"(__double_as_longlong(v)), "r"(bar), "r"(on)
+      : "memory");
+}
+__device__ __forceinline__ void st_async_if(unsigned on, unsigned addr, float v, unsigned bar) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n"
+      " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n}" ::"r"(
+          addr),
+      "r"(__float_as_uint(v)), "r"(bar), "r"(on)
+      : "memory");
+}
+
 // Every thread of the cluster; orders shared and global accesses of all its CTAs.
 __device__ __forceinline__ void cluster_sync(unsigned size) {
   if (size == 1) {
@@ -300,8 +317,10 @@ struct alignas(16) Exchange {
   }
 };
 
-// put_x (WHICH 0) or put_y (1) of one walk, its addresses in registers.
-template <typename V, int MODE, int WHICH>
+// put_x (WHICH 0) or put_y (1) of one walk, its addresses in registers. OWN: every lane goes
+// through its own targets (the chunk kernel's clusters of up to 16; the batched kernels' of mostly
+// 4 were 1-2% slower so).
+template <typename V, int MODE, int WHICH, bool OWN = false>
 struct Sender {
   Array<V, MODE != kInDevice> v;
   unsigned mask, bar, distance, size;
@@ -315,11 +334,27 @@ struct Sender {
     v.set(at.p, value);
     if constexpr (MODE != kInDevice) {
       if (size > 1) {
-        const unsigned m = sh_load_u16(mask + 2 * at.l);
-        for (unsigned q = 1; q < size; ++q) {
-          if ((m >> q) & 1u) {
-            const unsigned d = sh_load_u32(distance + 4 * q);
-            st_async(v.a + at.p * static_cast<int>(sizeof(V)) + d, value, bar + d);
+        unsigned m = sh_load_u16(mask + 2 * at.l);
+        if constexpr (OWN) {
+          // Each lane its own targets, two at a time (every target in turn by the whole warp takes
+          // 100 clocks each, 1,500 with 16 CTAs).
+          const unsigned a = v.a + at.p * static_cast<int>(sizeof(V));
+          while (m != 0u) {
+            const unsigned q0 = 31 - __clz(m);
+            m ^= 1u << q0;
+            const unsigned q1 = 31 - __clz(m | 1u);
+            const unsigned d0 = sh_load_u32(distance + 4 * q0);
+            const unsigned d1 = sh_load_u32(distance + 4 * q1);
+            st_async(a + d0, value, bar + d0);
+            st_async_if(m, a + d1, value, bar + d1);
+            m &= ~(1u << q1);
+          }
+        } else {
+          for (unsigned q = 1; q < size; ++q) {
+            if ((m >> q) & 1u) {
+              const unsigned d = sh_load_u32(distance + 4 * q);
+              st_async(v.a + at.p * static_cast<int>(sizeof(V)) + d, value, bar + d);
+            }
           }
         }
       }
@@ -330,9 +365,10 @@ struct Sender {
 // A CTA's share of an operator by rows.
 template <typename T>
 struct alignas(16) RowShare {
+  static constexpr bool kTasks = false;
   const int2* sl;  // per row (position): first nonzero, length
-  // Per slice: the place of its rows' first nonzeros (lane 0's; rows of at most 32), their number of
-  // steps, with kHasLong when the slice has longer rows.
+  // Per slice: the place of its rows' first nonzeros (lane 0's; rows of at most 32), their number
+  // of steps, with kHasLong when the slice has longer rows.
   const int2* desc;
   const int* idx;
   const T* val;
@@ -375,6 +411,27 @@ __device__ __forceinline__ void each_own(const RowShare<T>& A, const F& f) {
   }
 }
 
+// The bytes that arrive here per publication, from the entries that each CTA counted for each
+// other (ClusterShared::count); ends with a cluster barrier.
+template <typename V, int MODE>
+__device__ __forceinline__ void settle_counts(Exchange<V, MODE>& ex) {
+  ClusterShared& sh = *ex.sh;
+  ex.tx[0] = ex.tx[1] = 0;
+  __syncthreads();
+  if (threadIdx.x < 2 * ex.size) {
+    const unsigned which = threadIdx.x & 1u;
+    const unsigned q = threadIdx.x >> 1;
+    st_cluster(map_rank(shared_addr(&sh.incoming[which][q]), ex.rank ^ q), sh.count[which][q]);
+  }
+  cluster_sync(ex.size);
+  for (unsigned q = 0; q < ex.size; ++q) {
+    ex.tx[0] += sh.incoming[0][q] * static_cast<unsigned>(sizeof(V));
+    ex.tx[1] += sh.incoming[1][q] * static_cast<unsigned>(sizeof(V));
+  }
+  // Nobody overwrites the counts of the next LP before all have read these.
+  cluster_sync(ex.size);
+}
+
 // Fills the masks of the own rows and columns and the byte counts; ends with a cluster barrier.
 template <typename V, int MODE, typename T>
 __device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShare<T>& K,
@@ -410,19 +467,7 @@ __device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShar
       }
     });
   }
-  __syncthreads();
-  if (threadIdx.x < 2 * ex.size) {
-    const unsigned which = threadIdx.x & 1u;
-    const unsigned q = threadIdx.x >> 1;
-    st_cluster(map_rank(shared_addr(&sh.incoming[which][q]), ex.rank ^ q), sh.count[which][q]);
-  }
-  cluster_sync(ex.size);
-  for (unsigned q = 0; q < ex.size; ++q) {
-    ex.tx[0] += sh.incoming[0][q] * static_cast<unsigned>(sizeof(V));
-    ex.tx[1] += sh.incoming[1][q] * static_cast<unsigned>(sizeof(V));
-  }
-  // Nobody overwrites the counts of the next LP before all have read these.
-  cluster_sync(ex.size);
+  settle_counts(ex);
 }
 
 // K sums (or maxima, bit q of MAXMASK) over the cluster, in a fixed order; every thread of every
@@ -743,6 +788,17 @@ __device__ __forceinline__ bool walk_rows(const RowShare<T>& A, const Prod& prod
     return walk_one<NC, MAXRED>(A, prod, init, f, ready);
   } else {
     return walk_pairs<NC, MAXRED>(A, prod, init, f, ready);
+  }
+}
+
+// The walk of a step (NC, sums): a share of tasks has its own (sg_chunk.cu).
+template <typename Share, typename Prod, typename Init, typename F, typename Ready>
+__device__ __forceinline__ bool walk_step(const Share& A, const Prod& prod, const Init& init,
+                                          const F& f, const Ready& ready) {
+  if constexpr (Share::kTasks) {
+    return A.walk(prod, init, f, ready);
+  } else {
+    return walk_rows<true, false>(A, prod, init, f, ready);
   }
 }
 

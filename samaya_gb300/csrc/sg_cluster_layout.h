@@ -92,4 +92,80 @@ inline int place_of(const StartLen& sl, int k) {
   return sl.start + (sl.len <= 32 ? k << 5 : k);
 }
 
+// The other layout, for an LP on one cluster of few rows a CTA (sg_chunk.cu). The rows, by
+// decreasing length, are dealt out to the CTAs in turn; row l of CTA r has position
+// r ceil(rows / size) + l (the CTA's entries of the gathered vector lie side by side: l size + r,
+// tried first, sent every warp's 32 entries to one bank), and its nonzeros go to tasks, a warp's
+// work each: 32 >> lanes rows of the CTA, 2^lanes lanes to a row, `steps` steps; nonzero k of a
+// row is read at step k >> lanes by the row's lane k mod 2^lanes. Padding: value 0, index the other
+// operator's positions.
+struct Task {
+  int place;  // first element, in the CTA's block
+  int steps;
+  int first;  // own row
+  int rows;   // rows | lanes << 8
+};
+
+struct TaskLayout {
+  int per = 0;                // positions of a CTA
+  std::vector<int> perm, pos;  // position -> row (-1: none), row -> position
+  std::vector<StartLen> row;  // per position: first element (of the whole layout), log2 lanes
+  std::vector<Task> tasks;
+  std::vector<int> task_off, elem_off;  // per CTA: first task and element
+  std::vector<int> filled;  // and two numbers: rows with nonzeros, rows on several lanes
+  int most_tasks = 0, most_elems = 0;
+  int positions() const { return static_cast<int>(perm.size()); }
+};
+
+// limit: no row takes more steps (up to 32 lanes). 0: a row of at most 32 nonzeros by one lane,
+// longer ones by 32 (the sums of FP32 keep their order).
+inline TaskLayout make_tasks(const int* ptr, int rows, int size, int limit) {
+  TaskLayout t;
+  const RowOrder o = order_rows(ptr, rows);
+  t.per = (rows + size - 1) / size;
+  t.perm.assign(static_cast<size_t>(t.per) * size, -1);
+  t.pos.resize(rows);
+  t.row.assign(t.perm.size(), StartLen{0, 0});
+  t.task_off.assign(1, 0);
+  t.elem_off.assign(1, 0);
+  auto lanes_of = [&](int len) {
+    if (limit == 0) return len <= 32 ? 0 : 5;
+    int lanes = 0;
+    while (lanes < 5 && ((len - 1) >> lanes) >= limit) ++lanes;
+    return lanes;
+  };
+  for (int rank = 0; rank < size; ++rank) {
+    const int own = rows > rank ? (rows - rank - 1) / size + 1 : 0;
+    const int first = rank * t.per;
+    for (int l = 0; l < own; ++l) {
+      const int r = o.perm[static_cast<size_t>(l) * size + rank];
+      t.perm[first + l] = r;
+      t.pos[r] = first + l;
+    }
+    auto length = [&](int l) { return ptr[t.perm[first + l] + 1] - ptr[t.perm[first + l]]; };
+    int elems = 0, l = 0, count = 0, shared = 0;
+    while (l < own && length(l) > 0) {
+      const int lanes = lanes_of(length(l));
+      Task k{elems, ((length(l) - 1) >> lanes) + 1, l, 0};
+      int n = 0;
+      for (; n < (32 >> lanes) && l < own && length(l) > 0 && lanes_of(length(l)) == lanes;
+           ++n, ++l) {
+        t.row[first + l] = StartLen{t.elem_off.back() + elems + (n << lanes), lanes};
+      }
+      k.rows = n | lanes << 8;
+      if (lanes > 0) shared = l;
+      t.tasks.push_back(k);
+      ++count;
+      elems += k.steps * 32;
+    }
+    t.filled.push_back(l);
+    t.filled.push_back(shared);
+    t.task_off.push_back(static_cast<int>(t.tasks.size()));
+    t.elem_off.push_back(t.elem_off.back() + elems);
+    t.most_tasks = std::max(t.most_tasks, count);
+    t.most_elems = std::max(t.most_elems, elems);
+  }
+  return t;
+}
+
 }  // namespace sg

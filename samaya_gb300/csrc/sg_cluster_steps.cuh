@@ -97,11 +97,11 @@ __device__ __forceinline__ StepState<T, MODE, kRowArrays> row_state(const SolveS
 }
 
 // What the walks need of an instance, in shared memory (sh_copy).
-template <typename T, int MODE>
+template <typename T, int MODE, typename Share = RowShare<T>, typename State = SolveState<T, MODE>>
 struct StepContext {
-  MatShare<T> M;
+  MatShare<T, Share> M;
   Exchange<T, MODE> ex;
-  SolveState<T, MODE> S;
+  State S;
   Second<T> Z;
   T weight[64], rest[64];  // run_steps
 };
@@ -109,16 +109,16 @@ struct StepContext {
 // One PDHG iteration (FP64: sums since the restart in place of running averages, one addition
 // less each, and the row's own term as the sum's start). xs has been put, not waited for; so it
 // is afterwards.
-template <typename T, int MODE>
-__device__ __forceinline__ bool classic_step(const StepContext<T, MODE>* ctx, T tau, T sig,
+template <typename T, int MODE, typename Share, typename State>
+__device__ __forceinline__ bool classic_step(const StepContext<T, MODE, Share, State>* ctx, T tau, T sig,
                                              T ta, T tb) {
   constexpr bool kF64 = sizeof(T) == 8;
   {
     const auto K = sh_copy(&ctx->M.K);
     const auto ex = sh_copy(&ctx->ex);
     const auto R = row_state(sh_copy(&ctx->S));
-    const Sender<T, MODE, 1> y_out(ex);
-    const bool ok = walk_rows<true, false>(
+    const Sender<T, MODE, 1, Share::kTasks> y_out(ex);
+    const bool ok = walk_step(
         K, Gather<T, MODE>{ex.xs()},
         [&](const At& at) { return kF64 ? R.at(at).get(kBar) : T(0); },
         [&](const At& at, T s) {
@@ -159,8 +159,8 @@ __device__ __forceinline__ bool classic_step(const StepContext<T, MODE>* ctx, T 
   const auto Kt = sh_copy(&ctx->M.Kt);
   const auto ex = sh_copy(&ctx->ex);
   const auto C = col_state(sh_copy(&ctx->S));
-  const Sender<T, MODE, 0> x_out(ex);
-  return walk_rows<true, false>(
+  const Sender<T, MODE, 0, Share::kTasks> x_out(ex);
+  return walk_step(
       Kt, Gather<T, MODE>{ex.ys()},
       [&](const At& at) { return kF64 ? C.at(at).get(kCost) : T(0); },
       [&](const At& at, T s) {
@@ -180,8 +180,8 @@ __device__ __forceinline__ bool classic_step(const StepContext<T, MODE>* ctx, T 
 // halpern_primal / halpern_dual kernels compute it; the anchor is in the sums' place, and T(z)
 // (the point the evaluation, the restarts and the answer use) is written when it is `measured`.
 // ys has been put, not waited for; so it is afterwards.
-template <typename T, int MODE>
-__device__ __forceinline__ bool halpern_step(const StepContext<T, MODE>* ctx, T tau, T sig, T w,
+template <typename T, int MODE, typename Share, typename State>
+__device__ __forceinline__ bool halpern_step(const StepContext<T, MODE, Share, State>* ctx, T tau, T sig, T w,
                                              bool measured) {
   constexpr bool kF64 = sizeof(T) == 8;
   const Second<T>& Z = ctx->Z;
@@ -189,8 +189,8 @@ __device__ __forceinline__ bool halpern_step(const StepContext<T, MODE>* ctx, T 
     const auto Kt = sh_copy(&ctx->M.Kt);
     const auto ex = sh_copy(&ctx->ex);
     const auto C = col_state(sh_copy(&ctx->S));
-    const Sender<T, MODE, 0> x_out(ex);
-    const bool ok = walk_rows<true, false>(
+    const Sender<T, MODE, 0, Share::kTasks> x_out(ex);
+    const bool ok = walk_step(
         Kt, Gather<T, MODE>{ex.ys()},
         [&](const At& at) { return kF64 ? C.at(at).get(kCost) : T(0); },
         [&](const At& at, T s) {
@@ -209,8 +209,8 @@ __device__ __forceinline__ bool halpern_step(const StepContext<T, MODE>* ctx, T 
   const auto K = sh_copy(&ctx->M.K);
   const auto ex = sh_copy(&ctx->ex);
   const auto R = row_state(sh_copy(&ctx->S));
-  const Sender<T, MODE, 1> y_out(ex);
-  return walk_rows<true, false>(
+  const Sender<T, MODE, 1, Share::kTasks> y_out(ex);
+  return walk_step(
       K, Gather<T, MODE>{ex.xs()}, Zero<T>(),
       [&](const At& at, T s) {
         const auto e = R.at(at);
@@ -235,16 +235,17 @@ __device__ __forceinline__ bool halpern_step(const StepContext<T, MODE>* ctx, T 
 // `count` iterations, the last of them measured, before_last() just before it; xs (Halpern: ys)
 // put, not waited for, before and after. ctx->weight and rest hold the steps' weights. (Inlined:
 // in a called function every global load takes two more instructions for its descriptor.)
-template <typename T, int MODE, bool HALPERN, typename BeforeLast>
-__device__ __forceinline__ bool run_steps(const StepContext<T, MODE>* ctx, int count, T tau, T sig,
+template <bool HALPERN, typename T, int MODE, typename Share, typename State, typename BeforeLast>
+__device__ __forceinline__ bool run_steps(const StepContext<T, MODE, Share, State>* ctx,
+                                          int count, T tau, T sig,
                                           const BeforeLast& before_last) {
   bool ok = true;
   for (int i = 0; i < count && ok; ++i) {
     if (i == count - 1) before_last();
     if constexpr (HALPERN) {
-      ok = halpern_step<T, MODE>(ctx, tau, sig, ctx->weight[i], i == count - 1);
+      ok = halpern_step(ctx, tau, sig, ctx->weight[i], i == count - 1);
     } else {
-      ok = classic_step<T, MODE>(ctx, tau, sig, ctx->weight[i], ctx->rest[i]);
+      ok = classic_step(ctx, tau, sig, ctx->weight[i], ctx->rest[i]);
     }
   }
   return ok;

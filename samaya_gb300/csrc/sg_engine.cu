@@ -799,6 +799,25 @@ struct Carver {
   }
 };
 
+template <typename T>
+void take_chunk(Carver& c, DevChunk<T>* d) {
+  if (d->view.size == 0) return;
+  for (int q = 0; q < 2; ++q) {
+    const TaskLayout& l = d->layout[q];
+    auto& o = d->op[q];
+    c.take(&o.perm, l.perm.size());
+    c.take(&o.pos, l.pos.size());
+    c.take(&o.row, l.row.size());
+    c.take(&o.task, l.tasks.size());
+    c.take(&o.task_off, l.task_off.size());
+    c.take(&o.elem_off, l.elem_off.size());
+    c.take(&o.filled, l.filled.size());
+    c.take(&o.idx, l.elem_off.back());
+    c.take(&o.val, l.elem_off.back());
+  }
+  c.take(&d->second, static_cast<size_t>(d->view.np) + 2 * static_cast<size_t>(d->view.mp));
+}
+
 }  // namespace
 
 int Engine::alloc_all(std::string* err) {
@@ -846,19 +865,8 @@ int Engine::alloc_all(std::string* err) {
     for (double** p : {&rhs_ev_, &rs_, &rn_, &pu_, &u0_, &y_out_, &ray_out_}) c.take(p, m);
     for (double** p : {&cs_, &cn_, &pv_, &inv_cs_}) c.take(p, static_cast<size_t>(n_));
     c.take(&inv_rs_, m);
-    if (chunk_size_ > 0 || chunk32_size_ > 0) {
-      for (DevClusterOp* op : {&Kc_, &Ktc_}) {
-        c.take(&op->sl, op->sl_host.size());
-        c.take(&op->desc, op->desc_host.size());
-        c.take(&op->perm, op->order.perm.size());
-        c.take(&op->pos, op->order.pos.size());
-        c.take(&op->idx, static_cast<size_t>(op->elements));
-        c.take(&op->val, static_cast<size_t>(op->elements));
-        if (chunk32_size_ > 0) c.take(&op->val32, static_cast<size_t>(op->elements));
-      }
-      c.take(&chunk_second_, nt + m);
-      if (chunk32_size_ > 0) c.take(&chunk_second32_, nt + m);
-    }
+    take_chunk(c, &chunk64_);
+    take_chunk(c, &chunk32c_);
     c.take(&partial_, static_cast<size_t>(4096) * kMaxSums);
     c.take(&counter_, 8);
     c.take(&ctl_, 1);
@@ -900,94 +908,111 @@ int Engine::alloc_all(std::string* err) {
 // Whether the chunk's iterations run on a cluster (chunk_kernel), and on how many CTAs: up to where
 // 16 SMs take as long as the step launches do. Measured, us an iteration with its share of the
 // evaluation, w = 2 nnz + 5 (n + m), step launches against 4 / 8 / 16 CTAs:
-//   FP64  200 x 500 (w 9,500)        11.8 against 5.4 / 5.7 / 6.1
-//         777 x 2,049 (39,000)       12.2 against 7.1 / 6.0 / 6.5
-//         2,000 x 5,000 (95,000)     12.6 against 10.4 / 8.4 / 7.0
-//         5,000 x 10,000 (195,000)   12.9 against - / 13.3 / 10.6
-//   FP32  200 x 500                  9.7 against 4.4 / 4.7 / 5.2
-//         5,000 x 10,000             10.9 against 11.4 / 9.2 / 7.6
+//   FP64  200 x 500 (w 9,500)                9.1 against 3.4 / 3.3 / 3.5
+//         777 x 2,049 (39,000)               9.4 against  -  / 4.7 / 4.1
+//         facility 40 x 150 (97,000)        14.4 against 7.0 / 5.3 / 4.4
+//         2,000 x 5,000 (95,000)             9.6 against  -  / 7.6 / 6.1
+//         3,500 x 7,000 (137,000)            9.3 against  -  /  -  / 7.1
+//   FP32  200 x 500                          7.2 against 3.2 / 3.4 / 3.6
+//         777 x 2,049                        7.8 against 3.6 / 3.3 / 3.4
+//         2,000 x 5,000                      7.8 against 4.8 / 4.7 / 4.4
+//         5,000 x 10,000 (195,000)           8.1 against  -  / 8.2 / 7.4
+// The steps a row takes at most (make_tasks), FP64: 4 / 8 / 16 / 32 with 777 x 2,049 on 16 CTAs
+// 4.1 / 4.3 / 5.0 / 4.9, facility 40 x 150 4.3 / 4.3 / 4.4 / 4.9, 2,000 x 5,000 6.9 / 6.2 / 6.1 /
+// 6.0, 3,500 x 7,000 8.6 / 7.6 / 7.4 / 7.1.
 void Engine::plan_chunk() {
   if (m_ <= 0 || n_ <= 0 || nnz_ <= 0) return;
   const long long work = 2 * nnz_ + 5 * (static_cast<long long>(n_) + m_);
   constexpr long long kMost64 = 220000, kMost32 = 300000;
   if (work > kMost32) return;
-  const int size = work <= 20000 ? 4 : work <= 45000 ? 8 : 16;
-  Kc_.order = order_rows(K_.host_ptr.data(), m_);
-  Ktc_.order = order_rows(Kt_.host_ptr.data(), n_);
-  auto fits = [&](size_t elem) {
-    return chunk_fits(chunk_smem_bytes(n_, m_, Ktc_.order.slice, Kc_.order.slice, size, elem));
-  };
   auto longest = [](const std::vector<int>& ptr) {
     int most = 0;
     for (size_t r = 0; r + 1 < ptr.size(); ++r) most = std::max(most, ptr[r + 1] - ptr[r]);
     return most;
   };
-  if (work <= kMost64 && fits(sizeof(double))) chunk_size_ = size;
+  auto plan = [&](auto* c, bool fixed_order) {
+    const int size = work <= (fixed_order ? 12000 : 6000)    ? 4
+                     : work <= (fixed_order ? 50000 : 25000) ? 8
+                                                             : 16;
+    const int limit = fixed_order            ? 0
+                      : work <= 3000LL * size ? 4
+                      : work <= 7000LL * size ? 16
+                                              : 32;
+    c->layout[0] = make_tasks(K_.host_ptr.data(), m_, size, limit);
+    c->layout[1] = make_tasks(Kt_.host_ptr.data(), n_, size, limit);
+    c->view.n = n_;
+    c->view.m = m_;
+    c->view.size = size;
+    if (!place_chunk(&c->view, c->layout[0], c->layout[1])) c->view.size = 0;
+  };
+  if (work <= kMost64) plan(&chunk64_, false);
   // FP32 sums keep the step kernels' order: rows longer than kWarpRowMin have another. (The
   // refinement's inner problems have a right-hand side, which these steps do not read.)
-  if (switch_ && fits(sizeof(float)) &&
-      std::max(longest(K_.host_ptr), longest(Kt_.host_ptr)) <= kWarpRowMin) {
-    chunk32_size_ = size;
+  if (switch_ && std::max(longest(K_.host_ptr), longest(Kt_.host_ptr)) <= kWarpRowMin) {
+    plan(&chunk32c_, true);
   }
-  if (chunk_size_ == 0 && chunk32_size_ == 0) return;
-  for (auto p : {std::make_pair(&Kc_, &K_), std::make_pair(&Ktc_, &Kt_)}) {
-    DevClusterOp& c = *p.first;
-    c.sl_host.resize(p.second->rows);
-    c.desc_host.resize(slices_of(c.order));
-    c.elements =
-        place_rows(p.second->host_ptr.data(), c.order, c.sl_host.data(), c.desc_host.data());
-  }
-}
-
-// The layout's arrays (the column numbers by a kernel: the operators are in device memory).
-int Engine::upload_chunk(std::string* err) {
-  if (chunk_size_ == 0 && chunk32_size_ == 0) return kOk;
-  cudaStream_t s = stream_;
-  for (DevClusterOp* c : {&Kc_, &Ktc_}) {
-    const int other = c == &Kc_ ? n_ : m_;
-    auto up = [&](void* dst, const void* src, size_t bytes) {
-      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s);
-    };
-    SG_TRY(up(c->sl, c->sl_host.data(), c->sl_host.size() * sizeof(StartLen)));
-    SG_TRY(up(c->desc, c->desc_host.data(), c->desc_host.size() * sizeof(StartLen)));
-    SG_TRY(up(c->perm, c->order.perm.data(), c->order.perm.size() * sizeof(int)));
-    SG_TRY(up(c->pos, c->order.pos.data(), c->order.pos.size() * sizeof(int)));
-    // Padding: value 0, the other operator's entry past the last.
-    const std::vector<int> pad(static_cast<size_t>(c->elements), other);
-    SG_TRY(up(c->idx, pad.data(), pad.size() * sizeof(int)));
-    SG_TRY(cudaMemsetAsync(c->val, 0, c->elements * sizeof(double), s));
-    if (c->val32) SG_TRY(cudaMemsetAsync(c->val32, 0, c->elements * sizeof(float), s));
-  }
-  launch_chunk_indices(chunk_view64(), K_.view64(), Kt_.view64(), s);
-  SG_TRY(cudaGetLastError());
-  SG_TRY(cudaStreamSynchronize(s));
-  return kOk;
 }
 
 namespace {
 
+// The layout's arrays to the device (the column numbers by a kernel: the operators are there).
 template <typename T>
-ClusterOp<T> cluster_op(const DevClusterOp& c, T* val) {
-  return ClusterOp<T>{reinterpret_cast<const int2*>(c.sl), reinterpret_cast<const int2*>(c.desc),
-                      c.perm, c.pos, c.idx, val, c.order.slice};
+cudaError_t upload_chunk_arrays(DevChunk<T>* c, const OpView<T>& K, const OpView<T>& Kt,
+                                int* wait_error, std::vector<unsigned short>* pad,
+                                cudaStream_t s) {
+  if (c->view.size == 0) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+    const TaskLayout& l = c->layout[q];
+    const auto& o = c->op[q];
+    auto up = [&](void* dst, const auto& v) {
+      if (e == cudaSuccess && !v.empty()) {
+        e = cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, s);
+      }
+    };
+    up(o.perm, l.perm);
+    up(o.pos, l.pos);
+    up(o.row, l.row);
+    up(o.task, l.tasks);
+    up(o.task_off, l.task_off);
+    up(o.elem_off, l.elem_off);
+    up(o.filled, l.filled);
+    // Padding: value 0, the other operator's entry past the last.
+    pad[q].assign(l.elem_off.back(),
+                  static_cast<unsigned short>(q == 0 ? c->view.np : c->view.mp));
+    up(o.idx, pad[q]);
+    if (e == cudaSuccess) e = cudaMemsetAsync(o.val, 0, l.elem_off.back() * sizeof(T), s);
+    ChunkOp<T>& v = q == 0 ? c->view.K : c->view.Kt;
+    v.perm = o.perm;
+    v.pos = o.pos;
+    v.row = reinterpret_cast<const int2*>(o.row);
+    v.task = reinterpret_cast<const int4*>(o.task);
+    v.task_off = o.task_off;
+    v.elem_off = o.elem_off;
+    v.filled = o.filled;
+    v.idx = o.idx;
+    v.val = o.val;
+  }
+  c->view.second = c->second;
+  c->view.wait_error = wait_error;
+  if (e == cudaSuccess) {
+    launch_chunk_indices(c->view, K, Kt, s);
+    e = cudaGetLastError();
+  }
+  return e;
 }
 
 }  // namespace
 
-ChunkView<double> Engine::chunk_view64() const {
-  return ChunkView<double>{cluster_op(Kc_, Kc_.val), cluster_op(Ktc_, Ktc_.val), chunk_second_,
-                           n_, m_, chunk_size_,
-                           chunk_smem_bytes(n_, m_, Ktc_.order.slice, Kc_.order.slice,
-                                            std::max(chunk_size_, 1), sizeof(double)),
-                           wait_error_};
-}
-
-ChunkView<float> Engine::chunk_view32() const {
-  return ChunkView<float>{cluster_op(Kc_, Kc_.val32), cluster_op(Ktc_, Ktc_.val32),
-                          chunk_second32_, n_, m_, chunk32_size_,
-                          chunk_smem_bytes(n_, m_, Ktc_.order.slice, Kc_.order.slice,
-                                           std::max(chunk32_size_, 1), sizeof(float)),
-                          wait_error_};
+int Engine::upload_chunk(std::string* err) {
+  static_assert(sizeof(Task) == sizeof(int4) && sizeof(StartLen) == sizeof(int2), "device types");
+  if (chunk64_.view.size == 0 && chunk32c_.view.size == 0) return kOk;
+  std::vector<unsigned short> pad[4];
+  SG_TRY(upload_chunk_arrays(&chunk64_, K_.view64(), Kt_.view64(), wait_error_, pad, stream_));
+  SG_TRY(upload_chunk_arrays(&chunk32c_, K_.view32(), Kt_.view32(), wait_error_, pad + 2,
+                             stream_));
+  SG_TRY(cudaStreamSynchronize(stream_));
+  return kOk;
 }
 
 template <typename T>
@@ -1105,7 +1130,7 @@ int Engine::setup_device(const double* rhs_orig) {
     }
   }
   launch_apply_scaling(K, Kt, K_.val_orig, Kt_.val_orig, rs_, cs_, nnz_, s);
-  if (chunk_size_ > 0) launch_chunk_values(chunk_view64(), K, Kt, s);
+  if (chunk64_.view.size > 0) launch_chunk_values(chunk64_.view, K, Kt, s);
   launch_scale_vectors(n_, m_, cs_, rs_, cost_orig_, lower_orig_, upper_orig_, it64_.cost,
                        it64_.lower, it64_.upper, inv_cs_, inv_rs_, s);
   if (m_ > 0) {
@@ -1195,7 +1220,7 @@ int Engine::capture_chunk(bool detect) {
   if (g.exec != nullptr) return kOk;
   std::string* err = nullptr;
   SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  g.kernels = enqueue_chunk(ctl_, chunk_view64(), K_.step64(), K_.view64(), Kt_.view64(),
+  g.kernels = enqueue_chunk(ctl_, chunk64_.view, K_.step64(), K_.view64(), Kt_.view64(),
                             iter_view(it64_), eval_view(), red_view(), scratch_n_, grid_step_k_,
                             grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, detect, stream_);
   SG_TRY(cudaStreamEndCapture(stream_, &g.graph));
@@ -1211,7 +1236,7 @@ int Engine::capture_chunk32() {
   IterView<float> it = iter_view(it32_);
   it.rhs = it32_.rhs;
   SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  chunk32_.kernels = enqueue_chunk(ctl32_, chunk_view32(), K_.step32(), K_.view32(), Kt_.view32(), it,
+  chunk32_.kernels = enqueue_chunk(ctl32_, chunk32c_.view, K_.step32(), K_.view32(), Kt_.view32(), it,
                                    inner_eval_view(), red_view(), scratch_n_, grid_step_k_,
                                    grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, false,
                                    stream_);
@@ -1455,7 +1480,9 @@ int Engine::prepare_fp32() {
   const long long nb = nnz_;
   launch_convert(K_.val, K_.val32, nb, s);
   launch_convert(Kt_.val, Kt_.val32, nb, s);
-  if (chunk32_size_ > 0) launch_chunk_values(chunk_view32(), K_.view32(), Kt_.view32(), s);
+  if (chunk32c_.view.size > 0) {
+    launch_chunk_values(chunk32c_.view, K_.view32(), Kt_.view32(), s);
+  }
   launch_ir_begin(ctl32_, ctl_, s);
   launch_setup_norms(ctl32_, K_.view64(), Kt_.view64(), it64_.cost, red_view(), grid_k_, grid_t_,
                      s);

@@ -161,18 +161,19 @@ struct DevOp {
   OpView<float> step32() const { return OpView<float>{ptr, idx, val32, rows, step_tileset()}; }
 };
 
-// An operator in the cluster kernels' layout (sg_chunk.cu), beside its CSR arrays.
-struct DevClusterOp {
-  RowOrder order;
-  std::vector<StartLen> sl_host, desc_host;
-  long long elements = 0;
-  StartLen* sl = nullptr;
-  StartLen* desc = nullptr;
-  int* perm = nullptr;
-  int* pos = nullptr;
-  int* idx = nullptr;
-  double* val = nullptr;
-  float* val32 = nullptr;
+// An LP on one cluster (sg_chunk.cu) in one precision: host layouts, device arrays and the view.
+template <typename T>
+struct DevChunk {
+  TaskLayout layout[2];  // A, A'
+  struct Op {
+    int *perm, *pos, *task_off, *elem_off, *filled;
+    StartLen* row;
+    Task* task;
+    unsigned short* idx;
+    T* val;
+  } op[2] = {};
+  T* second = nullptr;
+  ChunkView<T> view{};
 };
 
 // Iterate storage of one precision.
@@ -297,16 +298,11 @@ class Engine {
   IrView ir_view();
   int finish_fp64(SolveInfo* info, double t0, long long iterations_before, double* x, double* y,
                   double* dual_ray, double* primal_ray);
-  // The cluster form of the chunk's iterations: whether and on how many CTAs (0: step launches),
-  // its arrays and views.
+  // The cluster form of the chunk's iterations, where the LP takes it (view.size > 0).
   void plan_chunk();
   int upload_chunk(std::string* err);
-  int chunk_size_ = 0, chunk32_size_ = 0;
-  DevClusterOp Kc_, Ktc_;
-  double* chunk_second_ = nullptr;
-  float* chunk_second32_ = nullptr;
-  ChunkView<double> chunk_view64() const;
-  ChunkView<float> chunk_view32() const;
+  DevChunk<double> chunk64_;
+  DevChunk<float> chunk32c_;
   int check(cudaError_t e, const char* what);
   TileShape default_shape(const DevOp& op) const;
   int set_tiles(DevOp* op, const TileShape& shape);

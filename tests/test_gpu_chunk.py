@@ -1,7 +1,8 @@
 """Small LPs whose iterations run on one cluster, at the edges of that rule and of the kernel:
-work 2 nnz + 5 (n + m) on both sides of 20,000, 45,000 (4, 8, 16 CTAs) and 220,000 (step
-launches), rows of 0 to 129 nonzeros (in FP32 a row of 129 takes the step launches), one row, and
-iteration limits inside a chunk, at its end and after a restart.
+work 2 nnz + 5 (n + m) on both sides of 6,000, 12,000, 25,000 and 50,000 (4, 8, 16 CTAs), 24,000,
+48,000 and 112,000 (lanes a row takes) and 220,000 (step launches), rows of 0 to 129 nonzeros (in
+FP32 a row of 129 takes the step launches), one row, and iteration limits inside a chunk, at its end
+and after a restart.
 
 Against the oracle after a fixed number of iterations, with the tolerances (and their reasons) of
 tests/test_gpu_batch_clusters.py: 1e-9 in FP64, 1e-3 for the FP32 phase of the precision switch,
@@ -29,14 +30,14 @@ LPS = {
     "one row": lambda: _lp(3, [2], 1),
     "edges": lambda: _lp(150, EDGES, 3),
     "up to 128": lambda: _lp(150, EDGES[:-1] * 5, 4),
-    "4 CTAs": lambda: _near(20000, -1, 5),
-    "8 CTAs": lambda: _near(20000, 1, 6),
-    "8 CTAs at most": lambda: _near(45000, -1, 7),
-    "16 CTAs": lambda: _near(45000, 1, 8),
-    "16 CTAs at most": lambda: _near(220000, -1, 9),
     "step launches": lambda: _near(220000, 1, 10),
     "few columns": lambda: _lp(40, _lengths(900, 0, 9, 11), 11),
 }
+
+
+for _k, _work in enumerate((6000, 12000, 24000, 25000, 48000, 50000, 112000, 220000)):
+    LPS[f"below {_work}"] = lambda w=_work, k=_k: _near(w, -1, 20 + k)
+    LPS[f"above {_work}"] = lambda w=_work, k=_k: _near(w, 1, 40 + k)
 
 
 @pytest.mark.parametrize("name", list(LPS))
