@@ -233,6 +233,118 @@ __device__ __forceinline__ void task_masks(const TaskShare<T>& A, int per, unsig
   }
 }
 
+// The LP's share of this CTA in shared memory, its masks and counts; ends with a cluster barrier.
+template <typename T>
+__device__ __forceinline__ void begin_cluster(const ChunkView<T>& c, ClusterShared& sh,
+                                              unsigned rank, unsigned size,
+                                              MatShare<T, TaskShare<T>>* m,
+                                              Exchange<T, kAllShared>* e) {
+  load_block(c.K, rank);
+  load_block(c.Kt, rank);
+  MatShare<T, TaskShare<T>>& M = *m;
+  M.m = c.m;
+  M.n = c.n;
+  M.kz = M.tz = 0;
+  M.kperm = c.K.perm;
+  M.tperm = c.Kt.perm;
+  M.K = task_share(c.K, c.m, rank, size, c.sums_at);
+  M.Kt = task_share(c.Kt, c.n, rank, size, c.sums_at);
+  M.nr = M.K.own;
+  M.nc = M.Kt.own;
+  Exchange<T, kAllShared>& ex = *e;
+  ex.sh = &sh;
+  ex.rank = rank;
+  ex.size = size;
+  ex.device = nullptr;
+  ex.xs_at = 0u;
+  ex.ys_at = (c.np + 1) * static_cast<unsigned>(sizeof(T));
+  ex.cmask_at = ex.ys_at + (c.mp + 1) * static_cast<unsigned>(sizeof(T));
+  ex.rmask_at = ex.cmask_at + M.nc * 2;
+  if (threadIdx.x == 0) ex.xs()[c.np] = ex.ys()[c.mp] = T(0);
+  for (int k = threadIdx.x; k < M.nc + M.nr; k += kChunkThreads) ex.cmask()[k] = 0;
+  if (threadIdx.x < 2 * kMaxCluster) (&sh.count[0][0])[threadIdx.x] = 0;
+  __syncthreads();
+  task_masks(M.Kt, c.K.per, ex.cmask(), sh, 0);
+  task_masks(M.K, c.Kt.per, ex.rmask(), sh, 1);
+  settle_counts(ex);
+}
+
+template <typename T>
+__device__ __forceinline__ FlatState<T> flat_state(const ChunkView<T>& c,
+                                                   const MatShare<T, TaskShare<T>>& M) {
+  const unsigned base = shared_addr(sg_smem);
+  return FlatState<T>{base + c.cols_at, base + c.rows_at,
+                      M.nc * static_cast<unsigned>(sizeof(T)),
+                      M.nr * static_cast<unsigned>(sizeof(T))};
+}
+
+// The power iteration of the setup (pdlp.cpp:36-103; power_spmv_kernel's products): 20 times
+// v = A' u, u = A v, and |u| / |v| of the last. The lengths are taken in the first iteration, whose
+// u is brought into [1, 2) and whose growth the later ones undo by a power of two (exact), and in
+// the last. 40 launches took 0.3 ms of a 200 x 500 LP's solve, one takes 0.08.
+__global__ void __launch_bounds__(kChunkThreads, 1)
+    chunk_power_kernel(Ctl* ctl, ChunkView<double> c, const double* u0, int iterations) {
+  __shared__ ClusterShared sh;
+  const unsigned rank = cluster_rank();
+  const unsigned size = cluster_size();
+  cluster_init(sh, size);
+  MatShare<double, TaskShare<double>> M;
+  Exchange<double, kAllShared> ex;
+  begin_cluster(c, sh, rank, size, &M, &ex);
+  const FlatState<double> S = flat_state(c, M);
+  const Sender<double, kAllShared, 0, true> x_out(ex);
+  const Sender<double, kAllShared, 1, true> y_out(ex);
+  const Gather<double, kAllShared> from_x{ex.xs()}, from_y{ex.ys()};
+  const Zero<double> zero;
+  each_own(M.K, [&](const At& at) { y_out.put(at, u0[M.kperm[at.p]]); });
+  double sigma = 0.0, growth = 1.0;
+  bool ok = true, vanished = false;
+  for (int k = 0; k < iterations && ok && !vanished; ++k) {
+    const bool lengths = k == 0 || k == iterations - 1;
+    double v2[1] = {0.0}, u2[1] = {0.0};
+    ok = M.Kt.walk(from_y, zero,
+                   [&](const At& at, double s) {
+                     x_out.put(at, s);
+                     if (lengths) v2[0] += s * s;
+                   },
+                   [&] { return ex.wait(1); });
+    ok = ok && M.K.walk(from_x, zero,
+                        [&](const At& at, double s) {
+                          if (lengths) {
+                            u2[0] += s * s;
+                            S.row(at).set(0, s);
+                          } else {
+                            y_out.put(at, s * growth);
+                          }
+                        },
+                        [&] { return ex.wait(0); });
+    if (lengths) {
+      // (Every CTA comes here: a wait that gave up counts as a length too.)
+      double all[3] = {v2[0], u2[0], ok ? 0.0 : 1.0};
+      cluster_reduce<3>(all, sh, rank, size);
+      ok = all[2] == 0.0;
+      const double vn = sqrt(all[0]), un = sqrt(all[1]);
+      vanished = vn == 0.0 || un == 0.0;
+      if (ok && !vanished) {
+        sigma = un / vn;
+        growth = inverse_power(sigma * sigma);
+        const double start = inverse_power(un);
+        if (k < iterations - 1) {
+          each_own(M.K, [&](const At& at) { y_out.put(at, S.row(at).get(0) * start); });
+        }
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    if (!ok) atomicExch(c.wait_error, 1);
+    if (rank == 0) {
+      ctl->power_sigma = sigma;
+      ctl->power_done = vanished ? 1 : 0;
+    }
+  }
+  cluster_sync(size);
+}
+
 template <typename T, bool HALPERN>
 __global__ void __launch_bounds__(kChunkThreads, 1)
     chunk_kernel(Ctl* ctl, ChunkView<T> c, IterView<T> it) {
@@ -250,41 +362,11 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   const unsigned size = cluster_size();
   cluster_init(sh, size);
   const int n = c.n;
-  load_block(c.K, rank);
-  load_block(c.Kt, rank);
   MatShare<T, TaskShare<T>> M;
-  M.m = c.m;
-  M.n = n;
-  M.kz = M.tz = 0;
-  M.kperm = c.K.perm;
-  M.tperm = c.Kt.perm;
-  M.K = task_share(c.K, c.m, rank, size, c.sums_at);
-  M.Kt = task_share(c.Kt, n, rank, size, c.sums_at);
-  M.nr = M.K.own;
-  M.nc = M.Kt.own;
-  const Second<T> Z{c.second, c.np, c.mp};
   Exchange<T, MODE> ex;
-  ex.sh = &sh;
-  ex.rank = rank;
-  ex.size = size;
-  ex.device = nullptr;
-  ex.xs_at = 0u;
-  ex.ys_at = (c.np + 1) * static_cast<unsigned>(sizeof(T));
-  ex.cmask_at = ex.ys_at + (c.mp + 1) * static_cast<unsigned>(sizeof(T));
-  ex.rmask_at = ex.cmask_at + M.nc * 2;
-  if (threadIdx.x == 0) ex.xs()[c.np] = ex.ys()[c.mp] = T(0);
-  for (int k = threadIdx.x; k < M.nc + M.nr; k += kChunkThreads) ex.cmask()[k] = 0;
-  if (threadIdx.x < 2 * kMaxCluster) (&sh.count[0][0])[threadIdx.x] = 0;
-  __syncthreads();
-  task_masks(M.Kt, c.K.per, ex.cmask(), sh, 0);
-  task_masks(M.K, c.Kt.per, ex.rmask(), sh, 1);
-  settle_counts(ex);
-  const unsigned base = shared_addr(sg_smem);
-  FlatState<T> S;
-  S.cols_at = base + c.cols_at;
-  S.rows_at = base + c.rows_at;
-  S.cols_bytes = M.nc * static_cast<unsigned>(sizeof(T));
-  S.rows_bytes = M.nr * static_cast<unsigned>(sizeof(T));
+  begin_cluster(c, sh, rank, size, &M, &ex);
+  const Second<T> Z{c.second, c.np, c.mp};
+  const FlatState<T> S = flat_state(c, M);
   if (threadIdx.x == 0) {
     ctx.M = M;
     ctx.ex = ex;
@@ -465,6 +547,12 @@ cudaError_t launch_chunk(Ctl* ctl, const ChunkView<T>& c, const IterView<T>& it,
     return launch_clusters(kernel, c.size, 1, kChunkThreads, c.smem, s, ctl, c, it);
   };
   return halpern ? go(chunk_kernel<T, true>) : go(chunk_kernel<T, false>);
+}
+
+cudaError_t launch_chunk_power(Ctl* ctl, const ChunkView<double>& c, const double* u0,
+                               int iterations, cudaStream_t s) {
+  return launch_clusters(chunk_power_kernel, c.size, 1, kChunkThreads, c.smem, s, ctl, c, u0,
+                         iterations);
 }
 
 template bool place_chunk<double>(ChunkView<double>*, const TaskLayout&, const TaskLayout&);

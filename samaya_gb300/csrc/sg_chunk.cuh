@@ -53,4 +53,9 @@ template <typename T>
 cudaError_t launch_chunk(Ctl* ctl, const ChunkView<T>& c, const IterView<T>& it, bool halpern,
                          cudaStream_t s);
 
+// The power iteration of a solve's setup on A_eq (the chunk's values), from u0: sigma into the
+// control block (launch_power_finish takes it).
+cudaError_t launch_chunk_power(Ctl* ctl, const ChunkView<double>& c, const double* u0,
+                               int iterations, cudaStream_t s);
+
 }  // namespace sg

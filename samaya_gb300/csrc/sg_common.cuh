@@ -170,6 +170,13 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// 2^-e for norm = f 2^e, f in [1, 2) (norm zero or not normal: 1).
+__device__ __forceinline__ double inverse_power(double norm) {
+  const int e = (__double2hiint(norm) >> 20) & 0x7ff;
+  if (e == 0 || e >= 0x7fe) return 1.0;
+  return __hiloint2double((0x7fe - e) << 20, 0);
+}
+
 template <typename T>
 __device__ __forceinline__ T ldg(const T* p) {
   return __ldg(p);

@@ -1133,11 +1133,18 @@ int Engine::setup_device(const double* rhs_orig) {
   if (chunk64_.view.size > 0) launch_chunk_values(chunk64_.view, K, Kt, s);
   launch_scale_vectors(n_, m_, cs_, rs_, cost_orig_, lower_orig_, upper_orig_, it64_.cost,
                        it64_.lower, it64_.upper, inv_cs_, inv_rs_, s);
-  if (m_ > 0) {
-    SG_TRY(cudaMemcpyAsync(pu_, u0_, static_cast<size_t>(m_) * sizeof(double),
-                           cudaMemcpyDeviceToDevice, s));
+  constexpr int kPowerIterations = 20;
+  if (chunk64_.view.size > 0) {
+    SG_TRY(launch_chunk_power(ctl_, chunk64_.view, u0_, kPowerIterations, s));
+    launch_power_finish(ctl_, s);
+  } else {
+    if (m_ > 0) {
+      SG_TRY(cudaMemcpyAsync(pu_, u0_, static_cast<size_t>(m_) * sizeof(double),
+                             cudaMemcpyDeviceToDevice, s));
+    }
+    launch_power_iteration(ctl_, K, Kt, pu_, pv_, red, kPowerIterations, grid_setup_k_,
+                           grid_setup_t_, s);
   }
-  launch_power_iteration(ctl_, K, Kt, pu_, pv_, red, 20, grid_setup_k_, grid_setup_t_, s);
   if (opt_.algorithm >= 1) {
     launch_primal_weight_init(ctl_, n_, m_, it64_.cost, it64_.lower, it64_.upper, red, s);
   }

@@ -1669,13 +1669,6 @@ struct StoreSqEpi {
   }
 };
 
-// 2^-e for norm = f 2^e, f in [1, 2) (norm zero or not normal: 1).
-__device__ __forceinline__ double inverse_power(double norm) {
-  const int e = (__double2hiint(norm) >> 20) & 0x7ff;
-  if (e == 0 || e >= 0x7fe) return 1.0;
-  return __hiloint2double((0x7fe - e) << 20, 0);
-}
-
 __global__ void __launch_bounds__(kBlock) power_spmv_kernel(Ctl* c, OpView<double> A,
                                                             const double* x, double* y,
                                                             RedView red, int which) {
@@ -2168,6 +2161,8 @@ void launch_setup_begin(Ctl* ctl, const Ctl& value, int n, int m, double* cs, do
   setup_begin_kernel<<<vec_grid(n + m), kBlock, 0, s>>>(ctl, value, n, m, cs, cn, rs, rn);
 }
 
+void launch_power_finish(Ctl* ctl, cudaStream_t s) { power_finish_kernel<<<1, 32, 0, s>>>(ctl); }
+
 void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt,
                             double* u, double* v, const RedView& red, int iters, int grid_k,
                             int grid_t, cudaStream_t s) {
@@ -2184,7 +2179,7 @@ void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<doub
       }
     }
   }
-  power_finish_kernel<<<1, 32, 0, s>>>(ctl);
+  launch_power_finish(ctl, s);
 }
 
 void launch_init_state(Ctl* ctl, cudaStream_t s) { init_state_kernel<<<1, 32, 0, s>>>(ctl); }

@@ -128,6 +128,8 @@ void launch_scale_vectors(int n, int m, const double* cs, const double* rs, cons
                           cudaStream_t s);
 void launch_setup_begin(Ctl* ctl, const Ctl& value, int n, int m, double* cs, double* cn,
                         double* rs, double* rn, cudaStream_t s);
+// The power iteration and, from its result, the operator norm and the step sizes.
+void launch_power_finish(Ctl* ctl, cudaStream_t s);
 void launch_power_iteration(Ctl* ctl, const OpView<double>& K, const OpView<double>& Kt,
                             double* u, double* v, const RedView& red, int iters, int grid_k,
                             int grid_t, cudaStream_t s);
