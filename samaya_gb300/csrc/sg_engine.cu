@@ -1215,7 +1215,7 @@ int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const Op
     launch_decide(ctl, s);
   }
   launch_restart(ctl, it, s);
-  return kernels + 2 + (detect ? 8 : 1) + 1;
+  return kernels + 1 + (detect ? 8 : 1) + 1;
 }
 
 }  // namespace

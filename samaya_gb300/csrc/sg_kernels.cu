@@ -716,9 +716,12 @@ struct EvalColEpi {
 
 // Stores the grid totals (the split rows' terms are added by grid_reduce).
 struct EvalFin {
-  double* out;
+  Ctl* c;
   __device__ __forceinline__ void operator()(const double (&tot)[kEvalSums]) const {
-    for (int q = 0; q < kEvalSums; ++q) out[q] = tot[q];
+    for (int q = 0; q < kEvalSums; ++q) {
+      c->eval_r[q] = tot[q];
+      c->eval_c[q] = 0.0;
+    }
   }
 };
 
@@ -729,62 +732,64 @@ __device__ __forceinline__ int eval_parity(const Ctl* ctl, int fixed_parity) {
   return static_cast<int>((ctl->t + steps) & 1);
 }
 
+// One launch over both operators: the first grid_t CTAs take the columns (rows of K'), the rest the
+// rows, and one reduction adds them up into eval_r (eval_c 0). (A launch each took 18 and 14 us on
+// a 200 x 500 LP, most of it in the two reductions.)
 template <typename T, int W0>
-__global__ void __launch_bounds__(kBlock) eval_rows_kernel(Ctl* ctl, OpView<T> K, IterView<T> it,
-                                                           EvalView ev, RedView red,
-                                                           int fixed_parity) {
+__global__ void __launch_bounds__(kBlock) eval_kernel(Ctl* ctl, OpView<T> K, OpView<T> Kt,
+                                                      IterView<T> it, EvalView ev, RedView red,
+                                                      int grid_t, int fixed_parity) {
   if (fixed_parity < 0 && ctl->done) return;
   const int cur = eval_parity(ctl, fixed_parity);
-  EvalRowEpi<T, W0> epi;
-  const int n = it.n;
-  epi.vr[0] = it.v(cur) + n;
-  epi.vr[1] = it.Verg + n;
-  epi.y[0] = it.y(cur);
-  epi.y[1] = it.Yerg;
-  epi.vr_rst = it.Vrst + n;
-  epi.y_rst = it.Yrst;
-  epi.ev = ev;
-  epi.n = n;
-  epi.long_terms = red.long_terms;
+  double acc[kEvalSums];
+  const int b = blockIdx.x;
+  if (b < grid_t) {
+    EvalColEpi<T, W0> epi;
+    epi.x[0] = it.v(cur);
+    epi.x[1] = it.Verg;
+    epi.x_rst = it.Vrst;
+    epi.ev = ev;
+    epi.m = it.m;
+    epi.long_terms = red.long_terms + static_cast<size_t>(K.ts.nlong) * kMaxSums;
 #pragma unroll
-  for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0;
-  if constexpr (W0 == 0) {
-    Gather2<T> g{it.v(cur), it.Verg};
-    run_tiles<T, double, 2>(K.ts, K.ptr, K.idx, K.val, g, epi);
-  } else {
-    Gather1<T, double> g{it.Verg};
-    run_tiles<T, double, 1>(K.ts, K.ptr, K.idx, K.val, g, epi);
-  }
-  EvalFin fin{ctl->eval_r};
-  grid_reduce<kEvalSums>(epi.acc, red.partial, red.counter, smem_red(), fin, red.long_terms,
-                         K.ts.nlong);
-}
-
-template <typename T, int W0>
-__global__ void __launch_bounds__(kBlock) eval_cols_kernel(Ctl* ctl, OpView<T> Kt, IterView<T> it,
-                                                           EvalView ev, RedView red,
-                                                           int fixed_parity) {
-  if (fixed_parity < 0 && ctl->done) return;
-  const int cur = eval_parity(ctl, fixed_parity);
-  EvalColEpi<T, W0> epi;
-  epi.x[0] = it.v(cur);
-  epi.x[1] = it.Verg;
-  epi.x_rst = it.Vrst;
-  epi.ev = ev;
-  epi.m = it.m;
-  epi.long_terms = red.long_terms;
+    for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0;
+    if constexpr (W0 == 0) {
+      Gather2<T> g{it.y(cur), it.Yerg};
+      run_tiles<T, double, 2>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi, b, grid_t);
+    } else {
+      Gather1<T, double> g{it.Yerg};
+      run_tiles<T, double, 1>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi, b, grid_t);
+    }
 #pragma unroll
-  for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0;
-  if constexpr (W0 == 0) {
-    Gather2<T> g{it.y(cur), it.Yerg};
-    run_tiles<T, double, 2>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+    for (int q = 0; q < kEvalSums; ++q) acc[q] = epi.acc[q];
   } else {
-    Gather1<T, double> g{it.Yerg};
-    run_tiles<T, double, 1>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+    EvalRowEpi<T, W0> epi;
+    const int n = it.n;
+    epi.vr[0] = it.v(cur) + n;
+    epi.vr[1] = it.Verg + n;
+    epi.y[0] = it.y(cur);
+    epi.y[1] = it.Yerg;
+    epi.vr_rst = it.Vrst + n;
+    epi.y_rst = it.Yrst;
+    epi.ev = ev;
+    epi.n = n;
+    epi.long_terms = red.long_terms;
+#pragma unroll
+    for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0;
+    if constexpr (W0 == 0) {
+      Gather2<T> g{it.v(cur), it.Verg};
+      run_tiles<T, double, 2>(K.ts, K.ptr, K.idx, K.val, g, epi, b - grid_t,
+                              gridDim.x - grid_t);
+    } else {
+      Gather1<T, double> g{it.Verg};
+      run_tiles<T, double, 1>(K.ts, K.ptr, K.idx, K.val, g, epi, b - grid_t,
+                              gridDim.x - grid_t);
+    }
+#pragma unroll
+    for (int q = 0; q < kEvalSums; ++q) acc[q] = epi.acc[q];
   }
-  EvalFin fin{ctl->eval_c};
-  grid_reduce<kEvalSums>(epi.acc, red.partial, red.counter, smem_red(), fin, red.long_terms,
-                         Kt.ts.nlong);
+  grid_reduce<kEvalSums>(acc, red.partial, red.counter, smem_red(), EvalFin{ctl},
+                         red.long_terms, K.ts.nlong + Kt.ts.nlong);
 }
 
 // The same sums for an FP32 operator, which is always an inner problem already in its own
@@ -896,71 +901,65 @@ struct EvalColEpi32 {
 };
 
 template <int W0>
-__global__ void __launch_bounds__(kBlock) eval_rows32_kernel(Ctl* ctl, OpView<float> K,
-                                                             IterView<float> it, RedView red,
-                                                             int fixed_parity) {
+__global__ void __launch_bounds__(kBlock) eval32_kernel(Ctl* ctl, OpView<float> K,
+                                                        OpView<float> Kt, IterView<float> it,
+                                                        RedView red, int grid_t,
+                                                        int fixed_parity) {
   if (fixed_parity < 0 && ctl->done) return;
   const int cur = eval_parity(ctl, fixed_parity);
-  const int n = it.n;
-  EvalRowEpi32<W0> epi;
-  epi.vr[0] = it.v(cur) + n;
-  epi.vr[1] = it.Verg + n;
-  epi.y[0] = it.y(cur);
-  epi.y[1] = it.Yerg;
-  epi.vr_rst = it.Vrst + n;
-  epi.y_rst = it.Yrst;
-  epi.c = it.cost + n;
-  epi.l = it.lower + n;
-  epi.u = it.upper + n;
-  epi.q = it.rhs;
-  epi.long_terms = red.long_terms;
-#pragma unroll
-  for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0f;
-  if constexpr (W0 == 0) {
-    Gather2f g{it.v(cur), it.Verg};
-    run_tiles<float, float, 2>(K.ts, K.ptr, K.idx, K.val, g, epi);
-  } else {
-    Gather1<float, float> g{it.Verg};
-    run_tiles<float, float, 1>(K.ts, K.ptr, K.idx, K.val, g, epi);
-  }
   double acc[kEvalSums];
+  const int b = blockIdx.x;
+  if (b < grid_t) {
+    EvalColEpi32<W0> epi;
+    epi.x[0] = it.v(cur);
+    epi.x[1] = it.Verg;
+    epi.x_rst = it.Vrst;
+    epi.c = it.cost;
+    epi.l = it.lower;
+    epi.u = it.upper;
+    epi.m = it.m;
+    epi.long_terms = red.long_terms + static_cast<size_t>(K.ts.nlong) * kMaxSums;
 #pragma unroll
-  for (int q = 0; q < kEvalSums; ++q) acc[q] = epi.acc[q];
-  EvalFin fin{ctl->eval_r};
-  grid_reduce<kEvalSums>(acc, red.partial, red.counter, smem_red(), fin, red.long_terms,
-                         K.ts.nlong);
-}
-
-template <int W0>
-__global__ void __launch_bounds__(kBlock) eval_cols32_kernel(Ctl* ctl, OpView<float> Kt,
-                                                             IterView<float> it, RedView red,
-                                                             int fixed_parity) {
-  if (fixed_parity < 0 && ctl->done) return;
-  const int cur = eval_parity(ctl, fixed_parity);
-  EvalColEpi32<W0> epi;
-  epi.x[0] = it.v(cur);
-  epi.x[1] = it.Verg;
-  epi.x_rst = it.Vrst;
-  epi.c = it.cost;
-  epi.l = it.lower;
-  epi.u = it.upper;
-  epi.m = it.m;
-  epi.long_terms = red.long_terms;
+    for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0f;
+    if constexpr (W0 == 0) {
+      Gather2f g{it.y(cur), it.Yerg};
+      run_tiles<float, float, 2>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi, b, grid_t);
+    } else {
+      Gather1<float, float> g{it.Yerg};
+      run_tiles<float, float, 1>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi, b, grid_t);
+    }
 #pragma unroll
-  for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0f;
-  if constexpr (W0 == 0) {
-    Gather2f g{it.y(cur), it.Yerg};
-    run_tiles<float, float, 2>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
+    for (int q = 0; q < kEvalSums; ++q) acc[q] = epi.acc[q];
   } else {
-    Gather1<float, float> g{it.Yerg};
-    run_tiles<float, float, 1>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, g, epi);
-  }
-  double acc[kEvalSums];
+    const int n = it.n;
+    EvalRowEpi32<W0> epi;
+    epi.vr[0] = it.v(cur) + n;
+    epi.vr[1] = it.Verg + n;
+    epi.y[0] = it.y(cur);
+    epi.y[1] = it.Yerg;
+    epi.vr_rst = it.Vrst + n;
+    epi.y_rst = it.Yrst;
+    epi.c = it.cost + n;
+    epi.l = it.lower + n;
+    epi.u = it.upper + n;
+    epi.q = it.rhs;
+    epi.long_terms = red.long_terms;
 #pragma unroll
-  for (int q = 0; q < kEvalSums; ++q) acc[q] = epi.acc[q];
-  EvalFin fin{ctl->eval_c};
-  grid_reduce<kEvalSums>(acc, red.partial, red.counter, smem_red(), fin, red.long_terms,
-                         Kt.ts.nlong);
+    for (int q = 0; q < kEvalSums; ++q) epi.acc[q] = 0.0f;
+    if constexpr (W0 == 0) {
+      Gather2f g{it.v(cur), it.Verg};
+      run_tiles<float, float, 2>(K.ts, K.ptr, K.idx, K.val, g, epi, b - grid_t,
+                                 gridDim.x - grid_t);
+    } else {
+      Gather1<float, float> g{it.Verg};
+      run_tiles<float, float, 1>(K.ts, K.ptr, K.idx, K.val, g, epi, b - grid_t,
+                                 gridDim.x - grid_t);
+    }
+#pragma unroll
+    for (int q = 0; q < kEvalSums; ++q) acc[q] = epi.acc[q];
+  }
+  grid_reduce<kEvalSums>(acc, red.partial, red.counter, smem_red(), EvalFin{ctl},
+                         red.long_terms, K.ts.nlong + Kt.ts.nlong);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1459,10 +1458,10 @@ __global__ void __launch_bounds__(kBlock) det_ray_rows_kernel(Ctl* c, OpView<T> 
 // Setup on the device (pdlp.cpp:36-187, 289-299, 377-394, 490-492), FP64.
 
 struct MaxNormEpi {
-  double acc[1];
-  __device__ __forceinline__ void row(int, const double (&s)[1]) { acc[0] = fmax(acc[0], sqrt(s[0])); }
+  double most;
+  __device__ __forceinline__ void row(int, const double (&s)[1]) { most = fmax(most, sqrt(s[0])); }
   __device__ __forceinline__ void long_row(int, int, const double (&s)[1]) {
-    acc[0] = fmax(acc[0], sqrt(s[0]));
+    most = fmax(most, sqrt(s[0]));
   }
 };
 
@@ -1470,13 +1469,24 @@ struct SqProd {
   __device__ __forceinline__ double operator()(int, double a, int) const { return a * a; }
 };
 
-__global__ void __launch_bounds__(kBlock) max_norm_kernel(OpView<double> A, RedView red,
-                                                          double* out) {
-  MaxNormEpi epi;
-  epi.acc[0] = 0.0;
-  run_tiles<double, double, 1>(A.ts, A.ptr, A.idx, A.val, SqProd{}, epi);
-  grid_reduce<1, 1u>(epi.acc, red.partial, red.counter, smem_red(),
-                     [out](const double (&t)[1]) { *out = t[0]; });
+// The largest column norm (rows of K', the first grid_t CTAs) and the largest row norm.
+__global__ void __launch_bounds__(kBlock) max_norm_kernel(Ctl* c, OpView<double> K,
+                                                          OpView<double> Kt, RedView red,
+                                                          int grid_t) {
+  MaxNormEpi epi{0.0};
+  const int b = blockIdx.x;
+  const bool cols = b < grid_t;
+  if (cols) {
+    run_tiles<double, double, 1>(Kt.ts, Kt.ptr, Kt.idx, Kt.val, SqProd{}, epi, b, grid_t);
+  } else {
+    run_tiles<double, double, 1>(K.ts, K.ptr, K.idx, K.val, SqProd{}, epi, b - grid_t,
+                                 gridDim.x - grid_t);
+  }
+  double most[2] = {cols ? epi.most : 0.0, cols ? 0.0 : epi.most};
+  grid_reduce<2, 3u>(most, red.partial, red.counter, smem_red(), [c](const double (&t)[2]) {
+    c->a_norm_max_col = t[0];
+    c->at_norm_max_row = t[1];
+  });
 }
 
 __global__ void __launch_bounds__(kBlock) sum_sq_kernel(const double* x, int len, RedView red,
@@ -1855,14 +1865,6 @@ void configure_kernels() {
   // Opt in to large dynamic shared memory; the launch sizes themselves follow each operator's
   // tile capacity, so occupancy is set by the actual size.
   const int big = 200 * 1024;
-  cudaFuncSetAttribute(eval_rows_kernel<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_rows_kernel<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_cols_kernel<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_cols_kernel<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_rows_kernel<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_rows_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_cols_kernel<float, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(eval_cols_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(det_ray_rows_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(det_ray_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(dual_step_kernel<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -1976,25 +1978,21 @@ template <typename T>
 void launch_eval(Ctl* ctl, const OpView<T>& K, const OpView<T>& Kt, const IterView<T>& it,
                  const EvalView& ev, const RedView& red, int grid_k, int grid_t,
                  int fixed_parity, cudaStream_t s, bool second_only) {
-  const size_t smk = tile_smem_bytes(K.ts, 2, 8);
-  const size_t smt = tile_smem_bytes(Kt.ts, 2, 8);
+  const size_t sm = tile_smem_bytes(K.ts, 2, 8);
+  const int grid = grid_t + grid_k;
   if constexpr (std::is_same<T, float>::value) {
     // FP32 operators carry their own (equilibrated) data: `ev` is not used.
     (void)ev;
     if (second_only) {
-      eval_rows32_kernel<1><<<grid_k, kBlock, smk, s>>>(ctl, K, it, red, fixed_parity);
-      eval_cols32_kernel<1><<<grid_t, kBlock, smt, s>>>(ctl, Kt, it, red, fixed_parity);
+      eval32_kernel<1><<<grid, kBlock, sm, s>>>(ctl, K, Kt, it, red, grid_t, fixed_parity);
     } else {
-      eval_rows32_kernel<0><<<grid_k, kBlock, smk, s>>>(ctl, K, it, red, fixed_parity);
-      eval_cols32_kernel<0><<<grid_t, kBlock, smt, s>>>(ctl, Kt, it, red, fixed_parity);
+      eval32_kernel<0><<<grid, kBlock, sm, s>>>(ctl, K, Kt, it, red, grid_t, fixed_parity);
     }
   } else {
     if (second_only) {
-      eval_rows_kernel<T, 1><<<grid_k, kBlock, smk, s>>>(ctl, K, it, ev, red, fixed_parity);
-      eval_cols_kernel<T, 1><<<grid_t, kBlock, smt, s>>>(ctl, Kt, it, ev, red, fixed_parity);
+      eval_kernel<T, 1><<<grid, kBlock, sm, s>>>(ctl, K, Kt, it, ev, red, grid_t, fixed_parity);
     } else {
-      eval_rows_kernel<T, 0><<<grid_k, kBlock, smk, s>>>(ctl, K, it, ev, red, fixed_parity);
-      eval_cols_kernel<T, 0><<<grid_t, kBlock, smt, s>>>(ctl, Kt, it, ev, red, fixed_parity);
+      eval_kernel<T, 0><<<grid, kBlock, sm, s>>>(ctl, K, Kt, it, ev, red, grid_t, fixed_parity);
     }
   }
 }
@@ -2037,14 +2035,8 @@ void launch_setup_norms(Ctl* ctl, const OpView<double>& K, const OpView<double>&
                         const double* cost, const RedView& red, int grid_k, int grid_t,
                         cudaStream_t s) {
   if (K.rows > 0) {
-    if (Kt.ts.ntiles > 0) {
-      max_norm_kernel<<<grid_t, kBlock, tile_smem_bytes(Kt.ts, 1, 8), s>>>(Kt, red,
-                                                                         &ctl->a_norm_max_col);
-    }
-    if (K.ts.ntiles > 0) {
-      max_norm_kernel<<<grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(K, red,
-                                                                        &ctl->at_norm_max_row);
-    }
+    max_norm_kernel<<<grid_t + grid_k, kBlock, tile_smem_bytes(K.ts, 1, 8), s>>>(ctl, K, Kt, red,
+                                                                                 grid_t);
   }
   const int nt = K.rows + Kt.rows;
   sum_sq_kernel<<<vec_grid(nt) < 1024 ? vec_grid(nt) : 1024, kBlock, 0, s>>>(cost, nt, red,
