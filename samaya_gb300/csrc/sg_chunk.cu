@@ -40,9 +40,17 @@ struct alignas(16) TaskShare {
   // sums of rows on several lanes, a shuffle tree's, go to shared memory, and a thread per row runs
   // f after them. (With a lane per row everywhere, as walk_one has it, an LP of 200 x 500 left 12
   // of 16 warps idle, and one warp's 20 nonzeros took 3,500 of an iteration's 7,800 clocks.)
-  template <typename Prod, typename Init, typename F, typename Ready>
+  // MAXRED: the maximum of the products, none negative (FP64: their bits compare as integers).
+  template <bool MAXRED = false, typename Prod, typename Init, typename F, typename Ready>
   __device__ __forceinline__ bool walk(const Prod& prod, const Init& init, const F& f,
                                        const Ready& ready) const {
+    auto join = [](T p, T q) {
+      if constexpr (MAXRED) {
+        return __double_as_longlong(p) > __double_as_longlong(q) ? p : q;
+      } else {
+        return p + q;
+      }
+    };
     // B steps' elements loaded while the B before are summed (of the same task or the warp's task
     // before).
     constexpr int B = sizeof(T) == 8 ? 4 : 8;
@@ -83,13 +91,13 @@ struct alignas(16) TaskShare {
         if (left >= B) {
           if constexpr (sizeof(T) == 8) keep_branch(0xffffffffu);
 #pragma unroll
-          for (int u = 0; u < B; ++u) s = s + prod(ca[u], static_cast<int>(cj[u]));
+          for (int u = 0; u < B; ++u) s = join(s, prod(ca[u], static_cast<int>(cj[u])));
         } else {
 #pragma unroll
           for (int u = 0; u < B - 1; ++u) {
             if (u < left) {
               if constexpr (sizeof(T) == 8) keep_branch(0xffffffffu);
-              s = s + prod(ca[u], static_cast<int>(cj[u]));
+              s = join(s, prod(ca[u], static_cast<int>(cj[u])));
             }
           }
         }
@@ -100,11 +108,11 @@ struct alignas(16) TaskShare {
         if (lane < (d.w & 255)) {
           const int l = d.z + lane;
           const At at{l, 0, l, first + l};
-          f(at, init(at) + s);
+          f(at, join(init(at), s));
         }
       } else {
         for (int o = (1 << lanes) >> 1; o > 0; o >>= 1) {
-          s = s + __shfl_xor_sync(0xffffffffu, s, o);
+          s = join(s, __shfl_xor_sync(0xffffffffu, s, o));
         }
         const int r = lane >> lanes;
         if ((lane & ((1 << lanes) - 1)) == 0 && r < (d.w & 255)) {
@@ -121,7 +129,7 @@ struct alignas(16) TaskShare {
       const int l = sum ? k : k - shared_rows + filled;
       const At at{l, 0, l, first + l};
       T s = init(at);
-      if (sum) s = s + sh_load(sums_at + l * static_cast<int>(sizeof(T)), T());
+      if (sum) s = join(s, sh_load(sums_at + l * static_cast<int>(sizeof(T)), T()));
       f(at, s);
     }
     return true;
@@ -276,6 +284,84 @@ __device__ __forceinline__ FlatState<T> flat_state(const ChunkView<T>& c,
   return FlatState<T>{base + c.cols_at, base + c.rows_at,
                       M.nc * static_cast<unsigned>(sizeof(T)),
                       M.nr * static_cast<unsigned>(sizeof(T))};
+}
+
+// The scaling passes of the setup (sg_kernels.cu: ruiz_pass_kernel, abs_pass_kernel) from the given
+// values: the scales are the gathered vectors, xs the columns', ys the rows'. Both statistics are
+// taken with the old scales; a cluster barrier, then every new scale is sent. Bound by latency;
+// 10 or 11 launches took 0.1 ms of a small LP's solve, one takes 0.03.
+template <bool RUIZ>
+__global__ void __launch_bounds__(kChunkThreads, 1)
+    chunk_scale_kernel(ChunkView<double> c, double* cs, double* rs) {
+  __shared__ ClusterShared sh;
+  const unsigned rank = cluster_rank();
+  const unsigned size = cluster_size();
+  cluster_init(sh, size);
+  MatShare<double, TaskShare<double>> M;
+  Exchange<double, kAllShared> ex;
+  begin_cluster(c, sh, rank, size, &M, &ex);
+  const FlatState<double> S = flat_state(c, M);
+  const Sender<double, kAllShared, 0, true> x_out(ex);
+  const Sender<double, kAllShared, 1, true> y_out(ex);
+  const Array<double, true> x(ex.xs()), y(ex.ys());
+  const Zero<double> zero;
+  for (int p = threadIdx.x; p < c.np; p += kChunkThreads) x.set(p, 1.0);
+  for (int p = threadIdx.x; p < c.mp; p += kChunkThreads) y.set(p, 1.0);
+  cluster_sync(size);
+  auto cols = [&](const At& at, double s) { S.col(at).set(0, s); };
+  auto rows = [&](const At& at, double s) { S.row(at).set(0, s); };
+  bool ok = true;
+  constexpr int kPasses = RUIZ ? 10 : 11;
+  // (A wait that gave up ends the passes for all CTAs together or not at all: no CTA may leave
+  // while others still send to it.)
+  for (int pass = 0; pass < kPasses; ++pass) {
+    double moved[1] = {0.0};
+    if constexpr (RUIZ) {
+      auto by_y = [&](double a, int j) { return (a * y.get(j)) * (a * y.get(j)); };
+      auto by_x = [&](double a, int j) { return (a * x.get(j)) * (a * x.get(j)); };
+      M.Kt.walk(by_y, zero, cols, Ready());
+      __syncthreads();
+      M.K.walk(by_x, zero, rows, Ready());
+    } else {
+      auto by_y = [&](double a, int j) { return fabs(a) * y.get(j); };
+      auto by_x = [&](double a, int j) { return fabs(a) * x.get(j); };
+      if (pass < 10) {
+        M.Kt.walk<true>(by_y, zero, cols, Ready());
+        __syncthreads();
+        M.K.walk<true>(by_x, zero, rows, Ready());
+      } else {
+        M.Kt.walk(by_y, zero, cols, Ready());
+        __syncthreads();
+        M.K.walk(by_x, zero, rows, Ready());
+      }
+    }
+    cluster_sync(size);
+    auto next = [&](double old, double stat) {
+      if constexpr (RUIZ) {
+        const double nv = sqrt(stat) * old;
+        const double s = nv > 0 ? fmax(1e-8, fmin(1e8, old / nv)) : old;
+        if (fabs(s - old) / fmax(fabs(old), 1.0) > 0.1) moved[0] = 1.0;
+        return s;
+      } else {
+        const double by = stat * old;
+        return by > 0.0 ? old * rsqrt(by) : old;
+      }
+    };
+    each_own(M.Kt, [&](const At& at) { x_out.put(at, next(x.get(at.p), S.col(at).get(0))); });
+    each_own(M.K, [&](const At& at) { y_out.put(at, next(y.get(at.p), S.row(at).get(0))); });
+    ok = ex.wait(0) && ok;
+    ok = ex.wait(1) && ok;
+    if constexpr (RUIZ) {
+      double all[2] = {moved[0], ok ? 0.0 : 1.0};
+      cluster_reduce<2, 3u>(all, sh, rank, size);
+      ok = all[1] == 0.0;
+      if (all[0] == 0.0 || !ok) break;
+    }
+  }
+  each_own(M.Kt, [&](const At& at) { cs[M.tperm[at.p]] = x.get(at.p); });
+  each_own(M.K, [&](const At& at) { rs[M.kperm[at.p]] = y.get(at.p); });
+  if (threadIdx.x == 0 && !ok) atomicExch(c.wait_error, 1);
+  cluster_sync(size);
 }
 
 // The power iteration of the setup (pdlp.cpp:36-103; power_spmv_kernel's products): 20 times
@@ -553,6 +639,16 @@ cudaError_t launch_chunk_power(Ctl* ctl, const ChunkView<double>& c, const doubl
                                int iterations, cudaStream_t s) {
   return launch_clusters(chunk_power_kernel, c.size, 1, kChunkThreads, c.smem, s, ctl, c, u0,
                          iterations);
+}
+
+cudaError_t launch_chunk_scale(const ChunkView<double>& c, const double* k_given,
+                               const double* t_given, bool ruiz, double* cs, double* rs,
+                               cudaStream_t s) {
+  ChunkView<double> g = c;
+  g.K.val = const_cast<double*>(k_given);
+  g.Kt.val = const_cast<double*>(t_given);
+  return launch_clusters(ruiz ? chunk_scale_kernel<true> : chunk_scale_kernel<false>, c.size, 1,
+                         kChunkThreads, c.smem, s, g, cs, rs);
 }
 
 template bool place_chunk<double>(ChunkView<double>*, const TaskLayout&, const TaskLayout&);

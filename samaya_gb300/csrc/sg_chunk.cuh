@@ -53,6 +53,11 @@ template <typename T>
 cudaError_t launch_chunk(Ctl* ctl, const ChunkView<T>& c, const IterView<T>& it, bool halpern,
                          cudaStream_t s);
 
+// The scaling passes of a solve's setup (the reference's Ruiz, or the enhanced ones) from the given
+// values in the chunk's layout.
+cudaError_t launch_chunk_scale(const ChunkView<double>& c, const double* k_given,
+                               const double* t_given, bool ruiz, double* cs, double* rs,
+                               cudaStream_t s);
 // The power iteration of a solve's setup on A_eq (the chunk's values), from u0: sigma into the
 // control block (launch_power_finish takes it).
 cudaError_t launch_chunk_power(Ctl* ctl, const ChunkView<double>& c, const double* u0,

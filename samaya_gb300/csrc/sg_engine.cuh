@@ -171,6 +171,7 @@ struct DevChunk {
     Task* task;
     unsigned short* idx;
     T* val;
+    T* given;  // FP64: the values before scaling
   } op[2] = {};
   T* second = nullptr;
   ChunkView<T> view{};

@@ -1636,24 +1636,30 @@ __device__ __forceinline__ double bound_over(double b, double scale) {
   return b;
 }
 
-// The equilibrated cost and bounds, and the scales' reciprocals.
+// The equilibrated cost and bounds, the evaluation's copies of the given ones, and the scales'
+// reciprocals.
 __global__ void scale_vectors_kernel(int n, int m, const double* cs, const double* rs,
                                      const double* cost, const double* lower, const double* upper,
                                      double* cost_eq, double* lower_eq, double* upper_eq,
+                                     double* cost_ev, double* lower_ev, double* upper_ev,
                                      double* inv_cs, double* inv_rs) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n + m; k += gridDim.x * blockDim.x) {
+    const double c0 = cost[k], lo = lower[k], up = upper[k];
+    cost_ev[k] = c0;
+    lower_ev[k] = lo;
+    upper_ev[k] = up;
     if (k < n) {
       const double c = cs[k];
       inv_cs[k] = 1.0 / c;
-      cost_eq[k] = cost[k] * c;
-      lower_eq[k] = bound_over(lower[k], c);
-      upper_eq[k] = bound_over(upper[k], c);
+      cost_eq[k] = c0 * c;
+      lower_eq[k] = bound_over(lo, c);
+      upper_eq[k] = bound_over(up, c);
     } else {
       const double r = rs[k - n];
       inv_rs[k - n] = 1.0 / r;
-      cost_eq[k] = cost[k] * r;
-      lower_eq[k] = lower[k] * r;
-      upper_eq[k] = upper[k] * r;
+      cost_eq[k] = c0 * r;
+      lower_eq[k] = lo * r;
+      upper_eq[k] = up * r;
     }
   }
 }
@@ -2128,11 +2134,12 @@ void launch_apply_scaling(const OpView<double>& K, const OpView<double>& Kt,
 
 void launch_scale_vectors(int n, int m, const double* cs, const double* rs, const double* cost,
                           const double* lower, const double* upper, double* cost_eq,
-                          double* lower_eq, double* upper_eq, double* inv_cs, double* inv_rs,
+                          double* lower_eq, double* upper_eq, double* cost_ev,
+                          double* lower_ev, double* upper_ev, double* inv_cs, double* inv_rs,
                           cudaStream_t s) {
-  scale_vectors_kernel<<<vec_grid(n + m), kBlock, 0, s>>>(n, m, cs, rs, cost, lower, upper,
-                                                          cost_eq, lower_eq, upper_eq, inv_cs,
-                                                          inv_rs);
+  scale_vectors_kernel<<<vec_grid(n + m), kBlock, 0, s>>>(
+      n, m, cs, rs, cost, lower, upper, cost_eq, lower_eq, upper_eq, cost_ev, lower_ev, upper_ev,
+      inv_cs, inv_rs);
 }
 
 // The start of a solve's setup: the control block, and both scale buffers at 1.

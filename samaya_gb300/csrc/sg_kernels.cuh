@@ -124,7 +124,8 @@ void launch_apply_scaling(const OpView<double>& K, const OpView<double>& Kt,
                           const double* cs, long long nnz, cudaStream_t s);
 void launch_scale_vectors(int n, int m, const double* cs, const double* rs, const double* cost,
                           const double* lower, const double* upper, double* cost_eq,
-                          double* lower_eq, double* upper_eq, double* inv_cs, double* inv_rs,
+                          double* lower_eq, double* upper_eq, double* cost_ev,
+                          double* lower_ev, double* upper_ev, double* inv_cs, double* inv_rs,
                           cudaStream_t s);
 void launch_setup_begin(Ctl* ctl, const Ctl& value, int n, int m, double* cs, double* cn,
                         double* rs, double* rn, cudaStream_t s);
