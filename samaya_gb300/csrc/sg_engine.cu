@@ -587,10 +587,10 @@ int Engine::set_tiles(DevOp* op, const TileShape& shape) {
   return kOk;
 }
 
-// Average device milliseconds of one step kernel (the dual step on K, or the primal step on
-// K'), in the precision of the solve, over `reps` launches after two warm-up launches. The
-// control block is set to run (it is re-initialised by every solve's setup).
-double Engine::time_step_kernel(bool dual, int reps) {
+// Average device milliseconds of an iteration's two step kernels, in the precision of the solve,
+// over `reps` iterations after two. The control block is set to run (it is re-initialised by every
+// solve's setup).
+double Engine::time_steps_in_turn(int reps) {
   Ctl* c = fp32_ ? ctl32_ : ctl_;
   Ctl h;
   memset(&h, 0, sizeof(h));
@@ -604,43 +604,31 @@ double Engine::time_step_kernel(bool dual, int reps) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  // The step kernels the solves run (classic or Halpern).
+  // The step kernels the solves run (classic or Halpern), in their order: a shape that is the best
+  // for its kernel alone need not be behind the other one.
   const bool halpern = opt_.algorithm == 2;
-  auto launch = [&](int j) {
-    const int gk = std::max(1, std::min(K_.step_tiles(), 65535));
-    const int gt = std::max(1, std::min(Kt_.ntiles, 65535));
-    if (fp32_) {
-      IterView<float> it = iter_view(it32_);
-      if (dual) {
-        if (halpern) {
-          launch_halpern_dual(c, K_.step32(), it, j, gk, stream_);
-        } else {
-          launch_dual_step(c, K_.step32(), it, j, gk, stream_);
-        }
-      } else if (halpern) {
-        launch_halpern_primal(c, Kt_.view32(), it, j, gt, stream_);
-      } else {
-        launch_primal_step(c, Kt_.view32(), it, j, gt, stream_);
-      }
+  const int gk = std::max(1, std::min(K_.step_tiles(), 65535));
+  const int gt = std::max(1, std::min(Kt_.ntiles, 65535));
+  auto pair = [&](const auto& K, const auto& Kt, const auto& it, int j) {
+    if (halpern) {
+      launch_halpern_primal(c, Kt, it, j, gt, stream_, j > 0);
+      launch_halpern_dual(c, K, it, j, gk, stream_, true);
     } else {
-      IterView<double> it = iter_view(it64_);
-      if (dual) {
-        if (halpern) {
-          launch_halpern_dual(c, K_.step64(), it, j, gk, stream_);
-        } else {
-          launch_dual_step(c, K_.step64(), it, j, gk, stream_);
-        }
-      } else if (halpern) {
-        launch_halpern_primal(c, Kt_.view64(), it, j, gt, stream_);
-      } else {
-        launch_primal_step(c, Kt_.view64(), it, j, gt, stream_);
-      }
+      launch_dual_step(c, K, it, j, gk, stream_, j > 0);
+      launch_primal_step(c, Kt, it, j, gt, stream_, true);
+    }
+  };
+  auto launch = [&](int j) {
+    if (fp32_) {
+      pair(K_.step32(), Kt_.view32(), iter_view(it32_), j);
+    } else {
+      pair(K_.step64(), Kt_.view64(), iter_view(it64_), j);
     }
   };
   launch(0);
   launch(1);
   cudaEventRecord(e0, stream_);
-  for (int r = 0; r < reps; ++r) launch(r & 1);
+  for (int r = 0; r < reps; ++r) launch(2 + r);
   cudaEventRecord(e1, stream_);
   float ms = -1.0f;
   if (cudaEventSynchronize(e1) == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
@@ -657,10 +645,17 @@ double Engine::time_step_kernel(bool dual, int reps) {
 // split of the medium rows); the fastest (by a margin over the built-in shape) is kept and
 // cached under the statistics.
 int Engine::tune_tiles(std::string* err) {
+  // Both operators have tiles while either is timed.
+  for (DevOp* op : {&K_, &Kt_}) {
+    if (set_tiles(op, default_shape(*op)) != kOk) {
+      if (err) *err = "tile upload failed";
+      return kErrCuda;
+    }
+  }
   for (int which = 0; which < 2; ++which) {
     DevOp* op = which == 0 ? &K_ : &Kt_;
     const TileShape base = default_shape(*op);
-    TileShape best = base;
+    TileShape best = base, in_place = base;
     // (Two nonzeros a column: the primal steps take no tiles, two_nonzero_columns.)
     const bool tune = opt_.autotune && op->nnz >= (1LL << 18) &&
                       !(which == 1 && op->uniform_len == 2);
@@ -692,8 +687,10 @@ int Engine::tune_tiles(std::string* err) {
         if (med / 2 > base.warp_min) splits.push_back(med / 2);
       }
       // Candidates: the built-in shape first, then (split, capacity, variant). A candidate
-      // replaces the best so far only when it is at least kTuneMargin faster (the best of
-      // three timed rounds each), so launch-to-launch noise keeps the built-in shape.
+      // replaces the best so far only when an iteration (both steps, in turn: time_steps_in_turn)
+      // is at least kTuneMargin faster (the best of three timed rounds each), so launch-to-launch
+      // noise keeps the built-in shape. (Timed alone, over and over, a dual step of the 301 x 703
+      // transportation LP gave shapes with which 256 iterations took 4.6 to 5.4 ms; so 4.2.)
       std::vector<TileShape> cands{base};
       for (int split : splits) {
         for (int ci = 0; ci < 4; ++ci) {
@@ -724,10 +721,8 @@ int Engine::tune_tiles(std::string* err) {
       }
       // Candidates that differ from the tiles in place only in the kernel variant reuse them
       // (the partition does not depend on the variant).
-      bool built = false;
-      TileShape in_place;
       for (const TileShape& sh : cands) {
-        if (built && sh.cap_nnz == in_place.cap_nnz && sh.cap_rows == in_place.cap_rows &&
+        if (sh.cap_nnz == in_place.cap_nnz && sh.cap_rows == in_place.cap_rows &&
             sh.warp_min == in_place.warp_min && sh.split == in_place.split &&
             sh.groups == in_place.groups && sh.staged == in_place.staged) {
           op->variant = sh.variant;
@@ -737,12 +732,11 @@ int Engine::tune_tiles(std::string* err) {
             if (err) *err = "autotune: tile upload failed";
             return rc;
           }
-          built = true;
-          in_place = sh;
         }
+        in_place = sh;
         double ms = -1.0;
         for (int round = 0; round < 3; ++round) {
-          const double t = time_step_kernel(which == 0, 8);
+          const double t = time_steps_in_turn(4);
           if (t < 0) {
             if (err) *err = std::string("autotune: ") + cudaGetErrorString(cudaGetLastError());
             return kErrCuda;
@@ -758,10 +752,12 @@ int Engine::tune_tiles(std::string* err) {
       g_shape_cache[key] = best;
       append_shape_file(key, best);
     }
-    const int rc = set_tiles(op, best);
-    if (rc != kOk) {
-      if (err) *err = "tile upload failed";
-      return rc;
+    if (!(best == in_place)) {
+      const int rc = set_tiles(op, best);
+      if (rc != kOk) {
+        if (err) *err = "tile upload failed";
+        return rc;
+      }
     }
   }
   dfree(long_terms_);

@@ -57,6 +57,10 @@ struct TileShape {
   int split = 0;            // kind-2 rows: nonzeros per warp of a team (0: a warp per row)
   int groups = 0;           // dual steps: runs of gather-neighbour rows as kind-3 row groups
   int staged = 0;           // dual steps: kind-1 segments streamed through shared memory
+  bool operator==(const TileShape& o) const {
+    return cap_nnz == o.cap_nnz && cap_rows == o.cap_rows && warp_min == o.warp_min &&
+           variant == o.variant && split == o.split && groups == o.groups && staged == o.staged;
+  }
 };
 
 struct SolveInfo {
@@ -316,7 +320,7 @@ class Engine {
   int seam_grid_k() const { return seam_step_set() ? grid_step_k_ : grid_full_k_; }
   int find_neighbours(std::string* err);
   int tune_tiles(std::string* err);
-  double time_step_kernel(bool dual, int reps);
+  double time_steps_in_turn(int reps);
 
   int m_ = 0, n_ = 0;
   long long nnz_ = 0;
