@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
         return s;
       } else {
         const double by = stat * old;
-        return by > 0.0 ? old * rsqrt(by) : old;
+        return by > 0.0 ? old / sqrt(by) : old;
       }
     };
     each_own(M.Kt, [&](const At& at) { x_out.put(at, next(x.get(at.p), S.col(at).get(0))); });

@@ -63,3 +63,32 @@ def test_setup_passes(engine, oracle, name):
             r = s.solve()
             one = oracle.pdlp_solve(*lp.arrays(), tol=1e-30, max_iter=1)
             assert _differs(r.x, one.x) <= 1e-9 and _differs(r.y, one.y) <= 1e-9
+
+
+@pytest.mark.parametrize("supplies, demands", [(7, 9), (60, 81), (200, 301)])
+def test_enhanced_scales_of_a_transportation_lp_to_the_bit(engine, supplies, demands):
+    """One cluster's passes and the tile kernels'. Every nonzero is 1 and a column holds two, so
+    the ten maximum passes are the same IEEE products, roots and quotients in any order; the rows'
+    sums of the last pass take up to `demands` terms in another order: with the three operations
+    after them (demands + 3) * 2^-53."""
+    n, m = supplies * demands, supplies + demands
+    rowidx = np.empty((n, 2), dtype=np.int32)
+    rowidx[:, 0] = np.repeat(np.arange(supplies), demands)
+    rowidx[:, 1] = supplies + np.tile(np.arange(demands), supplies)
+    lp = engine.LpProblem(
+        m=m, n=n, colptr=np.arange(0, 2 * n + 1, 2, dtype=np.int64), rowidx=rowidx.reshape(-1),
+        vals=np.ones(2 * n), cost=np.concatenate([np.arange(n) % 7 + 1.0, np.zeros(m)]),
+        lower=np.concatenate([np.zeros(n), np.ones(m)]),
+        upper=np.concatenate([np.full(n, np.inf), np.ones(m)]))
+    s = engine.PdlpSolver(lp, engine.PdlpOptions(
+        tol=1e-30, max_iterations=1, algorithm=engine.ENHANCED, autotune=False))
+    got = s.equilibration()
+    cs, rs = np.ones(lp.n), np.ones(lp.m)
+    cols, rows = np.repeat(np.arange(lp.n), np.diff(lp.colptr)), lp.rowidx
+    for k in range(11):
+        cn, rn = np.zeros(lp.n), np.zeros(lp.m)
+        (np.maximum if k < 10 else np.add).at(cn, cols, rs[rows])
+        (np.maximum if k < 10 else np.add).at(rn, rows, cs[cols])
+        cs, rs = cs / np.sqrt(cn * cs), rs / np.sqrt(rn * rs)
+    assert np.array_equal(got[0], cs)
+    assert np.all(np.abs(got[1] - rs) <= (demands + 3) * 2.0 ** -53 * rs)
