@@ -111,6 +111,7 @@ struct InstanceList {
 struct ClusterPlan {
   int size = 0;
   int clusters = 1;
+  int sms = 0;  // SMs of the device
   int threads = 256;
   InstanceList group[kModes];
   size_t smem[kModes] = {0, 0, 0};

@@ -447,6 +447,7 @@ int Batch::make_plan(Kind kind, ClusterPlan* plan) {
   }
   const int best = plan->size;
   plan->clusters = std::max(1, per_sm * sms_ / best);
+  plan->sms = sms_;
   plan->threads = fp32 ? kThreads32 : kThreads64;
   if (setup) {
     // One launch for all matrices; a matrix whose vectors do not fit leaves them in device

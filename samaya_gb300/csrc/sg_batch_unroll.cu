@@ -394,9 +394,9 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
 
 }  // namespace
 
-template <bool ADJOINT, int MODE>
-__global__ void __launch_bounds__(kThreads64, 2) unroll_kernel(BatchView b, UnrollView u,
-                                                               InstanceList list) {
+template <bool ADJOINT, int MODE, int PER_SM = 2>
+__global__ void __launch_bounds__(kThreads64, PER_SM) unroll_kernel(BatchView b, UnrollView u,
+                                                                    InstanceList list) {
   __shared__ ClusterShared sh;
   __shared__ Unroll<MODE> ctx;
   const unsigned rank = cluster_rank();
@@ -422,6 +422,17 @@ cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const Cluster
     auto go = [&](auto kernel) {
       return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], gst, b, u, list);
     };
+    // The adjoint's state in 128 registers, two CTAs to an SM, spills 780 bytes of loads. While
+    // every CTA finds an SM of its own the variant of 215 registers runs (200 iterations: 1 LP of
+    // 80 x 176 1.76 ms before, 1.53 now; 64 of 150 x 330 2.42 and 2.06; 1 of 500 x 1,100 2.56
+    // and 2.25). Clusters of 4 and more leave SMs of a GPC over: 16 clusters of 8 no longer ran
+    // side by side (2.63 ms with two CTAs to an SM, 3.87 without).
+    const int side_by_side = p.size <= 2   ? p.sms / p.size
+                             : p.size == 4 ? p.sms / p.size * 3 / 4
+                                           : p.sms / p.size / 2;
+    if (mode == kAllShared && adjoint && clusters <= side_by_side) {
+      return go(unroll_kernel<true, kAllShared, 1>);
+    }
     if (mode == kAllShared) {
       return adjoint ? go(unroll_kernel<true, kAllShared>) : go(unroll_kernel<false, kAllShared>);
     }

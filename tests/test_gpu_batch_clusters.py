@@ -110,3 +110,23 @@ def test_cluster_kernels_at_their_edges(engine, oracle, name):
         for got, ref in zip(grads, o.adjoint(lp.cost, lp.lower, lp.upper, ITERATIONS, w[part])):
             assert _differs(got[part], ref) <= 1e-9, k
         off += lp.n + lp.m
+
+
+@pytest.mark.parametrize("count", [1, 152, 153])
+def test_adjoint_with_an_sm_to_a_cta_and_with_two_ctas_to_one(engine, count):
+    """Up to one small LP per SM, and one more: the adjoint has a kernel for each. Every copy's
+    gradients against the oracle's, to 1e-9 as above."""
+    from oracle.unroll_oracle import UnrolledPdhg as UnrollOracle
+    from samaya_gb300.batch import BatchSolver
+    from samaya_gb300.diff import UnrolledPdhg
+    lp = _lp(40, [5, 1, 7, 40, 3] * 4, 9)
+    b = BatchSolver.from_problems([lp] * count)
+    un = UnrolledPdhg(b, iterations=30, checkpoint_every=16)
+    un.forward()
+    w = np.random.default_rng(12).standard_normal(lp.n + lp.m)
+    grads = un.adjoint(np.tile(w, count))
+    b.close()
+    o = UnrollOracle(lp.m, lp.n, lp.colptr, lp.rowidx, lp.vals)
+    for got, ref in zip(grads, o.adjoint(lp.cost, lp.lower, lp.upper, 30, w)):
+        for part in np.split(got, count):
+            assert _differs(part, ref) <= 1e-9
