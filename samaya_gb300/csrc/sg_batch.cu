@@ -263,6 +263,10 @@ cudaError_t launch_batch(const BatchView& b, const ClusterPlan& setup, const Clu
   });
 }
 
+bool setup_fits(const ClusterPlan& p) {
+  return clusters_fit(batch_setup_kernel, p.size, kThreads64, p.smem[0]);
+}
+
 cudaError_t launch_batch_setup(const BatchView& b, const ClusterPlan& setup, cudaStream_t s) {
   return launch_clusters(batch_setup_kernel, setup.size, b.nmat, kThreads64, setup.smem[0], s, b,
                          static_cast<unsigned>(setup.smem[0]));

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
 
 #include <string>
 #include <vector>
@@ -145,6 +146,14 @@ cudaError_t for_groups(const ClusterPlan& p, const GroupStreams& gs, cudaStream_
   return e;
 }
 
+// The largest cluster an engine or batch may take: SG_MAX_CLUSTER when it is created (1: none, the
+// step launches and a CTA per LP), up to kMaxCluster.
+inline int cluster_limit() {
+  const char* v = getenv("SG_MAX_CLUSTER");
+  const int most = v == nullptr ? kMaxCluster : atoi(v);
+  return most < 1 ? kMaxCluster : most < kMaxCluster ? most : kMaxCluster;
+}
+
 // Dynamic shared memory of a cluster kernel at most: a CTA's 227 KB less its static part.
 constexpr size_t kClusterSmemMax = 227 * 1024 - 8 * 1024;
 // FP64 kernels: a CTA's half of an SM's 228 KB (1 KB of each CTA is the system's).
@@ -190,6 +199,12 @@ cudaError_t launch_solve64(const BatchView& b, const ClusterPlan& p, int mode, c
 cudaError_t launch_solve32(const BatchView& b, const ClusterPlan& p, int mode, cudaStream_t s);
 cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const ClusterPlan& p,
                           int adjoint, const GroupStreams& gs, cudaStream_t s);
+// Whether the device can hold a cluster of the plan's size of each kernel that a plan of several
+// CTAs launches.
+bool setup_fits(const ClusterPlan& p);
+bool solve64_fits(const ClusterPlan& p, int algorithm);
+bool solve32_fits(const ClusterPlan& p, int algorithm);
+bool unroll_fits(const ClusterPlan& p, int adjoint);
 
 class Batch {
  public:
@@ -221,6 +236,8 @@ class Batch {
   int* wait_host_ = nullptr;  // pinned copy of the wait flag
   enum class Kind { kSetup, kSolve, kForward, kAdjoint };
   int make_plan(Kind kind, ClusterPlan* plan);
+  void plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<int>* lists);
+  int upload_lists(const std::vector<int>* lists, ClusterPlan* plan);
   GroupStreams groups_;
   cudaError_t finish(std::string* err);
   double time_limit_ = 0.0;

@@ -116,31 +116,55 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
-// A launch of `clusters` clusters of `size` CTAs.
+// The configuration of a launch of `clusters` clusters of `size` CTAs.
+struct ClusterLaunch {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  template <typename... Params>
+  cudaError_t set(void (*kernel)(Params...), int size, int clusters, int threads, size_t smem,
+                  cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(kClusterSmemMax));
+    if (e == cudaSuccess && size > 8) {
+      e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                               cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
+    cfg.gridDim = dim3(clusters * size);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return e;
+  }
+};
+
 template <typename... Params, typename... Args>
 cudaError_t launch_clusters(void (*kernel)(Params...), int size, int clusters, int threads,
                             size_t smem, cudaStream_t s, Args... args) {
-  cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(kClusterSmemMax));
-  if (e == cudaSuccess && size > 8) {
-    e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
-                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  ClusterLaunch l;
+  const cudaError_t e = l.set(kernel, size, clusters, threads, smem, s);
+  return e != cudaSuccess ? e : cudaLaunchKernelEx(&l.cfg, kernel, args...);
+}
+
+// Whether the device can hold a cluster of this kernel at all. A process that owns a slice of the
+// GPU may have no GPC with that many SMs to itself.
+template <typename... Params>
+bool clusters_fit(void (*kernel)(Params...), int size, int threads, size_t smem) {
+  if (size > cluster_limit()) return false;
+  ClusterLaunch l;
+  int clusters = 0;
+  if (l.set(kernel, size, 1, threads, smem, nullptr) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, kernel, &l.cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
-  if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(clusters * size);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = size;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  return clusters > 0;
 }
 
 }  // namespace

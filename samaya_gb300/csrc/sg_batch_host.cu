@@ -378,6 +378,27 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
 // 1,500 x 3,000: 34.9 / 20.0 / 10.4 / 7.4 / 6.7 with 1 / 2 / 4 / 8 / 16 CTAs; 160 LPs of
 // 500 x 1,200: 15.3 / 17.6 / 21.5 / 32.2 / 84.9).
 int Batch::make_plan(Kind kind, ClusterPlan* plan) {
+  auto holds = [&](const ClusterPlan& p) {
+    if (p.size == 1) return true;
+    switch (kind) {
+      case Kind::kSetup: return setup_fits(p);
+      case Kind::kSolve:
+        return v_.fp32 ? solve32_fits(p, v_.algorithm) : solve64_fits(p, v_.algorithm);
+      default: return unroll_fits(p, kind == Kind::kAdjoint);
+    }
+  };
+  // Smaller clusters where the device cannot hold one of the size that suits best.
+  std::vector<int> lists[kModes];
+  for (int most = cluster_limit();; most = plan->size / 2) {
+    plan_clusters(kind, most, plan, lists);
+    if (holds(*plan)) break;
+  }
+  return upload_lists(lists, plan);
+}
+
+// The plan with clusters of at most `most` CTAs, and its instances by mode.
+void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<int>* lists) {
+  *plan = ClusterPlan();
   const bool setup = kind == Kind::kSetup;
   const bool fp32 = kind == Kind::kSolve && v_.fp32;
   const size_t elem = fp32 ? sizeof(float) : sizeof(double);
@@ -420,7 +441,7 @@ int Batch::make_plan(Kind kind, ClusterPlan* plan) {
   double best_time = -1.0;
   for (int k = 0; k < 5; ++k) {
     const int size = sizes[k];
-    if (size > 1 && !fits) break;
+    if (size > most || (size > 1 && !fits)) break;
     // Clusters at once (SMs of a GPC left over by clusters of 8 and 16: an eighth or more).
     const int slots = std::max(1, per_sm * sms_ / size - (size >= 8 ? per_sm * sms_ / size / 8 : 0));
     const bool shared_sm = !fp32 && static_cast<long long>(std::min(count, slots)) * size > sms_;
@@ -456,11 +477,11 @@ int Batch::make_plan(Kind kind, ClusterPlan* plan) {
       const size_t vec = vector_bytes(g, best);
       if (vec <= kClusterSmemMax) plan->smem[0] = std::max(plan->smem[0], vec);
     }
-    return SG_OK;
+    return;
   }
   // Every instance in the mode that keeps the most in shared memory, FP64 ones within half of it
   // (two CTAs to an SM) as long as their vectors allow that.
-  std::vector<int> lists[kModes];
+  for (int mode = 0; mode < kModes; ++mode) lists[mode].clear();
   for (int i : order_) {
     const int g = inst_mat_[i];
     const size_t vec = vector_bytes(g, best);
@@ -471,7 +492,11 @@ int Batch::make_plan(Kind kind, ClusterPlan* plan) {
     const size_t need = mode == kAllShared ? all : mode == kVectorsShared ? vec : 0;
     lists[mode].push_back(i);
     plan->smem[mode] = std::max(plan->smem[mode], need);
+    ++plan->group[mode].count;
   }
+}
+
+int Batch::upload_lists(const std::vector<int>* lists, ClusterPlan* plan) {
   int used = 0;
   for (int mode = 0; mode < kModes; ++mode) {
     if (lists[mode].empty()) continue;
@@ -484,7 +509,6 @@ int Batch::make_plan(Kind kind, ClusterPlan* plan) {
       return SG_ERR_CUDA;
     }
     plan->group[mode].inst = d;
-    plan->group[mode].count = static_cast<int>(lists[mode].size());
   }
   if (used > 1 && groups_.fork == nullptr) {
     cudaError_t e = cudaEventCreateWithFlags(&groups_.fork, cudaEventDisableTiming);

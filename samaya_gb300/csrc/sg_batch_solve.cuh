@@ -452,14 +452,10 @@ __global__ void __launch_bounds__(solve_threads<T>(), sizeof(T) == 8 ? 2 : 1)
   cluster_sync(size);
 }
 
-template <typename T>
-cudaError_t launch_solve(const BatchView& b, const ClusterPlan& p, int mode, cudaStream_t s) {
-  const InstanceList list = p.group[mode];
-  const int clusters = list.count < p.clusters ? list.count : p.clusters;
-  auto go = [&](auto kernel) {
-    return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], s, b, list);
-  };
-  const bool h = b.algorithm == 2;
+// go() with the kernel of a mode.
+template <typename T, typename Go>
+auto with_solve_kernel(int algorithm, int mode, const Go& go) {
+  const bool h = algorithm == 2;
   if (mode == kAllShared) {
     return h ? go(batch_solve_kernel<T, kAllShared, true>)
              : go(batch_solve_kernel<T, kAllShared, false>);
@@ -470,6 +466,27 @@ cudaError_t launch_solve(const BatchView& b, const ClusterPlan& p, int mode, cud
   }
   return h ? go(batch_solve_kernel<T, kInDevice, true>)
            : go(batch_solve_kernel<T, kInDevice, false>);
+}
+
+template <typename T>
+cudaError_t launch_solve(const BatchView& b, const ClusterPlan& p, int mode, cudaStream_t s) {
+  const InstanceList list = p.group[mode];
+  const int clusters = list.count < p.clusters ? list.count : p.clusters;
+  return with_solve_kernel<T>(b.algorithm, mode, [&](auto kernel) {
+    return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], s, b, list);
+  });
+}
+
+template <typename T>
+bool solve_fits(const ClusterPlan& p, int algorithm) {
+  for (int mode = 0; mode < kModes; ++mode) {
+    if (p.group[mode].count > 0 && !with_solve_kernel<T>(algorithm, mode, [&](auto kernel) {
+          return clusters_fit(kernel, p.size, p.threads, p.smem[mode]);
+        })) {
+      return false;
+    }
+  }
+  return true;
 }
 
 }  // namespace sg

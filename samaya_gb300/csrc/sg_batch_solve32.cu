@@ -7,4 +7,8 @@ cudaError_t launch_solve32(const BatchView& b, const ClusterPlan& p, int mode, c
   return launch_solve<float>(b, p, mode, s);
 }
 
+bool solve32_fits(const ClusterPlan& p, int algorithm) {
+  return solve_fits<float>(p, algorithm);
+}
+
 }  // namespace sg

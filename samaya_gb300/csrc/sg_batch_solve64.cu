@@ -7,4 +7,8 @@ cudaError_t launch_solve64(const BatchView& b, const ClusterPlan& p, int mode, c
   return launch_solve<double>(b, p, mode, s);
 }
 
+bool solve64_fits(const ClusterPlan& p, int algorithm) {
+  return solve_fits<double>(p, algorithm);
+}
+
 }  // namespace sg

@@ -414,14 +414,43 @@ __global__ void __launch_bounds__(kThreads64, PER_SM) unroll_kernel(BatchView b,
   cluster_sync(size);
 }
 
+namespace {
+
+// go() with the kernel of a mode; `alone`: the adjoint's variant with an SM to a CTA.
+template <typename Go>
+auto with_unroll_kernel(int adjoint, int mode, bool alone, const Go& go) {
+  if (mode == kAllShared && adjoint && alone) return go(unroll_kernel<true, kAllShared, 1>);
+  if (mode == kAllShared) {
+    return adjoint ? go(unroll_kernel<true, kAllShared>) : go(unroll_kernel<false, kAllShared>);
+  }
+  if (mode == kVectorsShared) {
+    return adjoint ? go(unroll_kernel<true, kVectorsShared>)
+                   : go(unroll_kernel<false, kVectorsShared>);
+  }
+  return adjoint ? go(unroll_kernel<true, kInDevice>) : go(unroll_kernel<false, kInDevice>);
+}
+
+}  // namespace
+
+bool unroll_fits(const ClusterPlan& p, int adjoint) {
+  for (int mode = 0; mode < kModes; ++mode) {
+    for (bool alone : {false, true}) {
+      if (p.group[mode].count > 0 &&
+          !with_unroll_kernel(adjoint, mode, alone, [&](auto kernel) {
+            return clusters_fit(kernel, p.size, p.threads, p.smem[mode]);
+          })) {
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
 cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const ClusterPlan& p,
                           int adjoint, const GroupStreams& gs, cudaStream_t s) {
   return for_groups(p, gs, s, cudaSuccess, [&](int mode, cudaStream_t gst) {
     const InstanceList list = p.group[mode];
     const int clusters = list.count < p.clusters ? list.count : p.clusters;
-    auto go = [&](auto kernel) {
-      return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], gst, b, u, list);
-    };
     // The adjoint's state in 128 registers, two CTAs to an SM, spills 780 bytes of loads. While
     // every CTA finds an SM of its own the variant of 215 registers runs (200 iterations: 1 LP of
     // 80 x 176 1.76 ms before, 1.53 now; 64 of 150 x 330 2.42 and 2.06; 1 of 500 x 1,100 2.56
@@ -430,17 +459,9 @@ cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const Cluster
     const int side_by_side = p.size <= 2   ? p.sms / p.size
                              : p.size == 4 ? p.sms / p.size * 3 / 4
                                            : p.sms / p.size / 2;
-    if (mode == kAllShared && adjoint && clusters <= side_by_side) {
-      return go(unroll_kernel<true, kAllShared, 1>);
-    }
-    if (mode == kAllShared) {
-      return adjoint ? go(unroll_kernel<true, kAllShared>) : go(unroll_kernel<false, kAllShared>);
-    }
-    if (mode == kVectorsShared) {
-      return adjoint ? go(unroll_kernel<true, kVectorsShared>)
-                     : go(unroll_kernel<false, kVectorsShared>);
-    }
-    return adjoint ? go(unroll_kernel<true, kInDevice>) : go(unroll_kernel<false, kInDevice>);
+    return with_unroll_kernel(adjoint, mode, clusters <= side_by_side, [&](auto kernel) {
+      return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], gst, b, u, list);
+    });
   });
 }
 

@@ -614,6 +614,13 @@ bool place_chunk(ChunkView<T>* v, const TaskLayout& k, const TaskLayout& t) {
   return at <= kClusterSmemMax;
 }
 
+// (The scaling and power kernels take the same launch and less static shared memory.)
+template <typename T>
+bool chunk_fits(const ChunkView<T>& c, bool halpern) {
+  return halpern ? clusters_fit(chunk_kernel<T, true>, c.size, kChunkThreads, c.smem)
+                 : clusters_fit(chunk_kernel<T, false>, c.size, kChunkThreads, c.smem);
+}
+
 template <typename T>
 void launch_chunk_indices(const ChunkView<T>& c, const OpView<T>& K, const OpView<T>& Kt,
                           cudaStream_t s) {
@@ -653,6 +660,8 @@ cudaError_t launch_chunk_scale(const ChunkView<double>& c, const double* k_given
 
 template bool place_chunk<double>(ChunkView<double>*, const TaskLayout&, const TaskLayout&);
 template bool place_chunk<float>(ChunkView<float>*, const TaskLayout&, const TaskLayout&);
+template bool chunk_fits<double>(const ChunkView<double>&, bool);
+template bool chunk_fits<float>(const ChunkView<float>&, bool);
 template void launch_chunk_indices<double>(const ChunkView<double>&, const OpView<double>&,
                                            const OpView<double>&, cudaStream_t);
 template void launch_chunk_indices<float>(const ChunkView<float>&, const OpView<float>&,

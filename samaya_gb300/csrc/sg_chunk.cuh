@@ -40,6 +40,9 @@ struct ChunkView {
 // Sets the places in shared memory and smem; false when they do not fit.
 template <typename T>
 bool place_chunk(ChunkView<T>* v, const TaskLayout& k, const TaskLayout& t);
+// Whether the device can hold the placed chunk's cluster.
+template <typename T>
+bool chunk_fits(const ChunkView<T>& c, bool halpern);
 // The column numbers of both operators, from their CSR arrays.
 template <typename T>
 void launch_chunk_indices(const ChunkView<T>& c, const OpView<T>& K, const OpView<T>& Kt,

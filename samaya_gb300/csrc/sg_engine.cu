@@ -942,7 +942,10 @@ void Engine::plan_chunk() {
     c->view.n = n_;
     c->view.m = m_;
     c->view.size = size;
-    if (!place_chunk(&c->view, c->layout[0], c->layout[1])) c->view.size = 0;
+    if (!place_chunk(&c->view, c->layout[0], c->layout[1]) ||
+        !chunk_fits(c->view, opt_.algorithm == 2)) {
+      c->view.size = 0;
+    }
   };
   if (work <= kMost64) plan(&chunk64_, false);
   // FP32 sums keep the step kernels' order: rows longer than kWarpRowMin have another. (The
@@ -1200,18 +1203,18 @@ int Engine::equilibration(double* col_scale, double* row_scale, double* op_norm,
 // detection. Recorded once as a CUDA graph.
 namespace {
 
-// The kernels of one chunk; returns how many launches it records.
+// The kernels of one chunk; `count` is how many launches it records.
 // Ks is K over the active rows (the steps), K over every row (evaluation and detection);
 // c.size > 0: the iterations in one cluster launch.
 template <typename T>
-int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const OpView<T>& K,
-                  const OpView<T>& Kt,
-                  const IterView<T>& it, const EvalView& ev, const RedView& red,
-                  double* scratch_n, int gsk, int gst, int gk, int gt, bool halpern, bool detect,
-                  cudaStream_t s) {
+cudaError_t enqueue_chunk(int* count, Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks,
+                          const OpView<T>& K, const OpView<T>& Kt, const IterView<T>& it,
+                          const EvalView& ev, const RedView& red, double* scratch_n, int gsk,
+                          int gst, int gk, int gt, bool halpern, bool detect, cudaStream_t s) {
   int kernels = 0;
   if (c.size > 0) {
-    launch_chunk(ctl, c, it, halpern, s);
+    const cudaError_t e = launch_chunk(ctl, c, it, halpern, s);
+    if (e != cudaSuccess) return e;
     kernels = 1;
   }
   const bool both = Ks.ts.ntiles > 0 && Kt.ts.ntiles > 0;
@@ -1235,7 +1238,29 @@ int enqueue_chunk(Ctl* ctl, const ChunkView<T>& c, const OpView<T>& Ks, const Op
     launch_decide(ctl, s);
   }
   launch_restart(ctl, it, s);
-  return kernels + 1 + (detect ? 8 : 1) + 1;
+  *count = kernels + 1 + (detect ? 8 : 1) + 1;
+  return cudaGetLastError();
+}
+
+// The graph of what enqueue() launches on the stream. A launch that failed leaves no graph: a
+// graph without it would replay and count iterations that nobody makes.
+template <typename Graph, typename Enqueue>
+cudaError_t capture_graph(Graph* g, cudaStream_t s, const Enqueue& enqueue) {
+  cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return e;
+  const cudaError_t launched = enqueue();
+  cudaGraph_t graph = nullptr;
+  e = cudaStreamEndCapture(s, &graph);
+  if (launched != cudaSuccess) e = launched;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
+  if (e == cudaSuccess) {
+    g->graph = graph;
+  } else {
+    g->exec = nullptr;
+    if (graph != nullptr) cudaGraphDestroy(graph);
+    cudaGetLastError();
+  }
+  return e;
 }
 
 }  // namespace
@@ -1246,12 +1271,11 @@ int Engine::capture_chunk(bool detect) {
   ChunkGraph& g = chunk_[detect ? 1 : 0];
   if (g.exec != nullptr) return kOk;
   std::string* err = nullptr;
-  SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  g.kernels = enqueue_chunk(ctl_, chunk64_.view, K_.step64(), K_.view64(), Kt_.view64(),
-                            iter_view(it64_), eval_view(), red_view(), scratch_n_, grid_step_k_,
-                            grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, detect, stream_);
-  SG_TRY(cudaStreamEndCapture(stream_, &g.graph));
-  SG_TRY(cudaGraphInstantiate(&g.exec, g.graph, 0));
+  SG_TRY(capture_graph(&g, stream_, [&] {
+    return enqueue_chunk(&g.kernels, ctl_, chunk64_.view, K_.step64(), K_.view64(), Kt_.view64(),
+                         iter_view(it64_), eval_view(), red_view(), scratch_n_, grid_step_k_,
+                         grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, detect, stream_);
+  }));
   return kOk;
 }
 
@@ -1262,13 +1286,12 @@ int Engine::capture_chunk32() {
   std::string* err = nullptr;
   IterView<float> it = iter_view(it32_);
   it.rhs = it32_.rhs;
-  SG_TRY(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-  chunk32_.kernels = enqueue_chunk(ctl32_, chunk32c_.view, K_.step32(), K_.view32(), Kt_.view32(), it,
-                                   inner_eval_view(), red_view(), scratch_n_, grid_step_k_,
-                                   grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, false,
-                                   stream_);
-  SG_TRY(cudaStreamEndCapture(stream_, &chunk32_.graph));
-  SG_TRY(cudaGraphInstantiate(&chunk32_.exec, chunk32_.graph, 0));
+  SG_TRY(capture_graph(&chunk32_, stream_, [&] {
+    return enqueue_chunk(&chunk32_.kernels, ctl32_, chunk32c_.view, K_.step32(), K_.view32(),
+                         Kt_.view32(), it, inner_eval_view(), red_view(), scratch_n_,
+                         grid_step_k_, grid_step_t_, grid_k_, grid_t_, opt_.algorithm == 2, false,
+                         stream_);
+  }));
   return kOk;
 }
 
