@@ -61,7 +61,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
   for (int j = threadIdx.x; j < n; j += blockDim.x) xs[j] = 1.0;
   for (int i = threadIdx.x; i < m; i += blockDim.x) ys[i] = 1.0;
   cluster_sync(size);
-  bool ok = true;
+  bool ok = true;  // (no loop ends on it: they hold cluster barriers)
   if (m > 0 && n > 0) {
     // Both statistics are taken with the old scales, then every own scale is updated and sent.
     if (b.algorithm >= 1) {
@@ -69,7 +69,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
         const double* o;
         __device__ double operator()(double a, int j) const { return fabs(a) * o[j]; }
       };
-      for (int pass = 0; pass < 11 && ok; ++pass) {
+      for (int pass = 0; pass < 11; ++pass) {
         auto fc = [&](const At& at, double s) { cn[at.p] = s * xs[at.p]; };
         auto fr = [&](const At& at, double s) { rn[at.p] = s * ys[at.p]; };
         if (pass < 10) {
@@ -100,7 +100,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
           return v * v;
         }
       };
-      for (int pass = 0; pass < 10 && ok; ++pass) {
+      for (int pass = 0; pass < 10; ++pass) {
         walk_rows<true, false>(T0, Sq2{ys}, zero_init,
                                [&](const At& at, double s) { cn[at.p] = sqrt(s) * xs[at.p]; }, Ready());
         walk_rows<true, false>(K0, Sq2{xs}, zero_init,
@@ -183,7 +183,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
     ok = ex.wait(1) && ok;
     double sigma = 0.0;
     bool zero = false;
-    for (int it = 0; it < 20 && ok; ++it) {
+    for (int it = 0; it < 20; ++it) {
       double acc[1] = {0.0};
       walk_rows<false, false>(T, GatherT<double>{ys}, zero_init, [&](const At& at, double s) {
         ex.put_x(at, s);

@@ -135,10 +135,10 @@ __device__ __noinline__ bool evaluate_point(const EvalContext<T, MODE>* ctx, int
   return true;
 }
 
-// Runs one instance; false when a wait gave up. Storage, products and step sums in T (GB300's
-// FP64 pipe is small), the evaluation in FP64.
+// Runs one instance (a wait that gave up is in sh.fail). Storage, products and step sums in T
+// (GB300's FP64 pipe is small), the evaluation in FP64.
 template <typename T, int MODE, bool halpern>
-__device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
+__device__ void solve_instance(const BatchView& b, int inst, ClusterShared& sh,
                                EvalContext<T, MODE>* ctx, unsigned rank,
                                unsigned size) {
   constexpr bool kF64 = sizeof(T) == 8;
@@ -251,7 +251,6 @@ __device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
     t += steps;
     k_since += steps;
     ok = ok && ex.wait(halpern ? 1 : 0);
-    if (!ok) break;
     // Evaluation of the current and the average iterate; Halpern: only T(z) (the Halpern iterate
     // itself can leave the bounds).
     if (!halpern) {
@@ -259,14 +258,15 @@ __device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
       inv_k = 1.0 / static_cast<double>(k_since);
     }
     // a: the current iterate's 7 sums, the average's 7, the distances (v, y) of each, and
-    // whether the time limit has passed (asked by one thread, so that all agree).
+    // whether the time limit has passed (1, asked by one thread, so that all agree) and CTAs' waits
+    // gave up (2 each).
     double a[19];
 #pragma unroll
     for (int q = 0; q < 19; ++q) a[q] = 0.0;
-    for (int w = halpern ? 1 : 0; w < 2 && ok; ++w) {
+    for (int w = halpern ? 1 : 0; w < 2; ++w) {
       cluster_sync(size);  // every CTA has read xs and ys, their last entries in place
       double e[9];
-      ok = evaluate_point<T, MODE>(ctx, halpern ? 2 : w, inv_k, e);
+      ok = evaluate_point<T, MODE>(ctx, halpern ? 2 : w, inv_k, e) && ok;
       if (w == 0) {
 #pragma unroll
         for (int q = 0; q < 7; ++q) a[q] = e[q];
@@ -279,12 +279,16 @@ __device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
         a[17] = e[8];
       }
     }
-    if (!ok) break;
     if (rank == 0 && threadIdx.x == 0) {
       const unsigned long long deadline = *b.deadline;
       if (deadline != 0ull && globaltimer_ns() > deadline) a[18] = 1.0;
     }
+    if (threadIdx.x == 0 && !ok) a[18] += 2.0;
     cluster_reduce<19>(a, sh, rank, size);
+    if (a[18] >= 2.0) {
+      ok = false;
+      break;
+    }
     const Meas mc = finish7(a, mi.a_norm_max_col, mi.at_norm_max_row, c_norm, m);
     const Meas ma = finish7(a + 7, mi.a_norm_max_col, mi.at_norm_max_row, c_norm, m);
     const double tol = b.tol;
@@ -414,15 +418,16 @@ __device__ bool solve_instance(const BatchView& b, int inst, ClusterShared& sh,
     r.restarts = restarts;
   }
   if (!ok && threadIdx.x == 0) atomicExch(b.wait_error, 1);
-  return ok;
 }
 
-// The next position of the work queue, the same for every thread of the cluster.
+// The next position of the work queue, the same for every thread of the cluster; past its end when
+// a wait gave up in one of the CTAs.
 __device__ __forceinline__ int next_instance(unsigned* queue, ClusterShared& sh, unsigned rank,
                                              unsigned size) {
-  cluster_sync(size);  // the last instance is done, its position read by all
+  // The last instance is done, its position read by all.
+  const bool stopped = cluster_stopped(sh, size);
   if (rank == 0 && threadIdx.x == 0) {
-    const unsigned q = atomicAdd(queue, 1u);
+    const unsigned q = stopped ? 0x7fffffffu : atomicAdd(queue, 1u);
     for (unsigned p = 0; p < size; ++p) st_cluster(map_rank(shared_addr(&sh.next), p), q);
   }
   cluster_sync(size);
@@ -447,7 +452,7 @@ __global__ void __launch_bounds__(solve_threads<T>(), sizeof(T) == 8 ? 2 : 1)
   for (;;) {
     const int q = next_instance(b.queue + MODE, sh, rank, size);
     if (q >= list.count) break;
-    if (!solve_instance<T, MODE, HALPERN>(b, list.inst[q], sh, &ctx, rank, size)) break;
+    solve_instance<T, MODE, HALPERN>(b, list.inst[q], sh, &ctx, rank, size);
   }
   cluster_sync(size);
 }

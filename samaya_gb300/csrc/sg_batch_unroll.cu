@@ -264,8 +264,7 @@ __device__ bool unroll_forward(const BatchView& b, const UnrollView& u, int inst
   double* vo = u.v_out + p.vo;
   each_own(M.Kt, [&](const At& at) { vo[M.tperm[at.p]] = S.col(kUPoint, at) * p.cs[at.p]; });
   each_own(M.K, [&](const At& at) { vo[M.n + M.kperm[at.p]] = S.row(kUPoint, at) / p.rs[at.p]; });
-  cluster_sync(size);
-  return ok;
+  return !cluster_stopped(sh, size);
 }
 
 template <int MODE>
@@ -293,11 +292,12 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
   unsigned char* mask = u.mask + u.mask_off[inst];
   const long long stride = 2 * nt + M.m;
   bool ok = true;
-  for (int seg = u.nck - 1; seg >= 0 && ok; --seg) {
+  for (int seg = u.nck - 1; seg >= 0; --seg) {
     const int k0 = seg * u.every;
     const int len = min(u.every, u.iterations - k0);
     const double* c = ck + static_cast<long long>(seg) * stride;
-    cluster_sync(size);  // xs and ys of the segment before are read by all
+    // xs and ys of the segment before are read by all.
+    if (cluster_stopped(sh, size)) break;
     each_own(M.Kt, [&](const At& at) {
       S.col(kUPoint, at) = c[at.p];
       p.ex.put_x(at, c[nt + at.p]);
@@ -311,7 +311,6 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
       ok = unroll_step<MODE>(ctx, tau, sigma, mask + static_cast<long long>(t) * nt);
     }
     ok = ok && p.ex.wait(0);
-    if (!ok) break;
     cluster_sync(size);  // the last x_bar is in place everywhere: xs may be sent again
     auto col = [&](const At& at, double bh, const unsigned char* mk, const UnrollState<MODE>& S,
                    const Sender<double, MODE, 0>& x_out) {
@@ -321,7 +320,7 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
       const auto e = S.row_entry(at);
       e.set(kURows + kAG, adjoint_entry(e, kURows, bh, mk[M.n + at.p], tau));
     };
-    {
+    if (ok) {
       const unsigned char* mk = mask + static_cast<long long>(len - 1) * nt;
       const Sender<double, MODE, 0> x_out(p.ex);
       each_own(M.Kt, [&](const At& at) { col(at, S.acol(kAB, at), mk, S, x_out); });
@@ -388,8 +387,7 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
     gl[k] = S.arow(kAGl, at) * sc;
     gu[k] = S.arow(kAGu, at) * sc;
   });
-  cluster_sync(size);
-  return ok;
+  return !cluster_stopped(sh, size);
 }
 
 }  // namespace

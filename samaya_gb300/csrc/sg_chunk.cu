@@ -312,8 +312,6 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   auto rows = [&](const At& at, double s) { S.row(at).set(0, s); };
   bool ok = true;
   constexpr int kPasses = RUIZ ? 10 : 11;
-  // (A wait that gave up ends the passes for all CTAs together or not at all: no CTA may leave
-  // while others still send to it.)
   for (int pass = 0; pass < kPasses; ++pass) {
     double moved[1] = {0.0};
     if constexpr (RUIZ) {
@@ -385,7 +383,8 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   each_own(M.K, [&](const At& at) { y_out.put(at, u0[M.kperm[at.p]]); });
   double sigma = 0.0, growth = 1.0;
   bool ok = true, vanished = false;
-  for (int k = 0; k < iterations && ok && !vanished; ++k) {
+  // (A CTA whose wait gave up stays to the reduction of the last iteration, where all know.)
+  for (int k = 0; k < iterations && !vanished; ++k) {
     const bool lengths = k == 0 || k == iterations - 1;
     double v2[1] = {0.0}, u2[1] = {0.0};
     ok = M.Kt.walk(from_y, zero,
@@ -405,13 +404,13 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
                         },
                         [&] { return ex.wait(0); });
     if (lengths) {
-      // (Every CTA comes here: a wait that gave up counts as a length too.)
       double all[3] = {v2[0], u2[0], ok ? 0.0 : 1.0};
       cluster_reduce<3>(all, sh, rank, size);
       ok = all[2] == 0.0;
+      if (!ok) break;
       const double vn = sqrt(all[0]), un = sqrt(all[1]);
       vanished = vn == 0.0 || un == 0.0;
-      if (ok && !vanished) {
+      if (!vanished) {
         sigma = un / vn;
         growth = inverse_power(sigma * sigma);
         const double start = inverse_power(un);

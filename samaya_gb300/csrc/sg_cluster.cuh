@@ -29,6 +29,13 @@
 // after its sum, so that CTA's wait covers all of them (and the same with xs and ys exchanged).
 // A publication that does not alternate this way needs a cluster_sync before it.
 //
+// A wait is bounded, and it may give up in one CTA and not, or later, in another. A CTA whose wait
+// gave up (ClusterShared::fail, which ends its later waits at once) goes on through every cluster
+// barrier of the kernel, and all CTAs leave a loop that holds such barriers together: by a reduction
+// that carries the failure, or by cluster_stopped. One that left alone would arrive at its last
+// barrier in the place of an earlier one and end, and the others would then store into the shared
+// memory of a CTA that has ended.
+//
 // Every sum is taken in a fixed order, so a re-run is bit-identical.
 #pragma once
 
@@ -201,6 +208,7 @@ struct ClusterShared {
   unsigned incoming[2][kMaxCluster];   // entries each other CTA sends here
   unsigned distance[kMaxCluster];      // from a shared address here to the one in rank ^ q
   int fail;                            // a bounded wait gave up
+  unsigned stop;                       // in some CTA of the cluster (cluster_stopped)
   int next;                            // work queue position
 };
 
@@ -216,8 +224,19 @@ __device__ __forceinline__ void cluster_init(ClusterShared& sh, unsigned size) {
     for (unsigned q = 0; q < size; ++q) sh.distance[q] = map_rank(here, cluster_rank() ^ q) - here;
     sh.phase[0] = sh.phase[1] = 0;
     sh.fail = 0;
+    sh.stop = 0u;
   }
   cluster_sync(size);
+}
+
+// A cluster barrier after which every CTA knows whether a wait gave up in any of them, before it.
+// (Another cluster barrier lies between two of these, so that none is told of a later failure.)
+__device__ __forceinline__ bool cluster_stopped(ClusterShared& sh, unsigned size) {
+  if (threadIdx.x < size && sh.fail != 0) {
+    st_cluster(map_rank(shared_addr(&sh.stop), threadIdx.x), 1u);
+  }
+  cluster_sync(size);
+  return sh.stop != 0u;
 }
 
 // The kernels' dynamic shared memory. What lies there is kept as an offset into it: a 32-bit value,
@@ -287,8 +306,8 @@ struct alignas(16) Exchange {
     }
   }
   // After every thread of the CTA has put its entries: true when all entries read here have
-  // arrived, false when the bounded wait gave up (uniform over the CTA). Two waits for the same
-  // vector have a barrier of the CTA between them.
+  // arrived, false when the bounded wait gave up or one did before (uniform over the CTA). Two
+  // waits for the same vector have a barrier of the CTA between them.
   __device__ __forceinline__ bool wait(int which) const {
     if (size == 1) {
       __syncthreads();
@@ -296,12 +315,14 @@ struct alignas(16) Exchange {
     }
     const unsigned bar = shared_addr(&sh->bar[which]);
     const unsigned ph = sh->phase[which] & 1u;
-    if (threadIdx.x == 0) {
+    // (After a failure the barrier's phase may be open still: no arrival, no wait.)
+    const bool failed = sh->fail != 0;
+    if (threadIdx.x == 0 && !failed) {
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                    "r"(tx[which])
                    : "memory");
     }
-    unsigned ok = 0;
+    unsigned ok = failed ? 1 : 0;
     for (int k = 0; k < kClusterWaitTries && ok == 0; ++k) {
       asm volatile(
           "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
