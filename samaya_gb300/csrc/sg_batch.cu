@@ -88,8 +88,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
           const double old = ys[at.p];
           ex.put_y(at, rn[at.p] > 0.0 ? old / sqrt(rn[at.p]) : old);
         });
-        ok = ex.wait(0);
-        ok = ex.wait(1) && ok;
+        ok = ok && ex.wait(0) && ex.wait(1);
       }
     } else {
       // The reference's L2 Ruiz (pdlp.cpp:109-187).
@@ -115,8 +114,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
         };
         each_own(T0, [&](const At& at) { ex.put_x(at, rescaled(xs[at.p], cn[at.p])); });
         each_own(K0, [&](const At& at) { ex.put_y(at, rescaled(ys[at.p], rn[at.p])); });
-        ok = ex.wait(0);
-        ok = ex.wait(1) && ok;
+        ok = ok && ex.wait(0) && ex.wait(1);
         cluster_reduce<1, 1u>(changed, sh, rank, size);
         if (changed[0] == 0.0) break;
       }
@@ -180,7 +178,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
     cluster_reduce<1>(ss, sh, rank, size);
     double un = sqrt(ss[0]);
     each_own(K, [&](const At& at) { ex.put_y(at, b.power_start[M.kperm[at.p]] / un); });
-    ok = ex.wait(1) && ok;
+    ok = ok && ex.wait(1);
     double sigma = 0.0;
     bool zero = false;
     for (int it = 0; it < 20; ++it) {
@@ -189,7 +187,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
         ex.put_x(at, s);
         acc[0] += s * s;
       }, Ready());
-      ok = ex.wait(0);
+      ok = ok && ex.wait(0);
       cluster_reduce<1>(acc, sh, rank, size);
       const double vn = sqrt(acc[0]);
       if (vn == 0.0) {
@@ -211,7 +209,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
       sigma = un / vn;
       const double inv = 1.0 / un;
       each_own(K, [&](const At& at) { ex.put_y(at, rn[at.p] * inv); });
-      ok = ex.wait(1);
+      ok = ok && ex.wait(1);
     }
     if (!zero) {
       const double la = sigma * 1.01;

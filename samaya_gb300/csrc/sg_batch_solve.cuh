@@ -86,9 +86,7 @@ __device__ __noinline__ bool evaluate_point(const EvalContext<T, MODE>* ctx, int
   for (int q = 0; q < 9; ++q) e[q] = 0.0;
   each_own(M.Kt, [&](const At& at) { ex.put_x(at, vx(at)); });
   each_own(M.K, [&](const At& at) { ex.put_y(at, vy(at)); });
-  bool good = ex.wait(0);
-  good = ex.wait(1) && good;
-  if (!good) return false;
+  if (!ex.wait(0) || !ex.wait(1)) return false;
   const int m = M.m;
   walk_rows<true, false>(M.K, GatherD<T>{ex.xs()}, Zero<double>(), [&](const At& at, double s) {
     const int k = G.n + G.kperm[at.p];
@@ -265,8 +263,8 @@ __device__ void solve_instance(const BatchView& b, int inst, ClusterShared& sh,
     for (int q = 0; q < 19; ++q) a[q] = 0.0;
     for (int w = halpern ? 1 : 0; w < 2; ++w) {
       cluster_sync(size);  // every CTA has read xs and ys, their last entries in place
-      double e[9];
-      ok = evaluate_point<T, MODE>(ctx, halpern ? 2 : w, inv_k, e) && ok;
+      double e[9] = {};
+      ok = ok && evaluate_point<T, MODE>(ctx, halpern ? 2 : w, inv_k, e);
       if (w == 0) {
 #pragma unroll
         for (int q = 0; q < 7; ++q) a[q] = e[q];

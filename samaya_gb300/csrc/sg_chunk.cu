@@ -347,8 +347,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
     };
     each_own(M.Kt, [&](const At& at) { x_out.put(at, next(x.get(at.p), S.col(at).get(0))); });
     each_own(M.K, [&](const At& at) { y_out.put(at, next(y.get(at.p), S.row(at).get(0))); });
-    ok = ex.wait(0) && ok;
-    ok = ex.wait(1) && ok;
+    ok = ok && ex.wait(0) && ex.wait(1);
     if constexpr (RUIZ) {
       double all[2] = {moved[0], ok ? 0.0 : 1.0};
       cluster_reduce<2, 3u>(all, sh, rank, size);
@@ -387,12 +386,12 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
   for (int k = 0; k < iterations && !vanished; ++k) {
     const bool lengths = k == 0 || k == iterations - 1;
     double v2[1] = {0.0}, u2[1] = {0.0};
-    ok = M.Kt.walk(from_y, zero,
-                   [&](const At& at, double s) {
-                     x_out.put(at, s);
-                     if (lengths) v2[0] += s * s;
-                   },
-                   [&] { return ex.wait(1); });
+    ok = ok && M.Kt.walk(from_y, zero,
+                         [&](const At& at, double s) {
+                           x_out.put(at, s);
+                           if (lengths) v2[0] += s * s;
+                         },
+                         [&] { return ex.wait(1); });
     ok = ok && M.K.walk(from_x, zero,
                         [&](const At& at, double s) {
                           if (lengths) {

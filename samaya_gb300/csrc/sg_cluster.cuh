@@ -30,9 +30,9 @@
 // A publication that does not alternate this way needs a cluster_sync before it.
 //
 // A wait is bounded, and it may give up in one CTA and not, or later, in another. A CTA whose wait
-// gave up (ClusterShared::fail, which ends its later waits at once) goes on through every cluster
-// barrier of the kernel, and all CTAs leave a loop that holds such barriers together: by a reduction
-// that carries the failure, or by cluster_stopped. One that left alone would arrive at its last
+// gave up (ClusterShared::fail) waits no more and goes on through every cluster barrier of the
+// kernel, and all CTAs leave a loop that holds such barriers together: by a reduction that carries
+// the failure, or by cluster_stopped. (A look at `fail` in the wait itself took 1% of every solve.) One that left alone would arrive at its last
 // barrier in the place of an earlier one and end, and the others would then store into the shared
 // memory of a CTA that has ended.
 //
@@ -306,8 +306,9 @@ struct alignas(16) Exchange {
     }
   }
   // After every thread of the CTA has put its entries: true when all entries read here have
-  // arrived, false when the bounded wait gave up or one did before (uniform over the CTA). Two
-  // waits for the same vector have a barrier of the CTA between them.
+  // arrived, false when the bounded wait gave up (uniform over the CTA; no wait follows that one, as
+  // its phase may be open still). Two waits for the same vector have a barrier of the CTA between
+  // them.
   __device__ __forceinline__ bool wait(int which) const {
     if (size == 1) {
       __syncthreads();
@@ -315,14 +316,12 @@ struct alignas(16) Exchange {
     }
     const unsigned bar = shared_addr(&sh->bar[which]);
     const unsigned ph = sh->phase[which] & 1u;
-    // (After a failure the barrier's phase may be open still: no arrival, no wait.)
-    const bool failed = sh->fail != 0;
-    if (threadIdx.x == 0 && !failed) {
+    if (threadIdx.x == 0) {
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                    "r"(tx[which])
                    : "memory");
     }
-    unsigned ok = failed ? 1 : 0;
+    unsigned ok = 0;
     for (int k = 0; k < kClusterWaitTries && ok == 0; ++k) {
       asm volatile(
           "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"

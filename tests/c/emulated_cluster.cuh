@@ -66,7 +66,8 @@ struct alignas(16) Exchange {
     for (unsigned r = 0; r < size; ++r) emu::cluster.touch(r);
   }
   bool wait(int) const {
-    if (sh->fail == 0 && emu::waits++ >= emu::fail_at) {
+    if (sh->fail != 0) emu::cluster.stray = true;  // none after one that gave up
+    if (emu::waits++ >= emu::fail_at) {
       sh->fail = 1;
       emu::cluster.failed = true;
     }
