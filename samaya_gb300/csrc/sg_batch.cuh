@@ -113,7 +113,7 @@ struct ClusterPlan {
   int size = 0;
   int clusters = 1;
   int sms = 0;  // SMs of the device
-  int threads = 256;
+  int threads[kModes] = {kThreads64, kThreads64, kThreads64};
   InstanceList group[kModes];
   size_t smem[kModes] = {0, 0, 0};
 };

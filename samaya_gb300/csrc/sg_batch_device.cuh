@@ -67,20 +67,21 @@ struct MatShare {
   int nr, nc;              // own rows and columns, whole slices
 };
 
-template <typename T>
-__device__ __forceinline__ MatShare<T> mat_share(const BatchView& b, int g, const T* kval,
-                                                 const T* tval, unsigned rank, unsigned size) {
-  MatShare<T> s;
+template <typename T, typename Share = RowShare<T>>
+__device__ __forceinline__ MatShare<T, Share> mat_share(const BatchView& b, int g, const T* kval,
+                                                        const T* tval, unsigned rank,
+                                                        unsigned size) {
+  MatShare<T, Share> s;
   s.m = b.mat_m[g];
   s.n = b.mat_n[g];
   s.kz = b.mat_k_off[g];
   s.tz = b.mat_t_off[g];
   s.kperm = b.k_perm + b.mat_row_off[g];
   s.tperm = b.t_perm + b.mat_col_off[g];
-  s.K = RowShare<T>{b.k_sl + b.mat_row_off[g], b.k_desc + b.mat_kd_off[g], b.k_idx + s.kz,
-                    kval + s.kz, s.m, b.mat_slice[2 * g], rank, size};
-  s.Kt = RowShare<T>{b.t_sl + b.mat_col_off[g], b.t_desc + b.mat_td_off[g], b.t_idx + s.tz,
-                     tval + s.tz, s.n, b.mat_slice[2 * g + 1], rank, size};
+  s.K = Share{b.k_sl + b.mat_row_off[g], b.k_desc + b.mat_kd_off[g], b.k_idx + s.kz,
+              kval + s.kz, s.m, b.mat_slice[2 * g], rank, size};
+  s.Kt = Share{b.t_sl + b.mat_col_off[g], b.t_desc + b.mat_td_off[g], b.t_idx + s.tz,
+               tval + s.tz, s.n, b.mat_slice[2 * g + 1], rank, size};
   s.nr = s.K.own();
   s.nc = s.Kt.own();
   return s;
@@ -88,10 +89,10 @@ __device__ __forceinline__ MatShare<T> mat_share(const BatchView& b, int g, cons
 
 // Shared memory, in order: the gathered vectors, the masks (clusters of several CTAs), the state.
 // The vectors sit at the same place in every CTA of a cluster.
-template <typename V, int MODE, typename T>
-__device__ __forceinline__ Exchange<V, MODE> make_exchange(const MatShare<T>& s, ClusterShared& sh,
-                                                           V* spill, unsigned rank,
-                                                           unsigned size) {
+template <typename V, int MODE, typename T, typename Share>
+__device__ __forceinline__ Exchange<V, MODE> make_exchange(const MatShare<T, Share>& s,
+                                                           ClusterShared& sh, V* spill,
+                                                           unsigned rank, unsigned size) {
   Exchange<V, MODE> ex;
   ex.sh = &sh;
   ex.rank = rank;

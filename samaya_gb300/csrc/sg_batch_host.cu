@@ -373,10 +373,11 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
 
 // Cluster size, shared memory and clusters of one kernel: the size with the shortest estimated
 // finish when the instances go to the clusters largest first. The estimate of an iteration, in
-// microseconds, is fitted to measured ones of random LPs from 100 x 250 to 5,000 x 10,000 and
-// facility-location LPs, 1 to 600 of them, at every size (within 20%; e.g. FP64, 1 LP of
-// 1,500 x 3,000: 34.9 / 20.0 / 10.4 / 7.4 / 6.7 with 1 / 2 / 4 / 8 / 16 CTAs; 160 LPs of
-// 500 x 1,200: 15.3 / 17.6 / 21.5 / 32.2 / 84.9).
+// microseconds, is fitted to measured ones of random LPs (FP64 from 100 x 250, FP32 from 20 x 50, to
+// 5,000 x 10,000) and facility-location LPs, 1 to 600 of them, at every size (within 20%; e.g. FP64,
+// 1 LP of 1,500 x 3,000: 34.9 / 20.0 / 10.4 / 7.4 / 6.7 with 1 / 2 / 4 / 8 / 16 CTAs; 160 LPs of 500 x
+// 1,200: 15.3 / 17.6 / 21.5 / 32.2 / 84.9; FP32, 1 LP of 20 x 50: 1.7 / 2.2 / 2.2 / 2.4 / 2.9, of 2,000 x
+// 5,000: 14.7 / 9.0 / 5.3 / 4.0 / 3.9).
 int Batch::make_plan(Kind kind, ClusterPlan* plan) {
   auto holds = [&](const ClusterPlan& p) {
     if (p.size == 1) return true;
@@ -425,14 +426,14 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
     const int g = setup ? i : inst_mat_[i];
     const double rows = static_cast<double>(mat_m_[g]) + mat_n_[g];
     const double nnz = static_cast<double>(mat_nnz_[g]);
-    work[i] = {fp32 ? 2.7e-4 * (2 * nnz + 3 * rows) : 5.6e-4 * (2 * nnz + 5 * rows), g};
+    work[i] = {(fp32 ? 1.5e-4 : 5.6e-4) * (2 * nnz + 5 * rows), g};
     fits = fits && vector_bytes(g, 2) <= kClusterSmemMax;
   }
   std::sort(work.begin(), work.end(), std::greater<std::pair<double, int>>());
   // The sizes' exchanges and epilogues.
   const int sizes[5] = {1, 2, 4, 8, 16};
   const double fixed64[5] = {0.7, 2.2, 3.4, 4.2, 5.2};
-  const double fixed32[5] = {5.4, 6.4, 6.8, 7.7, 8.7};
+  const double fixed32[5] = {1.4, 2.0, 2.1, 2.6, 3.4};
   // The setup's passes end in reductions over the cluster (the same unit: a thirtieth of it; 64
   // LPs of 500 x 1,200: 0.66 / 0.55 / 0.61 / 1.09 ms with 1 / 2 / 4 / 8 CTAs).
   const double fixed_setup[5] = {5.5, 9.0, 9.9, 10.6, 11.3};
@@ -442,8 +443,10 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   for (int k = 0; k < 5; ++k) {
     const int size = sizes[k];
     if (size > most || (size > 1 && !fits)) break;
-    // Clusters at once (SMs of a GPC left over by clusters of 8 and 16: an eighth or more).
-    const int slots = std::max(1, per_sm * sms_ / size - (size >= 8 ? per_sm * sms_ / size / 8 : 0));
+    // Clusters at once (SMs of a GPC left over by clusters of 8 and 16: an eighth or more; a quarter
+    // with an SM to a CTA, where 16 clusters of 8 no longer run side by side).
+    const int whole = per_sm * sms_ / size;
+    const int slots = std::max(1, whole - (size >= 8 ? whole / (fp32 ? 4 : 8) : 0));
     const bool shared_sm = !fp32 && static_cast<long long>(std::min(count, slots)) * size > sms_;
     // Largest first, each to the cluster that is free first.
     std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
@@ -469,7 +472,6 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   const int best = plan->size;
   plan->clusters = std::max(1, per_sm * sms_ / best);
   plan->sms = sms_;
-  plan->threads = fp32 ? kThreads32 : kThreads64;
   if (setup) {
     // One launch for all matrices; a matrix whose vectors do not fit leaves them in device
     // memory.
@@ -482,6 +484,7 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   // Every instance in the mode that keeps the most in shared memory, FP64 ones within half of it
   // (two CTAs to an SM) as long as their vectors allow that.
   for (int mode = 0; mode < kModes; ++mode) lists[mode].clear();
+  int most_rows = 0;
   for (int i : order_) {
     const int g = inst_mat_[i];
     const size_t vec = vector_bytes(g, best);
@@ -493,7 +496,21 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
     lists[mode].push_back(i);
     plan->smem[mode] = std::max(plan->smem[mode], need);
     ++plan->group[mode].count;
+    if (mode == kAllShared) most_rows = std::max(most_rows, (mat_m_[g] + mat_n_[g]) / best);
   }
+  if (!fp32) return;
+  // Threads of an FP32 CTA by the largest LP's rows and columns a CTA. Few: 256 threads, all in
+  // registers (every kernel of 512 spilled, the averaging one 1,600 bytes of loads a thread, and an
+  // iteration of 64 LPs of 60 x 120 took 6.9 us; so 2.3). More: 384 (256 LPs of facility location
+  // 40 x 120, averaging, 192 iterations: 10.6 ms with 256, 7.1 with 384, 8.6 with 512). The Halpern
+  // iteration, whose rows take fewer registers, has use for 512 from 3,000 on, to hide the loads of
+  // longer rows (facility location 40 x 80 5.4 with 384, 5.3 with 512; 40 x 160 11.2 and 10.0; but
+  // 160 random LPs of 1,200 x 3,000 6.8 and 7.6).
+  const bool halpern = v_.algorithm == 2;
+  plan->threads[kAllShared] = most_rows <= 1600             ? kThreads32Few
+                              : !halpern || most_rows < 3000 ? kThreads32Mid
+                                                             : kThreads32;
+  plan->threads[kVectorsShared] = plan->threads[kInDevice] = kThreads32;
 }
 
 int Batch::upload_lists(const std::vector<int>* lists, ClusterPlan* plan) {

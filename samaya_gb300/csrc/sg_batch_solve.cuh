@@ -50,19 +50,19 @@ struct Given {
 
 // What the evaluation needs beside the steps' context; evaluate_point is a call of its own, so
 // that its registers are not the step's.
-template <typename T, int MODE>
-struct EvalContext : StepContext<T, MODE> {
+template <typename T, int MODE, typename Share>
+struct EvalContext : StepContext<T, MODE, Share> {
   Given G;
 };
 
 // One iterate's sums (7 evaluation sums in the original space, pdlp.cpp:411-488, and the restart
 // distances of v and y) into e: which 0 the current point, 1 the average, 2 Halpern's T(z). The
 // evaluated vectors take the place of xs and ys.
-template <typename T, int MODE>
-__device__ __noinline__ bool evaluate_point(const EvalContext<T, MODE>* ctx, int which,
+template <typename T, int MODE, typename Share>
+__device__ __noinline__ bool evaluate_point(const EvalContext<T, MODE, Share>* ctx, int which,
                                             double inv_k, double (&e)[9]) {
   constexpr bool kF64 = sizeof(T) == 8;
-  const MatShare<T>& M = ctx->M;
+  const MatShare<T, Share>& M = ctx->M;
   const Exchange<T, MODE>& ex = ctx->ex;
   const SolveState<T, MODE>& S = ctx->S;
   const Second<T>& Z = ctx->Z;
@@ -135,9 +135,9 @@ __device__ __noinline__ bool evaluate_point(const EvalContext<T, MODE>* ctx, int
 
 // Runs one instance (a wait that gave up is in sh.fail). Storage, products and step sums in T
 // (GB300's FP64 pipe is small), the evaluation in FP64.
-template <typename T, int MODE, bool halpern>
+template <typename T, int MODE, bool halpern, typename Share>
 __device__ void solve_instance(const BatchView& b, int inst, ClusterShared& sh,
-                               EvalContext<T, MODE>* ctx, unsigned rank,
+                               EvalContext<T, MODE, Share>* ctx, unsigned rank,
                                unsigned size) {
   constexpr bool kF64 = sizeof(T) == 8;
   const int g = b.inst_mat[inst];
@@ -145,7 +145,7 @@ __device__ void solve_instance(const BatchView& b, int inst, ClusterShared& sh,
                                                   : static_cast<const void*>(b.k_val32));
   const T* tval = reinterpret_cast<const T*>(kF64 ? static_cast<const void*>(b.t_val)
                                                   : static_cast<const void*>(b.t_val32));
-  MatShare<T> M = mat_share<T>(b, g, kval, tval, rank, size);
+  MatShare<T, Share> M = mat_share<T, Share>(b, g, kval, tval, rank, size);
   const int m = M.m;
   const int n = M.n;
   const long long nt = static_cast<long long>(n) + m;
@@ -244,7 +244,7 @@ __device__ void solve_instance(const BatchView& b, int inst, ClusterShared& sh,
       ctx->rest[threadIdx.x] = static_cast<T>(1.0 - 1.0 / (k + 1.0));
     }
     __syncthreads();
-    ok = run_steps<halpern, T, MODE, RowShare<T>, SolveState<T, MODE>>(
+    ok = run_steps<halpern, T, MODE, Share, SolveState<T, MODE>>(
         ctx, static_cast<int>(steps), static_cast<T>(tau), static_cast<T>(sigma), [] {});
     t += steps;
     k_since += steps;
@@ -264,7 +264,7 @@ __device__ void solve_instance(const BatchView& b, int inst, ClusterShared& sh,
     for (int w = halpern ? 1 : 0; w < 2; ++w) {
       cluster_sync(size);  // every CTA has read xs and ys, their last entries in place
       double e[9] = {};
-      ok = ok && evaluate_point<T, MODE>(ctx, halpern ? 2 : w, inv_k, e);
+      ok = ok && evaluate_point<T, MODE, Share>(ctx, halpern ? 2 : w, inv_k, e);
       if (w == 0) {
 #pragma unroll
         for (int q = 0; q < 7; ++q) a[q] = e[q];
@@ -434,57 +434,68 @@ __device__ __forceinline__ int next_instance(unsigned* queue, ClusterShared& sh,
 
 }  // namespace
 
-template <typename T>
-constexpr int solve_threads() {
-  return sizeof(T) == 8 ? kThreads64 : kThreads32;
-}
-
-template <typename T, int MODE, bool HALPERN>
-__global__ void __launch_bounds__(solve_threads<T>(), sizeof(T) == 8 ? 2 : 1)
+template <typename T, int MODE, bool HALPERN, int THREADS>
+__global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 2 : 1)
     batch_solve_kernel(BatchView b, InstanceList list) {
+  // (FP32 with 512 threads: 128 registers and one slice's loads on their way are too few.)
+  using Share = RowShare<T, sizeof(T) == 4 && THREADS == kThreads32>;
   __shared__ ClusterShared sh;
-  __shared__ EvalContext<T, MODE> ctx;
+  __shared__ EvalContext<T, MODE, Share> ctx;
   const unsigned rank = cluster_rank();
   const unsigned size = cluster_size();
   cluster_init(sh, size);
   for (;;) {
     const int q = next_instance(b.queue + MODE, sh, rank, size);
     if (q >= list.count) break;
-    solve_instance<T, MODE, HALPERN>(b, list.inst[q], sh, &ctx, rank, size);
+    solve_instance<T, MODE, HALPERN, Share>(b, list.inst[q], sh, &ctx, rank, size);
   }
   cluster_sync(size);
 }
 
-// go() with the kernel of a mode.
+// go() with the kernel of a mode and number of threads (Batch::plan_clusters).
 template <typename T, typename Go>
-auto with_solve_kernel(int algorithm, int mode, const Go& go) {
+auto with_solve_kernel(int algorithm, int mode, int threads, const Go& go) {
   const bool h = algorithm == 2;
-  if (mode == kAllShared) {
-    return h ? go(batch_solve_kernel<T, kAllShared, true>)
-             : go(batch_solve_kernel<T, kAllShared, false>);
+  if constexpr (sizeof(T) == 4) {
+    if (mode == kAllShared && threads == kThreads32Few) {
+      return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads32Few>)
+               : go(batch_solve_kernel<T, kAllShared, false, kThreads32Few>);
+    }
+    if (mode == kAllShared && threads == kThreads32Mid) {
+      return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads32Mid>)
+               : go(batch_solve_kernel<T, kAllShared, false, kThreads32Mid>);
+    }
+    if (mode == kAllShared) return go(batch_solve_kernel<T, kAllShared, true, kThreads32>);
+  } else if (mode == kAllShared) {
+    return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads64>)
+             : go(batch_solve_kernel<T, kAllShared, false, kThreads64>);
   }
+  constexpr int kMost = sizeof(T) == 4 ? kThreads32 : kThreads64;
   if (mode == kVectorsShared) {
-    return h ? go(batch_solve_kernel<T, kVectorsShared, true>)
-             : go(batch_solve_kernel<T, kVectorsShared, false>);
+    return h ? go(batch_solve_kernel<T, kVectorsShared, true, kMost>)
+             : go(batch_solve_kernel<T, kVectorsShared, false, kMost>);
   }
-  return h ? go(batch_solve_kernel<T, kInDevice, true>)
-           : go(batch_solve_kernel<T, kInDevice, false>);
+  return h ? go(batch_solve_kernel<T, kInDevice, true, kMost>)
+           : go(batch_solve_kernel<T, kInDevice, false, kMost>);
 }
 
 template <typename T>
 cudaError_t launch_solve(const BatchView& b, const ClusterPlan& p, int mode, cudaStream_t s) {
   const InstanceList list = p.group[mode];
   const int clusters = list.count < p.clusters ? list.count : p.clusters;
-  return with_solve_kernel<T>(b.algorithm, mode, [&](auto kernel) {
-    return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], s, b, list);
+  const int threads = p.threads[mode];
+  return with_solve_kernel<T>(b.algorithm, mode, threads, [&](auto kernel) {
+    return launch_clusters(kernel, p.size, clusters, threads, p.smem[mode], s, b, list);
   });
 }
 
 template <typename T>
 bool solve_fits(const ClusterPlan& p, int algorithm) {
   for (int mode = 0; mode < kModes; ++mode) {
-    if (p.group[mode].count > 0 && !with_solve_kernel<T>(algorithm, mode, [&](auto kernel) {
-          return clusters_fit(kernel, p.size, p.threads, p.smem[mode]);
+    const int threads = p.threads[mode];
+    if (p.group[mode].count > 0 &&
+        !with_solve_kernel<T>(algorithm, mode, threads, [&](auto kernel) {
+          return clusters_fit(kernel, p.size, threads, p.smem[mode]);
         })) {
       return false;
     }

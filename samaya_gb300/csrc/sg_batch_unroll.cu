@@ -435,7 +435,7 @@ bool unroll_fits(const ClusterPlan& p, int adjoint) {
     for (bool alone : {false, true}) {
       if (p.group[mode].count > 0 &&
           !with_unroll_kernel(adjoint, mode, alone, [&](auto kernel) {
-            return clusters_fit(kernel, p.size, p.threads, p.smem[mode]);
+            return clusters_fit(kernel, p.size, p.threads[mode], p.smem[mode]);
           })) {
         return false;
       }
@@ -458,7 +458,7 @@ cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const Cluster
                              : p.size == 4 ? p.sms / p.size * 3 / 4
                                            : p.sms / p.size / 2;
     return with_unroll_kernel(adjoint, mode, clusters <= side_by_side, [&](auto kernel) {
-      return launch_clusters(kernel, p.size, clusters, p.threads, p.smem[mode], gst, b, u, list);
+      return launch_clusters(kernel, p.size, clusters, p.threads[mode], p.smem[mode], gst, b, u, list);
     });
   });
 }

@@ -46,10 +46,13 @@
 
 namespace sg {
 
-// Threads per CTA, 128 registers each. FP64 kernels, bound by the FP64 pipe, take 256, so that
-// two CTAs share an SM and one's exchange overlaps the other's sums; FP32 steps, bound by the
-// latency of the nonzeros' loads, 512.
+// Threads per CTA. FP64 kernels, bound by the FP64 pipe, take 256 of 128 registers, so that two CTAs
+// share an SM and one's exchange overlaps the other's sums. An FP32 solve has an SM to a CTA and is
+// bound by the latency of its chains; how many threads share the registers follows the rows
+// (Batch::plan_clusters): 256 of 255 registers, 384 of 168, 512 of 128.
 constexpr int kThreads64 = 256;
+constexpr int kThreads32Few = 256;
+constexpr int kThreads32Mid = 384;
 constexpr int kThreads32 = 512;
 constexpr int kMaxWarps = kThreads32 / 32;
 constexpr int kMaxCluster = 16;
@@ -382,8 +385,8 @@ struct Sender {
   }
 };
 
-// A CTA's share of an operator by rows.
-template <typename T>
+// A CTA's share of an operator by rows. PAIRS: walked two slices at a time (walk_pairs).
+template <typename T, bool PAIRS = false>
 struct alignas(16) RowShare {
   static constexpr bool kTasks = false;
   const int2* sl;  // per row (position): first nonzero, length
@@ -422,8 +425,8 @@ __device__ __forceinline__ int nonzero_at(int start, int len, int k) {
 }
 
 // f(at) for every own row of the share (thread tid takes own rows tid, tid + threads, ...).
-template <typename T, typename F>
-__device__ __forceinline__ void each_own(const RowShare<T>& A, const F& f) {
+template <typename T, bool PAIRS, typename F>
+__device__ __forceinline__ void each_own(const RowShare<T, PAIRS>& A, const F& f) {
   const int own = A.own();
   for (int l = threadIdx.x; l < own; l += blockDim.x) {
     const At at{l >> A.slice, l & ((1 << A.slice) - 1), l, A.position(l)};
@@ -453,9 +456,9 @@ __device__ __forceinline__ void settle_counts(Exchange<V, MODE>& ex) {
 }
 
 // Fills the masks of the own rows and columns and the byte counts; ends with a cluster barrier.
-template <typename V, int MODE, typename T>
-__device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShare<T>& K,
-                                            const RowShare<T>& Kt) {
+template <typename V, int MODE, typename T, bool PAIRS>
+__device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShare<T, PAIRS>& K,
+                                            const RowShare<T, PAIRS>& Kt) {
   ClusterShared& sh = *ex.sh;
   ex.tx[0] = ex.tx[1] = 0;
   if (ex.size == 1) {
@@ -468,7 +471,7 @@ __device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShar
   for (int which = 0; which < 2; ++which) {
     // Column j is read by the CTAs that own the rows of its nonzeros, row i by the CTAs that
     // own the columns of its nonzeros.
-    const RowShare<T>& A = which == 0 ? Kt : K;
+    const RowShare<T, PAIRS>& A = which == 0 ? Kt : K;
     const int other = which == 0 ? K.slice : Kt.slice;
     unsigned short* mask = which == 0 ? ex.cmask() : ex.rmask();
     each_own(A, [&](const At& at) {
@@ -558,8 +561,8 @@ __device__ __forceinline__ void keep_branch(unsigned mask) { __syncwarp(mask); }
 // their loads overlap: lane l takes nonzeros l, l + 32, ..., and the shuffle trees of the rows are
 // folded into one (each step halves the sums a lane carries: 6 additions in place of 20, 9 in
 // place of 40); every row's tree is the same as alone.
-template <bool NC, bool MAXRED, typename T, typename ACC, typename Prod>
-__device__ __forceinline__ ACC long_rows(const RowShare<T> A, const Prod& prod, bool valid,
+template <bool NC, bool MAXRED, typename T, bool PAIRS, typename ACC, typename Prod>
+__device__ __forceinline__ ACC long_rows(const RowShare<T, PAIRS> A, const Prod& prod, bool valid,
                                          int p, ACC s) {
   constexpr int kTogether = sizeof(ACC) == 8 ? 4 : 8;
   const int lane = threadIdx.x & 31;
@@ -639,12 +642,12 @@ __device__ __forceinline__ ACC long_rows(const RowShare<T> A, const Prod& prod, 
 // so that the updates of a slice run side by side. ready() waits for the gathered vector after
 // the first loads are on their way (every thread calls it once; false ends the walk).
 //
-// FP64 storage (walk_one): a slice at a time, four steps' nonzeros loaded while the four before
-// are summed (of the same slice or the warp's slice before).
+// walk_one: a slice at a time, four steps' nonzeros loaded while the four before are summed (of the
+// same slice or the warp's slice before).
 template <bool NC, bool MAXRED, typename T, typename Prod, typename Init, typename F,
           typename Ready>
-__device__ __forceinline__ bool walk_one(const RowShare<T> A, const Prod& prod,
-                                          const Init& init, const F& f, const Ready& ready) {
+__device__ __forceinline__ bool walk_one(const RowShare<T, false> A, const Prod& prod,
+                                         const Init& init, const F& f, const Ready& ready) {
   using ACC = decltype(prod(T(), 0));
   constexpr int B = kBatch;
   const int lane = threadIdx.x & 31;
@@ -723,10 +726,10 @@ __device__ __forceinline__ bool walk_one(const RowShare<T> A, const Prod& prod,
   return true;
 }
 
-// FP32 storage (walk_pairs): two slices at a time, so that 16 loads a thread are on their way.
+// walk_pairs: two slices at a time, so that 16 loads a thread are on their way.
 template <bool NC, bool MAXRED, typename T, typename Prod, typename Init, typename F,
           typename Ready>
-__device__ __forceinline__ bool walk_pairs(const RowShare<T> A, const Prod& prod,
+__device__ __forceinline__ bool walk_pairs(const RowShare<T, true> A, const Prod& prod,
                                            const Init& init, const F& f, const Ready& ready) {
   using ACC = decltype(prod(T(), 0));
   constexpr int B = kBatch;
@@ -800,14 +803,14 @@ __device__ __forceinline__ bool walk_pairs(const RowShare<T> A, const Prod& prod
   return true;
 }
 
-template <bool NC, bool MAXRED, typename T, typename Prod, typename Init, typename F,
+template <bool NC, bool MAXRED, typename T, bool PAIRS, typename Prod, typename Init, typename F,
           typename Ready>
-__device__ __forceinline__ bool walk_rows(const RowShare<T>& A, const Prod& prod,
+__device__ __forceinline__ bool walk_rows(const RowShare<T, PAIRS>& A, const Prod& prod,
                                           const Init& init, const F& f, const Ready& ready) {
-  if constexpr (sizeof(T) == 8) {
-    return walk_one<NC, MAXRED>(A, prod, init, f, ready);
-  } else {
+  if constexpr (PAIRS) {
     return walk_pairs<NC, MAXRED>(A, prod, init, f, ready);
+  } else {
+    return walk_one<NC, MAXRED>(A, prod, init, f, ready);
   }
 }
 

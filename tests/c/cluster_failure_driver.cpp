@@ -111,8 +111,8 @@ int main() {
             const BatchView b = p.view(which == 1 || which == 3 ? 2 : 0);
             const InstanceList list{p.order, kInstances};
             if (which < 2) batch_setup_kernel(b, 1u << 20);
-            if (which == 2) batch_solve_kernel<double, kAllShared, false>(b, list);
-            if (which == 3) batch_solve_kernel<double, kAllShared, true>(b, list);
+            if (which == 2) batch_solve_kernel<double, kAllShared, false, kThreads64>(b, list);
+            if (which == 3) batch_solve_kernel<double, kAllShared, true, kThreads64>(b, list);
             if (which == 4) unroll_kernel<false, kAllShared>(b, p.unroll(), list);
             if (which == 5) unroll_kernel<true, kAllShared>(b, p.unroll(), list);
           });

@@ -37,7 +37,7 @@ def test_every_cta_leaves_together(tmp_path):
         "sg_batch.cu": _cut(_text("sg_batch.cu"),
                             "__global__ void batch_deadline_kernel") + "}\n",
         "sg_batch_solve.cuh": _cut(_text("sg_batch_solve.cuh"),
-                                   "// go() with the kernel of a mode.") + "}\n",
+                                   "// go() with the kernel of a mode and") + "}\n",
         "sg_batch_unroll.cu": _cut(_text("sg_batch_unroll.cu"),
                                    "namespace {\n\n// go() with the kernel of a mode") + "}\n",
     }
