@@ -1937,22 +1937,28 @@ void launch_dual_step(const Ctl* ctl, const OpView<T>& K, const IterView<T>& it,
                  ctl, K, it, j, grid, dual_smem_bytes<T>(K.ts), behind, s);
 }
 
-// The launch of a primal step: columns of two nonzeros, or tiles.
+// The launch of a primal step: columns of two nonzeros, or tiles. In FP64 two_nonzero_columns takes
+// 80,000 columns and more, when every SM has a CTA of 512: fewer keep more of the FP64 pipes busy in
+// tiles (transportation LPs, 320 iterations, ms, by columns against tiles: 100 x 200 3.89 and 3.62,
+// 150 x 400 5.53 and 5.22, 200 x 500 6.10 and 6.20, 301 x 703 5.10 and 5.52, 500 x 1,000 7.46 and
+// 8.08). In FP32 all (50 x 130 3.70 and 3.81, 60 x 200 3.30 and 3.29, 100 x 200 3.10 and 3.20, 500 x
+// 1,000 5.32 and 5.55).
 template <typename T>
-int primal_variant(const TileSet& ts) {
-  return ts.uniform_len == 2 ? 3 : ts.variant == 1 ? 1 : 0;
+int primal_variant(const OpView<T>& Kt) {
+  const bool wide = Kt.ts.uniform_len == 2 && (sizeof(T) == 4 || Kt.rows >= 80000);
+  return wide ? 3 : Kt.ts.variant == 1 ? 1 : 0;
 }
 template <typename T>
 int primal_grid(const OpView<T>& Kt, int grid) {
   constexpr int kColumns = kBlock * kWide<T>;
-  return Kt.ts.uniform_len == 2 ? (Kt.rows + kColumns - 1) / kColumns : grid;
+  return primal_variant(Kt) == 3 ? (Kt.rows + kColumns - 1) / kColumns : grid;
 }
 
 template <typename T>
 void launch_primal_step(const Ctl* ctl, const OpView<T>& Kt, const IterView<T>& it, int j,
                         int grid, cudaStream_t s, bool behind) {
   if (Kt.ts.ntiles == 0) return;
-  const int v = primal_variant<T>(Kt.ts);
+  const int v = primal_variant(Kt);
   launch_step<T>(v == 3   ? primal_step_kernel<T, 3>
                  : v == 1 ? primal_step_kernel<T, 1>
                           : primal_step_kernel<T, 0>,
@@ -1964,7 +1970,7 @@ template <typename T>
 void launch_halpern_primal(const Ctl* ctl, const OpView<T>& Kt, const IterView<T>& it, int j,
                            int grid, cudaStream_t s, bool behind) {
   if (Kt.ts.ntiles == 0) return;
-  const int v = primal_variant<T>(Kt.ts);
+  const int v = primal_variant(Kt);
   launch_step<T>(v == 3   ? halpern_primal_kernel<T, 3>
                  : v == 1 ? halpern_primal_kernel<T, 1>
                           : halpern_primal_kernel<T, 0>,
