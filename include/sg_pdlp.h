@@ -92,7 +92,10 @@ typedef struct sg_pdlp_opts {
                                 the power-law LP's long rows, which are bound by their
                                 scattered gathers, not by the nonzero stream) */
   int tile_nnz;              /* built-in rule: nonzeros per tile (a power of two from 256 to
-                                16384); 0 (default): about 8 tiles per SM */
+                                16384); 0 (default): about 8 tiles per SM. (A small LP's
+                                iterations run on one thread-block cluster, without tiles, unless
+                                tile_nnz, tile_split, row_groups 1 or segment_staging asks for a
+                                shape of the step launches.) */
 } sg_pdlp_opts;
 
 /* Algorithm variants. REFERENCE follows samaya's PDLP step for step (L2 Ruiz, fixed step

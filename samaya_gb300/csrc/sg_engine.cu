@@ -916,11 +916,16 @@ int Engine::alloc_all(std::string* err) {
 //         777 x 2,049                        7.8 against 3.6 / 3.3 / 3.4
 //         2,000 x 5,000                      7.8 against 4.8 / 4.7 / 4.4
 //         5,000 x 10,000 (195,000)           8.1 against  -  / 8.2 / 7.4
+// A caller who asks for a shape of the step launches gets them.
 // The steps a row takes at most (make_tasks), FP64: 4 / 8 / 16 / 32 with 777 x 2,049 on 16 CTAs
 // 4.1 / 4.3 / 5.0 / 4.9, facility 40 x 150 4.3 / 4.3 / 4.4 / 4.9, 2,000 x 5,000 6.9 / 6.2 / 6.1 /
 // 6.0, 3,500 x 7,000 8.6 / 7.6 / 7.4 / 7.1.
 void Engine::plan_chunk() {
   if (m_ <= 0 || n_ <= 0 || nnz_ <= 0) return;
+  if (opt_.tile_nnz > 0 || opt_.tile_split > 0 || opt_.row_groups > 0 ||
+      opt_.segment_staging > 0) {
+    return;
+  }
   const long long work = 2 * nnz_ + 5 * (static_cast<long long>(n_) + m_);
   constexpr long long kMost64 = 220000, kMost32 = 300000;
   if (work > kMost32) return;
