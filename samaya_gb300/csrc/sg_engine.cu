@@ -905,8 +905,9 @@ int Engine::alloc_all(std::string* err) {
 }
 
 // Whether the chunk's iterations run on a cluster (chunk_kernel), and on how many CTAs: up to where
-// 16 SMs take as long as the step launches do. Measured, us an iteration with its share of the
-// evaluation, w = 2 nnz + 5 (n + m), step launches against 4 / 8 / 16 CTAs:
+// 16 SMs take as long as the step launches do or, in FP64, their shared memory is full. Measured, us
+// an iteration with its share of the evaluation, w = 2 nnz + 5 (n + m), step launches against 4 / 8
+// / 16 CTAs:
 //   FP64  200 x 500 (w 9,500)                9.1 against 3.4 / 3.3 / 3.5
 //         777 x 2,049 (39,000)               9.4 against  -  / 4.7 / 4.1
 //         facility 40 x 150 (97,000)        14.4 against 7.0 / 5.3 / 4.4
@@ -916,6 +917,13 @@ int Engine::alloc_all(std::string* err) {
 //         777 x 2,049                        7.8 against 3.6 / 3.3 / 3.4
 //         2,000 x 5,000                      7.8 against 4.8 / 4.7 / 4.4
 //         5,000 x 10,000 (195,000)           8.1 against  -  / 8.2 / 7.4
+// Where the sides meet, 320 iterations, ms, step launches against 16 CTAs.
+// FP64, the largest that fit: 3,500 x 8,500 of 6 a column (w 162,000) 3.89 against 3.30; 2,500 x 5,500
+// of 16 (216,000) 7.86 against 4.14. But a row is one warp's chain of additions, 63 ns for every 32
+// nonzeros, as much as 66 w a nonzero: 2,000 x 5,000 with one row of 2,600 / 3,000 / 3,400 / 4,000 3.92 /
+// 3.89 / 3.95 / 3.95 against 3.59 / 3.83 / 4.08 / 4.47, 100 x 6,000 with one of 3,000 / 4,500 4.06 / 4.08
+// against 4.10 / 4.99, 300 x 4,000 of 3,000 / 4,000 4.30 / 4.28 against 3.72 / 4.34, 1,000 x 3,500 of 3,500
+// 4.48 against 4.00.
 // A caller who asks for a shape of the step launches gets them.
 // The steps a row takes at most (make_tasks), FP64: 4 / 8 / 16 / 32 with 777 x 2,049 on 16 CTAs
 // 4.1 / 4.3 / 5.0 / 4.9, facility 40 x 150 4.3 / 4.3 / 4.4 / 4.9, 2,000 x 5,000 6.9 / 6.2 / 6.1 /
@@ -926,14 +934,16 @@ void Engine::plan_chunk() {
       opt_.segment_staging > 0) {
     return;
   }
-  const long long work = 2 * nnz_ + 5 * (static_cast<long long>(n_) + m_);
-  constexpr long long kMost64 = 220000, kMost32 = 300000;
+  const long long entries = static_cast<long long>(n_) + m_;
+  const long long work = 2 * nnz_ + 5 * entries;
+  constexpr long long kMost64 = 220000, kMostChain64 = 310000, kMost32 = 300000;
   if (work > kMost32) return;
-  auto longest = [](const std::vector<int>& ptr) {
-    int most = 0;
-    for (size_t r = 0; r + 1 < ptr.size(); ++r) most = std::max(most, ptr[r + 1] - ptr[r]);
-    return most;
-  };
+  int longest = 0;
+  for (const std::vector<int>* ptr : {&K_.host_ptr, &Kt_.host_ptr}) {
+    for (size_t r = 0; r + 1 < ptr->size(); ++r) {
+      longest = std::max(longest, (*ptr)[r + 1] - (*ptr)[r]);
+    }
+  }
   auto plan = [&](auto* c, bool fixed_order) {
     const int size = work <= (fixed_order ? 12000 : 6000)    ? 4
                      : work <= (fixed_order ? 50000 : 25000) ? 8
@@ -952,12 +962,10 @@ void Engine::plan_chunk() {
       c->view.size = 0;
     }
   };
-  if (work <= kMost64) plan(&chunk64_, false);
+  if (work <= kMost64 && work + 66LL * longest <= kMostChain64) plan(&chunk64_, false);
   // FP32 sums keep the step kernels' order: rows longer than kWarpRowMin have another. (The
   // refinement's inner problems have a right-hand side, which these steps do not read.)
-  if (switch_ && std::max(longest(K_.host_ptr), longest(Kt_.host_ptr)) <= kWarpRowMin) {
-    plan(&chunk32c_, true);
-  }
+  if (switch_ && longest <= kWarpRowMin) plan(&chunk32c_, true);
 }
 
 namespace {

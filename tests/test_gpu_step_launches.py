@@ -2,7 +2,7 @@
 which share no step code: a caller who asks for a shape of the step launches (here tile_nnz) gets
 them. The cluster's iterations, the batch's (the cluster's steps, one LP to a cluster) and the step
 launches end at the same points past restarts; the rows that a solve leaves out of the step launches
-change no bit of them.
+change no bit of them; and an LP with one long row takes them by itself.
 
 Tolerances, of (1 + max |value|): test_gpu_batch_clusters.py's 2e-10 for 100 iterations in FP64, times
 4 for 400 and times 10 for primal weights that restarts move (they come from the iterates), 8e-9: 1e-8.
@@ -90,3 +90,14 @@ def test_inert_rows_left_out_of_the_step_launches(engine, algorithm, precision):
             assert _on_steps(out[-1])
         a, b = out
         assert np.array_equal(a.x, b.x) and np.array_equal(a.y, b.y)
+
+
+@pytest.mark.parametrize("longest,on_steps", [(4141, False), (4142, True), (5000, True)])
+def test_one_long_row(engine, oracle, longest, on_steps):
+    """A row is a warp's chain on the cluster; step launches split it."""
+    lp = _lp(5000, [longest] + [6] * 200, longest)
+    assert (2 * lp.nnz + 5 * (lp.n + lp.m) + 66 * longest > 310000) == on_steps
+    r = _solve(engine, lp, 100, algorithm=engine.REFERENCE)
+    assert _on_steps(r) == on_steps
+    ref = oracle.pdlp_solve(*lp.arrays(), tol=1e-30, max_iter=100)
+    assert _differs(r.x, ref.x) <= 1e-8 and _differs(r.y, ref.y) <= 1e-8
