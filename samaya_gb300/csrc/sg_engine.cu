@@ -917,7 +917,15 @@ int Engine::alloc_all(std::string* err) {
 //         777 x 2,049                        7.8 against 3.6 / 3.3 / 3.4
 //         2,000 x 5,000                      7.8 against 4.8 / 4.7 / 4.4
 //         5,000 x 10,000 (195,000)           8.1 against  -  / 8.2 / 7.4
-// Where the sides meet, 320 iterations, ms, step launches against 16 CTAs.
+// Where the sides meet, 320 iterations, ms, step launches against 16 CTAs. FP32, by 2 nnz + 8 (n + m)
+// (the rows' and columns' own work weighs more than in FP64, whose additions take the pipe):
+//   6 a column   5,000 x 10,000 (240,000)    3.52 against 3.35
+//                5,000 x 12,000 (280,000)    3.74 against 3.58
+//                5,500 x 13,000 (304,000)    3.80 against 3.76
+//                6,000 x 14,000 (328,000)    3.70 against 3.92
+//                7,000 x 14,500 (346,000)    3.61 against 4.01
+//   14, 16, 18   3,000 x 7,000 (276,000)     5.73 against 4.59, (304,000) 5.73 against 5.25,
+//                (332,000) 5.95 and more (rows past 32 nonzeros take the step launches longer)
 // FP64, the largest that fit: 3,500 x 8,500 of 6 a column (w 162,000) 3.89 against 3.30; 2,500 x 5,500
 // of 16 (216,000) 7.86 against 4.14. But a row is one warp's chain of additions, 63 ns for every 32
 // nonzeros, as much as 66 w a nonzero: 2,000 x 5,000 with one row of 2,600 / 3,000 / 3,400 / 4,000 3.92 /
@@ -936,8 +944,10 @@ void Engine::plan_chunk() {
   }
   const long long entries = static_cast<long long>(n_) + m_;
   const long long work = 2 * nnz_ + 5 * entries;
-  constexpr long long kMost64 = 220000, kMostChain64 = 310000, kMost32 = 300000;
-  if (work > kMost32) return;
+  constexpr long long kMost64 = 220000, kMostChain64 = 310000;
+  const long long most32 = nnz_ > 32LL * m_ ? 330000 : 300000;
+  const bool small32 = switch_ && 2 * nnz_ + 8 * entries <= most32;
+  if (work > kMost64 && !small32) return;
   int longest = 0;
   for (const std::vector<int>* ptr : {&K_.host_ptr, &Kt_.host_ptr}) {
     for (size_t r = 0; r + 1 < ptr->size(); ++r) {
@@ -965,7 +975,7 @@ void Engine::plan_chunk() {
   if (work <= kMost64 && work + 66LL * longest <= kMostChain64) plan(&chunk64_, false);
   // FP32 sums keep the step kernels' order: rows longer than kWarpRowMin have another. (The
   // refinement's inner problems have a right-hand side, which these steps do not read.)
-  if (switch_ && longest <= kWarpRowMin) plan(&chunk32c_, true);
+  if (small32 && longest <= kWarpRowMin) plan(&chunk32c_, true);
 }
 
 namespace {

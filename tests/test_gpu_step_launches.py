@@ -101,3 +101,16 @@ def test_one_long_row(engine, oracle, longest, on_steps):
     assert _on_steps(r) == on_steps
     ref = oracle.pdlp_solve(*lp.arrays(), tol=1e-30, max_iter=100)
     assert _differs(r.x, ref.x) <= 1e-8 and _differs(r.y, ref.y) <= 1e-8
+
+
+@pytest.mark.parametrize("m,n,on_steps", [(5400, 12000, False), (5900, 13400, True)])
+def test_fp32_limit(engine, m, n, on_steps):
+    """2 nnz + 8 (n + m) below and above 300,000: the same iterations on both sides."""
+    rng = np.random.default_rng(m)
+    lp = _lp(n, rng.multinomial(6 * n, np.full(m, 1.0 / m)), m)
+    assert (2 * lp.nnz + 8 * (lp.n + lp.m) > 300000) == on_steps
+    options = dict(precision=engine.FP32_THEN_FP64, algorithm=engine.HALPERN)
+    r = _solve(engine, lp, 100, **options)
+    assert _on_steps(r) == on_steps
+    ref = _solve(engine, lp, 100, tile_nnz=512, **options)
+    assert _differs(r.x, ref.x) <= 1e-3 and _differs(r.y, ref.y) <= 1e-3
