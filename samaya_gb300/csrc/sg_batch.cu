@@ -25,10 +25,12 @@ namespace sg {
 // in all) when the matrices fill the chip, by the exchanges when a single matrix is set up.
 namespace {
 
-template <int MODE>
+template <int MODE, int WALK>
 __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
                              unsigned rank, unsigned size) {
-  MatShare<double> M = mat_share<double>(b, g, b.k_val0, b.t_val0, rank, size);
+  using Share = RowShare<double, WALK>;
+  MatShare<double, Share> M =
+      mat_share<double, Share>(b, g, b.k_val0, b.t_val0, rank, size);
   const int m = M.m;
   const int n = M.n;
   // By position: scales, their reciprocals, scratch.
@@ -40,8 +42,8 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
   double* rn = irs;
   Exchange<double, MODE> ex = make_exchange<double, MODE>(
       M, sh, b.spill + b.mat_col_off[g] + b.mat_row_off[g] + 2 * g, rank, size);
-  const RowShare<double>& K0 = M.K;
-  const RowShare<double>& T0 = M.Kt;
+  const Share& K0 = M.K;
+  const Share& T0 = M.Kt;
   const Zero<double> zero_init;
   // Relative-residual scales of the original matrix (pdlp.cpp:377-394).
   double norms[2] = {0.0, 0.0};
@@ -124,7 +126,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
   double* kv = b.k_val + M.kz;
   double* tv = b.t_val + M.tz;
   {
-    auto scale_rows = [&](const RowShare<double>& A, const double* own, const double* other,
+    auto scale_rows = [&](const Share& A, const double* own, const double* other,
                           double* out, float* out32, double* scale) {
       const int lane = threadIdx.x & 31;
       const int stride = 1 << A.slice;
@@ -146,7 +148,7 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
           if (out32 != nullptr) out32[q] = static_cast<float>(v);
         };
         if (sl.y <= 32) {
-          for (int k = 0; k < sl.y; ++k) put(sl.x + (k << 5), own_scale);
+          for (int k = 0; k < sl.y; ++k) put(A.place(sl, k), own_scale);
         }
         unsigned pending = __ballot_sync(0xffffffffu, sl.y > 32);
         while (pending != 0u) {
@@ -166,9 +168,9 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
   // Power iteration (pdlp.cpp:36-103): ys holds u, xs holds v = A_eq' u.
   double L = 1.0;
   if (m > 0) {
-    RowShare<double> K = K0;
+    Share K = K0;
     K.val = kv;
-    RowShare<double> T = T0;
+    Share T = T0;
     T.val = tv;
     double ss[1] = {0.0};
     each_own(K, [&](const At& at) {
@@ -230,7 +232,9 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
 
 }  // namespace
 
-__global__ void __launch_bounds__(kThreads64, 2) batch_setup_kernel(BatchView b, unsigned smem_bytes) {
+template <int WALK>
+__global__ void __launch_bounds__(kThreads64, 2) batch_setup_kernel(BatchView b,
+                                                                    unsigned smem_bytes) {
   __shared__ ClusterShared sh;
   const unsigned rank = cluster_rank();
   const unsigned size = cluster_size();
@@ -238,9 +242,9 @@ __global__ void __launch_bounds__(kThreads64, 2) batch_setup_kernel(BatchView b,
   const int g = blockIdx.x / size;
   if (cluster_vector_bytes(b.mat_n[g], b.mat_m[g], b.mat_slice[2 * g + 1], b.mat_slice[2 * g],
                            static_cast<int>(size), sizeof(double)) <= smem_bytes) {
-    setup_matrix<kVectorsShared>(b, g, sh, rank, size);
-  } else {
-    setup_matrix<kInDevice>(b, g, sh, rank, size);
+    setup_matrix<kVectorsShared, WALK>(b, g, sh, rank, size);
+  } else if constexpr (WALK == kWalkOne) {
+    setup_matrix<kInDevice, WALK>(b, g, sh, rank, size);
   }
   cluster_sync(size);  // no CTA leaves while another may still send to it
 }
@@ -262,12 +266,14 @@ cudaError_t launch_batch(const BatchView& b, const ClusterPlan& setup, const Clu
 }
 
 bool setup_fits(const ClusterPlan& p) {
-  return clusters_fit(batch_setup_kernel, p.size, kThreads64, p.smem[0]);
+  return p.small ? clusters_fit(batch_setup_kernel<kWalkLanes>, p.size, kThreads64, p.smem[0])
+                 : clusters_fit(batch_setup_kernel<kWalkOne>, p.size, kThreads64, p.smem[0]);
 }
 
 cudaError_t launch_batch_setup(const BatchView& b, const ClusterPlan& setup, cudaStream_t s) {
-  return launch_clusters(batch_setup_kernel, setup.size, b.nmat, kThreads64, setup.smem[0], s, b,
-                         static_cast<unsigned>(setup.smem[0]));
+  return launch_clusters(
+      setup.small ? batch_setup_kernel<kWalkLanes> : batch_setup_kernel<kWalkOne>, setup.size,
+      b.nmat, kThreads64, setup.smem[0], s, b, static_cast<unsigned>(setup.smem[0]));
 }
 
 }  // namespace sg

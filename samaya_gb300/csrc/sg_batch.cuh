@@ -113,6 +113,7 @@ struct ClusterPlan {
   int size = 0;
   int clusters = 1;
   int sms = 0;  // SMs of the device
+  bool small = false;  // the kernels of kWalkLanes (every instance in kAllShared)
   int threads[kModes] = {kThreads64, kThreads64, kThreads64};
   InstanceList group[kModes];
   size_t smem[kModes] = {0, 0, 0};
@@ -231,6 +232,7 @@ class Batch {
   int sms_ = 148;
   long long total_vec_ = 0, total_rows_ = 0;
   std::vector<int> mat_m_, mat_n_, inst_mat_, mat_slice_, order_;
+  bool small_ = false;  // the layout of kWalkLanes
   std::vector<long long> mat_nnz_;
   ClusterPlan setup_plan_, solve_plan_, forward_plan_, adjoint_plan_;
   int* wait_host_ = nullptr;  // pinned copy of the wait flag

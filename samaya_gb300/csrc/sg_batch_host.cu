@@ -114,6 +114,14 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   std::vector<RowOrder> korder(nmat), torder(nmat);
   std::vector<std::vector<int>> kptr(nmat);
   int max_m = 0;
+  // LPs of at most 512 rows and columns take several lanes a row (kWalkLanes; 32 >> slice): 64
+  // unrolled LPs of 40 x 88, 200 iterations forward and backward, 2.54 ms with a lane a row, 1.95
+  // now, of 110 x 242 2.83 and 2.47; 160 solves of 60 x 120, 192 iterations, 1.82 and 1.64 in FP64,
+  // 1.59 and 1.52 in FP32. (Kernels that allow for both took 1% longer on the larger ones.)
+  bool small = true;
+  for (int g = 0; g < nmat; ++g) {
+    small = small && static_cast<long long>(mat_m[g]) + mat_n[g] <= 512;
+  }
   for (int g = 0; g < nmat; ++g) {
     const int m = mat_m[g], n = mat_n[g];
     max_m = std::max(max_m, m);
@@ -132,8 +140,8 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
     for (int i = 0; i < m; ++i) kp[i + 1] += kp[i];
     std::vector<int> tp(static_cast<size_t>(n) + 1);
     for (int j = 0; j <= n; ++j) tp[j] = static_cast<int>(cp[j]);
-    korder[g] = order_rows(kp.data(), m);
-    torder[g] = order_rows(tp.data(), n);
+    korder[g] = order_rows(kp.data(), m, small);
+    torder[g] = order_rows(tp.data(), n, small);
     slice[2 * g] = korder[g].slice;
     slice[2 * g + 1] = torder[g].slice;
     kd_off[g + 1] = kd_off[g] + slices_of(korder[g]);
@@ -168,10 +176,11 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
       const StartLen& ts = tsl[col_off[g] + tpos];
       for (long long p = cp[j]; p < cp[j + 1]; ++p) {
         const int kpos = korder[g].pos[ri[p]];
-        const long long tq = t_off[g] + place_of(ts, static_cast<int>(p - cp[j]));
+        const long long tq = t_off[g] + place_of(ts, static_cast<int>(p - cp[j]), torder[g]);
         tidx[tq] = kpos;
         tval[tq] = va[p];
-        const long long kq = k_off[g] + place_of(ksl[row_off[g] + kpos], done[ri[p]]++);
+        const long long kq =
+            k_off[g] + place_of(ksl[row_off[g] + kpos], done[ri[p]]++, korder[g]);
         kidx[kq] = tpos;
         kval[kq] = va[p];
       }
@@ -362,6 +371,7 @@ int Batch::create(Batch** out, int nmat, const int* mat_m, const int* mat_n,
   b->mat_n_.assign(mat_n, mat_n + nmat);
   b->inst_mat_.assign(inst_mat, inst_mat + count);
   b->mat_slice_ = slice;
+  b->small_ = small;
   b->mat_nnz_.resize(nmat);
   for (int g = 0; g < nmat; ++g) b->mat_nnz_[g] = nnz_off[g + 1] - nnz_off[g];
   b->order_ = std::move(order);
@@ -472,6 +482,7 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   const int best = plan->size;
   plan->clusters = std::max(1, per_sm * sms_ / best);
   plan->sms = sms_;
+  plan->small = small_;
   if (setup) {
     // One launch for all matrices; a matrix whose vectors do not fit leaves them in device
     // memory.
@@ -514,6 +525,10 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
 }
 
 int Batch::upload_lists(const std::vector<int>* lists, ClusterPlan* plan) {
+  // (Small LPs' vectors and state are 60 KB at most.)
+  if (plan->small && !(lists[kInDevice].empty() && lists[kVectorsShared].empty())) {
+    return SG_ERR_INTERNAL;
+  }
   int used = 0;
   for (int mode = 0; mode < kModes; ++mode) {
     if (lists[mode].empty()) continue;

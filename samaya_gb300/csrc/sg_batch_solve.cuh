@@ -434,11 +434,10 @@ __device__ __forceinline__ int next_instance(unsigned* queue, ClusterShared& sh,
 
 }  // namespace
 
-template <typename T, int MODE, bool HALPERN, int THREADS>
+template <typename T, int MODE, bool HALPERN, int THREADS, int WALK = kWalkOne>
 __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 2 : 1)
     batch_solve_kernel(BatchView b, InstanceList list) {
-  // (FP32 with 512 threads: 128 registers and one slice's loads on their way are too few.)
-  using Share = RowShare<T, sizeof(T) == 4 && THREADS == kThreads32>;
+  using Share = RowShare<T, WALK>;
   __shared__ ClusterShared sh;
   __shared__ EvalContext<T, MODE, Share> ctx;
   const unsigned rank = cluster_rank();
@@ -452,10 +451,17 @@ __global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 2 : 1)
   cluster_sync(size);
 }
 
-// go() with the kernel of a mode and number of threads (Batch::plan_clusters).
+// go() with the kernel of a mode and number of threads (Batch::plan_clusters). FP32 with 512 threads
+// walks two slices at a time: 128 registers and one slice's loads on their way are too few.
 template <typename T, typename Go>
-auto with_solve_kernel(int algorithm, int mode, int threads, const Go& go) {
+auto with_solve_kernel(int algorithm, int mode, const ClusterPlan& p, const Go& go) {
   const bool h = algorithm == 2;
+  const int threads = p.threads[mode];
+  if (p.small) {
+    constexpr int kFew = sizeof(T) == 4 ? kThreads32Few : kThreads64;
+    return h ? go(batch_solve_kernel<T, kAllShared, true, kFew, kWalkLanes>)
+             : go(batch_solve_kernel<T, kAllShared, false, kFew, kWalkLanes>);
+  }
   if constexpr (sizeof(T) == 4) {
     if (mode == kAllShared && threads == kThreads32Few) {
       return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads32Few>)
@@ -465,37 +471,37 @@ auto with_solve_kernel(int algorithm, int mode, int threads, const Go& go) {
       return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads32Mid>)
                : go(batch_solve_kernel<T, kAllShared, false, kThreads32Mid>);
     }
-    if (mode == kAllShared) return go(batch_solve_kernel<T, kAllShared, true, kThreads32>);
+    if (mode == kAllShared) {
+      return go(batch_solve_kernel<T, kAllShared, true, kThreads32, kWalkPairs>);
+    }
   } else if (mode == kAllShared) {
     return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads64>)
              : go(batch_solve_kernel<T, kAllShared, false, kThreads64>);
   }
   constexpr int kMost = sizeof(T) == 4 ? kThreads32 : kThreads64;
+  constexpr int kWalk = sizeof(T) == 4 ? kWalkPairs : kWalkOne;
   if (mode == kVectorsShared) {
-    return h ? go(batch_solve_kernel<T, kVectorsShared, true, kMost>)
-             : go(batch_solve_kernel<T, kVectorsShared, false, kMost>);
+    return h ? go(batch_solve_kernel<T, kVectorsShared, true, kMost, kWalk>)
+             : go(batch_solve_kernel<T, kVectorsShared, false, kMost, kWalk>);
   }
-  return h ? go(batch_solve_kernel<T, kInDevice, true, kMost>)
-           : go(batch_solve_kernel<T, kInDevice, false, kMost>);
+  return h ? go(batch_solve_kernel<T, kInDevice, true, kMost, kWalk>)
+           : go(batch_solve_kernel<T, kInDevice, false, kMost, kWalk>);
 }
 
 template <typename T>
 cudaError_t launch_solve(const BatchView& b, const ClusterPlan& p, int mode, cudaStream_t s) {
   const InstanceList list = p.group[mode];
   const int clusters = list.count < p.clusters ? list.count : p.clusters;
-  const int threads = p.threads[mode];
-  return with_solve_kernel<T>(b.algorithm, mode, threads, [&](auto kernel) {
-    return launch_clusters(kernel, p.size, clusters, threads, p.smem[mode], s, b, list);
+  return with_solve_kernel<T>(b.algorithm, mode, p, [&](auto kernel) {
+    return launch_clusters(kernel, p.size, clusters, p.threads[mode], p.smem[mode], s, b, list);
   });
 }
 
 template <typename T>
 bool solve_fits(const ClusterPlan& p, int algorithm) {
   for (int mode = 0; mode < kModes; ++mode) {
-    const int threads = p.threads[mode];
-    if (p.group[mode].count > 0 &&
-        !with_solve_kernel<T>(algorithm, mode, threads, [&](auto kernel) {
-          return clusters_fit(kernel, p.size, threads, p.smem[mode]);
+    if (p.group[mode].count > 0 && !with_solve_kernel<T>(algorithm, mode, p, [&](auto kernel) {
+          return clusters_fit(kernel, p.size, p.threads[mode], p.smem[mode]);
         })) {
       return false;
     }

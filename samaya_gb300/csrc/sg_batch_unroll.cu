@@ -89,9 +89,9 @@ struct alignas(16) UnrollState {
   __device__ __forceinline__ double& arow(int k, const At& at) const { return row(kURows + k, at); }
 };
 
-template <int MODE>
+template <int MODE, int WALK>
 struct Unroll {
-  MatShare<double> M;
+  MatShare<double, RowShare<double, WALK>> M;
   Exchange<double, MODE> ex;
   UnrollState<MODE> S;
   const double *cs, *rs;
@@ -99,15 +99,16 @@ struct Unroll {
   long long vo, nt;
 };
 
-template <int MODE>
-__device__ __forceinline__ Unroll<MODE> unroll_begin(const BatchView& b, const UnrollView& u,
+template <int MODE, int WALK>
+__device__ __forceinline__ Unroll<MODE, WALK> unroll_begin(const BatchView& b, const UnrollView& u,
                                                      int inst, bool adjoint, ClusterShared& sh,
                                                      unsigned rank,
                                                      unsigned size) {
-  Unroll<MODE> p;
+  using Share = RowShare<double, WALK>;
+  Unroll<MODE, WALK> p;
   const int g = b.inst_mat[inst];
-  p.M = mat_share<double>(b, g, b.k_val, b.t_val, rank, size);
-  MatShare<double>& M = p.M;
+  p.M = mat_share<double, Share>(b, g, b.k_val, b.t_val, rank, size);
+  MatShare<double, Share>& M = p.M;
   p.nt = static_cast<long long>(M.n) + M.m;
   p.cs = b.cs + b.mat_col_off[g];
   p.rs = b.rs + b.mat_row_off[g];
@@ -150,8 +151,8 @@ __device__ __forceinline__ Unroll<MODE> unroll_begin(const BatchView& b, const U
 // projections. An equality row's logical is its bound from the first step on: a warp of such rows
 // skips the logicals unless the mask is kept (which side its z lies on depends on the dual). xs
 // has been put, not waited for; so it is afterwards.
-template <int MODE>
-__device__ __forceinline__ bool unroll_step(const Unroll<MODE>* p, double tau, double sigma,
+template <int MODE, int WALK>
+__device__ __forceinline__ bool unroll_step(const Unroll<MODE, WALK>* p, double tau, double sigma,
                                             unsigned char* mask) {
   {
     const auto K = sh_copy(&p->M.K);
@@ -224,14 +225,14 @@ __device__ __forceinline__ double adjoint_entry(const Entry& e, int from, double
   return gh;
 }
 
-template <int MODE>
+template <int MODE, int WALK>
 __device__ bool unroll_forward(const BatchView& b, const UnrollView& u, int inst,
-                               ClusterShared& sh, Unroll<MODE>* ctx, unsigned rank,
+                               ClusterShared& sh, Unroll<MODE, WALK>* ctx, unsigned rank,
                                unsigned size) {
-  const Unroll<MODE> p = unroll_begin<MODE>(b, u, inst, false, sh, rank, size);
+  const Unroll<MODE, WALK> p = unroll_begin<MODE, WALK>(b, u, inst, false, sh, rank, size);
   if (threadIdx.x == 0) *ctx = p;
   const UnrollState<MODE>& S = p.S;
-  const MatShare<double>& M = p.M;
+  const auto& M = p.M;
   const long long nt = p.nt;
   each_own(M.Kt, [&](const At& at) { S.col(kUPoint, at) = 0.0; });
   each_own(M.K, [&](const At& at) {
@@ -257,7 +258,7 @@ __device__ bool unroll_forward(const BatchView& b, const UnrollView& u, int inst
       });
       __syncthreads();  // read above by other threads than update them
     }
-    ok = unroll_step<MODE>(ctx, p.eta, p.eta, nullptr);
+    ok = unroll_step(ctx, p.eta, p.eta, nullptr);
   }
   if (ok) ok = p.ex.wait(0);
   __syncthreads();
@@ -267,14 +268,14 @@ __device__ bool unroll_forward(const BatchView& b, const UnrollView& u, int inst
   return !cluster_stopped(sh, size);
 }
 
-template <int MODE>
+template <int MODE, int WALK>
 __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst,
-                               ClusterShared& sh, Unroll<MODE>* ctx, unsigned rank,
+                               ClusterShared& sh, Unroll<MODE, WALK>* ctx, unsigned rank,
                                unsigned size) {
-  const Unroll<MODE> p = unroll_begin<MODE>(b, u, inst, true, sh, rank, size);
+  const Unroll<MODE, WALK> p = unroll_begin<MODE, WALK>(b, u, inst, true, sh, rank, size);
   if (threadIdx.x == 0) *ctx = p;
   const UnrollState<MODE>& S = p.S;
-  const MatShare<double>& M = p.M;
+  const auto& M = p.M;
   const long long nt = p.nt;
   const double tau = p.eta, sigma = p.eta;
   const double* gv = u.grad_v + p.vo;
@@ -308,7 +309,7 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
       S.row(kUDual, at) = c[2 * nt + at.p];
     });
     for (int t = 0; t < len && ok; ++t) {
-      ok = unroll_step<MODE>(ctx, tau, sigma, mask + static_cast<long long>(t) * nt);
+      ok = unroll_step(ctx, tau, sigma, mask + static_cast<long long>(t) * nt);
     }
     ok = ok && p.ex.wait(0);
     cluster_sync(size);  // the last x_bar is in place everywhere: xs may be sent again
@@ -392,20 +393,20 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
 
 }  // namespace
 
-template <bool ADJOINT, int MODE, int PER_SM = 2>
+template <bool ADJOINT, int MODE, int PER_SM = 2, int WALK = kWalkOne>
 __global__ void __launch_bounds__(kThreads64, PER_SM) unroll_kernel(BatchView b, UnrollView u,
                                                                     InstanceList list) {
   __shared__ ClusterShared sh;
-  __shared__ Unroll<MODE> ctx;
+  __shared__ Unroll<MODE, WALK> ctx;
   const unsigned rank = cluster_rank();
   const unsigned size = cluster_size();
   cluster_init(sh, size);
   bool ok = true;
   for (int q = blockIdx.x / size; q < list.count && ok; q += gridDim.x / size) {
     if constexpr (ADJOINT) {
-      ok = unroll_adjoint<MODE>(b, u, list.inst[q], sh, &ctx, rank, size);
+      ok = unroll_adjoint<MODE, WALK>(b, u, list.inst[q], sh, &ctx, rank, size);
     } else {
-      ok = unroll_forward<MODE>(b, u, list.inst[q], sh, &ctx, rank, size);
+      ok = unroll_forward<MODE, WALK>(b, u, list.inst[q], sh, &ctx, rank, size);
     }
   }
   if (!ok && threadIdx.x == 0) atomicExch(b.wait_error, 1);
@@ -416,7 +417,12 @@ namespace {
 
 // go() with the kernel of a mode; `alone`: the adjoint's variant with an SM to a CTA.
 template <typename Go>
-auto with_unroll_kernel(int adjoint, int mode, bool alone, const Go& go) {
+auto with_unroll_kernel(int adjoint, int mode, bool alone, bool small, const Go& go) {
+  if (small && adjoint && alone) return go(unroll_kernel<true, kAllShared, 1, kWalkLanes>);
+  if (small) {
+    return adjoint ? go(unroll_kernel<true, kAllShared, 2, kWalkLanes>)
+                   : go(unroll_kernel<false, kAllShared, 2, kWalkLanes>);
+  }
   if (mode == kAllShared && adjoint && alone) return go(unroll_kernel<true, kAllShared, 1>);
   if (mode == kAllShared) {
     return adjoint ? go(unroll_kernel<true, kAllShared>) : go(unroll_kernel<false, kAllShared>);
@@ -434,7 +440,7 @@ bool unroll_fits(const ClusterPlan& p, int adjoint) {
   for (int mode = 0; mode < kModes; ++mode) {
     for (bool alone : {false, true}) {
       if (p.group[mode].count > 0 &&
-          !with_unroll_kernel(adjoint, mode, alone, [&](auto kernel) {
+          !with_unroll_kernel(adjoint, mode, alone, p.small, [&](auto kernel) {
             return clusters_fit(kernel, p.size, p.threads[mode], p.smem[mode]);
           })) {
         return false;
@@ -457,7 +463,8 @@ cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const Cluster
     const int side_by_side = p.size <= 2   ? p.sms / p.size
                              : p.size == 4 ? p.sms / p.size * 3 / 4
                                            : p.sms / p.size / 2;
-    return with_unroll_kernel(adjoint, mode, clusters <= side_by_side, [&](auto kernel) {
+    const bool alone = clusters <= side_by_side;
+    return with_unroll_kernel(adjoint, mode, alone, p.small, [&](auto kernel) {
       return launch_clusters(kernel, p.size, clusters, p.threads[mode], p.smem[mode], gst, b, u, list);
     });
   });

@@ -6,7 +6,9 @@
 // (sg_cluster_layout.h): its rows are renumbered by decreasing length and taken in slices of 32
 // (8 where most nonzeros sit in long rows). Rows of at most 32 nonzeros are stored slice by slice
 // with their k-th nonzeros side by side (start + 32 k), so that a warp's loads are whole lines and
-// the lanes of a slice end together; longer rows are stored row by row. Slice s belongs to CTA
+// the lanes of a slice end together; longer rows are stored row by row. (Small LPs, kWalkLanes: 8, 16
+// or 32 rows to a slice, row r's nonzeros on lane r and every 2^slice-th after it in turn.) Slice s
+// belongs to CTA
 // s mod C of the cluster: sorted slices dealt out in turn balance the CTAs.
 // Rows of random LPs hold 15 +- 4 nonzeros: unsorted, a warp's longest row keeps it half as long
 // again, and the FP64 pipe (below) is busy for every lane that has nothing to add.
@@ -385,8 +387,12 @@ struct Sender {
   }
 };
 
-// A CTA's share of an operator by rows. PAIRS: walked two slices at a time (walk_pairs).
-template <typename T, bool PAIRS = false>
+// How a share's slices are walked: one at a time, two (walk_pairs), or one whose rows take 32 >> slice
+// lanes each.
+enum : int { kWalkOne = 0, kWalkPairs = 1, kWalkLanes = 2 };
+
+// A CTA's share of an operator by rows.
+template <typename T, int WALK = kWalkOne>
 struct alignas(16) RowShare {
   static constexpr bool kTasks = false;
   const int2* sl;  // per row (position): first nonzero, length
@@ -412,6 +418,14 @@ struct alignas(16) RowShare {
     return __ldg(desc + (ls * static_cast<int>(size) + static_cast<int>(rank)));
   }
   __host__ __device__ __forceinline__ int own() const { return slices() << slice; }
+  // Nonzero k of a row (its first, length): the place.
+  __device__ __forceinline__ int place(const int2& row, int k) const {
+    if (row.y > 32) return row.x + k;
+    if constexpr (WALK == kWalkLanes) {
+      return row.x + ((k >> (5 - slice)) << 5) + ((k & ((32 >> slice) - 1)) << slice);
+    }
+    return row.x + (k << 5);
+  }
   __device__ __forceinline__ int position(int l) const {
     return ((((l >> slice) * static_cast<int>(size)) + static_cast<int>(rank)) << slice) +
            (l & ((1 << slice) - 1));
@@ -419,14 +433,9 @@ struct alignas(16) RowShare {
 };
 constexpr int kHasLong = 256;  // as place_rows sets it
 
-// Nonzero k of a row: its place.
-__device__ __forceinline__ int nonzero_at(int start, int len, int k) {
-  return start + (len <= 32 ? k << 5 : k);
-}
-
 // f(at) for every own row of the share (thread tid takes own rows tid, tid + threads, ...).
-template <typename T, bool PAIRS, typename F>
-__device__ __forceinline__ void each_own(const RowShare<T, PAIRS>& A, const F& f) {
+template <typename T, int WALK, typename F>
+__device__ __forceinline__ void each_own(const RowShare<T, WALK>& A, const F& f) {
   const int own = A.own();
   for (int l = threadIdx.x; l < own; l += blockDim.x) {
     const At at{l >> A.slice, l & ((1 << A.slice) - 1), l, A.position(l)};
@@ -456,9 +465,9 @@ __device__ __forceinline__ void settle_counts(Exchange<V, MODE>& ex) {
 }
 
 // Fills the masks of the own rows and columns and the byte counts; ends with a cluster barrier.
-template <typename V, int MODE, typename T, bool PAIRS>
-__device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShare<T, PAIRS>& K,
-                                            const RowShare<T, PAIRS>& Kt) {
+template <typename V, int MODE, typename T, int WALK>
+__device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShare<T, WALK>& K,
+                                            const RowShare<T, WALK>& Kt) {
   ClusterShared& sh = *ex.sh;
   ex.tx[0] = ex.tx[1] = 0;
   if (ex.size == 1) {
@@ -471,14 +480,14 @@ __device__ __forceinline__ void build_masks(Exchange<V, MODE>& ex, const RowShar
   for (int which = 0; which < 2; ++which) {
     // Column j is read by the CTAs that own the rows of its nonzeros, row i by the CTAs that
     // own the columns of its nonzeros.
-    const RowShare<T, PAIRS>& A = which == 0 ? Kt : K;
+    const RowShare<T, WALK>& A = which == 0 ? Kt : K;
     const int other = which == 0 ? K.slice : Kt.slice;
     unsigned short* mask = which == 0 ? ex.cmask() : ex.rmask();
     each_own(A, [&](const At& at) {
       const int2 sl = __ldg(A.sl + at.p);
       unsigned m = 0;
       for (int k = 0; k < sl.y; ++k) {
-        const int j = __ldg(A.idx + nonzero_at(sl.x, sl.y, k));
+        const int j = __ldg(A.idx + A.place(sl, k));
         m |= 1u << (((j >> other) & static_cast<int>(ex.size - 1)) ^ static_cast<int>(ex.rank));
       }
       m &= ~1u;
@@ -556,13 +565,23 @@ __device__ __forceinline__ T ld_mat(const T* p) {
 // every lane off (measured on a walk of no rows: 8 of them, 1,400 clocks beside 15 busy warps).
 __device__ __forceinline__ void keep_branch(unsigned mask) { __syncwarp(mask); }
 
+// The parts of a slice's rows, on every 2^slice-th lane, added up (or their maximum).
+template <bool MAXRED, typename ACC>
+__device__ __forceinline__ ACC join_lanes(ACC s, int slice) {
+  for (int o = 16; o >= 1 << slice; o >>= 1) {
+    const ACC got = __shfl_xor_sync(0xffffffffu, s, o);
+    s = MAXRED ? fmax(s, got) : s + got;
+  }
+  return s;
+}
+
 // s + the sum (or maximum) over the nonzeros of the slice's longer rows (lanes with a row, at
 // position p; the others keep s), by the whole warp, four (FP64) or eight rows at a time so that
 // their loads overlap: lane l takes nonzeros l, l + 32, ..., and the shuffle trees of the rows are
 // folded into one (each step halves the sums a lane carries: 6 additions in place of 20, 9 in
 // place of 40); every row's tree is the same as alone.
-template <bool NC, bool MAXRED, typename T, bool PAIRS, typename ACC, typename Prod>
-__device__ __forceinline__ ACC long_rows(const RowShare<T, PAIRS> A, const Prod& prod, bool valid,
+template <bool NC, bool MAXRED, typename T, int WALK, typename ACC, typename Prod>
+__device__ __forceinline__ ACC long_rows(const RowShare<T, WALK> A, const Prod& prod, bool valid,
                                          int p, ACC s) {
   constexpr int kTogether = sizeof(ACC) == 8 ? 4 : 8;
   const int lane = threadIdx.x & 31;
@@ -638,15 +657,16 @@ __device__ __forceinline__ ACC long_rows(const RowShare<T, PAIRS> A, const Prod&
 // f(at, s) for every own row of the share, s = init(at) + the sum of prod(val, idx) over the row's
 // nonzeros (or the maximum, with init 0). A row of at most 32 nonzeros is summed by its thread in
 // index order, as many steps as its slice's longest (a shorter row's padding adds 0 times the
-// gathered vector's last entry, 0); longer rows by long_rows. Then every row's own lane runs f,
-// so that the updates of a slice run side by side. ready() waits for the gathered vector after
+// gathered vector's last entry, 0), with kWalkLanes by its lanes and a tree over them; longer rows
+// by long_rows. Then every row's (first) lane runs f, so that the updates of a slice run side by
+// side. ready() waits for the gathered vector after
 // the first loads are on their way (every thread calls it once; false ends the walk).
 //
 // walk_one: a slice at a time, four steps' nonzeros loaded while the four before are summed (of the
 // same slice or the warp's slice before).
-template <bool NC, bool MAXRED, typename T, typename Prod, typename Init, typename F,
+template <bool NC, bool MAXRED, typename T, int WALK, typename Prod, typename Init, typename F,
           typename Ready>
-__device__ __forceinline__ bool walk_one(const RowShare<T, false> A, const Prod& prod,
+__device__ __forceinline__ bool walk_one(const RowShare<T, WALK> A, const Prod& prod,
                                          const Init& init, const F& f, const Ready& ready) {
   using ACC = decltype(prod(T(), 0));
   constexpr int B = kBatch;
@@ -718,6 +738,7 @@ __device__ __forceinline__ bool walk_one(const RowShare<T, false> A, const Prod&
       }
       if (!more) break;
     }
+    if constexpr (WALK == kWalkLanes) s = join_lanes<MAXRED>(s, A.slice);
     if (d.y >= kHasLong) s = long_rows<NC, MAXRED>(A, prod, valid, at.p, s);
     if (valid) f(at, s);
     d = dn;
@@ -729,7 +750,7 @@ __device__ __forceinline__ bool walk_one(const RowShare<T, false> A, const Prod&
 // walk_pairs: two slices at a time, so that 16 loads a thread are on their way.
 template <bool NC, bool MAXRED, typename T, typename Prod, typename Init, typename F,
           typename Ready>
-__device__ __forceinline__ bool walk_pairs(const RowShare<T, true> A, const Prod& prod,
+__device__ __forceinline__ bool walk_pairs(const RowShare<T, kWalkPairs> A, const Prod& prod,
                                            const Init& init, const F& f, const Ready& ready) {
   using ACC = decltype(prod(T(), 0));
   constexpr int B = kBatch;
@@ -803,11 +824,11 @@ __device__ __forceinline__ bool walk_pairs(const RowShare<T, true> A, const Prod
   return true;
 }
 
-template <bool NC, bool MAXRED, typename T, bool PAIRS, typename Prod, typename Init, typename F,
+template <bool NC, bool MAXRED, typename T, int WALK, typename Prod, typename Init, typename F,
           typename Ready>
-__device__ __forceinline__ bool walk_rows(const RowShare<T, PAIRS>& A, const Prod& prod,
+__device__ __forceinline__ bool walk_rows(const RowShare<T, WALK>& A, const Prod& prod,
                                           const Init& init, const F& f, const Ready& ready) {
-  if constexpr (PAIRS) {
+  if constexpr (WALK == kWalkPairs) {
     return walk_pairs<NC, MAXRED>(A, prod, init, f, ready);
   } else {
     return walk_one<NC, MAXRED>(A, prod, init, f, ready);

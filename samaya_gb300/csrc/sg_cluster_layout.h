@@ -1,7 +1,7 @@
 // Host side of the cluster kernels' operator layout (see sg_cluster.cuh): rows renumbered by
-// decreasing length, rows of at most 32 nonzeros interleaved by slices (padded to the slice's
-// longest; a padding element is 0 in the gathered vector's last entry, one past the other
-// operator's rows), longer rows row by row.
+// decreasing length, rows of at most 32 nonzeros interleaved by slices, a lane or several to a row
+// (padded to the slice's longest; a padding element is 0 in the gathered vector's last entry, one
+// past the other operator's rows), longer rows row by row.
 #pragma once
 
 #include <stdint.h>
@@ -19,11 +19,12 @@ struct StartLen {
 // The numbering of one operator's rows.
 struct RowOrder {
   int slice = 5;          // log2 of the rows of a slice
+  int lanes = 1;          // lanes of a row of at most 32 nonzeros
   std::vector<int> perm;  // position -> row
   std::vector<int> pos;   // row -> position
 };
 
-inline RowOrder order_rows(const int* ptr, int rows) {
+inline RowOrder order_rows(const int* ptr, int rows, bool small = false) {
   RowOrder o;
   long long in_long = 0;
   int longest = 0;
@@ -36,6 +37,12 @@ inline RowOrder order_rows(const int* ptr, int rows) {
   // facility-location LP, 40-160 nonzeros each) occupies every warp. (Not where the padding of
   // its shorter rows, three of four places, could pass 32-bit offsets.)
   o.slice = rows > 0 && 2 * in_long > ptr[rows] && ptr[rows] < (1 << 28) ? 3 : 5;
+  // Small LPs (Batch::create): one CTA has more warps than the operator has slices of 32, and an
+  // iteration is mostly the chain of a row's additions: 8 or 16 rows to a slice, 4 or 2 lanes a row.
+  if (small) {
+    if (rows <= 128) o.slice = rows <= 64 ? 3 : std::min(o.slice, 4);
+    o.lanes = 32 >> o.slice;
+  }
   // Stable counting sort by decreasing length.
   std::vector<int> at(static_cast<size_t>(longest) + 2, 0);
   for (int r = 0; r < rows; ++r) ++at[longest - (ptr[r + 1] - ptr[r]) + 1];
@@ -74,7 +81,7 @@ inline long long place_rows(const int* ptr, const RowOrder& o, StartLen* sl, Sta
         has_long = true;
         continue;
       }
-      width = std::max(width, sl[p].len);
+      width = std::max(width, (sl[p].len + o.lanes - 1) / o.lanes);
       sl[p].start = static_cast<int>(at + (p - first));
     }
     desc[first >> o.slice] = {width > 0 ? static_cast<int>(at) : 0, width | (has_long ? 256 : 0)};
@@ -87,9 +94,10 @@ inline int slices_of(const RowOrder& o) {
   return (static_cast<int>(o.perm.size()) + (1 << o.slice) - 1) >> o.slice;
 }
 
-// The place of nonzero k of the row at position p.
-inline int place_of(const StartLen& sl, int k) {
-  return sl.start + (sl.len <= 32 ? k << 5 : k);
+// The place of nonzero k of the row at position p (RowShare::place on the device).
+inline int place_of(const StartLen& sl, int k, const RowOrder& o) {
+  if (sl.len > 32) return sl.start + k;
+  return sl.start + ((k / o.lanes) << 5) + ((k % o.lanes) << o.slice);
 }
 
 // The other layout, for an LP on one cluster of few rows a CTA (sg_chunk.cu). The rows, by

@@ -81,7 +81,8 @@ struct Sender {
   explicit Sender(const Exchange<V, MODE>& e) : ex(e) {}
   void put(const At&, V) const { ex.store(); }
 };
-template <typename T, bool B = false>
+enum : int { kWalkOne = 0, kWalkPairs = 1, kWalkLanes = 2 };
+template <typename T, int WALK = kWalkOne>
 struct alignas(16) RowShare {
   static constexpr bool kTasks = false;
   const int2 *sl, *desc;
@@ -91,6 +92,7 @@ struct alignas(16) RowShare {
   unsigned rank, size;
   int slices() const { return 1; }
   int own() const { return 1; }
+  int place(const int2& row, int k) const { return row.x + k; }
 };
 // One own row, at position 0.
 template <typename S, typename F>
