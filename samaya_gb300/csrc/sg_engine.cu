@@ -330,19 +330,30 @@ int Engine::create_from_device(Engine** out, const DeviceLp& d, const Options& o
 
 namespace {
 
-// Row-length statistics of an operator: the autotuner's cache key.
-struct ShapeKey {
+// Row-length statistics of an operator, over the rows that a step runs over.
+struct RowStats {
   int rows;
-  long long nnz;
   int max_len;
   long long over32, over128, over4096;
+  bool operator<(const RowStats& o) const {
+    return std::tie(rows, max_len, over32, over128, over4096) <
+           std::tie(o.rows, o.max_len, o.over32, o.over128, o.over4096);
+  }
+};
+
+// The autotuner's cache key: all that the timed iteration depends on, both operators and both steps'
+// kernels (time_steps_in_turn).
+struct ShapeKey {
+  int which;    // 0: K, 1: K'
+  int halpern;
+  RowStats own, other;
+  long long nnz;
   int fp32;
   int groups;   // the row-group option (0 tuned, 1 built-in, -1 never)
   int staging;  // the segment-staging option (1 staged, -1 direct)
   bool operator<(const ShapeKey& o) const {
-    return std::tie(rows, nnz, max_len, over32, over128, over4096, fp32, groups, staging) <
-           std::tie(o.rows, o.nnz, o.max_len, o.over32, o.over128, o.over4096, o.fp32,
-                    o.groups, o.staging);
+    return std::tie(which, halpern, own, other, nnz, fp32, groups, staging) <
+           std::tie(o.which, o.halpern, o.own, o.other, o.nnz, o.fp32, o.groups, o.staging);
   }
 };
 
@@ -352,8 +363,10 @@ bool g_shape_file_read = false;
 
 // SG_TILE_CACHE names a text file that carries the tuner's choices across processes (so that a
 // profiler run, whose launches cannot be timed, uses the shapes a plain run picked): one line
-// per operator, the key's nine fields then the shape's seven. Read once per process, appended
-// after each tuning. Call with g_shape_mu held.
+// per operator of 16 fields, the key (the first field holds the format, the step kernels and the
+// operators' rows) then the shape's seven. Lines of another format are not read: their shapes were
+// chosen for a step timed alone. Read once per process, appended after each tuning. Call with
+// g_shape_mu held.
 void read_shape_file() {
   if (g_shape_file_read) return;
   g_shape_file_read = true;
@@ -361,12 +374,20 @@ void read_shape_file() {
   if (path == nullptr || *path == '\0') return;
   FILE* f = std::fopen(path, "r");
   if (f == nullptr) return;
-  ShapeKey k{};
-  TileShape sh;
-  while (std::fscanf(f, "%d %lld %d %lld %lld %lld %d %d %d %d %d %d %d %d %d %d", &k.rows,
-                     &k.nnz, &k.max_len, &k.over32, &k.over128, &k.over4096, &k.fp32,
-                     &k.groups, &k.staging, &sh.cap_nnz, &sh.cap_rows, &sh.warp_min,
-                     &sh.variant, &sh.split, &sh.groups, &sh.staged) == 16) {
+  char line[512];
+  while (std::fgets(line, sizeof(line), f) != nullptr) {
+    ShapeKey k{};
+    TileShape sh;
+    if (std::sscanf(line,
+                    "v2:%d:%d:%d:%d:%d:%lld:%lld:%lld %lld %d %lld %lld %lld %d %d %d %d %d %d %d "
+                    "%d %d %d",
+                    &k.which, &k.halpern, &k.own.rows, &k.other.rows, &k.other.max_len,
+                    &k.other.over32, &k.other.over128, &k.other.over4096, &k.nnz, &k.own.max_len,
+                    &k.own.over32, &k.own.over128, &k.own.over4096, &k.fp32, &k.groups, &k.staging,
+                    &sh.cap_nnz, &sh.cap_rows, &sh.warp_min, &sh.variant, &sh.split, &sh.groups,
+                    &sh.staged) != 23) {
+      continue;
+    }
     if (sh.cap_nnz >= 256 && sh.cap_nnz <= 4 * kTileNnz && sh.cap_rows >= 1 &&
         sh.cap_rows <= kTileRows && sh.warp_min >= 32 && (sh.variant == 0 || sh.variant == 1) &&
         sh.split >= 0 && (sh.groups == 0 || sh.groups == 1) &&
@@ -382,16 +403,20 @@ void append_shape_file(const ShapeKey& k, const TileShape& sh) {
   if (path == nullptr || *path == '\0') return;
   FILE* f = std::fopen(path, "a");
   if (f == nullptr) return;
-  std::fprintf(f, "%d %lld %d %lld %lld %lld %d %d %d %d %d %d %d %d %d %d\n", k.rows, k.nnz,
-               k.max_len, k.over32, k.over128, k.over4096, k.fp32, k.groups, k.staging,
-               sh.cap_nnz, sh.cap_rows, sh.warp_min, sh.variant, sh.split, sh.groups, sh.staged);
+  std::fprintf(f,
+               "v2:%d:%d:%d:%d:%d:%lld:%lld:%lld %lld %d %lld %lld %lld %d %d %d %d %d %d %d %d %d "
+               "%d\n",
+               k.which, k.halpern, k.own.rows, k.other.rows, k.other.max_len, k.other.over32,
+               k.other.over128, k.other.over4096, k.nnz, k.own.max_len, k.own.over32,
+               k.own.over128, k.own.over4096, k.fp32, k.groups, k.staging, sh.cap_nnz,
+               sh.cap_rows, sh.warp_min, sh.variant, sh.split, sh.groups, sh.staged);
   std::fclose(f);
 }
 
-ShapeKey shape_key(const DevOp& op, bool fp32, int groups, int staging) {
+RowStats row_stats(const DevOp& op) {
   // The rows the step kernel runs over (inert rows left out are empty).
   const int rows = op.act_rows != nullptr ? static_cast<int>(op.act_list.size()) : op.rows;
-  ShapeKey k{rows, op.nnz, 0, 0, 0, 0, fp32 ? 1 : 0, groups, staging};
+  RowStats k{rows, 0, 0, 0, 0};
   for (int r = 0; r < op.rows; ++r) {
     const int len = op.host_ptr[r + 1] - op.host_ptr[r];
     k.max_len = std::max(k.max_len, len);
@@ -662,7 +687,14 @@ int Engine::tune_tiles(std::string* err) {
     ShapeKey key{};
     bool cached = false;
     if (tune) {
-      key = shape_key(*op, fp32_, opt_.row_groups, opt_.segment_staging);
+      key = ShapeKey{which,
+                     opt_.algorithm == 2 ? 1 : 0,
+                     row_stats(*op),
+                     row_stats(which == 0 ? Kt_ : K_),
+                     op->nnz,
+                     fp32_ ? 1 : 0,
+                     opt_.row_groups,
+                     opt_.segment_staging};
       std::lock_guard<std::mutex> lock(g_shape_mu);
       read_shape_file();
       auto it = g_shape_cache.find(key);

@@ -55,6 +55,6 @@ def test_choices_are_kept_by_iteration(tmp_path):
     out = _run(path)
     lines = path.read_text().splitlines()
     assert lines[0] == old and len(lines) == 7
-    assert len({x.split()[0] for x in lines[1:]}) == 6
+    assert len({tuple(x.split()[:9]) for x in lines[1:]}) == 6
     assert _run(path) == out
     assert path.read_text().splitlines() == lines
