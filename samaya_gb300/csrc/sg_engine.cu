@@ -672,9 +672,10 @@ double Engine::time_steps_in_turn(int reps) {
 int Engine::tune_tiles(std::string* err) {
   // Both operators have tiles while either is timed.
   for (DevOp* op : {&K_, &Kt_}) {
-    if (set_tiles(op, default_shape(*op)) != kOk) {
+    const int rc = set_tiles(op, default_shape(*op));
+    if (rc != kOk) {
       if (err) *err = "tile upload failed";
-      return kErrCuda;
+      return rc;
     }
   }
   for (int which = 0; which < 2; ++which) {
