@@ -21,7 +21,10 @@ int Batch::alloc(T** p, size_t count) {
   *p = nullptr;
   const cudaError_t e =
       cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
-  if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? SG_ERR_OUT_OF_MEMORY : SG_ERR_CUDA;
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next call
+    return e == cudaErrorMemoryAllocation ? SG_ERR_OUT_OF_MEMORY : SG_ERR_CUDA;
+  }
   allocs_.push_back(*p);
   return SG_OK;
 }
@@ -628,10 +631,14 @@ int Batch::unroll(int iterations, int every, double* v_out, std::string* err) {
     mask_off[i + 1] = mask_off[i] + (static_cast<long long>(every) * nt + 15) / 16 * 16;
   }
   auto fail = [&](cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported here, not by the next call
     if (err) *err = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? SG_ERR_OUT_OF_MEMORY : SG_ERR_CUDA;
   };
   if (u_.iterations != iterations || u_.every != every || u_.ck == nullptr) {
+    // (Where an allocation below fails, neither the adjoint nor a later call finds half of them.)
+    unrolled_ = false;
+    u_.iterations = 0;
     for (void* p : {static_cast<void*>(u_.ck), static_cast<void*>(u_.mask),
                     const_cast<void*>(static_cast<const void*>(u_.ck_off)),
                     const_cast<void*>(static_cast<const void*>(u_.mask_off))}) {
@@ -662,7 +669,7 @@ int Batch::unroll(int iterations, int every, double* v_out, std::string* err) {
     u_.ck_off = cko;
     u_.mask_off = mko;
     if (e != cudaSuccess) return fail(e, "unroll buffers");
-    if (u_.v_out == nullptr) {
+    if (u_.grad_v == nullptr) {  // the last of them
       for (double** p : {&u_.v_out, &u_.grad_cost, &u_.grad_lower, &u_.grad_upper}) {
         const int rc = alloc(p, total_vec_);
         if (rc != SG_OK) {

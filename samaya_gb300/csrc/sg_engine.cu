@@ -29,7 +29,10 @@ double now_s() {
 template <typename T>
 cudaError_t dalloc(T** p, size_t count) {
   *p = nullptr;
-  return cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
+  const cudaError_t e =
+      cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next call
+  return e;
 }
 
 template <typename T>
