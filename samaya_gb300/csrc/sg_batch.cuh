@@ -155,6 +155,10 @@ inline int cluster_limit() {
   return most < 1 ? kMaxCluster : most < kMaxCluster ? most : kMaxCluster;
 }
 
+// The clusters that a device was found to hold with kClusterSmemMax (sg_batch_host.cu): whether this
+// one is among them, after `add` it is. Safe from several threads.
+bool known_to_fit(const void* kernel, int device, int size, int threads, bool add);
+
 // Dynamic shared memory of a cluster kernel at most: a CTA's 227 KB less its static part.
 constexpr size_t kClusterSmemMax = 227 * 1024 - 8 * 1024;
 // FP64 kernels: a CTA's half of an SM's 228 KB (1 KB of each CTA is the system's).

@@ -5,9 +5,12 @@
 #include <algorithm>
 #include <functional>
 #include <limits>
+#include <mutex>
 #include <numeric>
 #include <queue>
 #include <random>
+#include <set>
+#include <tuple>
 #include <utility>
 
 #include "../../include/sg_pdlp.h"
@@ -15,6 +18,15 @@
 #include "sg_cluster_layout.h"
 
 namespace sg {
+
+bool known_to_fit(const void* kernel, int device, int size, int threads, bool add) {
+  static std::mutex mu;
+  static std::set<std::tuple<const void*, int, int, int>> known;  // kernels x devices x sizes
+  std::lock_guard<std::mutex> lock(mu);
+  const std::tuple<const void*, int, int, int> key{kernel, device, size, threads};
+  if (add) known.insert(key);
+  return known.count(key) != 0;
+}
 
 template <typename T>
 int Batch::alloc(T** p, size_t count) {
