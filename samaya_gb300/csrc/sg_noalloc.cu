@@ -57,7 +57,7 @@ __device__ __forceinline__ int lower_bound_ptr(const int* ptr, int m, long long 
   const int lane = threadIdx.x & 31;
   int lo = 0, hi = m;
   while (lo < hi) {
-    const int step = (hi - lo + 31) >> 5;
+    const int step = static_cast<int>((static_cast<unsigned>(hi - lo) + 31u) >> 5);
     const long long at = lo + static_cast<long long>(lane + 1) * step - 1;
     const bool below = at < hi && static_cast<long long>(ptr[at]) < key;
     const int c = __popc(__ballot_sync(0xffffffffu, below));
@@ -135,17 +135,18 @@ __global__ void __launch_bounds__(kThreads) spmv_chunk_kernel(int m, const int* 
   }
   __syncthreads();
   const int r_begin = range[0];
-  const int r_end = range[1];
-  auto end_of = [&](int r) {
+  // (Unsigned: the numbers past the last row are no int beyond 2^31 - 256 rows.)
+  const unsigned r_end = static_cast<unsigned>(range[1]);
+  auto end_of = [&](unsigned r) {
     const long long e = ptr[r + 1];
     return e > k1 && !last_chunk && !whole ? k1 : e;
   };
   // Rows side by side, `rows` at a time; every lane of a warp stays in the loop for the shuffles.
   const int width = 1 << lanes;
   const int part = threadIdx.x & (width - 1);
-  const int rows = kThreads >> lanes;
-  for (int base = r_begin; base < r_end; base += rows) {
-    const int r = base + (threadIdx.x >> lanes);
+  const unsigned rows = kThreads >> lanes;
+  for (unsigned base = static_cast<unsigned>(r_begin); base < r_end; base += rows) {
+    const unsigned r = base + (threadIdx.x >> lanes);
     const long long b = r < r_end ? ptr[r] : 0;
     const long long e = r < r_end ? end_of(r) : 0;
     // (A last chunk that runs on to a count beyond the grid's may hold more long rows than the
@@ -154,7 +155,7 @@ __global__ void __launch_bounds__(kThreads) spmv_chunk_kernel(int m, const int* 
     if (e - b > kLongRow && part == 0) slot = atomicAdd(&nlongs, 1) + 1;
     slot = __shfl_sync(0xffffffffu, slot, lane & ~(width - 1));
     const bool listed = slot > 0 && slot <= static_cast<int>(sizeof(longs) / sizeof(longs[0]));
-    if (listed && part == 0) longs[slot - 1] = r;
+    if (listed && part == 0) longs[slot - 1] = static_cast<int>(r);
     double s = listed ? 0.0 : partial(b, e, part, width, idx, val, x);
     for (int o = width >> 1; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, width);
     if (r < r_end && !listed && part == 0) y[r] = s;
