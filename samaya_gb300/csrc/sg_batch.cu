@@ -232,9 +232,9 @@ __device__ void setup_matrix(const BatchView& b, int g, ClusterShared& sh,
 
 }  // namespace
 
-template <int WALK>
-__global__ void __launch_bounds__(kThreads64, 2) batch_setup_kernel(BatchView b,
-                                                                    unsigned smem_bytes) {
+template <int WALK, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kThreads64 ? 2 : 1)
+    batch_setup_kernel(BatchView b, unsigned smem_bytes) {
   __shared__ ClusterShared sh;
   const unsigned rank = cluster_rank();
   const unsigned size = cluster_size();
@@ -265,15 +265,23 @@ cudaError_t launch_batch(const BatchView& b, const ClusterPlan& setup, const Clu
   });
 }
 
+namespace {
+
+auto setup_kernel(const ClusterPlan& p) {
+  return p.small                       ? batch_setup_kernel<kWalkLanes, kThreads64>
+         : p.threads[0] == kThreads64 ? batch_setup_kernel<kWalkOne, kThreads64>
+                                       : batch_setup_kernel<kWalkOne, kThreads64Large>;
+}
+
+}  // namespace
+
 bool setup_fits(const ClusterPlan& p) {
-  return p.small ? clusters_fit(batch_setup_kernel<kWalkLanes>, p.size, kThreads64, p.smem[0])
-                 : clusters_fit(batch_setup_kernel<kWalkOne>, p.size, kThreads64, p.smem[0]);
+  return clusters_fit(setup_kernel(p), p.size, p.threads[0], p.smem[0]);
 }
 
 cudaError_t launch_batch_setup(const BatchView& b, const ClusterPlan& setup, cudaStream_t s) {
-  return launch_clusters(
-      setup.small ? batch_setup_kernel<kWalkLanes> : batch_setup_kernel<kWalkOne>, setup.size,
-      b.nmat, kThreads64, setup.smem[0], s, b, static_cast<unsigned>(setup.smem[0]));
+  return launch_clusters(setup_kernel(setup), setup.size, b.nmat, setup.threads[0], setup.smem[0], s,
+                         b, static_cast<unsigned>(setup.smem[0]));
 }
 
 }  // namespace sg

@@ -429,8 +429,6 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   const bool fp32 = kind == Kind::kSolve && v_.fp32;
   const size_t elem = fp32 ? sizeof(float) : sizeof(double);
   const int count = setup ? static_cast<int>(mat_m_.size()) : v_.count;
-  // Two FP64 CTAs share an SM; FP32 ones take it for themselves.
-  const int per_sm = fp32 ? 1 : 2;
   const size_t limit = fp32 ? kClusterSmemMax : kClusterSmemHalf;
   auto vector_bytes = [&](int g, int size) {
     return cluster_vector_bytes(mat_n_[g], mat_m_[g], mat_slice_[2 * g + 1], mat_slice_[2 * g],
@@ -447,14 +445,22 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   };
   std::vector<std::pair<double, int>> work(count);  // an iteration's time by one CTA, the matrix
   bool fits = true;  // every instance's gathered vectors in shared memory
+  size_t most_vectors = 0;
   for (int i = 0; i < count; ++i) {
     const int g = setup ? i : inst_mat_[i];
     const double rows = static_cast<double>(mat_m_[g]) + mat_n_[g];
     const double nnz = static_cast<double>(mat_nnz_[g]);
     work[i] = {(fp32 ? 1.5e-4 : 5.6e-4) * (2 * nnz + 5 * rows), g};
     fits = fits && vector_bytes(g, 2) <= kClusterSmemMax;
+    most_vectors = std::max(most_vectors, vector_bytes(g, 1));
   }
   std::sort(work.begin(), work.end(), std::greater<std::pair<double, int>>());
+  // Two FP64 CTAs share an SM, unless an LP's vectors leave no room for a second one: then one of 512
+  // threads has it (128 iterations of facility-location LPs with 256 and with 512: 16 of
+  // 60 x 240 7.8 and 4.7 ms, 64 of 100 x 400 72.0 and 42.5; 256 random LPs of 5,000 x 12,500 67.3 and
+  // 42.8). FP32 CTAs take an SM each.
+  const bool alone = !fp32 && most_vectors > kClusterSmemHalf;
+  const int per_sm = fp32 || alone ? 1 : 2;
   // The sizes' exchanges and epilogues.
   const int sizes[5] = {1, 2, 4, 8, 16};
   const double fixed64[5] = {0.7, 2.2, 3.4, 4.2, 5.2};
@@ -471,8 +477,8 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
     // Clusters at once (SMs of a GPC left over by clusters of 8 and 16: an eighth or more; a quarter
     // with an SM to a CTA, where 16 clusters of 8 no longer run side by side).
     const int whole = per_sm * sms_ / size;
-    const int slots = std::max(1, whole - (size >= 8 ? whole / (fp32 ? 4 : 8) : 0));
-    const bool shared_sm = !fp32 && static_cast<long long>(std::min(count, slots)) * size > sms_;
+    const int slots = std::max(1, whole - (size >= 8 ? whole / (per_sm == 1 ? 4 : 8) : 0));
+    const bool shared_sm = per_sm == 2 && static_cast<long long>(std::min(count, slots)) * size > sms_;
     // Largest first, each to the cluster that is free first.
     std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
     for (int c = 0; c < std::min(count, slots); ++c) free_at.push(0.0);
@@ -483,22 +489,27 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
       // The FP64 pipe of a shared SM; a state left in device memory (160 LPs of 2,000 x 4,000:
       // 72 us with 2 CTAs, 48 with 4, which hold it).
       if (shared_sm) t = setup ? 1.25 * t : std::max(t, 1.15 * own);
-      if (!setup && !fp32 && all_bytes(w.second, size) > limit) t *= 1.45;
+      if (!setup && per_sm == 2 && all_bytes(w.second, size) > limit) t *= 1.45;
       t += free_at.top();
       free_at.pop();
       free_at.push(t);
       end = std::max(end, t);
     }
-    if (best_time < 0 || end < best_time) {
+    // (Where the state stays in device memory, a larger cluster's gain is partly the memory's: 256
+    // nodes of 100 x 400 in FP32 54.1 ms with clusters of four, estimated alike, 42.8 with one CTA.)
+    const bool close = !setup && all_bytes(work[0].second, size) > limit;
+    if (best_time < 0 || end < (close ? 0.95 : 1.0) * best_time) {
       best_time = end;
       plan->size = size;
     }
   }
   const int best = plan->size;
-  plan->clusters = std::max(1, per_sm * sms_ / best);
+  plan->clusters = std::max(1, (fp32 ? 1 : 2) * sms_ / best);
   plan->sms = sms_;
   plan->small = small_;
+  if (alone) plan->threads[kVectorsShared] = plan->threads[kInDevice] = kThreads64Large;
   if (setup) {
+    plan->threads[0] = alone ? kThreads64Large : kThreads64;
     // One launch for all matrices; a matrix whose vectors do not fit leaves them in device
     // memory.
     for (int g = 0; g < count; ++g) {

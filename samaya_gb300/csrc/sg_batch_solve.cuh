@@ -435,7 +435,7 @@ __device__ __forceinline__ int next_instance(unsigned* queue, ClusterShared& sh,
 }  // namespace
 
 template <typename T, int MODE, bool HALPERN, int THREADS, int WALK = kWalkOne>
-__global__ void __launch_bounds__(THREADS, sizeof(T) == 8 ? 2 : 1)
+__global__ void __launch_bounds__(THREADS, sizeof(T) == 8 && THREADS == kThreads64 ? 2 : 1)
     batch_solve_kernel(BatchView b, InstanceList list) {
   using Share = RowShare<T, WALK>;
   __shared__ ClusterShared sh;
@@ -478,8 +478,14 @@ auto with_solve_kernel(int algorithm, int mode, const ClusterPlan& p, const Go& 
     return h ? go(batch_solve_kernel<T, kAllShared, true, kThreads64>)
              : go(batch_solve_kernel<T, kAllShared, false, kThreads64>);
   }
-  constexpr int kMost = sizeof(T) == 4 ? kThreads32 : kThreads64;
+  constexpr int kMost = sizeof(T) == 4 ? kThreads32 : kThreads64Large;
   constexpr int kWalk = sizeof(T) == 4 ? kWalkPairs : kWalkOne;
+  if constexpr (sizeof(T) == 8) {
+    if (mode == kVectorsShared && threads == kThreads64) {
+      return h ? go(batch_solve_kernel<T, kVectorsShared, true, kThreads64>)
+               : go(batch_solve_kernel<T, kVectorsShared, false, kThreads64>);
+    }
+  }
   if (mode == kVectorsShared) {
     return h ? go(batch_solve_kernel<T, kVectorsShared, true, kMost, kWalk>)
              : go(batch_solve_kernel<T, kVectorsShared, false, kMost, kWalk>);

@@ -393,8 +393,8 @@ __device__ bool unroll_adjoint(const BatchView& b, const UnrollView& u, int inst
 
 }  // namespace
 
-template <bool ADJOINT, int MODE, int PER_SM = 2, int WALK = kWalkOne>
-__global__ void __launch_bounds__(kThreads64, PER_SM) unroll_kernel(BatchView b, UnrollView u,
+template <bool ADJOINT, int MODE, int PER_SM = 2, int WALK = kWalkOne, int THREADS = kThreads64>
+__global__ void __launch_bounds__(THREADS, PER_SM) unroll_kernel(BatchView b, UnrollView u,
                                                                     InstanceList list) {
   __shared__ ClusterShared sh;
   __shared__ Unroll<MODE, WALK> ctx;
@@ -417,9 +417,9 @@ namespace {
 
 // go() with the kernel of a mode; `alone`: the adjoint's variant with an SM to a CTA.
 template <typename Go>
-auto with_unroll_kernel(int adjoint, int mode, bool alone, bool small, const Go& go) {
-  if (small && adjoint && alone) return go(unroll_kernel<true, kAllShared, 1, kWalkLanes>);
-  if (small) {
+auto with_unroll_kernel(int adjoint, int mode, bool alone, const ClusterPlan& p, const Go& go) {
+  if (p.small && adjoint && alone) return go(unroll_kernel<true, kAllShared, 1, kWalkLanes>);
+  if (p.small) {
     return adjoint ? go(unroll_kernel<true, kAllShared, 2, kWalkLanes>)
                    : go(unroll_kernel<false, kAllShared, 2, kWalkLanes>);
   }
@@ -427,11 +427,17 @@ auto with_unroll_kernel(int adjoint, int mode, bool alone, bool small, const Go&
   if (mode == kAllShared) {
     return adjoint ? go(unroll_kernel<true, kAllShared>) : go(unroll_kernel<false, kAllShared>);
   }
-  if (mode == kVectorsShared) {
+  if (mode == kVectorsShared && p.threads[mode] == kThreads64) {
     return adjoint ? go(unroll_kernel<true, kVectorsShared>)
                    : go(unroll_kernel<false, kVectorsShared>);
   }
-  return adjoint ? go(unroll_kernel<true, kInDevice>) : go(unroll_kernel<false, kInDevice>);
+  constexpr int kMost = kThreads64Large;
+  if (mode == kVectorsShared) {
+    return adjoint ? go(unroll_kernel<true, kVectorsShared, 1, kWalkOne, kMost>)
+                   : go(unroll_kernel<false, kVectorsShared, 1, kWalkOne, kMost>);
+  }
+  return adjoint ? go(unroll_kernel<true, kInDevice, 1, kWalkOne, kMost>)
+                 : go(unroll_kernel<false, kInDevice, 1, kWalkOne, kMost>);
 }
 
 }  // namespace
@@ -440,7 +446,7 @@ bool unroll_fits(const ClusterPlan& p, int adjoint) {
   for (int mode = 0; mode < kModes; ++mode) {
     for (bool alone : {false, true}) {
       if (p.group[mode].count > 0 &&
-          !with_unroll_kernel(adjoint, mode, alone, p.small, [&](auto kernel) {
+          !with_unroll_kernel(adjoint, mode, alone, p, [&](auto kernel) {
             return clusters_fit(kernel, p.size, p.threads[mode], p.smem[mode]);
           })) {
         return false;
@@ -464,7 +470,7 @@ cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const Cluster
                              : p.size == 4 ? p.sms / p.size * 3 / 4
                                            : p.sms / p.size / 2;
     const bool alone = clusters <= side_by_side;
-    return with_unroll_kernel(adjoint, mode, alone, p.small, [&](auto kernel) {
+    return with_unroll_kernel(adjoint, mode, alone, p, [&](auto kernel) {
       return launch_clusters(kernel, p.size, clusters, p.threads[mode], p.smem[mode], gst, b, u, list);
     });
   });

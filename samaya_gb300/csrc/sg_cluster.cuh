@@ -49,10 +49,12 @@
 namespace sg {
 
 // Threads per CTA. FP64 kernels, bound by the FP64 pipe, take 256 of 128 registers, so that two CTAs
-// share an SM and one's exchange overlaps the other's sums. An FP32 solve has an SM to a CTA and is
+// share an SM and one's exchange overlaps the other's sums; 512 where the gathered vectors leave no
+// room for a second CTA (Batch::plan_clusters). An FP32 solve has an SM to a CTA and is
 // bound by the latency of its chains; how many threads share the registers follows the rows
 // (Batch::plan_clusters): 256 of 255 registers, 384 of 168, 512 of 128.
 constexpr int kThreads64 = 256;
+constexpr int kThreads64Large = 512;
 constexpr int kThreads32Few = 256;
 constexpr int kThreads32Mid = 384;
 constexpr int kThreads32 = 512;

@@ -110,7 +110,7 @@ int main() {
           const bool ok = run(size, fail_at, [&] {
             const BatchView b = p.view(which == 1 || which == 3 ? 2 : 0);
             const InstanceList list{p.order, kInstances};
-            if (which < 2) batch_setup_kernel<kWalkOne>(b, 1u << 20);
+            if (which < 2) batch_setup_kernel<kWalkOne, kThreads64>(b, 1u << 20);
             if (which == 2) batch_solve_kernel<double, kAllShared, false, kThreads64>(b, list);
             if (which == 3) batch_solve_kernel<double, kAllShared, true, kThreads64>(b, list);
             if (which == 4) unroll_kernel<false, kAllShared>(b, p.unroll(), list);

@@ -6,7 +6,7 @@
 
 namespace sg {
 
-constexpr int kThreads64 = 256, kThreads32Few = 256, kThreads32Mid = 384, kThreads32 = 512;
+constexpr int kThreads64 = 256, kThreads64Large = 512, kThreads32Few = 256, kThreads32Mid = 384, kThreads32 = 512;
 constexpr int kMaxCluster = 16;
 enum : int { kInDevice = 0, kVectorsShared = 1, kAllShared = 2, kModes = 3 };
 enum : int { kOptimal = 0, kIterationLimit = 3, kTimeLimit = 4, kNumericalError = 5 };
