@@ -445,21 +445,24 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
   };
   std::vector<std::pair<double, int>> work(count);  // an iteration's time by one CTA, the matrix
   bool fits = true;  // every instance's gathered vectors in shared memory
-  size_t most_vectors = 0;
+  double all_work = 0.0, alone_work = 0.0;  // of LPs whose vectors leave an SM no second CTA
   for (int i = 0; i < count; ++i) {
     const int g = setup ? i : inst_mat_[i];
     const double rows = static_cast<double>(mat_m_[g]) + mat_n_[g];
     const double nnz = static_cast<double>(mat_nnz_[g]);
     work[i] = {(fp32 ? 1.5e-4 : 5.6e-4) * (2 * nnz + 5 * rows), g};
     fits = fits && vector_bytes(g, 2) <= kClusterSmemMax;
-    most_vectors = std::max(most_vectors, vector_bytes(g, 1));
+    all_work += work[i].first;
+    if (vector_bytes(g, 1) > kClusterSmemHalf) alone_work += work[i].first;
   }
   std::sort(work.begin(), work.end(), std::greater<std::pair<double, int>>());
-  // Two FP64 CTAs share an SM, unless an LP's vectors leave no room for a second one: then one of 512
-  // threads has it (128 iterations of facility-location LPs with 256 and with 512: 16 of
+  // Two FP64 CTAs share an SM, unless most of the work is in LPs whose vectors leave no room for a
+  // second one: then one of 512 threads has it (128 iterations of facility-location LPs with 256 and with 512: 16 of
   // 60 x 240 7.8 and 4.7 ms, 64 of 100 x 400 72.0 and 42.5; 256 random LPs of 5,000 x 12,500 67.3 and
-  // 42.8). FP32 CTAs take an SM each.
-  const bool alone = !fp32 && most_vectors > kClusterSmemHalf;
+  // 42.8). With less of them the others' sharing counts for more: 512 LPs of 100 to 5,000 rows, 41% of the
+  // work in such ones, to 1e-4, 3.18 s as two to an SM and 3.46 otherwise, Halpern 8.24 and 12.9. FP32
+  // CTAs take an SM each.
+  const bool alone = !fp32 && alone_work > 0.5 * all_work;
   const int per_sm = fp32 || alone ? 1 : 2;
   // The sizes' exchanges and epilogues.
   const int sizes[5] = {1, 2, 4, 8, 16};
@@ -497,7 +500,7 @@ void Batch::plan_clusters(Kind kind, int most, ClusterPlan* plan, std::vector<in
     }
     // (Where the state stays in device memory, a larger cluster's gain is partly the memory's: 256
     // nodes of 100 x 400 in FP32 54.1 ms with clusters of four, estimated alike, 42.8 with one CTA.)
-    const bool close = !setup && all_bytes(work[0].second, size) > limit;
+    const bool close = fp32 && all_bytes(work[0].second, size) > limit;
     if (best_time < 0 || end < (close ? 0.95 : 1.0) * best_time) {
       best_time = end;
       plan->size = size;

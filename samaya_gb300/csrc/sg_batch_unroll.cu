@@ -19,7 +19,7 @@ namespace sg {
 //
 // Bound by the FP64 pipe and, with four CTAs to an LP, by the exchanges: 64 LPs of 500 x 1,200,
 // 256 iterations forward and backward: 11.0 ms with a CTA per LP and block barriers, 7.1 with
-// clusters of two, 6.4 with four.
+// clusters of two, 6.2 with four.
 
 namespace {
 
@@ -461,11 +461,11 @@ cudaError_t launch_unroll(const BatchView& b, const UnrollView& u, const Cluster
   return for_groups(p, gs, s, cudaSuccess, [&](int mode, cudaStream_t gst) {
     const InstanceList list = p.group[mode];
     const int clusters = list.count < p.clusters ? list.count : p.clusters;
-    // The adjoint's state in 128 registers, two CTAs to an SM, spills 780 bytes of loads. While
-    // every CTA finds an SM of its own the variant of 215 registers runs (200 iterations: 1 LP of
-    // 80 x 176 1.76 ms before, 1.53 now; 64 of 150 x 330 2.42 and 2.06; 1 of 500 x 1,100 2.56
-    // and 2.25). Clusters of 4 and more leave SMs of a GPC over: 16 clusters of 8 no longer ran
-    // side by side (2.63 ms with two CTAs to an SM, 3.87 without).
+    // The adjoint's values take 215 registers; with 128, two CTAs to an SM, some are read anew. While
+    // every CTA finds an SM of its own the variant of 215 runs (the adjoint of 200 iterations: 1 LP of
+    // 300 x 660 2.08 ms, 2.31 without; 64 of 150 x 330 2.07 and 2.33). Clusters of 4 and more leave SMs
+    // of a GPC over: 16 clusters of 8 no longer ran side by side (2.63 ms with two CTAs to an SM, 3.87
+    // without).
     const int side_by_side = p.size <= 2   ? p.sms / p.size
                              : p.size == 4 ? p.sms / p.size * 3 / 4
                                            : p.sms / p.size / 2;
