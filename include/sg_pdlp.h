@@ -104,8 +104,7 @@ typedef struct sg_pdlp_opts {
  * and starts the primal weight at |c| / |b|; everything else is the same. HALPERN is ENHANCED
  * with the reflected Halpern iteration z+ = lambda (2 T(z) - z) + (1 - lambda) z0 in place
  * of the running average (T the PDHG map, z0 the restart point, lambda = (k+1)/(k+2));
- * termination, restarts and the answer use T(z); no infeasibility / unboundedness checks.
- * The batched engine runs HALPERN requests as ENHANCED. */
+ * termination, restarts and the answer use T(z); no infeasibility / unboundedness checks. */
 enum {
   SG_ALGORITHM_REFERENCE = 0,
   SG_ALGORITHM_ENHANCED = 1,
@@ -149,7 +148,9 @@ int sg_pdlp_available(int* cc_major, int* cc_minor, char* name, size_t name_len)
  * row index out of range, a value or cost that is not finite, a NaN bound); the row-major
  * copy of A is then built on the device (a stable sort by row: the CSR sg_csc_to_csr gives).
  * Matrices with 2^31 - 1 or more nonzeros are refused (SG_ERR_TOO_LARGE), as the reference
- * refuses them (pdhg_core.cu:176-178). */
+ * refuses them (pdhg_core.cu:176-178). A small LP iterates on one thread-block cluster where the
+ * device can hold it; the environment variable SG_MAX_CLUSTER, read here and by sg_batch_create,
+ * caps the cluster's CTAs (1: none). */
 int sg_pdlp_create(sg_pdlp** handle, int m, int n, const int64_t* a_colptr,
                    const int32_t* a_rowidx, const double* a_val, const double* cost,
                    const double* lower, const double* upper, const sg_pdlp_opts* opts);
